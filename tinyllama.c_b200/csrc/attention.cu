@@ -205,7 +205,16 @@ attention_warp_kernel(const T* __restrict__ q, const T* __restrict__ k_pages, co
       const int page = table[kp / TLC_PAGE];
       const T* kr = k_pages + (((size_t)page * KV + g) * TLC_PAGE + kp % TLC_PAGE) * hd;
       float dot = 0.f;
-      for (int d = 0; d < hd; d++) dot = fmaf(to_f32(kr[d]), qs[d], dot);
+      if (sizeof(T) == 4 && hd % 4 == 0 && ((uintptr_t)k_pages & 15) == 0) {     // 16 bytes a load, eight of them in flight
+        const float4* k4 = reinterpret_cast<const float4*>(kr);
+#pragma unroll 8
+        for (int d4 = 0; d4 < hd / 4; d4++) {
+          const float4 kv = k4[d4], qv = *reinterpret_cast<const float4*>(qs + 4 * d4);
+          dot = fmaf(kv.w, qv.w, fmaf(kv.z, qv.z, fmaf(kv.y, qv.y, fmaf(kv.x, qv.x, dot))));
+        }
+      } else {
+        for (int d = 0; d < hd; d++) dot = fmaf(to_f32(kr[d]), qs[d], dot);
+      }
       s = capped_score(dot, softcap);
     }
     const float m_new = fmaxf(m, warp_max(s));
@@ -309,11 +318,25 @@ attention_decode_partial_kernel(const T* __restrict__ q, const T* __restrict__ k
   for (int hg = 0; hg < DEC_MAXG; hg++) s[hg] = 0.f;
   if (valid) {
     const T* kr = k_pages + (((size_t)table[kp / TLC_PAGE] * KV + g) * TLC_PAGE + kp % TLC_PAGE) * hd;
-    for (int d = 0; d < hd; d++) {
-      const float kv = to_f32(kr[d]);
+    if (sizeof(T) == 4 && hd % 4 == 0 && ((uintptr_t)k_pages & 15) == 0) {       // 16 bytes a load, eight of them in flight
+      const float4* k4 = reinterpret_cast<const float4*>(kr);
+#pragma unroll 8
+      for (int d4 = 0; d4 < hd / 4; d4++) {
+        const float4 kv = k4[d4];
 #pragma unroll
-      for (int hg = 0; hg < DEC_MAXG; hg++)
-        if (hg < G) s[hg] = fmaf(kv, qs[hg * hd + d], s[hg]);
+        for (int hg = 0; hg < DEC_MAXG; hg++)
+          if (hg < G) {
+            const float4 qv = *reinterpret_cast<const float4*>(qs + hg * hd + 4 * d4);
+            s[hg] = fmaf(kv.w, qv.w, fmaf(kv.z, qv.z, fmaf(kv.y, qv.y, fmaf(kv.x, qv.x, s[hg]))));
+          }
+      }
+    } else {
+      for (int d = 0; d < hd; d++) {
+        const float kv = to_f32(kr[d]);
+#pragma unroll
+        for (int hg = 0; hg < DEC_MAXG; hg++)
+          if (hg < G) s[hg] = fmaf(kv, qs[hg * hd + d], s[hg]);
+      }
     }
   }
   // per head: maximum and sum over the block's keys
@@ -335,13 +358,20 @@ attention_decode_partial_kernel(const T* __restrict__ q, const T* __restrict__ k
     float acc[DEC_MAXG];
 #pragma unroll
     for (int hg = 0; hg < DEC_MAXG; hg++) acc[hg] = 0.f;
-    for (int j = 0; j < nk; j++) {
-      const int kj = k0 + j;
-      if (kj < start && kj >= kept) continue;   // outside the window: its page may have been given back
-      const float vv = to_f32(v_pages[(((size_t)table[kj / TLC_PAGE] * KV + g) * TLC_PAGE + kj % TLC_PAGE) * hd + d]);
+    for (int j = 0; j < nk; j += 8) {             // k0 starts a page: eight keys lie in one
+      const size_t at = (((size_t)table[(k0 + j) / TLC_PAGE] * KV + g) * TLC_PAGE + (k0 + j) % TLC_PAGE) * hd + d;
+      float vv[8];
 #pragma unroll
-      for (int hg = 0; hg < DEC_MAXG; hg++)
-        if (hg < G) acc[hg] = fmaf(ps[hg * DEC_KEYS + j], vv, acc[hg]);
+      for (int u = 0; u < 8; u++) {
+        const int kj = k0 + j + u;
+        const bool ok = j + u < nk && (kj >= start || kj < kept);      // outside the window its page may have been given back
+        vv[u] = ok ? to_f32(v_pages[at + (size_t)u * hd]) : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; u++)
+#pragma unroll
+        for (int hg = 0; hg < DEC_MAXG; hg++)
+          if (hg < G) acc[hg] = fmaf(ps[hg * DEC_KEYS + j + u], vv[u], acc[hg]);
     }
 #pragma unroll
     for (int hg = 0; hg < DEC_MAXG; hg++)

@@ -147,10 +147,267 @@ gemm_skinny_bf16x8_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __
   }
 }
 
+// ---- 32-bit operands in 16-byte pieces (rows of a multiple of 4 values on 16-byte boundaries) -----------------------
+// Two kernels that do what the two general ones above do, in true 32-bit arithmetic with the sums in the same number of
+// terms.  What bounded the general ones was loads: one 4-byte load a lane in flight (a one-token step of two
+// sequences read its weights at 0.75 TB/s), and shared-memory reads a product (4 x 4 results a thread: 17 TFLOP/s).
+
+// 16 bytes that this kernel reads once: they leave the first-level cache to the activations.
+__device__ __forceinline__ float4 load_once(const float4* p) {
+  float4 v;
+  asm("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+
+// Few rows: a warp takes COLS output columns and reads their weight rows 512 bytes at a time, U pieces a column in flight
+// (the first ones before the wait on the previous kernel); an activation piece serves COLS columns.
+// 2 rows, 2048 -> 8240 (67 MB): 90 -> 12.7 us, 4096 -> 2048 (34 MB): 95 -> 12.4 us; 8 rows 216 -> 19 and 237 -> 50 us.
+template <typename TO, int MT, int COLS, int U>
+__global__ void __launch_bounds__(256)
+gemm_skinny_f32x4_kernel(const float* __restrict__ a, int lda, const float* __restrict__ w, int ldw, TO* __restrict__ out,
+                         int ldo, const float* __restrict__ colscale, const float* __restrict__ colbias, TlcEpi accumulate,
+                         int M, int N, int K, int m_base) {
+  asm volatile("griddepcontrol.launch_dependents;");
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n0 = (blockIdx.x * 8 + warp) * COLS;
+  const int K4 = K >> 2;
+  const float4* wr[COLS];
+#pragma unroll
+  for (int c = 0; c < COLS; c++) wr[c] = reinterpret_cast<const float4*>(w + (size_t)min(n0 + c, N - 1) * ldw);   // clamped rows are never stored
+  float acc[MT][COLS];
+#pragma unroll
+  for (int m = 0; m < MT; m++)
+#pragma unroll
+    for (int c = 0; c < COLS; c++) acc[m][c] = 0.f;
+  for (int i0 = lane; i0 - lane < K4; i0 += 32 * U) {
+    float4 wv[COLS][U];
+#pragma unroll
+    for (int u = 0; u < U; u++)
+#pragma unroll
+      for (int c = 0; c < COLS; c++) wv[c][u] = i0 + 32 * u < K4 ? load_once(wr[c] + i0 + 32 * u) : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i0 == lane) tlc_wait(a, out);
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      if (i0 + 32 * u < K4) {
+#pragma unroll
+        for (int m = 0; m < MT; m++) {
+          if (m_base + m < M) {
+            const float4 x = *(reinterpret_cast<const float4*>(a + (size_t)(m_base + m) * lda) + i0 + 32 * u);
+#pragma unroll
+            for (int c = 0; c < COLS; c++) {
+              acc[m][c] = fmaf(x.x, wv[c][u].x, acc[m][c]);
+              acc[m][c] = fmaf(x.y, wv[c][u].y, acc[m][c]);
+              acc[m][c] = fmaf(x.z, wv[c][u].z, acc[m][c]);
+              acc[m][c] = fmaf(x.w, wv[c][u].w, acc[m][c]);
+            }
+          }
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < MT; m++) {
+#pragma unroll
+    for (int c = 0; c < COLS; c++) {
+      float v = warp_sum(acc[m][c]);
+      const int n = n0 + c;
+      if (lane == 0 && m_base + m < M && n < N) {
+        if (colscale) v *= colscale[n];
+        if (colbias) v += colbias[n];
+        TO* o = out + (size_t)(m_base + m) * ldo + n;
+        if (accumulate) v += to_f32(*o);
+        *o = from_f32<TO>(v);
+      }
+    }
+  }
+}
+
+// Two products of a pair of accumulators in one instruction, each rounded as fmaf rounds it.
+__device__ __forceinline__ void fma_pair(float2& d, float2 a, float2 b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;"
+      : "+l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
+}
+
+// Many rows: a tile of 64 rows x 16 CT columns, 128 threads with 8 x CT results each (CT 8 or 4); two K-steps of 16 in
+// shared memory, the next one in registers.  With KG = 4 four groups of 128 threads take a quarter of K each and the
+// first adds the others' sums to its own: outputs of few columns have too few tiles to keep an SM's schedulers busy.
+// 310 rows: 2048 -> 8192: 595 -> 311 us (33 TFLOP/s), 4096 -> 2048: 920 -> 270 us; 1,200 rows 1633 -> 878 and 1185 -> 626 us.
+constexpr int FT_M = 64, FT_K = 16, FT_LD = 4;
+template <typename TO, int CT, int KG>
+__global__ void __launch_bounds__(128 * KG)
+gemm_tiled_f32x4_kernel(const float* __restrict__ a, int lda, const float* __restrict__ w, int ldw, TO* __restrict__ out,
+                        int ldo, const float* __restrict__ colscale, const float* __restrict__ colbias, TlcEpi accumulate,
+                        int M, int N, int K) {
+  tlc_pdl(a, out);
+  constexpr int TN = 16 * CT, LA = FT_M + FT_LD, LW = TN + FT_LD;
+  constexpr int PA = FT_M * FT_K / 4 / 128, PW = TN * FT_K / 4 / 128;   // 16-byte pieces a thread brings of each operand
+  extern __shared__ __align__(16) float ft_sm[];
+  const int grp = threadIdx.x >> 7, tid = threadIdx.x & 127;
+  float* As = ft_sm + grp * 2 * FT_K * (LA + LW);            // [2][FT_K][LA]
+  float* Ws = As + 2 * FT_K * LA;                            // [2][FT_K][LW]
+  const int m0 = blockIdx.y * FT_M, n0 = blockIdx.x * TN;
+  const int tx = tid & 15, ty = tid >> 4;
+  const int steps = (K + FT_K - 1) / FT_K, per = (steps + KG - 1) / KG;
+  const int s_begin = min(steps, grp * per), s_end = min(steps, s_begin + per);
+  float4 ra[PA], rw[PW];
+  auto load = [&](int s) {
+#pragma unroll
+    for (int i = 0; i < PA; i++) {
+      const int q = tid + 128 * i, r = m0 + (q >> 2), k = s * FT_K + (q & 3) * 4;
+      ra[i] = (r < M && k < K) ? *reinterpret_cast<const float4*>(a + (size_t)r * lda + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int i = 0; i < PW; i++) {
+      const int q = tid + 128 * i, r = n0 + (q >> 2), k = s * FT_K + (q & 3) * 4;
+      rw[i] = (r < N && k < K) ? __ldg(reinterpret_cast<const float4*>(w + (size_t)r * ldw + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  };
+  auto store = [&](int buf) {
+#pragma unroll
+    for (int i = 0; i < PA; i++) {
+      const int q = tid + 128 * i;
+      float* d = As + buf * FT_K * LA + (q & 3) * 4 * LA + (q >> 2);
+      d[0] = ra[i].x; d[LA] = ra[i].y; d[2 * LA] = ra[i].z; d[3 * LA] = ra[i].w;
+    }
+#pragma unroll
+    for (int i = 0; i < PW; i++) {
+      const int q = tid + 128 * i;
+      float* d = Ws + buf * FT_K * LW + (q & 3) * 4 * LW + (q >> 2);
+      d[0] = rw[i].x; d[LW] = rw[i].y; d[2 * LW] = rw[i].z; d[3 * LW] = rw[i].w;
+    }
+  };
+  float2 acc[8][CT / 2];
+#pragma unroll
+  for (int i = 0; i < 8; i++)
+#pragma unroll
+    for (int j = 0; j < CT / 2; j++) acc[i][j] = make_float2(0.f, 0.f);
+  // all groups go through the same number of barriers
+  if (s_begin < s_end) { load(s_begin); store(0); }
+  __syncthreads();
+#pragma unroll 1
+  for (int i = 0; i < per; i++) {
+    const int s = s_begin + i, buf = i & 1;
+    if (s + 1 < s_end) load(s + 1);
+    if (s < s_end) {
+      const float* Ab = As + buf * FT_K * LA + ty * 8;
+      const float* Wb = Ws + buf * FT_K * LW + tx * 4;
+#pragma unroll
+      for (int k = 0; k < FT_K; k++) {
+        const float4 a0 = *reinterpret_cast<const float4*>(Ab + k * LA), a1 = *reinterpret_cast<const float4*>(Ab + k * LA + 4);
+        const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+        float2 wv[CT / 2];
+#pragma unroll
+        for (int h = 0; h < CT / 4; h++) {
+          const float4 b = *reinterpret_cast<const float4*>(Wb + k * LW + h * 64);
+          wv[2 * h] = make_float2(b.x, b.y);
+          wv[2 * h + 1] = make_float2(b.z, b.w);
+        }
+#pragma unroll
+        for (int r = 0; r < 8; r++)
+#pragma unroll
+          for (int j = 0; j < CT / 2; j++) fma_pair(acc[r][j], make_float2(av[r], av[r]), wv[j]);
+      }
+    }
+    if (s + 1 < s_end) store(buf ^ 1);
+    __syncthreads();
+  }
+  if constexpr (KG > 1) {
+    float* part = ft_sm;                                     // the other groups' sums, [KG - 1][8 * CT][128]
+    if (grp > 0) {
+      float* mine = part + (grp - 1) * 8 * CT * 128 + tid;
+#pragma unroll
+      for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int j = 0; j < CT / 2; j++) {
+          mine[((i * CT) + 2 * j) * 128] = acc[i][j].x;
+          mine[((i * CT) + 2 * j + 1) * 128] = acc[i][j].y;
+        }
+    }
+    __syncthreads();
+    if (grp > 0) return;
+#pragma unroll
+    for (int q = 0; q < KG - 1; q++) {                       // in the order of K
+      const float* other = part + q * 8 * CT * 128 + tid;
+#pragma unroll
+      for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int j = 0; j < CT / 2; j++) {
+          acc[i][j].x += other[((i * CT) + 2 * j) * 128];
+          acc[i][j].y += other[((i * CT) + 2 * j + 1) * 128];
+        }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const int m = m0 + ty * 8 + i;
+    if (m >= M) continue;
+#pragma unroll
+    for (int j = 0; j < CT; j++) {
+      const int n = n0 + tx * 4 + (j >> 2) * 64 + (j & 3);
+      if (n >= N) continue;
+      float v = (j & 1) ? acc[i][j >> 1].y : acc[i][j >> 1].x;
+      if (colscale) v *= colscale[n];
+      if (colbias) v += colbias[n];
+      TO* o = out + (size_t)m * ldo + n;
+      if (accumulate) v += to_f32(*o);
+      *o = from_f32<TO>(v);
+    }
+  }
+}
+constexpr int ft_smem(int CT, int KG) { return KG * 2 * FT_K * (FT_M + 16 * CT + 2 * FT_LD) * 4; }
+static_assert(ft_smem(4, 4) >= 3 * 8 * 4 * 128 * 4 && ft_smem(8, 1) <= 48 * 1024, "the other groups' sums reuse the operands' memory");
+
+// Kernels that ask for more than 48 KB of shared memory, prepared outside any stream capture.
+int tlc_linear_simt_init() {
+  if (cudaFuncSetAttribute(gemm_tiled_f32x4_kernel<float, 4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, ft_smem(4, 4)) != cudaSuccess ||
+      cudaFuncSetAttribute(gemm_tiled_f32x4_kernel<__nv_bfloat16, 4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, ft_smem(4, 4)) != cudaSuccess)
+    return tlc_fail(-2, "linear(32 bits): cannot reserve %d bytes of shared memory", ft_smem(4, 4));
+  return 0;
+}
+
+template <typename TO>
+static void launch_simt_f32x4(const float* a, int lda, const float* w, int ldw, TO* out, int ldo, const float* colscale,
+                              const float* colbias, TlcEpi accumulate, int M, int N, int K, cudaStream_t stream) {
+  static int sms = 0;
+  if (sms == 0) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
+  if (M > 16) {
+    // 128 columns a tile where that still makes two blocks an SM, else 64 columns and K in four parts
+    const unsigned my = (unsigned)((M + FT_M - 1) / FT_M);
+    if ((long long)my * ((N + 127) / 128) >= 2 * sms)
+      tlc_launch(gemm_tiled_f32x4_kernel<TO, 8, 1>, dim3((N + 127) / 128, my), dim3(128), ft_smem(8, 1), stream, a, lda, w, ldw, out, ldo, colscale,
+                 colbias, accumulate, M, N, K);
+    else
+      tlc_launch(gemm_tiled_f32x4_kernel<TO, 4, 4>, dim3((N + 63) / 64, my), dim3(512), ft_smem(4, 4), stream, a, lda, w, ldw, out, ldo, colscale,
+                 colbias, accumulate, M, N, K);
+    return;
+  }
+  // A warp's columns share its activations: a read of them costs as much as one of the weights, so up to 2 rows take two
+  // columns and more rows four, where that still makes two blocks an SM.
+  auto blocks_of = [&](int cols) { return (unsigned)((N + 8 * cols - 1) / (8 * cols)); };
+#define TLC_SK4(MT_, C_, U_) tlc_launch(gemm_skinny_f32x4_kernel<TO, MT_, C_, U_>, dim3(blocks_of(C_)), dim3(256), 0, stream, a, lda, w, ldw, out, ldo, \
+                                        colscale, colbias, accumulate, M, N, K, mb)
+  for (int mb = 0; mb < M; mb += 8) {
+    const int rows = M - mb;
+    const bool two = blocks_of(2) >= 2 * (unsigned)sms;
+    if (rows <= 2) { if (two) TLC_SK4(2, 2, 4); else TLC_SK4(2, 1, 8); }
+    else if (rows <= 4) { if (two) TLC_SK4(4, 2, 4); else TLC_SK4(4, 2, 2); }
+    else { if (two) TLC_SK4(8, 4, 2); else TLC_SK4(8, 2, 2); }
+  }
+#undef TLC_SK4
+}
+
 template <typename TA, typename TW, typename TO>
 static int launch_simt(const void* a, int lda, const void* w, int ldw, void* out, int ldo, const float* colscale,
                        const float* colbias, TlcEpi accumulate, int M, int N, int K, cudaStream_t stream) {
   constexpr int MT = 8;
+  if constexpr (std::is_same<TA, float>::value && std::is_same<TW, float>::value) {
+    if (K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)a % 16 == 0) && ((uintptr_t)w % 16 == 0)) {
+      launch_simt_f32x4<TO>((const float*)a, lda, (const float*)w, ldw, (TO*)out, ldo, colscale, colbias, accumulate, M, N, K, stream);
+      TLC_CHECK_LAUNCH("linear(simt)");
+      return 0;
+    }
+  }
   if (M <= 16) {
     const bool vec = std::is_same<TA, __nv_bfloat16>::value && std::is_same<TW, __nv_bfloat16>::value && (K % 8 == 0) &&
                      (lda % 8 == 0) && (ldw % 8 == 0) && ((uintptr_t)a % 16 == 0) && ((uintptr_t)w % 16 == 0);

@@ -26,6 +26,7 @@
 #include <mutex>
 #include <unordered_map>
 
+int tlc_linear_simt_init();      // gemm_simt.cu
 // gemm_tcgen05_few_rows.cu
 int tlc_linear_few_rows_run(const void* a, int lda, const void* w, int ldw, void* out, int out_dtype, int ldo,
                             const float* colscale, const float* colbias, TlcEpi accumulate, int M, int N, int K,
@@ -545,6 +546,7 @@ int count_pairs() {
 int init_once() {
   std::lock_guard<std::mutex> lk(g_mu);
   if (g_encode) return 0;
+  if (int rc = tlc_linear_simt_init()) return rc;
   if (int rc = configure<float, 128, 6>()) return rc;
   if (int rc = configure<__nv_bfloat16, 128, 6>()) return rc;
   if (int rc = configure<float, 256, 4>()) return rc;
