@@ -46,3 +46,31 @@ def test_linear_of_32_bit_rows_in_pieces_of_16_bytes(M, N, K):
     """Few rows (one or two columns a warp, two or four from five rows on; more than eight rows in two launches), then
     tiles of 64 x 128 or of 64 x 64 with K in four parts: K shorter than a step, parts without a step, edges in M and N."""
     _run(M, N, K, torch.float32)
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 16424, 72), (4, 16500, 2056), (5, 16384, 4096), (8, 18950, 136), (9, 16390, 520), (16, 16400, 264), (17, 16385, 200), (32, 20000, 72)])
+def test_linear_of_a_vocabulary_with_few_rows(M, N, K):
+    """Outputs of 128 tiles of 128 weight rows and more: 16 or 32 activation rows on the narrow side, last tiles past N."""
+    _run(M, N, K, torch.bfloat16)
+
+
+@pytest.mark.parametrize("split", [1, 2, 4, 8])
+@pytest.mark.parametrize("M,N,K", [(9, 300, 520), (16, 1000, 1096), (13, 128, 136), (24, 2064, 328)])
+def test_linear_with_16_or_32_rows_on_the_narrow_side_and_a_fixed_split(M, N, K, split):
+    """The sums of 1 to 8 blocks: fewer K-steps than blocks, a share of the rows that some blocks do not have; the gated form."""
+    from tinyllama_c_b200 import ops
+    ops.linear_few_rows(True, split)
+    try:
+        _run(M, N, K, torch.bfloat16, pad=3)
+        if N % 16 == 0:
+            g = torch.Generator().manual_seed(N + M)
+            a, w = torch.randn(M, K, generator=g).bfloat16().cuda(), (torch.randn(N, K, generator=g) * 0.05).bfloat16().cuda()
+            out = torch.empty(M, N // 2, device="cuda")
+            ops.linear_swiglu(a, w, out)
+            gu = (a.double() @ w.double().T).view(M, N // 16, 2, 8)
+            ref = (torch.nn.functional.silu(gu[:, :, 0]) * gu[:, :, 1]).reshape(M, N // 2)
+            # sums of K terms (relative 2^-13 at the most here) through a product and a SiLU of slope at most 1.1
+            assert (out.double() - ref).abs().max().item() <= 3 * (K + 8) * 2.0 ** -24 * 8 * (1 + gu.abs().max().item()) ** 2
+            ops.check_errors()
+    finally:
+        ops.linear_few_rows(True, 0)

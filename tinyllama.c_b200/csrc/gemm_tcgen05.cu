@@ -814,7 +814,7 @@ extern "C" int tlc_linear_swiglu(const void* a, int a_dtype, int lda, const void
   TLC_REQUIRE(K > 0 && lda >= K && ldw >= K && ldo >= N / 2, "linear: bad sizes M=%d N=%d K=%d lda=%d ldw=%d ldo=%d", M, N, K,
               lda, ldw, ldo);
   if (out_dtype != TLC_F32 && out_dtype != TLC_BF16) return tlc_fail(-1, "linear: unknown output dtype %d", out_dtype);
-  if (min_rows_for_tensor_cores <= 128 && tlc_linear_few_rows_ok(a_dtype, lda, a, w_dtype, ldw, w, M, N, K)) {
+  if (min_rows_for_tensor_cores <= 128 && tlc_linear_few_rows_ok(a_dtype, lda, a, w_dtype, ldw, w, M, N, K, 0)) {
     if (int rc = init_once()) return rc;
     return tlc_linear_few_rows_swiglu(a, lda, w, ldw, out, out_dtype, ldo, colscale, colbias, M, N, K, act, stream);
   }
@@ -849,12 +849,12 @@ extern "C" int tlc_linear(const void* a, int a_dtype, int lda, const void* w, in
                           int out_dtype, int ldo, const float* colscale, const float* colbias, int accumulate, int M,
                           int N, int K, int min_rows_for_tensor_cores, cudaStream_t stream) {
   if (M == 0 || N == 0) return 0;
-  // Up to 32 rows the weight-streaming kernel is always best.  From 33 to 64 rows it re-reads the
-  // activations once per 16 output columns, which only pays while the tiled kernel would have too
+  // What the kernel of few rows leaves: up to 32 rows the weight-streaming mma.sync kernel.  From 33 to 64 rows it
+  // re-reads the activations once per 16 output columns, which only pays while the tiled kernel would have too
   // few tiles to keep the GPU busy (narrow outputs) and too few K-steps to share among blocks.
   // (a threshold above 128 rows keeps every tensor-core kernel out, this one too)
   if (min_rows_for_tensor_cores <= 128 && (out_dtype == TLC_F32 || out_dtype == TLC_BF16) &&
-      tlc_linear_few_rows_ok(a_dtype, lda, a, w_dtype, ldw, w, M, N, K)) {
+      tlc_linear_few_rows_ok(a_dtype, lda, a, w_dtype, ldw, w, M, N, K, out_dtype == TLC_F32 && !accumulate)) {
     TLC_REQUIRE(K > 0 && lda >= K && ldw >= K && ldo >= N, "linear: bad sizes M=%d N=%d K=%d lda=%d ldw=%d ldo=%d", M, N, K,
                 lda, ldw, ldo);
     if (int rc = init_once()) return rc;

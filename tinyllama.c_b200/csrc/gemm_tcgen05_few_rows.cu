@@ -1,21 +1,28 @@
-// bfloat16 linear layer for 17..128 rows (decode steps of that many sequences, short prompts) on the 5th-generation tensor cores,
+// bfloat16 linear layer for up to 128 rows (decode steps of that many sequences, short prompts) on the 5th-generation tensor cores,
 // with the WEIGHTS on the M side of tcgen05.mma:  out[M, N] (+)= (A[M, K] @ W[N, K]^T) * colscale + colbias.
 //
 // With so few rows the time is the time to stream the weights once.  The product for prompts puts the activations
 // on the 128-row side and pads them, and has too few tiles for the GPU where N is small; the weight-streaming
 // mma.sync kernel of the smallest batches re-reads the activations for every 16 output columns.  Here a tile is
-// 128 weight rows x 32, 64 or 128 activation rows: D[n, m] = sum_k W[n, k] A[m, k], an accumulator of 128 lanes x NB
+// 128 weight rows x 16, 32, 64 or 128 activation rows: D[n, m] = sum_k W[n, k] A[m, k], an accumulator of 128 lanes x NB
 // columns of tensor memory.  Weight tiles [128, 64] and activation tiles [NB, 64] arrive by TMA (128-byte
 // swizzle, rows past the matrices read as zero) in a ring of shared-memory stages; one thread issues the
 // products; four warps take the result out of tensor memory, a thread per weight row.
 //
 // N / 128 tiles do not fill 148 SMs (65 for N = 8240, 16 for N = 2048), so the K-steps of a tile are shared
-// among the 2, 4 or 8 blocks of a thread-block CLUSTER: every block leaves its partial sums [NB, 128] in its own
-// shared memory, the cluster meets at a barrier, and block r adds up rows r * NB / split ... of all blocks'
-// sums, read through distributed shared memory in the order of the ranks (so the result does not depend on
-// timing), applies the epilogue and stores.  A second barrier keeps every block's shared memory alive until
-// all have read it.  With SWIGLU the weight rows come in groups of 16 = 8 gate rows and their 8 up rows, and the
-// block writes silu(gate) * up ([M, N / 2]).
+// among the up to 8 blocks of a thread-block CLUSTER: every block leaves its partial sums [NB, 128] in its own
+// shared memory, the cluster meets at a barrier, and block r adds up its share of the rows of all blocks' sums,
+// read through distributed shared memory in the order of the ranks (so the result does not depend on
+// timing), applies the epilogue and stores: a warp a row, a lane four weight rows in 16-byte pieces (a thread a weight
+// row instead, with 4-byte reads: 64 x 2048 x 8240 12.6 us, so 10.6).  What the sums are added to is asked for while the
+// products run.  A second barrier keeps every block's shared memory alive until all have read it.  A block that has the
+// whole of K writes from tensor memory.  With SWIGLU the weight rows come in groups of 16 = 8 gate rows and their
+// 8 up rows, and the block writes silu(gate) * up ([M, N / 2]).
+//
+// What bounds it: the stream of the weights; a copy loop of the same boxes without products takes 26.7 us for 24576 x 3072
+// (151 MB), the product of 64 rows 34.9 (40.3 with four stages for every width and the 4-byte reads).  Where a block has few K-steps, the chain from the wait on the
+// kernel before to the last store (activations, products, the meeting of the sums: 3 to 4 us) counts as much as the
+// stream: 64 rows, 4096 -> 2048 8.2 us (9.7 before), of which the 17 MB are 2.6.
 //
 // Every mbarrier wait is bounded (codes 31-33 of the error word); a block whose wait ran out still goes to both
 // cluster barriers, so that no block of its cluster waits for it.
@@ -50,6 +57,17 @@ __device__ __forceinline__ const float* in_rank(const float* p, int rank) {
   return reinterpret_cast<const float*>((uintptr_t)q);
 }
 
+__device__ __forceinline__ float4 read4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 read4(const __nv_bfloat16* p) {
+  const uint2 u = *reinterpret_cast<const uint2*>(p);
+  return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
+}
+__device__ __forceinline__ void write4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void write4(__nv_bfloat16* p, float4 v) {
+  const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+  *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const unsigned*>(&lo), *reinterpret_cast<const unsigned*>(&hi));
+}
+
 template <typename TO, int NB, int STAGES, bool SWIGLU>
 __global__ void __launch_bounds__(FR_THREADS, 2)
 gemm_few_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
@@ -57,6 +75,8 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                      const float* __restrict__ colbias, TlcEpi accumulate, int M, int N, int K, int split, ErrWords* err) {
   asm volatile("griddepcontrol.launch_dependents;");
   using S = FrSmem<NB, STAGES>;
+  constexpr int CW = NB < 32 ? 16 : 32;                     // columns of tensor memory an epilogue warp reads at a time
+  constexpr int TCOLS = NB < 32 ? 32 : NB;                  // (tensor memory comes in 32 columns or more)
   extern __shared__ uint8_t fr_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)fr_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* w_tiles = smem;
@@ -81,7 +101,7 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(NB) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TCOLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -142,69 +162,131 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
       if (ok && n_k > 0) umma_commit(acc_full);
       else if (n_k == 0) mbar_arrive(acc_full);             // nothing to wait for: the epilogue takes zeros
     }
-  } else {                                                  // ---- epilogue warps 2..5: the block's sums into shared memory ----
+  } else {                                                  // ---- epilogue warps 2..5 ----
     const int quarter = warp & 3;                           // a warp may touch lanes 32 * (warp % 4) .. + 31 only
     const int row = quarter * 32 + lane;                    // weight row of the tile
     asm volatile("griddepcontrol.wait;" ::: "memory");      // `out` may still be read or written by the previous kernel
-    mbar_wait(acc_full, 0, err, 33, wait_limit);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    auto read_columns = [&](int c, uint32_t (&r)[CW]) {
+      const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(c * CW);
+      if constexpr (CW == 32) tmem_ld32(at, r);
+      else tmem_ld16(at, r);
+    };
+    if (split == 1) {
+      // the block has the whole sum: out of tensor memory and straight to the output, a lane a weight row
+      const int n = n0 + row;
+      const bool n_in = n < N, add = !SWIGLU && accumulate;
+      const float cs = (colscale && n_in) ? colscale[n] : 1.0f, cb = (colbias && n_in) ? colbias[n] : 0.0f;
+      mbar_wait(acc_full, 0, err, 33, wait_limit);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-    for (int c = 0; c < NB / 32; c++) {
-      uint32_t r[32];
-      tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(c * 32), r);
+      for (int c = 0; c < NB / CW; c++) {
+        float old[CW];
 #pragma unroll
-      for (int j = 0; j < 32; j++) part[(c * 32 + j) * WM + row] = n_k > 0 ? __uint_as_float(r[j]) : 0.f;
-    }
-  }
-  __syncwarp();                                             // the loader's and the issuer's warps are whole again
-  // every block's sums are in its shared memory (the stages are free: every product that read them is complete)
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  if (split > 1) {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-  } else {
-    __syncthreads();
-  }
-  if (warp >= 2) {
-    const int row = (warp & 3) * 32 + lane;
-    const int rows_per = NB / split;                        // activation rows this block finishes
-    const bool second = SWIGLU && (row & 8);                // an up row: its gate row's thread writes the feature
-    const int n = n0 + row;
-    if (!second && n + (SWIGLU ? 8 : 0) < N) {
-      const float cs = colscale ? colscale[n] : 1.0f, cb = colbias ? colbias[n] : 0.0f;
-      const float cs2 = (SWIGLU && colscale) ? colscale[n + 8] : 1.0f, cb2 = (SWIGLU && colbias) ? colbias[n + 8] : 0.0f;
-      const float* src[8];                                  // the sums of every rank, this thread's weight row
-      for (int q = 0; q < 8; q++) src[q] = (q < split ? (split > 1 ? in_rank(part, q) : part) : part) + row;
-      constexpr int RB = 4;                                 // rows whose loads are issued together
-      for (int m0 = rank * rows_per; m0 < min(M, (rank + 1) * rows_per); m0 += RB) {
-        float x[RB][8], x2[RB][8];
+        for (int j = 0; j < CW; j++) old[j] = (add && n_in && c * CW + j < M) ? to_f32(out[(size_t)(c * CW + j) * ldo + n]) : 0.f;
+        uint32_t r[CW];
+        read_columns(c, r);
+#pragma unroll
+        for (int j = 0; j < CW; j++) {
+          const int m = c * CW + j;
+          if (m >= M) break;
+          const float v = __uint_as_float(r[j]) * cs + cb;
+          if (SWIGLU) {                                     // the up rows sit eight lanes above their gate rows
+            const float u = __shfl_down_sync(0xffffffffu, v, 8);
+            if (!(row & 8) && n + 8 < N) out[(size_t)m * ldo + (n0 >> 1) + ((row >> 4) << 3) + (row & 7)] = from_f32<TO>(glu_epilogue<false>(accumulate, v, u));      // (with SWIGLU the argument carries the activation's code)
+          } else if (n_in) {
+            out[(size_t)m * ldo + n] = from_f32<TO>(add ? v + old[j] : v);
+          }
+        }
+      }
+    } else {
+      // Rows m_begin .. m_end are this block's to finish: a warp takes every fourth of them, a lane four weight rows of it
+      // (16-byte reads of every rank's sums, all of a group of RB rows in flight together).  What the sums are added to
+      // is asked for while the products run.
+      const int rows_per = (NB + split - 1) / split, m_begin = rank * rows_per, m_end = min(min(M, NB), m_begin + rows_per);
+      const int n = n0 + 4 * lane;
+      const bool add = !SWIGLU && accumulate;
+      const bool vec = n + 4 <= N && ((size_t)ldo * sizeof(TO)) % (4 * sizeof(TO)) == 0 && ((uintptr_t)out) % (4 * sizeof(TO)) == 0;
+      auto column = [&](const float* p, float none) {
+        return make_float4(p && n < N ? p[n] : none, p && n + 1 < N ? p[n + 1] : none, p && n + 2 < N ? p[n + 2] : none, p && n + 3 < N ? p[n + 3] : none);
+      };
+      const float4 cs = column(colscale, 1.0f), cb = column(colbias, 0.0f);
+      constexpr int RB = 2;                                 // rows of a group
+      auto before = [&](int m) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (add && m < m_end) {
+          const TO* o = out + (size_t)m * ldo + n;
+          if (vec) v = read4(o);
+          else v = make_float4(n < N ? to_f32(o[0]) : 0.f, n + 1 < N ? to_f32(o[1]) : 0.f, n + 2 < N ? to_f32(o[2]) : 0.f, n + 3 < N ? to_f32(o[3]) : 0.f);
+        }
+        return v;
+      };
+      float4 old[RB];
+#pragma unroll
+      for (int i = 0; i < RB; i++) old[i] = before(m_begin + quarter + 4 * i);
+      mbar_wait(acc_full, 0, err, 33, wait_limit);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+      for (int c = 0; c < NB / CW; c++) {
+        uint32_t r[CW];
+        read_columns(c, r);
+#pragma unroll
+        for (int j = 0; j < CW; j++) part[(c * CW + j) * WM + row] = n_k > 0 ? __uint_as_float(r[j]) : 0.f;
+      }
+      // every block's sums are in its shared memory (the stages are free: every product that read them is complete)
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+      asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+      const float* src[8];                                  // the sums of every rank, this lane's weight rows
+#pragma unroll
+      for (int q = 0; q < 8; q++) src[q] = in_rank(part, min(q, split - 1)) + 4 * lane;
+#pragma unroll 1
+      for (int m0 = m_begin + quarter; m0 < m_end; m0 += 4 * RB) {
+        float4 x[RB][8];
 #pragma unroll
         for (int i = 0; i < RB; i++)
 #pragma unroll
-          for (int q = 0; q < 8; q++) {
-            const bool in = q < split && m0 + i < M && i < rows_per;
-            x[i][q] = in ? src[q][(m0 + i) * WM] : 0.f;
-            x2[i][q] = (SWIGLU && in) ? src[q][(m0 + i) * WM + 8] : 0.f;
-          }
+          for (int q = 0; q < 8; q++)
+            x[i][q] = (q < split && m0 + 4 * i < m_end) ? *reinterpret_cast<const float4*>(src[q] + (m0 + 4 * i) * WM) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int i = 0; i < RB; i++) {
-        const int m = m0 + i;
-        if (m >= M || i >= rows_per) break;
-        float v = 0.f, v2 = 0.f;
+          const int m = m0 + 4 * i;
+          if (m >= m_end) break;                            // (the same for the whole warp)
+          float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int q = 0; q < 8; q++) { v += x[i][q]; v2 += x2[i][q]; }     // in the order of the ranks; absent ranks add zero
-        v = v * cs + cb;
-        if (SWIGLU) {
-          v2 = v2 * cs2 + cb2;
-          out[(size_t)m * ldo + (n0 >> 1) + ((row >> 4) << 3) + (row & 7)] = from_f32<TO>(glu_epilogue<false>(accumulate, v, v2));      // (with SWIGLU the argument carries the activation's code)
-        } else {
-          TO* o = out + (size_t)m * ldo + n;
-          if (accumulate) v += to_f32(*o);
-          *o = from_f32<TO>(v);
+          for (int q = 0; q < 8; q++) { v.x += x[i][q].x; v.y += x[i][q].y; v.z += x[i][q].z; v.w += x[i][q].w; }   // in the order of the ranks; absent ranks add zero
+          v = make_float4(v.x * cs.x + cb.x, v.y * cs.y + cb.y, v.z * cs.z + cb.z, v.w * cs.w + cb.w);
+          if (SWIGLU) {                                     // the up rows sit two lanes above their gate rows
+            const float4 u = make_float4(__shfl_down_sync(0xffffffffu, v.x, 2), __shfl_down_sync(0xffffffffu, v.y, 2),
+                                         __shfl_down_sync(0xffffffffu, v.z, 2), __shfl_down_sync(0xffffffffu, v.w, 2));
+            if (!(lane & 2) && n + 8 < N) {                 // (N is a multiple of 16: the four features are there or none is)
+              TO* o = out + (size_t)m * ldo + (n0 >> 1) + ((lane >> 2) << 3) + (lane & 1) * 4;
+              const float4 y = make_float4(glu_epilogue<false>(accumulate, v.x, u.x), glu_epilogue<false>(accumulate, v.y, u.y),
+                                           glu_epilogue<false>(accumulate, v.z, u.z), glu_epilogue<false>(accumulate, v.w, u.w));
+              if (((uintptr_t)o) % (4 * sizeof(TO)) == 0) write4(o, y);
+              else { o[0] = from_f32<TO>(y.x); o[1] = from_f32<TO>(y.y); o[2] = from_f32<TO>(y.z); o[3] = from_f32<TO>(y.w); }
+            }
+          } else {
+            if (add) { v.x += old[i].x; v.y += old[i].y; v.z += old[i].z; v.w += old[i].w; }
+            TO* o = out + (size_t)m * ldo + n;
+            if (vec) write4(o, v);
+            else {
+              if (n < N) o[0] = from_f32<TO>(v.x);
+              if (n + 1 < N) o[1] = from_f32<TO>(v.y);
+              if (n + 2 < N) o[2] = from_f32<TO>(v.z);
+              if (n + 3 < N) o[3] = from_f32<TO>(v.w);
+            }
+          }
         }
-        }
+#pragma unroll
+        for (int i = 0; i < RB; i++) old[i] = before(m0 + 4 * (RB + i));
       }
     }
+  }
+  __syncwarp();                                             // the loader's and the issuer's warps are whole again
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  if (split > 1 && warp < 2) {                              // the epilogue warps met above
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
   }
   // no block leaves while another may still read its sums
   if (split > 1) {
@@ -213,7 +295,7 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
   } else {
     __syncthreads();
   }
-  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(NB) : "memory");
+  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TCOLS) : "memory");
 }
 
 int g_few_rows = 1;                     // test hook: 0 = never this kernel
@@ -261,10 +343,11 @@ int launch_few(const CUtensorMap& mw, const CUtensorMap& mx, void* out, int ldo,
   return 0;
 }
 
-constexpr int FR_STAGES = 4;
+// Stages of a block's ring: as many as leave room for a second block on the SM (113 KB each).
+constexpr int fr_stages(int NB) { return NB == 16 ? 6 : NB == 32 ? 5 : NB == 64 ? 4 : 3; }
 
 // How many blocks share a tile's K-steps: as many (2, 4, 8) as bring the grid closest to two blocks an SM (what
-// fits with four stages) without passing it, each with at least 4 K-steps.
+// fits beside one another) without passing it, each with at least 4 K-steps.
 int pick_split(int N, int K, int NB, int sms) {
   const int tiles = (N + WM - 1) / WM, num_k = (K + FBK - 1) / FBK;
   int split = 1;
@@ -277,43 +360,58 @@ int run_few(const void* a, int lda, const void* w, int ldw, void* out, int out_d
             const float* colbias, TlcEpi accumulate, int M, int N, int K, int force_split, cudaStream_t stream) {
   static int sms = 0;
   if (sms == 0) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
-  const int NB = M <= 32 ? 32 : M <= 64 ? 64 : 128;
+  const int NB = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
   const int split = force_split > 0 ? force_split : pick_split(N, K, NB, sms);
   CUtensorMap mw, mx;
   if (int rc = tlc_tensor_map_bf16(w, N, K, ldw, FBK, WM, &mw)) return rc;
   if (int rc = tlc_tensor_map_bf16(a, M, K, lda, FBK, NB, &mx)) return rc;
-  // (with 128 activation rows a stage is 32 KB: three of them, so that two blocks still share an SM)
-#define TLC_FEW(TO_, NB_) launch_few<TO_, NB_, (NB_ == 128 ? 3 : FR_STAGES), SWIGLU>(mw, mx, out, ldo, colscale, colbias, accumulate, M, N, K, split, stream)
-  if (out_dtype == TLC_F32) return NB == 32 ? TLC_FEW(float, 32) : NB == 64 ? TLC_FEW(float, 64) : TLC_FEW(float, 128);
-  if (out_dtype == TLC_BF16) return NB == 32 ? TLC_FEW(__nv_bfloat16, 32) : NB == 64 ? TLC_FEW(__nv_bfloat16, 64) : TLC_FEW(__nv_bfloat16, 128);
+#define TLC_FEW(TO_, NB_) launch_few<TO_, NB_, fr_stages(NB_), SWIGLU>(mw, mx, out, ldo, colscale, colbias, accumulate, M, N, K, split, stream)
+#define TLC_FEW_NB(TO_) (NB == 16 ? TLC_FEW(TO_, 16) : NB == 32 ? TLC_FEW(TO_, 32) : NB == 64 ? TLC_FEW(TO_, 64) : TLC_FEW(TO_, 128))
+  if (out_dtype == TLC_F32) return TLC_FEW_NB(float);
+  if (out_dtype == TLC_BF16) return TLC_FEW_NB(__nv_bfloat16);
+#undef TLC_FEW_NB
 #undef TLC_FEW
   return tlc_fail(-1, "linear: unknown output dtype %d", out_dtype);
 }
 
+// bfloat16 operands with 16-byte aligned rows, up to 128 rows, where this kernel is the quickest (microseconds in a captured
+// loop over operand sets larger than the L2):
+//   * from 17 rows on, an output that is wide enough, 32 tiles of 128 weight rows, 16 with more than 32 rows, and not more
+//     tiles than two an SM (96 rows, 3072 -> 130048: 141 with the tiles of the product for prompts, 149 here).  At 64 rows
+//     2048 -> 8240 10.6, 4096 -> 2048 8.2, 2560 -> 16384 with SwiGLU 20.7, 3072 -> 24576 34.9;
+//   * up to 32 rows, a plain 32-bit output of 128 tiles or more, a vocabulary: there the weight-streaming mma.sync kernel
+//     re-reads the activations for every 16 columns, and its rounds of K (2,048; from 9 rows on 1,024) may end in a part
+//     of one (32 rows, 3072 -> 130048: 221 with that kernel, 126 here; 16 rows, 2560 -> 65536: 68 and 53; 8 rows, 3072 ->
+//     130048 141 and 120; 1 row 138 and 117).  Up to 4 rows with full rounds it is as quick (2048 -> 65536: 40.9 and 42.1)
+//     and keeps them.
+// Narrower outputs of up to 32 rows would gain as well (32 rows, 12288 -> 3072: 31.6 and 15.9), but their sums would be made
+// in another order, and what a layer rounds to 16 bits after them would move the tokens that a model picks; a logit is
+// not rounded again.
+// With a forced split (tests) any output of at least one tile qualifies, from 9 rows on.
+int few_rows_ok(int a_dtype, int lda, const void* a, int w_dtype, int ldw, const void* w, int M, int N, int K, bool plain32) {
+  static int sms = 0;
+  if (sms == 0) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
+  if (!g_few_rows || a_dtype != TLC_BF16 || w_dtype != TLC_BF16 || M > g_max_rows || K % 8 != 0 || lda % 8 != 0 || ldw % 8 != 0 ||
+      (uintptr_t)a % 16 != 0 || (uintptr_t)w % 16 != 0 || tlc_error_words() == nullptr)
+    return 0;
+  const int tiles = (N + WM - 1) / WM;
+  if (g_force_split > 0) return M > 8 && N >= WM;
+  if (M <= 32 && plain32 && tiles >= 128) return M > 4 || K % 2048 != 0;
+  return M > 16 && N >= (g_min_tiles > 0 ? g_min_tiles : M > 32 ? 16 : 32) * WM && tiles <= 2 * sms;
+}
+
 }  // namespace
 
-// Test hooks: whether products of 17..64 rows may take this kernel; a fixed number of blocks per tile (0: chosen).
+// Test hooks: whether products of up to 128 rows may take this kernel; a fixed number of blocks per tile (0: chosen).
 extern "C" void tlc_linear_few_rows(int on) { g_few_rows = on; }
 extern "C" void tlc_linear_few_rows_split(int split) { g_force_split = split; }
 extern "C" void tlc_linear_few_rows_min_tiles(int tiles) { g_min_tiles = tiles; }
 extern "C" void tlc_linear_few_rows_max_rows(int rows) { g_max_rows = rows; }
 
-// bfloat16 operands with 16-byte aligned rows, 17..64 rows, and an output that is wide enough: from 32 tiles of 128
-// weight rows on, from 16 with more than 32 rows.  Measured at 48 and 64 rows, microseconds in a captured loop over
-// operand sets larger than the L2: N = 8240, K = 2048: 11.5 against 14.2 for the kernels that run these sizes
-// otherwise; N = 8192 with SwiGLU 12.3 against 13.5; N = 2048, K = 4096: 12.0 against 12.0 alone, but inside the
-// captured decode step at batch 64 the two products with N = 2048 make 4.08 -> 3.79 ms a step (the
-// weight-streaming kernel re-reads 64 rows of activations per 16 columns), at batch 32 and 24 2.40 -> 2.44 and
-// 2.13 -> 2.17.  With a forced split (tests) any output of at least one tile qualifies.
-extern "C" int tlc_linear_few_rows_ok(int a_dtype, int lda, const void* a, int w_dtype, int ldw, const void* w, int M, int N, int K) {
-  // more tiles than two an SM (a vocabulary-sized output: 512 tiles) are better served by the persistent tiles of
-  // the product for prompts: 55 us against 62 for 64 x 65,536 x 2,048
-  static int sms = 0;
-  if (sms == 0) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
-  if (g_force_split == 0 && (N + WM - 1) / WM > 2 * sms) return 0;
-  return g_few_rows && a_dtype == TLC_BF16 && w_dtype == TLC_BF16 && M > 16 && M <= g_max_rows && N >= (g_force_split > 0 ? 1 : g_min_tiles > 0 ? g_min_tiles : M > 32 ? 16 : 32) * WM &&
-         K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0 && ((uintptr_t)a % 16 == 0) && ((uintptr_t)w % 16 == 0) &&
-         tlc_error_words() != nullptr;
+// plain32: the output is 32-bit and overwritten, not added to.
+extern "C" int tlc_linear_few_rows_ok(int a_dtype, int lda, const void* a, int w_dtype, int ldw, const void* w, int M, int N, int K,
+                                      int plain32) {
+  return few_rows_ok(a_dtype, lda, a, w_dtype, ldw, w, M, N, K, plain32 != 0);
 }
 
 int tlc_linear_few_rows_run(const void* a, int lda, const void* w, int ldw, void* out, int out_dtype, int ldo,
