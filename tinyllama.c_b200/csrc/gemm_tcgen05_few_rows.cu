@@ -344,7 +344,7 @@ int launch_few(const CUtensorMap& mw, const CUtensorMap& mx, void* out, int ldo,
 }
 
 // Stages of a block's ring: as many as leave room for a second block on the SM (113 KB each).
-constexpr int fr_stages(int NB) { return NB == 16 ? 6 : NB == 32 ? 5 : NB == 64 ? 4 : 3; }
+constexpr int fr_stages(int NB) { return NB == 16 ? 6 : NB <= 64 ? 4 : 3; }
 
 // How many blocks share a tile's K-steps: as many (2, 4, 8) as bring the grid closest to two blocks an SM (what
 // fits beside one another) without passing it, each with at least 4 K-steps.
