@@ -16,6 +16,14 @@
 // (row, key/value head) the block writes the output itself, otherwise partial results go to scratch and
 // the last block to arrive merges them.
 //
+// Where the grid is small (CLUSTER_BLOCKS) the splits of a (row, key/value head), up to 8, are one thread-block cluster: each
+// block leaves its outputs and statistics in its own shared memory, the cluster meets at a barrier, and block r merges
+// its share of the outputs from all of them, read through distributed shared memory in the order of the splits.  Through
+// scratch and an arrival counter the merge is five trips to memory one after the other: one sequence of 128 tokens, a
+// step of the 1.5B sizes 1036 us, as a cluster 924.  More blocks go through scratch: a cluster's blocks start together and stay
+// until the last has read, and beside another mixer's kernel that costs more than it saves (8 sequences, 128 blocks: a step
+// 1280 us through scratch, 1322 as clusters).
+//
 // Arrival counting: every block of a (row, kv head) adds one to arrivals[row * KV + kv head] with
 // atomicInc modulo the number of splits, so the counter is back at zero when the kernel ends and needs
 // no clearing between launches.  It must be zero before the first launch.
@@ -63,6 +71,13 @@ __device__ __forceinline__ unsigned pack_bf16(float lo, float hi) {
   return *reinterpret_cast<const unsigned*>(&v);
 }
 
+// The same shared-memory word in the block of another rank of the cluster, for ordinary loads.
+template <typename T> __device__ __forceinline__ const T* fm_in_rank(const T* p, int rank) {
+  unsigned long long q;
+  asm("mapa.u64 %0, %1, %2;" : "=l"(q) : "l"((unsigned long long)(uintptr_t)p), "r"(rank));
+  return reinterpret_cast<const T*>((uintptr_t)q);
+}
+
 template <int HD, int CK, int STAGES>
 struct FmSmem {
   static constexpr int ROWB = HD * 2;                       // bytes of a key or value row
@@ -76,7 +91,7 @@ struct FmSmem {
 // HD: head size; CK: keys of a chunk (a multiple of 16); STAGES: chunks of a warp in shared memory.
 // A block takes `passes` rounds of FM_NW chunks, one per warp.  Within a row of shared memory the
 // 16-byte pieces are stored at piece ^ (row & 7): ldmatrix then reads eight rows without bank conflicts.
-template <int HD, int CK, int STAGES>
+template <int HD, int CK, int STAGES, bool CLUSTER>
 __global__ void __launch_bounds__(FM_NT)
 attention_decode_fused_kernel(const float* __restrict__ qkv, int ld, int q_off, int k_off, int v_off,
                             __nv_bfloat16* __restrict__ k_pages, __nv_bfloat16* __restrict__ v_pages,
@@ -111,9 +126,15 @@ attention_decode_fused_kernel(const float* __restrict__ qkv, int ld, int q_off, 
   float* ml = part_ml + (((size_t)t * H + (size_t)g * G) * n_splits + split) * 2;
   const bool empty = kbase >= n_keys || (kbase + span <= start && kbase >= kept);     // the same for all threads of the block
   __shared__ int s_last;
+  __shared__ float2 s_ml[CLUSTER ? FM_MAXG : 1];           // a cluster's block: maximum and sum of each head over its keys
   if (empty) {
-    tlc_wait(ml);
-    if (tid < G) { ml[(size_t)tid * n_splits * 2] = -INFINITY; ml[(size_t)tid * n_splits * 2 + 1] = 0.f; }
+    if constexpr (CLUSTER) {
+      tlc_wait(out, head_gate);
+      if (tid < FM_MAXG) s_ml[tid] = make_float2(-INFINITY, 0.f);
+    } else {
+      tlc_wait(ml);
+      if (tid < G) { ml[(size_t)tid * n_splits * 2] = -INFINITY; ml[(size_t)tid * n_splits * 2 + 1] = 0.f; }
+    }
   } else {
     unsigned char* wsm = smraw + (size_t)w * L::WARP;                                // this warp's stages
     unsigned char* qsm = smraw + (size_t)FM_NW * L::WARP;                            // [8][HD] bfloat16
@@ -337,7 +358,10 @@ attention_decode_fused_kernel(const float* __restrict__ qkv, int ld, int q_off, 
         }
       }
       const size_t th = (size_t)t * H + (size_t)g * G + hg;
-      if (n_splits == 1) {
+      if constexpr (CLUSTER) {
+        reinterpret_cast<float*>(smraw)[hg * HD + d] = o;        // over the first warp's share of this value, which only this thread reads
+        if (d == 0) s_ml[hg] = make_float2(M, l);
+      } else if (n_splits == 1) {
         out[(size_t)t * out_ld + ((size_t)g * G + hg) * HD + d] =
             __float2bfloat16_rn(o * (tlc_head_gate(head_gate, gate_ld, t, g * G + hg) / l));
       } else {
@@ -345,6 +369,55 @@ attention_decode_fused_kernel(const float* __restrict__ qkv, int ld, int q_off, 
         if (d == 0) { ml[(size_t)hg * n_splits * 2] = M; ml[(size_t)hg * n_splits * 2 + 1] = l; }
       }
     }
+  }
+  if constexpr (CLUSTER) {
+    // ---- the blocks of the cluster meet; each merges its share of the outputs ----
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    const int per = (G * HD + n_splits - 1) / n_splits, first = split * per, last = min(G * HD, first + per);
+    const float2* ml_of[8];
+    const float* o_of[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      ml_of[q] = fm_in_rank(s_ml, min(q, n_splits - 1));
+      o_of[q] = fm_in_rank(reinterpret_cast<const float*>(smraw), min(q, n_splits - 1));
+    }
+    for (int idx = first + tid; idx < last; idx += FM_NT) {
+      const int hg = idx / HD, d = idx % HD;
+      float2 st[8];
+      float o[8];
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        st[q] = q < n_splits ? ml_of[q][hg] : make_float2(-INFINITY, 0.f);
+        o[q] = q < n_splits ? o_of[q][idx] : 0.f;
+      }
+      // the arithmetic of attention_merge_splits, sum by sum, so that both give the same bits (its sum over the splits is a
+      // warp's: lanes 4 apart, then 2, then 1)
+      const float sv = (sink && sink_values) ? sink_values[g * G + hg] : 0.f;
+      float M = -INFINITY;
+#pragma unroll
+      for (int q = 0; q < 8; q++) M = fmaxf(M, st[q].x);
+      if (sink) M = fmaxf(M, sv);
+      float e[8], x[8];
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        e[q] = st[q].y > 0.f ? expf(st[q].x - M) : 0.f;                // (a block without keys has left no outputs)
+        x[q] = __fmul_rn(st[q].y, e[q]);
+      }
+      float l = ((x[0] + x[4]) + (x[2] + x[6])) + ((x[1] + x[5]) + (x[3] + x[7]));
+      if (sink) l += expf(sv - M);
+      const float inv = tlc_head_gate(head_gate, gate_ld, t, g * G + hg) / l;
+      float acc = 0.f;
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        const float wq = __fmul_rn(e[q], inv);
+        if (wq != 0.f) acc = fmaf(o[q], wq, acc);
+      }
+      out[(size_t)t * out_ld + ((size_t)g * G + hg) * HD + d] = __float2bfloat16_rn(acc);
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // every block's shared memory stays until all have read it
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    return;
   }
   if (n_splits == 1) return;                      // one block per (row, kv head): it wrote the output itself
   // ---- the last block of this (row, kv head) merges the splits ----
@@ -360,19 +433,36 @@ attention_decode_fused_kernel(const float* __restrict__ qkv, int ld, int q_off, 
   attention_merge_splits<HD, FM_NT>(part_o, part_ml, out, reinterpret_cast<float*>(smraw), smem_floats, t, g, G, H, n_splits, out_ld, sink, sink_values, head_gate, gate_ld);
 }
 
+constexpr int CLUSTER_BLOCKS = 32;
 int g_fused_passes = 0;       // > 0: rounds a block takes, for tests (0: chosen from the grid)
 
-template <int HD, int CK, int STAGES, typename... Args>
+template <int HD, int CK, int STAGES, bool CLUSTER, typename... Args>
 cudaError_t launch_fused(dim3 grid, int passes, cudaStream_t stream, Args... args) {
   static bool raised[64] = {};          // per device: the kernel uses more than 48 KB of shared memory
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !raised[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(attention_decode_fused_kernel<HD, CK, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaError_t e = cudaFuncSetAttribute(attention_decode_fused_kernel<HD, CK, STAGES, CLUSTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     if (e != cudaSuccess) return e;
     raised[dev] = true;
   }
-  return tlc_launch(attention_decode_fused_kernel<HD, CK, STAGES>, grid, dim3(FM_NT), FmSmem<HD, CK, STAGES>::bytes(passes), stream, args...);
+  if constexpr (!CLUSTER)
+    return tlc_launch(attention_decode_fused_kernel<HD, CK, STAGES, CLUSTER>, grid, dim3(FM_NT), FmSmem<HD, CK, STAGES>::bytes(passes), stream, args...);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(FM_NT);
+  cfg.dynamicSmemBytes = FmSmem<HD, CK, STAGES>::bytes(passes);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = grid.z;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = g_tlc_pdl ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, attention_decode_fused_kernel<HD, CK, STAGES, CLUSTER>, args...);
 }
 
 }  // namespace
@@ -424,16 +514,19 @@ extern "C" int tlc_attention_decode_fused(const float* qkv, int ld, int q_off, i
   // blocks fit an SM, and the model's step at batch 8 took 1.82 ms instead of 1.44.
   const size_t smem = hd == 64 ? FmSmem<64, 32, 4>::bytes(passes) : hd == 128 ? FmSmem<128, 32, 2>::bytes(passes) : FmSmem<256, 16, 2>::bytes(passes);
   TLC_REQUIRE(smem <= 200 * 1024, "attention(decode, fused): %d keys need %zu bytes of shared memory", max_keys, smem);
+  const int clustered = n_splits > 1 && n_splits <= 8 && rows * n_splits <= CLUSTER_BLOCKS;
   dim3 grid(T, KV, n_splits);
   __nv_bfloat16 *kp = (__nv_bfloat16*)k_pages, *vp = (__nv_bfloat16*)v_pages, *op = (__nv_bfloat16*)out;
   cudaError_t e = cudaSuccess;
-#define TLC_FM_LAUNCH(HDV, CKV, STV)                                                                                   \
-  e = launch_fused<HDV, CKV, STV>(grid, passes, stream, qkv, ld, q_off, k_off, v_off, kp, vp, inv_freq, rope_dim, write_kv, \
+#define TLC_FM_LAUNCH_AS(HDV, CKV, STV, CLV)                                                                                   \
+  e = launch_fused<HDV, CKV, STV, CLV>(grid, passes, stream, qkv, ld, q_off, k_off, v_off, kp, vp, inv_freq, rope_dim, write_kv, \
                                 block_table, max_pages, positions, row_seq, slots, part_o, part_ml, arrivals, op, H, KV, \
                                 scale, window, n_splits, passes, out_ld, softcap, sink, keep_first, sink_values, chunk, head_gate, gate_ld)
+#define TLC_FM_LAUNCH(HDV, CKV, STV) do { if (clustered) TLC_FM_LAUNCH_AS(HDV, CKV, STV, true); else TLC_FM_LAUNCH_AS(HDV, CKV, STV, false); } while (0)
   if (hd == 64) TLC_FM_LAUNCH(64, 32, 4);
   else if (hd == 128) TLC_FM_LAUNCH(128, 32, 2);
   else TLC_FM_LAUNCH(256, 16, 2);
+#undef TLC_FM_LAUNCH_AS
 #undef TLC_FM_LAUNCH
   if (e != cudaSuccess) return tlc_fail(-2, "attention(decode, fused): %s", cudaGetErrorString(e));
   TLC_CHECK_LAUNCH("attention(decode)");

@@ -41,22 +41,39 @@ __device__ __forceinline__ void attention_merge_splits(const float* part_o, cons
       for (int s = lane; s < n_splits; s += 32) e[2 * s] = e[2 * s + 1] > 0.f ? expf(e[2 * s] - m) * inv : 0.f;
     }
     __syncthreads();
-    for (int idx = tid; idx < G * HD; idx += NT) {
-      const int hg = idx / HD, d = idx % HD;
-      const size_t th = (size_t)t * H + (size_t)g * G + hg;
-      const float* e = sh + (size_t)2 * hg * n_splits;
-      const float* po = part_o + th * n_splits * HD + d;
-      float acc = 0.f;
-      int s = 0;
-      for (; s + 8 <= n_splits; s += 8) {
-        float v[8];
+    // four outputs of a thread at a time, eight splits of each: 32 loads in flight, all unconditional (past the last split or
+    // output they read the last one, with weight 0); one output after the other, 32 splits were 16 trips to memory in a row
+    constexpr int NI = 4, NS = 8;
+    for (int base = tid; base < G * HD; base += NI * NT) {
+      const float* po[NI];
+      const float* e[NI];
+      float acc[NI];
 #pragma unroll
-        for (int u = 0; u < 8; u++) v[u] = __ldcg(po + (size_t)(s + u) * HD);
-#pragma unroll
-        for (int u = 0; u < 8; u++) { const float w = e[2 * (s + u)]; acc = w != 0.f ? fmaf(v[u], w, acc) : acc; }
+      for (int i = 0; i < NI; i++) {
+        const int idx = min(base + i * NT, G * HD - 1), hg = idx / HD;
+        po[i] = part_o + ((size_t)t * H + (size_t)g * G + hg) * n_splits * HD + idx % HD;
+        e[i] = sh + (size_t)2 * hg * n_splits;
+        acc[i] = 0.f;
       }
-      for (; s < n_splits; s++) { const float w = e[2 * s]; const float v = __ldcg(po + (size_t)s * HD); acc = w != 0.f ? fmaf(v, w, acc) : acc; }
-      out[(size_t)t * out_ld + ((size_t)g * G + hg) * HD + d] = __float2bfloat16_rn(acc);
+      for (int s0 = 0; s0 < n_splits; s0 += NS) {
+        float v[NI][NS];
+#pragma unroll
+        for (int u = 0; u < NS; u++)
+#pragma unroll
+          for (int i = 0; i < NI; i++) v[i][u] = __ldcg(po[i] + (size_t)min(s0 + u, n_splits - 1) * HD);
+#pragma unroll
+        for (int u = 0; u < NS; u++)
+#pragma unroll
+          for (int i = 0; i < NI; i++) {
+            const float w = s0 + u < n_splits ? e[i][2 * (s0 + u)] : 0.f;
+            acc[i] = w != 0.f ? fmaf(v[i][u], w, acc[i]) : acc[i];
+          }
+      }
+#pragma unroll
+      for (int i = 0; i < NI; i++) {
+        const int idx = base + i * NT;
+        if (idx < G * HD) out[(size_t)t * out_ld + (size_t)g * G * HD + idx] = __float2bfloat16_rn(acc[i]);
+      }
     }
     return;
   }
