@@ -326,12 +326,18 @@ extern "C" int tlc_mamba_conv(const void* proj, int dtype, int ld, int xbc_off, 
 // grid (segment, Hs, ceil(P / (4*RP))), 128 threads: each warp owns RP rows p of one head's state
 // [P, N], each lane the columns lane, lane+32, ... (NPL of them) in registers.  Rows run in
 // order; the inputs of SCAN_TT rows are staged in shared memory at a time.
-#define SCAN_TT 8
+#define SCAN_TT 4
 #define SCAN_PLAIN 0
 #define SCAN_CHUNK_STATE 1
 #define SCAN_CHUNK_OUT 3
+__device__ __forceinline__ void scan_copy16(float* dst, const float* src, bool on) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(on ? 16 : 0) : "memory");   // (0: zeros)
+}
+__device__ __forceinline__ void scan_copy4(float* dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
 template <int NPL, int RP>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, 7)
 ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dt, const float* __restrict__ dA,
                 const float* __restrict__ Dskip, float* __restrict__ state, float* __restrict__ chunk_state,
                 const int* __restrict__ seg_start, const int* __restrict__ seg_seq,
@@ -388,33 +394,54 @@ ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dt, con
     }
   }
   if (mode == SCAN_PLAIN) tlc_wait(xbc, dt, dA, y);
-  // shared staging: per row  B[N] | C[N] | x[rows_per_block] | dt | dA
-  const int per_tok = 2 * N + rows_per_block + 2;
+  // Shared staging: per row  B[N] | C[N] | x[rows_per_block] | dt | dA, the rows SCAN_TT at a time, in two buffers: the
+  // copies of a batch, in pieces of 16 bytes where the rows are laid out in them, are on their way while the batch
+  // before it is worked on, so that a row costs its arithmetic and not a trip to memory (a loop over the rows, each with
+  // its own loads, made a row of a 23-token prompt take 2 us).
+  const int per_tok = 2 * N + rows_per_block + 4;            // (a multiple of 4 where N is one)
   const float Dh = Dskip[h];
-  for (int tt0 = 0; tt0 < n_tok; tt0 += SCAN_TT) {
+  const bool quads = N % 4 == 0 && P % 4 == 0 && Cd % 4 == 0 && ((uintptr_t)xbc & 15) == 0;
+  const int nq = N >> 2, row_q = 2 * nq + RP;                // pieces of a row: B, C, x (4 RP values)
+  auto fetch = [&](int tt0, float* buf) {
     const int nt = min(SCAN_TT, n_tok - tt0);
-    __syncthreads();
-    for (int k = 0; k < nt; k++) {
-      const float* row = xbc + (size_t)(t0 + tt0 + k) * Cd;
-      float* dst = sm + (size_t)k * per_tok;
-      const float* Bg = row + Di + (size_t)g * N;
-      const float* Cg = row + Di + (size_t)G * N + (size_t)g * N;
-      for (int e = threadIdx.x; e < N; e += blockDim.x) {
-        dst[e] = Bg[e];
-        dst[N + e] = want_y ? Cg[e] : 0.f;
+    if (quads) {
+      for (int idx = threadIdx.x; idx < nt * row_q; idx += 128) {
+        const int k = idx / row_q, q = idx - k * row_q;
+        const float* row = xbc + (size_t)(t0 + tt0 + k) * Cd;
+        const int p = p_blk + 4 * (q - 2 * nq);
+        const float* src = row;
+        bool on = true;
+        if (q < nq) src = row + Di + (size_t)g * N + 4 * q;
+        else if (q < 2 * nq) { src = row + Di + (size_t)G * N + (size_t)g * N + 4 * (q - nq); on = want_y; }
+        else { on = p < P; if (on) src = row + (size_t)h * P + p; }
+        scan_copy16(buf + (size_t)k * per_tok + 4 * q, src, on);
       }
-      if (threadIdx.x < rows_per_block) {
-        const int p = p_blk + threadIdx.x;
-        dst[2 * N + threadIdx.x] = p < P ? row[(size_t)h * P + p] : 0.f;
-      } else if (threadIdx.x == 32 + rows_per_block) {
-        dst[2 * N + rows_per_block] = dt[(size_t)(t0 + tt0 + k) * Hs + h];
-      } else if (threadIdx.x == 64 + rows_per_block) {
-        dst[2 * N + rows_per_block + 1] = dA[(size_t)(t0 + tt0 + k) * Hs + h];
+    } else {
+#pragma unroll 4
+      for (int idx = threadIdx.x; idx < nt * (per_tok - 4); idx += 128) {
+        const int k = idx / (per_tok - 4), e = idx - k * (per_tok - 4);
+        const float* row = xbc + (size_t)(t0 + tt0 + k) * Cd;
+        float v = 0.f;
+        if (e < N) v = row[Di + (size_t)g * N + e];
+        else if (e < 2 * N) { if (want_y) v = row[Di + (size_t)G * N + (size_t)g * N + (e - N)]; }
+        else if (p_blk + e - 2 * N < P) v = row[(size_t)h * P + p_blk + (e - 2 * N)];
+        buf[(size_t)k * per_tok + e] = v;
       }
     }
-    __syncthreads();
+    if (threadIdx.x < 2 * SCAN_TT && (threadIdx.x >> 1) < nt)
+      scan_copy4(buf + (size_t)(threadIdx.x >> 1) * per_tok + 2 * N + rows_per_block + (threadIdx.x & 1),
+                 ((threadIdx.x & 1) ? dA : dt) + (size_t)(t0 + tt0 + (threadIdx.x >> 1)) * Hs + h);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fetch(0, sm);
+  for (int tt0 = 0, turn = 0; tt0 < n_tok; tt0 += SCAN_TT, turn ^= 1) {
+    const int nt = min(SCAN_TT, n_tok - tt0);
+    float* smb = sm + (size_t)turn * SCAN_TT * per_tok;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                                         // this batch is here, and every warp is done with the one before it
+    if (tt0 + SCAN_TT < n_tok) fetch(tt0 + SCAN_TT, sm + (size_t)(turn ^ 1) * SCAN_TT * per_tok);
     for (int k = 0; k < nt; k++) {
-      const float* tk = sm + (size_t)k * per_tok;
+      const float* tk = smb + (size_t)k * per_tok;
       const float dtv = tk[2 * N + rows_per_block], dAv = tk[2 * N + rows_per_block + 1];
       float Bv[NPL], Cv[NPL];
 #pragma unroll
@@ -571,7 +598,7 @@ static int launch_scan(const float* xbc, const float* dt, const float* dA, const
                        int P, int N, int G, int Cd, cudaStream_t stream) {
   constexpr int RP = 4;
   dim3 grid(n_seg, Hs, (P + 4 * RP - 1) / (4 * RP));
-  const size_t smem = (size_t)SCAN_TT * (2 * N + 4 * RP + 2) * sizeof(float);
+  const size_t smem = (size_t)2 * SCAN_TT * (2 * N + 4 * RP + 4) * sizeof(float);
   tlc_launch(ssm_scan_kernel<NPL, RP>, dim3(grid), dim3(128), smem, stream, xbc, dt, dA, Dskip, state, chunk_state, seg_start, seg_seq,
                                                         seq_seg_start, slots, start_pos, y, chunk_decay, mode, Hs, P, N, G,
                                                         Cd);
