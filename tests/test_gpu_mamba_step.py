@@ -1,0 +1,46 @@
+"""One-token steps of the Mamba2 mixer in one kernel: the same bits as the convolution and the scan as two kernels."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("bf16_run", [False, True])
+@pytest.mark.parametrize("Hs,P,N,G,K,bias", [(4, 16, 68, 1, 4, True), (2, 20, 128, 2, 3, False), (6, 4, 132, 3, 2, True), (3, 64, 256, 1, 4, True),
+                                             (8, 36, 72, 4, 4, False), (120, 36, 72, 4, 4, False), (64, 64, 256, 1, 4, True)])
+def test_step_kernel_against_convolution_and_scan(Hs, P, N, G, K, bias, bf16_run):
+    """State columns that fill a warp's loads or not, rows of a head that end inside a block (of 16 rows, with many heads
+    of 32), several groups, sequences at position 0 (zero window, zero state) beside ones that continue, slots in any
+    order; y, the states and, after the norm that follows, all windows."""
+    from tinyllama_c_b200 import ops
+    g = torch.Generator().manual_seed(Hs * 1009 + N)
+    B, Di = 5, Hs * P
+    Cd = Di + 2 * G * N
+    rnd = lambda *s: torch.randn(*s, generator=g).cuda()  # noqa: E731
+    width = (Di + Cd + Hs + 11) // 4 * 4
+    proj = rnd(B, width)
+    w, cb = rnd(Cd, K), rnd(Cd) if bias else None
+    dt_bias, A, D, norm_w = rnd(Hs), -rnd(Hs).abs() - 0.1, rnd(Hs), rnd(Di)
+    conv0, state0 = rnd(7, K - 1, Cd), rnd(7, Hs, P, N)
+    slots = torch.tensor([3, 0, 6, 2, 5], dtype=torch.int32).cuda()
+    start = torch.tensor([9, 0, 130, 1, 0], dtype=torch.int32).cuda()
+    ar = torch.arange(B + 1, dtype=torch.int32).cuda()
+    z, eps = proj[:, :Di], 1e-5
+    got = []
+    for fused in (False, True):
+        conv, state, y = conv0.clone(), state0.clone(), torch.full((B, Di), 7.0, device="cuda")
+        out = torch.empty(B, Di, device="cuda", dtype=torch.bfloat16 if bf16_run else torch.float32)
+        if fused:
+            assert ops.mamba_step_ok(proj, Di, Hs, P, N, G, K)
+            ops.mamba_step(proj, Di, Di + Cd, w, cb, dt_bias, A, D, conv, state, slots, start, y, Hs, P, N, G, bf16_run)
+            ops.gated_rmsnorm(y, z, norm_w, eps, G, False, out, 0.5, window=(proj, Di, conv, slots, start, Di, Cd - Di))
+        else:
+            xbc, dt, dA = torch.empty(B, Cd, device="cuda"), torch.empty(B, Hs, device="cuda"), torch.empty(B, Hs, device="cuda")
+            ops.mamba_conv(proj, Di, Di + Cd, w, cb, dt_bias, A, conv, ar, ar[:B].contiguous(), slots, start, xbc, dt, dA, True, bf16_run)
+            ops.ssm_scan(xbc, dt, dA, D, state, ar, slots, start, y, Hs, P, N, G)
+            ops.gated_rmsnorm(y, z, norm_w, eps, G, False, out, 0.5)
+        torch.cuda.synchronize()
+        ops.check_errors()
+        got.append((y, state, conv, out))
+    for a, b, name in zip(got[0], got[1], ("y", "states", "windows", "gated output")):
+        assert torch.equal(a, b), name

@@ -282,17 +282,51 @@ gated_rmsnorm_kernel(const float* __restrict__ y, const float* __restrict__ y2, 
   }
 }
 
+// After a one-token step of the scan: the convolution windows that the scan's blocks share (see mamba_step_kernel) advance
+// here, behind all of them.  Row b of the step is sequence b's only one: window row j <- j + 1 (zeros at the sequence's
+// start), the last one <- the raw sample.  rows: blocks of the launch that norm; the T blocks behind them advance windows.
+struct WindowStep {
+  float* state;
+  const float* proj;
+  const int* slots;
+  const int* start_pos;
+  int ld, off, Cd, c0, n, K, rows;
+};
+__device__ __forceinline__ void advance_window(const WindowStep& ws, int b) {
+  const bool has_state = ws.start_pos[b] > 0;
+  float* st = ws.state + (size_t)ws.slots[b] * (ws.K - 1) * ws.Cd + ws.c0;
+  const float* raw = ws.proj + (size_t)b * ws.ld + ws.off + ws.c0;
+  for (int c = threadIdx.x; c < ws.n; c += blockDim.x) {
+    const float last = raw[c];
+    float v[2];                                          // (2 to 4 taps)
+#pragma unroll
+    for (int k = 0; k < 2; k++) v[k] = (k < ws.K - 2 && has_state) ? st[(size_t)(k + 1) * ws.Cd + c] : 0.f;
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+      if (k < ws.K - 1) st[(size_t)k * ws.Cd + c] = k < ws.K - 2 ? v[k < 2 ? k : 0] : last;
+  }
+}
+__global__ void __launch_bounds__(256) window_step_kernel(WindowStep ws) {
+  tlc_pdl(ws.state, ws.proj);
+  advance_window(ws, blockIdx.x);
+}
+
 // Groups whose width is a multiple of 4 (up to 16384), 32-bit gate: NT threads take PT float4 each;
 // the weight is fetched before the wait on the previous kernel.
 template <typename TO, int NT, int PT>
 __global__ void __launch_bounds__(NT)
 gated_rmsnorm_vec_kernel(const float* __restrict__ y, const float* __restrict__ y2, const float* __restrict__ z, int ldz, const float* __restrict__ w,
                          float eps, int Di, int gs, int mode, TO* __restrict__ out, int out_ld,
-                         float out_scale) {
+                         float out_scale, WindowStep ws) {
   asm volatile("griddepcontrol.launch_dependents;");
   __shared__ float red[33];
   const bool norm_before_gate = mode & TLC_GATE_NORM_FIRST, sig = mode & TLC_GATE_SIGMOID;
   const int t = blockIdx.x, g = blockIdx.y;
+  if (t >= ws.rows) {
+    tlc_wait(ws.state, ws.proj);
+    if (g == 0) advance_window(ws, t - ws.rows);
+    return;
+  }
   const int n4 = gs >> 2;
   float4 wv[PT], v[PT], gate[PT];
 #pragma unroll
@@ -377,10 +411,13 @@ gated_rmsnorm_warp_kernel(const float* __restrict__ y, const float* __restrict__
     Out4<TO>::put(o, v.x * s * wv.x, v.y * s * wv.y, v.z * s * wv.z, v.w * s * wv.w);
 }
 
-extern "C" int tlc_gated_rmsnorm(const float* y, const float* y2, const void* z, int z_dtype, int ldz, const float* w, float eps, int T,
-                                 int Di, int n_groups, int mode, void* out, int out_dtype, int out_ld,
-                                 float out_scale, cudaStream_t stream) {
+static int gated_rmsnorm_launch(const float* y, const float* y2, const void* z, int z_dtype, int ldz, const float* w, float eps, int T,
+                                int Di, int n_groups, int mode, void* out, int out_dtype, int out_ld, float out_scale,
+                                WindowStep ws, cudaStream_t stream) {
   if (T == 0) return 0;
+  const bool windows = ws.state != nullptr;
+  ws.rows = T;
+  auto windows_alone = [&]() { if (windows) tlc_launch(window_step_kernel, dim3(T), dim3(256), 0, stream, ws); };
   if (out_ld <= 0) out_ld = Di;                          // elements between rows of out (0: dense)
   TLC_REQUIRE(n_groups > 0 && Di % n_groups == 0, "gated_rmsnorm: width %d is not a multiple of %d groups", Di, n_groups);
   const int gs = Di / n_groups;
@@ -394,12 +431,14 @@ extern "C" int tlc_gated_rmsnorm(const float* y, const float* y2, const void* z,
       TLC_DISPATCH_DTYPE(out_dtype, TO, tlc_launch(gated_rmsnorm_warp_kernel<TO>, dim3((unsigned)((n_rows + 7) / 8)), dim3(256), 0, stream,
                                                    y, y2, (const float*)z, ldz, w, eps, n_rows, n_groups, Di, gs, mode,
                                                    (TO*)out, out_ld, out_scale));
+      windows_alone();
       TLC_CHECK_LAUNCH("gated_rmsnorm");
       return 0;
     }
+    if (windows) grid.x = 2 * T;
 #define TLC_GRMS_LAUNCH(NT, PT)                                                                                         \
   TLC_DISPATCH_DTYPE(out_dtype, TO, tlc_launch(gated_rmsnorm_vec_kernel<TO, NT, PT>, grid, dim3(NT), 0, stream, y, y2,    \
-                                               (const float*)z, ldz, w, eps, Di, gs, mode, (TO*)out, out_ld, out_scale))
+                                               (const float*)z, ldz, w, eps, Di, gs, mode, (TO*)out, out_ld, out_scale, ws))
     if (T >= VEC_MANY_ROWS) { TLC_VEC_SHAPES_MANY(n4, TLC_GRMS_LAUNCH) } else { TLC_VEC_SHAPES(n4, TLC_GRMS_LAUNCH) }
 #undef TLC_GRMS_LAUNCH
     TLC_CHECK_LAUNCH("gated_rmsnorm");
@@ -407,8 +446,24 @@ extern "C" int tlc_gated_rmsnorm(const float* y, const float* y2, const void* z,
   }
   TLC_DISPATCH_DTYPE(z_dtype, TZ, TLC_DISPATCH_DTYPE(out_dtype, TO, tlc_launch(gated_rmsnorm_kernel<TZ, TO>, dim3(grid), dim3(256), 0, stream, 
       y, y2, (const TZ*)z, ldz, w, eps, Di, gs, mode, (TO*)out, out_ld, out_scale)));
+  windows_alone();
   TLC_CHECK_LAUNCH("gated_rmsnorm");
   return 0;
+}
+
+extern "C" int tlc_gated_rmsnorm(const float* y, const float* y2, const void* z, int z_dtype, int ldz, const float* w, float eps, int T,
+                                 int Di, int n_groups, int mode, void* out, int out_dtype, int out_ld,
+                                 float out_scale, cudaStream_t stream) {
+  return gated_rmsnorm_launch(y, y2, z, z_dtype, ldz, w, eps, T, Di, n_groups, mode, out, out_dtype, out_ld, out_scale, WindowStep{}, stream);
+}
+
+extern "C" int tlc_gated_rmsnorm_step(const float* y, const float* z, int ldz, const float* w, float eps, int T, int Di, int n_groups,
+                                      int mode, void* out, int out_dtype, int out_ld, float out_scale, const float* proj, int ld,
+                                      int xbc_off, float* conv_state, const int* slots, const int* start_pos, int Cd, int c0,
+                                      int n_channels, int K, cudaStream_t stream) {
+  TLC_REQUIRE(K >= 2 && K <= 4 && c0 >= 0 && n_channels >= 0 && c0 + n_channels <= Cd, "gated_rmsnorm_step: windows of %d taps, channels %d + %d of %d", K, c0, n_channels, Cd);
+  const WindowStep ws{conv_state, proj, slots, start_pos, ld, xbc_off, Cd, c0, n_channels, K, 0};
+  return gated_rmsnorm_launch(y, nullptr, z, TLC_F32, ldz, w, eps, T, Di, n_groups, mode, out, out_dtype, out_ld, out_scale, ws, stream);
 }
 
 // ---- gated product: out = act(gate) * up, gate|up side by side in one row -----------------

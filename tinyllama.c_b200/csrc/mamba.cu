@@ -9,6 +9,7 @@
 // position 0 starts from a zero window and a zero state, any other continues from its
 // slot.  Convolution, dt, the decay and the state are 32-bit.
 #include "common.cuh"
+#include "mbarrier.cuh"
 
 #define CONV_MAX_TAPS 16
 
@@ -650,4 +651,192 @@ extern "C" int tlc_ssm_scan_chunked(const float* xbc, const float* dt, const flo
                                          stream)) return rc;
   return scan_dispatch(xbc, dt, dA, Dskip, state, chunk_state, seg_start, seg_seq, seq_seg_start, slots, start_pos, y,
                        chunk_decay, SCAN_CHUNK_OUT, n_seg, Hs, P, N, G, Cd, stream);
+}
+
+// ---- one-token steps: convolution and scan in one kernel ---------------------------------------------------------------
+// Every sequence brings one row.  A block owns ROWS rows p of a head's state, which lie side by side in memory: one bulk
+// copy brings them into shared memory, the threads update them there, one bulk copy takes them back.  The state, the
+// stored windows of the channels that the block needs and the convolution's weights do not depend on the kernel before
+// this one and are asked for ahead of the wait on it; after it come the row's projection, the convolution of the
+// block's channels (B and C of the head's group, a thread four channels; x of its rows, the fifth warp), dt and the decay.
+// B and C are convolved by every block of the group: 512 channels of L2 reads beside up to 64 KB of state, instead of a
+// kernel of their own (2 to 5 us a layer) and a trip through memory.
+//
+// The windows of the x channels are the block's own to advance.  Those of B and C are read by all the blocks of (sequence,
+// group), so the mixer's next kernel advances them (tlc_gated_rmsnorm_step).
+// What bounds it: the state, read and written once.  A step of the 1.5B sizes at batch 64 (403 MB of states a layer) takes 2.97 ms, with the two
+// kernels 3.45; at batch 8 1.18 and 1.27; of the 3B sizes at batch 16 3.29 and 3.41; of the 7B sizes at batch 32 7.01 and 7.27.
+template <int NPL, int ROWS>
+struct StepSmem {
+  static constexpr int STATE = ROWS * 32 * NPL * 4;                       // at most
+  static constexpr int OPS = (2 * 32 * NPL + ROWS + 4) * 4;               // B[N] | C[N] | x[ROWS] | dt | dA
+  static constexpr int TOTAL = STATE + OPS + 16;                          // + the mbarrier
+};
+template <int NPL, int ROWS, int KT>
+__global__ void __launch_bounds__(160)
+mamba_step_kernel(const float* __restrict__ proj, int ld, int xbc_off, int dt_off, const float* __restrict__ w,
+                  const float* __restrict__ bias, const float* __restrict__ dt_bias, const float* __restrict__ A,
+                  const float* __restrict__ Dskip, float* conv_state, float* state, const int* __restrict__ slots,
+                  const int* __restrict__ start_pos, float* __restrict__ y, int Hs, int P, int N, int G, int Cd, int bf16_run,
+                  ErrWords* err) {
+  asm volatile("griddepcontrol.launch_dependents;");
+  constexpr int RP = ROWS / 4;                       // rows of a warp
+  extern __shared__ __align__(128) unsigned char step_sm[];
+  float* ss = reinterpret_cast<float*>(step_sm);                                        // [rows][N]
+  float* sm = reinterpret_cast<float*>(step_sm + StepSmem<NPL, ROWS>::STATE);
+  const uint32_t bar = smem_u32(step_sm + StepSmem<NPL, ROWS>::STATE + StepSmem<NPL, ROWS>::OPS);
+  const int b = blockIdx.x, h = blockIdx.y, p_blk = blockIdx.z * ROWS;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int Di = Hs * P, g = h / (Hs / G), nq = N >> 2;
+  const int rows = min(ROWS, P - p_blk);
+  const bool has_state = start_pos[b] > 0;
+  const int slot = slots[b];
+  float* win = conv_state + (size_t)slot * (KT - 1) * Cd;
+  float* S = state + (((size_t)slot * Hs + h) * P + p_blk) * N;
+  const uint32_t bytes = (uint32_t)(rows * N * 4);
+  if (threadIdx.x == 0 && has_state) {
+    mbar_init(bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    mbar_expect_tx(bar, bytes);
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(ss)), "l"(S),
+                 "r"(bytes), "r"(bar) : "memory");
+  }
+  // the four channels this thread convolves (-1: none), and where their values go
+  int c = -1, dst = 0;
+  if (warp < 4) {
+    const int q = threadIdx.x;
+    if (q < nq) c = Di + g * N + 4 * q;
+    else if (q < 2 * nq) c = Di + G * N + g * N + 4 * (q - nq);
+    dst = 4 * q;
+  } else if (lane < RP && 4 * lane < rows) {
+    c = h * P + p_blk + 4 * lane;
+    dst = 2 * N + 4 * lane;
+  }
+  float4 prev[KT - 1], wk[KT], bv = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int k = 0; k < KT - 1; k++)
+    prev[k] = c >= 0 && has_state ? *reinterpret_cast<const float4*>(win + (size_t)k * Cd + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int k = 0; k < KT; k++) wk[k] = c >= 0 ? __ldg(reinterpret_cast<const float4*>(w + (size_t)c * KT) + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+  if (bias && c >= 0) bv = __ldg(reinterpret_cast<const float4*>(bias + c));
+  const float db = dt_bias[h], Ah = A[h], Dh = Dskip[h];
+  const long long wait_limit = mbar_wait_limit(err);
+  tlc_wait(proj, y);
+  const float* row = proj + (size_t)b * ld;
+  if (c >= 0) {
+    const float4 cur = *reinterpret_cast<const float4*>(row + xbc_off + c);
+    // the taps of channel c + i are the KT weights from (c + i) * KT on
+    float wf[4 * KT];
+#pragma unroll
+    for (int k = 0; k < KT; k++) { wf[4 * k] = wk[k].x; wf[4 * k + 1] = wk[k].y; wf[4 * k + 2] = wk[k].z; wf[4 * k + 3] = wk[k].w; }
+    auto conv1 = [&](int i, float b0, auto get) {
+      float sum = b0;
+#pragma unroll
+      for (int k = 0; k < KT - 1; k++) sum = fmaf(get(prev[k]), wf[i * KT + k], sum);
+      sum = silu_f(fmaf(get(cur), wf[i * KT + KT - 1], sum));
+      return bf16_run ? as_operand<true>(sum) : sum;
+    };
+    float4 v;
+    v.x = conv1(0, bv.x, [](const float4& u) { return u.x; });
+    v.y = conv1(1, bv.y, [](const float4& u) { return u.y; });
+    v.z = conv1(2, bv.z, [](const float4& u) { return u.z; });
+    v.w = conv1(3, bv.w, [](const float4& u) { return u.w; });
+    *reinterpret_cast<float4*>(sm + dst) = v;
+    if (warp == 4) {                                 // x of this block's rows: nobody else reads that window
+#pragma unroll
+      for (int k = 0; k < KT - 1; k++) *reinterpret_cast<float4*>(win + (size_t)k * Cd + c) = k < KT - 2 ? prev[k < KT - 2 ? k + 1 : 0] : cur;
+    }
+  }
+  if (warp == 4 && lane == 31) {
+    const float dtv = softplus_f(row[dt_off + h] + db);
+    sm[2 * N + ROWS] = dtv;
+    sm[2 * N + ROWS + 1] = expf(dtv * Ah);
+  }
+  __syncthreads();                                   // (also behind the mbarrier's initialisation)
+  if (warp < 4) {
+    if (has_state && !mbar_wait(bar, 0, err, 41, wait_limit)) mbar_wait(bar, 0, err, 41, wait_limit);   // (reported; the copy still lands before the block ends)
+    const float dtv = sm[2 * N + ROWS], dAv = sm[2 * N + ROWS + 1];
+    float4 Bv[NPL / 4], Cv[NPL / 4];
+#pragma unroll
+    for (int j = 0; j < NPL / 4; j++) {
+      const int n = 4 * lane + 128 * j;
+      Bv[j] = n < N ? *reinterpret_cast<const float4*>(sm + n) : make_float4(0.f, 0.f, 0.f, 0.f);
+      Cv[j] = n < N ? *reinterpret_cast<const float4*>(sm + N + n) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float sum[RP];
+#pragma unroll
+    for (int r = 0; r < RP; r++) {
+      const int p = warp * RP + r;
+      const float xdt = p < rows ? sm[2 * N + p] * dtv : 0.f;
+      float a = 0.f;
+#pragma unroll
+      for (int j = 0; j < NPL / 4; j++) {
+        const int n = 4 * lane + 128 * j;
+        if (n < N && p < rows) {
+          float4* at = reinterpret_cast<float4*>(ss + p * N + n);
+          float4 u = has_state ? *at : make_float4(0.f, 0.f, 0.f, 0.f);
+          u.x = fmaf(u.x, dAv, Bv[j].x * xdt); u.y = fmaf(u.y, dAv, Bv[j].y * xdt);
+          u.z = fmaf(u.z, dAv, Bv[j].z * xdt); u.w = fmaf(u.w, dAv, Bv[j].w * xdt);
+          a = fmaf(u.x, Cv[j].x, a); a = fmaf(u.y, Cv[j].y, a); a = fmaf(u.z, Cv[j].z, a); a = fmaf(u.w, Cv[j].w, a);
+          *at = u;
+        }
+      }
+      sum[r] = a;
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the threads' stores, before the copy reads them
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    if (threadIdx.x == 0) {
+      asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(S), "r"(smem_u32(ss)), "r"(bytes) : "memory");
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    }
+#pragma unroll
+    for (int r = 0; r < RP; r++) sum[r] = warp_sum(sum[r]);
+    if (lane < RP) {
+      float v = sum[0];
+#pragma unroll
+      for (int r = 1; r < RP; r++) if (lane == r) v = sum[r];
+      const int p = warp * RP + lane;
+      if (p < rows) y[(size_t)b * Di + (size_t)h * P + p_blk + p] = v + sm[2 * N + p] * Dh;
+    }
+    // complete, not only read: the next step's copy of this state starts when this kernel has ended
+    if (threadIdx.x == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+  }
+}
+
+constexpr int STEP_BLOCKS = 4096;
+
+// Whether mamba_step_kernel takes these sizes: 65..256 state columns and the other sizes in pieces of 16 bytes (smaller
+// states leave lanes idle: they keep the two kernels), 2 to 4 taps.
+extern "C" int tlc_mamba_step_ok(int Hs, int P, int N, int G, int Cd, int K) {
+  return N > 64 && N <= 256 && N % 4 == 0 && P % 4 == 0 && Cd % 4 == 0 && K >= 2 && K <= 4 && G > 0 && Hs % G == 0 && Hs <= 65535 && Hs * P + 2 * G * N == Cd;
+}
+
+extern "C" int tlc_mamba_step(const float* proj, int ld, int xbc_off, int dt_off, const float* w, const float* bias,
+                              const float* dt_bias, const float* A, const float* Dskip, float* conv_state, float* state,
+                              const int* slots, const int* start_pos, float* y, int B, int Hs, int P, int N, int G, int Cd, int K,
+                              int bf16_run, cudaStream_t stream) {
+  if (B == 0) return 0;
+  TLC_REQUIRE(tlc_mamba_step_ok(Hs, P, N, G, Cd, K), "mamba_step: %d heads of %d, state %d, %d groups, %d taps are outside the kernel's range", Hs, P, N, G, K);
+  const void* aligned[] = {proj, w, bias, conv_state, state};
+  for (const void* p : aligned) TLC_REQUIRE(((uintptr_t)p & 15) == 0, "mamba_step: operands must start on 16-byte boundaries");
+  TLC_REQUIRE(ld % 4 == 0 && xbc_off % 4 == 0, "mamba_step: rows of the projection must start on 16-byte boundaries");
+  TLC_REQUIRE(tlc_error_words() != nullptr, "mamba_step: the library is not set up (tlc_linear_init)");
+  // 16 rows a block (18.6 KB of shared memory), and 32 where that still makes STEP_BLOCKS blocks: then the convolution that every
+  // block makes for itself counts, and the kernels beside this one no longer do.  A step of the 1.5B sizes at batch 64 (6,144 blocks
+  // of 32 rows): 2.96 ms, with 16 rows 3.12; of the 7B sizes at batch 32 (3,072): 7.17 and 7.03; of 1.5B at batch 8 (768): 1.51 and
+  // 1.18; of 3B at batch 16 (2,048): 4.71 and 3.29, blocks of 35 KB leave the attention kernel, which runs beside this one and
+  // needs 131 KB of an SM's shared memory, no room until the last of them has started, and the products too little of
+  // the first-level cache that their weight loads are in flight through.
+#define TLC_STEP(NPL_, ROWS_, KT_)                                                                                                       \
+  tlc_launch(mamba_step_kernel<NPL_, ROWS_, KT_>, dim3(B, Hs, (P + ROWS_ - 1) / ROWS_), dim3(160), StepSmem<NPL_, ROWS_>::TOTAL, stream,  \
+             proj, ld, xbc_off, dt_off, w, bias, dt_bias, A, Dskip, conv_state, state, slots, start_pos, y, Hs, P, N, G, Cd, bf16_run,     \
+             tlc_error_words())
+#define TLC_STEP_K(NPL_, ROWS_) do { if (K == 4) TLC_STEP(NPL_, ROWS_, 4); else if (K == 3) TLC_STEP(NPL_, ROWS_, 3); else TLC_STEP(NPL_, ROWS_, 2); } while (0)
+  const bool wide = (long long)B * Hs * ((P + 31) / 32) >= STEP_BLOCKS;
+  if (N <= 128) { if (wide) TLC_STEP_K(4, 32); else TLC_STEP_K(4, 16); }
+  else { if (wide) TLC_STEP_K(8, 32); else TLC_STEP_K(8, 16); }
+#undef TLC_STEP_K
+#undef TLC_STEP
+  TLC_CHECK_LAUNCH("mamba_step");
+  return 0;
 }

@@ -97,6 +97,12 @@ int tlc_difference_join(const void* att, int dtype, int ld_in, int hd, void* out
 int tlc_gated_rmsnorm(const float* y, const float* y2, const void* z, int z_dtype, int ldz, const float* w, float eps, int T,
                       int Di, int n_groups, int mode, void* out, int out_dtype, int out_ld,
                       float out_scale, cudaStream_t stream);
+/* The same with z in 32 bits, after tlc_mamba_step: also advances the windows of channels c0 .. c0 + n_channels - 1 of
+ * conv_state [n_slots, K-1, Cd] by the row's raw samples, columns xbc_off + c of its projection. */
+int tlc_gated_rmsnorm_step(const float* y, const float* z, int ldz, const float* w, float eps, int T, int Di, int n_groups,
+                           int mode, void* out, int out_dtype, int out_ld, float out_scale, const float* proj, int ld,
+                           int xbc_off, float* conv_state, const int* slots, const int* start_pos, int Cd, int c0,
+                           int n_channels, int K, cudaStream_t stream);
 /* out[T, F] = silu(gate) * up; gu holds gate | up as halves, or (interleave) 8 gates then their 8 ups. */
 int tlc_swiglu(const void* gu, int in_dtype, int ld, int F, int T, void* out, int dtype, int interleave,
                cudaStream_t stream);
@@ -246,6 +252,14 @@ int tlc_mamba_conv(const void* proj, int dtype, int ld, int xbc_off, int dt_off,
                    const int* cu_seqlens, const int* row_seq, const int* slots, const int* start_pos,
                    void* xbc_out, int xbc_dtype, float* dt_out, float* dA_out, int T, int B, int Cd, int K,
                    int Hs, int single_rows, int quick, int all_fresh, cudaStream_t stream);
+/* Steps in which every sequence brings one row (row b is sequence b's): tlc_mamba_conv and tlc_ssm_scan in one kernel, for
+ * 32-bit projections and the sizes of tlc_mamba_step_ok.  The windows of the B and C channels stay as they were: the
+ * kernel that follows, tlc_gated_rmsnorm_step, advances them. */
+int tlc_mamba_step_ok(int Hs, int P, int N, int G, int Cd, int K);
+int tlc_mamba_step(const float* proj, int ld, int xbc_off, int dt_off, const float* w, const float* bias,
+                   const float* dt_bias, const float* A, const float* Dskip, float* conv_state, float* state,
+                   const int* slots, const int* start_pos, float* y, int B, int Hs, int P, int N, int G, int Cd, int K,
+                   int bf16_run, cudaStream_t stream);
 /* S = S * dA + B (x dt), y = S.C + x D, row by row from each slot's state [n_slots, Hs, P, N] (zero at
  * position 0), which is updated in place. */
 int tlc_ssm_scan(const float* xbc, const float* dt, const float* dA, const float* Dskip, float* state,

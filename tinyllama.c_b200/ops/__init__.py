@@ -86,6 +86,11 @@ _SIGNATURES = {
     "tlc_attention_prefill_tc_splits": (_i, [_i, _i, _i]),
     "tlc_mamba_conv": (_i, [_vp, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _vp, _vp, _i, _i,
                             _i, _i, _i, _i, _i, _i, _vp]),
+    "tlc_mamba_step_ok": (_i, [_i, _i, _i, _i, _i, _i]),
+    "tlc_mamba_step": (_i, [_vp, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i,
+                            _i, _vp]),
+    "tlc_gated_rmsnorm_step": (_i, [_vp, _vp, _i, _vp, _f, _i, _i, _i, _i, _vp, _i, _i, _f, _vp, _i, _i, _vp, _vp, _vp, _i, _i, _i,
+                                    _i, _vp]),
     "tlc_ssm_scan": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp]),
     "tlc_ssm_scan_chunked": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i,
                                   _vp]),
@@ -307,10 +312,12 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float, out: torch.Tensor
 
 def gated_rmsnorm(y: torch.Tensor, z: torch.Tensor, weight: Optional[torch.Tensor], eps: float, n_groups: int,
                   norm_before_gate: bool, out: torch.Tensor, out_scale: float = 1.0,
-                  y_add: Optional[torch.Tensor] = None, gate: str = "silu") -> None:
+                  y_add: Optional[torch.Tensor] = None, gate: str = "silu", window=None) -> None:
     """Gate y by silu(z) (or, gate "sigmoid", by sigmoid(z)) and RMS-normalise per group (either order); weight None = gate only.  The
     result is multiplied by out_scale; out [T, Di] may be a range of the columns of a wider buffer.
-    y_add: a second summand of the input (the scan of prompts leaves its outputs as two), same shape as y."""
+    y_add: a second summand of the input (the scan of prompts leaves its outputs as two), same shape as y.
+    window (after mamba_step): (proj, xbc_off, conv_state, slots, start_pos, first channel, number of channels); the stored
+    windows of these channels advance by the rows' raw samples in the same kernel."""
     _gpu(y, z, weight, out, y_add)
     T, Di = y.shape
     if y.dtype != torch.float32 or not y.is_contiguous():
@@ -321,6 +328,21 @@ def gated_rmsnorm(y: torch.Tensor, z: torch.Tensor, weight: Optional[torch.Tenso
     if z.shape != y.shape:
         raise KernelError("gated_rmsnorm: gate and input differ in shape")
     _f32vec(weight, Di, "gated_rmsnorm weight")
+    if window is not None:
+        proj, off, conv_state, slots, start_pos, c0, n = window
+        _gpu(proj, conv_state, slots, start_pos)
+        Cd, K = conv_state.shape[2], conv_state.shape[1] + 1
+        if y_add is not None or z.dtype != torch.float32 or proj.dtype != torch.float32 or conv_state.dtype != torch.float32 \
+                or not conv_state.is_contiguous() or proj.shape[0] != T or slots.numel() != T or start_pos.numel() != T \
+                or off < 0 or c0 < 0 or c0 + n > Cd or off + Cd > proj.shape[1]:
+            raise KernelError("gated_rmsnorm: windows advance by a float32 projection of one row a sequence")
+        _i32(slots, "slots")
+        _i32(start_pos, "start_pos")
+        _call("tlc_gated_rmsnorm_step", y.data_ptr(), z.data_ptr(), _rows(z, "gate"), _p(weight), float(eps), T, Di, int(n_groups),
+              int(bool(norm_before_gate)) | (2 if gate == "sigmoid" else 0), out.data_ptr(), dtype_code(out.dtype), out_ld,
+              float(out_scale), proj.data_ptr(), _rows(proj, "proj"), off, conv_state.data_ptr(), slots.data_ptr(),
+              start_pos.data_ptr(), Cd, c0, n, K, _stream())
+        return
     _call("tlc_gated_rmsnorm", y.data_ptr(), _p(y_add), z.data_ptr(), dtype_code(z.dtype), _rows(z, "gate"), _p(weight),
           float(eps), T, Di, int(n_groups), int(bool(norm_before_gate)) | (2 if gate == "sigmoid" else 0), out.data_ptr(),
           dtype_code(out.dtype), out_ld, float(out_scale), _stream())
@@ -880,6 +902,44 @@ def mamba_conv(proj: torch.Tensor, xbc_off: int, dt_off: int, w: torch.Tensor, b
           row_seq.data_ptr(), slots.data_ptr(), start_pos.data_ptr(), xbc_out.data_ptr(), dtype_code(xbc_out.dtype),
           dt_out.data_ptr(), dA_out.data_ptr(), T, B, Cd, K, Hs, int(bool(single_rows)), int(bool(bf16_run)),
           int(bool(all_fresh)), _stream())
+
+
+def mamba_step_ok(proj: torch.Tensor, xbc_off: int, Hs: int, P: int, N: int, G: int, K: int) -> bool:
+    """Whether mamba_step takes this projection and these sizes."""
+    return bool(proj.is_cuda and proj.dtype == torch.float32 and proj.stride(0) % 4 == 0 and xbc_off % 4 == 0
+                and proj.data_ptr() % 16 == 0 and library().tlc_mamba_step_ok(Hs, P, N, G, Hs * P + 2 * G * N, K))
+
+
+def mamba_step(proj: torch.Tensor, xbc_off: int, dt_off: int, w: torch.Tensor, bias: Optional[torch.Tensor],
+               dt_bias: torch.Tensor, A: torch.Tensor, Dskip: torch.Tensor, conv_state: torch.Tensor, state: torch.Tensor,
+               slots: torch.Tensor, start_pos: torch.Tensor, y: torch.Tensor, Hs: int, P: int, N: int, G: int,
+               bf16_run: bool = False) -> None:
+    """mamba_conv and ssm_scan of a step in which every sequence brings one row (row b of proj is sequence b's), in one
+    kernel: the states advance in place, y [T, Hs*P] is before gating.  Of the windows those of the x channels advance here;
+    the B and C channels' stay as they were until gated_rmsnorm gets them as `window`, which must follow.  See
+    mamba_step_ok for what it takes."""
+    _gpu(proj, w, bias, dt_bias, A, Dskip, conv_state, state, slots, start_pos, y)
+    T = proj.shape[0]
+    Cd, K = w.shape
+    if slots.numel() != T or start_pos.numel() != T:
+        raise KernelError("mamba_step: every sequence brings exactly one row")
+    if Cd != Hs * P + 2 * G * N:
+        raise KernelError("mamba_step: the convolution's width does not match Hs*P + 2*G*N")
+    if proj.dtype != torch.float32 or xbc_off < 0 or dt_off < 0 or max(xbc_off + Cd, dt_off + Hs) > proj.shape[1]:
+        raise KernelError("mamba_step: a float32 projection with x|B|C and dt inside its rows")
+    for t, n, name in ((w, Cd * K, "conv weight"), (bias, Cd, "conv bias"), (dt_bias, Hs, "dt_bias"), (A, Hs, "A"), (Dskip, Hs, "D")):
+        _f32vec(t, n, name)
+    for t, name in ((slots, "slots"), (start_pos, "start_pos")):
+        _i32(t, name)
+    if conv_state.dtype != torch.float32 or not conv_state.is_contiguous() or tuple(conv_state.shape[1:]) != (K - 1, Cd):
+        raise KernelError("mamba_step: conv_state must be contiguous float32 [n_slots, K-1, Cd]")
+    if state.dtype != torch.float32 or not state.is_contiguous() or tuple(state.shape[1:]) != (Hs, P, N):
+        raise KernelError("mamba_step: state must be contiguous float32 [n_slots, Hs, P, N]")
+    if y.dtype != torch.float32 or not y.is_contiguous() or tuple(y.shape) != (T, Hs * P):
+        raise KernelError(f"mamba_step: y must be contiguous float32 {(T, Hs * P)}")
+    _call("tlc_mamba_step", proj.data_ptr(), _rows(proj, "proj"), xbc_off, dt_off, w.data_ptr(), _p(bias), dt_bias.data_ptr(),
+          A.data_ptr(), Dskip.data_ptr(), conv_state.data_ptr(), state.data_ptr(), slots.data_ptr(), start_pos.data_ptr(),
+          y.data_ptr(), T, Hs, P, N, G, Cd, K, int(bool(bf16_run)), _stream())
 
 
 def ssd_walk_blocks(blocks: int) -> None:

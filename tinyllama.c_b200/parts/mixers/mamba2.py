@@ -24,7 +24,7 @@ from ..linear import StackedLinear
 
 @register_mixer("mamba2")
 class Mamba2Mixer(Part):
-    single_token_launches = 3      # convolution, scan, gated norm: what a one-token step launches in mix()
+    single_token_launches = 3      # convolution, scan (or both in one), gated norm: what a one-token step launches in mix(), at most
 
     def __init__(self, hidden: int, d_ssm: int, n_heads: int, d_head: int, n_groups: int, d_state: int, d_conv: int,
                  prefix: str, eps: float, conv_bias: bool = True, proj_bias: bool = False, rms_norm: bool = True,
@@ -150,6 +150,13 @@ class Mamba2Mixer(Part):
         conv_state = cache.state[self.cache_key + ".conv"]
         ssm_state = cache.state[self.cache_key + ".ssm"]
         new = lambda tag, shape, dtype: scratch_buf(f"mamba2.{self.cache_key}.{tag}", shape, dtype, proj.device)   # (two mixers of a layer have two keys)
+        y = new("y", (T, self.Di), f32)
+        if step.max_new == 1 and T == step.n_seqs and ops.mamba_step_ok(proj, self.Di, self.Hs, self.P, self.N, self.G, self.K):
+            # one token per sequence: convolution and scan in one kernel
+            ops.mamba_step(proj, self.Di, self.Di + self.Cd, self.conv_w, self.conv_b, self.dt_bias, self.A, self.D, conv_state,
+                           ssm_state, step.slots, step.start_pos, y, self.Hs, self.P, self.N, self.G, self.dtype == torch.bfloat16)
+            return self._gate(y, proj, None, out, out_scale, join, new,
+                              (proj, self.Di, conv_state, step.slots, step.start_pos, self.Di, self.Cd - self.Di))
         # prompts cut into chunks of a bfloat16 run: the scan in matrix form, whose operands x|B|C the convolution
         # writes in bfloat16 at once; everything else scans 32-bit values
         chunks = step.chunks.get(self.scan_chunk)
@@ -163,17 +170,23 @@ class Mamba2Mixer(Part):
                        step.cu_seqlens, step.row_seq, step.slots, step.start_pos, xbc, dt, dA,
                        step.max_new == 1, self.dtype == torch.bfloat16,
                        len(step.host_start) == step.n_seqs and not any(step.host_start))
-        y = new("y", (T, self.Di), f32)
         # in matrix form the outputs may come as two summands, the one that needs no state computed beside the walk
         # over the chunks; the gated norm adds them
         y_part = new("y_part", (T, self.Di), f32) if matrix_form else None
         in_two = ops.ssm_scan(xbc, dt, dA, self.D, ssm_state, step.cu_seqlens, step.slots, step.start_pos, y, self.Hs,
                               self.P, self.N, self.G, chunks, self.A if matrix_form else None, y_part)
-        gated = out if out is not None else new("gated", (T, self.Di), self.dtype)
+        return self._gate(y, proj, y_part if in_two else None, out, out_scale, join, new)
+
+    def _gate(self, y: torch.Tensor, proj: torch.Tensor, y_part: Optional[torch.Tensor], out: Optional[torch.Tensor], out_scale: float,
+              join: Optional[Callable[[], None]], new: Callable, window=None) -> torch.Tensor:
+        """The mixer's last kernel: the gate and the grouped norm of y (+ y_part); after mamba_step it also advances the
+        windows of `window`."""
+        gated = out if out is not None else new("gated", (y.shape[0], self.Di), self.dtype)
         if join is not None:
             join()
+        more = {} if window is None else {"window": window}
         ops.gated_rmsnorm(y, proj[:, :self.Di], self.norm_w, self.eps, self.norm_groups, self.norm_before_gate, gated,
-                          out_scale, y_part if in_two else None)
+                          out_scale, y_part, **more)
         return gated
 
     def output(self, gated: torch.Tensor, residual: torch.Tensor) -> None:
