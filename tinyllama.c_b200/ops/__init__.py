@@ -97,6 +97,7 @@ _SIGNATURES = {
     "tlc_ssd_ok": (_i, [_i, _i, _i, _i, _i]),
     "tlc_ssd_walk_override": (None, [_i]),
     "tlc_ssd_walk_blocks": (None, [_i]),
+    "tlc_ssd_first_chunks": (None, [_i]),
     "tlc_ssd_scratch_floats": (_ll, [_i, _i, _i, _i, _i, _i]),
     "tlc_ssm_scan_ssd": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i,
                               _i, _i, _vp, _vp]),
@@ -940,6 +941,12 @@ def mamba_step(proj: torch.Tensor, xbc_off: int, dt_off: int, w: torch.Tensor, b
     _call("tlc_mamba_step", proj.data_ptr(), _rows(proj, "proj"), xbc_off, dt_off, w.data_ptr(), _p(bias), dt_bias.data_ptr(),
           A.data_ptr(), Dskip.data_ptr(), conv_state.data_ptr(), state.data_ptr(), slots.data_ptr(), start_pos.data_ptr(),
           y.data_ptr(), T, Hs, P, N, G, Cd, K, int(bool(bf16_run)), _stream())
+
+
+def ssd_first_chunks(mode: int) -> None:
+    """First chunks of sequences that start in the step, matrix form on tcgen05: 0 = in a kernel of their own where that pays,
+    1 = never, 2 = always; for tests."""
+    library().tlc_ssd_first_chunks(int(mode))
 
 
 def ssd_walk_blocks(blocks: int) -> None:
