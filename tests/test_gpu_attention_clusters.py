@@ -6,7 +6,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("T", [1, 3])
-@pytest.mark.parametrize("n_splits", [2, 3, 5, 8, 9, 13])
+@pytest.mark.parametrize("n_splits", [2, 3, 5, 6, 7, 8, 9, 13])
 def test_attention_splits_that_meet_in_a_cluster_or_through_scratch(n_splits, T):
     """One round of chunks a block: up to 8 splits of a (row, key/value head) merge as a cluster while the grid has at most 32
     blocks, others through scratch; rows whose sequences end inside the first, a middle and the last split; with and

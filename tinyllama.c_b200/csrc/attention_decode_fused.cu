@@ -372,8 +372,10 @@ attention_decode_fused_kernel(const float* __restrict__ qkv, int ld, int q_off, 
   }
   if constexpr (CLUSTER) {
     // ---- the blocks of the cluster meet; each merges its share of the outputs ----
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    // (not the .aligned forms: the loops before both meetings may leave a warp lane by lane, a share of the outputs is no
+    // multiple of 32 with 3, 5, 6 or 7 splits)
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
     const int per = (G * HD + n_splits - 1) / n_splits, first = split * per, last = min(G * HD, first + per);
     const float2* ml_of[8];
     const float* o_of[8];
@@ -415,8 +417,8 @@ attention_decode_fused_kernel(const float* __restrict__ qkv, int ld, int q_off, 
       }
       out[(size_t)t * out_ld + ((size_t)g * G + hg) * HD + d] = __float2bfloat16_rn(acc);
     }
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // every block's shared memory stays until all have read it
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");   // every block's shared memory stays until all have read it
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
     return;
   }
   if (n_splits == 1) return;                      // one block per (row, kv head): it wrote the output itself
