@@ -167,6 +167,7 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     const int row = quarter * 32 + lane;                    // weight row of the tile
     asm volatile("griddepcontrol.wait;" ::: "memory");      // `out` may still be read or written by the previous kernel
     auto read_columns = [&](int c, uint32_t (&r)[CW]) {
+      __syncwarp();                                         // (the reads want a whole warp; waits, loads and stores by lane lie before them)
       const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(c * CW);
       if constexpr (CW == 32) tmem_ld32(at, r);
       else tmem_ld16(at, r);
