@@ -784,6 +784,7 @@ mamba_step_kernel(const float* __restrict__ proj, int ld, int xbc_off, int dt_of
       sum[r] = a;
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the threads' stores, before the copy reads them
+    __syncwarp();                                                    // (bar.sync wants whole warps)
     asm volatile("bar.sync 1, 128;" ::: "memory");
     if (threadIdx.x == 0) {
       asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(S), "r"(smem_u32(ss)), "r"(bytes) : "memory");
