@@ -44,3 +44,39 @@ def test_step_kernel_against_convolution_and_scan(Hs, P, N, G, K, bias, bf16_run
         got.append((y, state, conv, out))
     for a, b, name in zip(got[0], got[1], ("y", "states", "windows", "gated output")):
         assert torch.equal(a, b), name
+
+
+def test_step_whose_waits_run_out_leaves_whole_states():
+    """With a limit of one clock cycle a block whose state has not landed at once gives up: every block of rows keeps the
+    state that it had or gets the new one, never a part of it, and check_errors raises if one was kept."""
+    from tinyllama_c_b200 import ops
+    Hs, P, N, G, K, B = 64, 64, 256, 1, 4, 5
+    Di, Cd = Hs * P, Hs * P + 2 * G * N
+    g = torch.Generator().manual_seed(41)
+    rnd = lambda *s: torch.randn(*s, generator=g).cuda()  # noqa: E731
+    proj, w, dt_bias, A, D = rnd(B, Di + Cd + Hs), rnd(Cd, K), rnd(Hs), -rnd(Hs).abs() - 0.1, rnd(Hs)
+    conv0, state0 = rnd(B, K - 1, Cd), rnd(B, Hs, P, N)
+    slots = torch.arange(B, dtype=torch.int32).cuda()
+    start = torch.full((B,), 9, dtype=torch.int32).cuda()
+
+    def step(state):
+        conv, y = conv0.clone(), torch.empty(B, Di, device="cuda")
+        ops.mamba_step(proj, Di, Di + Cd, w, None, dt_bias, A, D, conv, state, slots, start, y, Hs, P, N, G)
+        torch.cuda.synchronize()
+        return state.view(-1, 16, N)
+
+    old, new = state0.view(-1, 16, N), step(state0.clone())
+    ops.check_errors()
+    try:
+        ops.wait_limit_cycles(1)
+        for _ in range(5):
+            got = step(state0.clone())
+            kept = (got == old).flatten(1).all(1)
+            assert ((got == new).flatten(1).all(1) | kept).all(), "a state in parts"
+            if kept.any():
+                with pytest.raises(ops.KernelError, match="41"):
+                    ops.check_errors()
+            else:
+                ops.check_errors()
+    finally:
+        ops.wait_limit_cycles(0)

@@ -669,7 +669,7 @@ extern "C" int tlc_ssm_scan_chunked(const float* xbc, const float* dt, const flo
 template <int NPL, int ROWS>
 struct StepSmem {
   static constexpr int STATE = ROWS * 32 * NPL * 4;                       // at most
-  static constexpr int OPS = (2 * 32 * NPL + ROWS + 4) * 4;               // B[N] | C[N] | x[ROWS] | dt | dA
+  static constexpr int OPS = (2 * 32 * NPL + ROWS + 4) * 4;               // B[N] | C[N] | x[ROWS] | dt | dA | whether a wait ran out
   static constexpr int TOTAL = STATE + OPS + 16;                          // + the mbarrier
 };
 template <int NPL, int ROWS, int KT>
@@ -685,6 +685,7 @@ mamba_step_kernel(const float* __restrict__ proj, int ld, int xbc_off, int dt_of
   float* ss = reinterpret_cast<float*>(step_sm);                                        // [rows][N]
   float* sm = reinterpret_cast<float*>(step_sm + StepSmem<NPL, ROWS>::STATE);
   const uint32_t bar = smem_u32(step_sm + StepSmem<NPL, ROWS>::STATE + StepSmem<NPL, ROWS>::OPS);
+  int* ran_out = reinterpret_cast<int*>(sm + 2 * N + ROWS + 2);
   const int b = blockIdx.x, h = blockIdx.y, p_blk = blockIdx.z * ROWS;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int Di = Hs * P, g = h / (Hs / G), nq = N >> 2;
@@ -751,10 +752,15 @@ mamba_step_kernel(const float* __restrict__ proj, int ld, int xbc_off, int dt_of
     const float dtv = softplus_f(row[dt_off + h] + db);
     sm[2 * N + ROWS] = dtv;
     sm[2 * N + ROWS + 1] = expf(dtv * Ah);
+    *ran_out = 0;
   }
   __syncthreads();                                   // (also behind the mbarrier's initialisation)
   if (warp < 4) {
-    if (has_state && !mbar_wait(bar, 0, err, 41, wait_limit)) mbar_wait(bar, 0, err, 41, wait_limit);   // (reported; the copy still lands before the block ends)
+    // A wait that ran out is reported (the host raises): its warp leaves its rows alone and the block stores none, so that the
+    // slot keeps the state it had.
+    bool landed = !has_state || mbar_wait(bar, 0, err, 41, wait_limit);
+    if (!landed) *ran_out = 1;
+    landed = __all_sync(0xffffffffu, landed);
     const float dtv = sm[2 * N + ROWS], dAv = sm[2 * N + ROWS + 1];
     float4 Bv[NPL / 4], Cv[NPL / 4];
 #pragma unroll
@@ -772,7 +778,7 @@ mamba_step_kernel(const float* __restrict__ proj, int ld, int xbc_off, int dt_of
 #pragma unroll
       for (int j = 0; j < NPL / 4; j++) {
         const int n = 4 * lane + 128 * j;
-        if (n < N && p < rows) {
+        if (n < N && p < rows && landed) {
           float4* at = reinterpret_cast<float4*>(ss + p * N + n);
           float4 u = has_state ? *at : make_float4(0.f, 0.f, 0.f, 0.f);
           u.x = fmaf(u.x, dAv, Bv[j].x * xdt); u.y = fmaf(u.y, dAv, Bv[j].y * xdt);
@@ -786,7 +792,8 @@ mamba_step_kernel(const float* __restrict__ proj, int ld, int xbc_off, int dt_of
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the threads' stores, before the copy reads them
     __syncwarp();                                                    // (bar.sync wants whole warps)
     asm volatile("bar.sync 1, 128;" ::: "memory");
-    if (threadIdx.x == 0) {
+    const bool store = *(volatile int*)ran_out == 0;
+    if (threadIdx.x == 0 && store) {
       asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(S), "r"(smem_u32(ss)), "r"(bytes) : "memory");
       asm volatile("cp.async.bulk.commit_group;" ::: "memory");
     }
@@ -801,6 +808,8 @@ mamba_step_kernel(const float* __restrict__ proj, int ld, int xbc_off, int dt_of
     }
     // complete, not only read: the next step's copy of this state starts when this kernel has ended
     if (threadIdx.x == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    // the copy that was waited for in vain is still on its way into this block's memory: it gets the default limit once more
+    if (threadIdx.x == 0 && !store) mbar_wait(bar, 0, err, 41, wait_limit > TLC_WAIT_LIMIT_CYCLES ? wait_limit : TLC_WAIT_LIMIT_CYCLES);
   }
 }
 
