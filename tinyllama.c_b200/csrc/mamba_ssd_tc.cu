@@ -361,7 +361,7 @@ struct FirstSmem {
   static constexpr int N = 128 * NTILES;
   static constexpr int BT_SLAB = N * 128, BT = 0, BT_BYTES = 2 * BT_SLAB;               // [N rows n][128 j], slabs of 64 j
   static constexpr int X_SLAB = PF * 128, XW = BT + BT_BYTES, XW_BYTES = 2 * X_SLAB;    // (w x)^T [PF rows p][128 j]
-  static constexpr int BARS = XW + XW_BYTES;                                            // 2 mbarriers, tmem slot
+  static constexpr int BARS = XW + XW_BYTES;                                            // 2 mbarriers, tmem slot, whether B^T did not come
   static constexpr int TOTAL = BARS + 32 + 1024;                                        // + alignment slack
 };
 
@@ -381,12 +381,14 @@ ssd_first_chunk_kernel(const __grid_constant__ CUtensorMap map_bt, const __nv_bf
   if (start_pos[b] > 0 || seq_seg_start[b + 1] <= c0) return;           // the same for the whole block
   uint64_t* bars = reinterpret_cast<uint64_t*>(sm + L_::BARS);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2);
+  volatile int* absent = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const uint32_t sm0 = smem_u32(sm), bar_bt = smem_u32(bars), bar_s = smem_u32(bars + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int Di = Hs * P, g = h / (Hs / G);
   const int t0 = seg_start[c0], L = seg_start[c0 + 1] - t0;
-  const long long wait_limit = mbar_wait_limit(err);
+  const long long wait_limit = mbar_wait_limit(err), last_limit = wait_limit > TLC_WAIT_LIMIT_CYCLES ? wait_limit : TLC_WAIT_LIMIT_CYCLES;
   if (tid == 0) {
+    *absent = 0;
     mbar_init(bar_bt, 1);
     mbar_init(bar_s, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -431,8 +433,7 @@ ssd_first_chunk_kernel(const __grid_constant__ CUtensorMap map_bt, const __nv_bf
   const uint32_t tmem = *tmem_slot;
   if (tid == 0) {
     constexpr uint32_t idesc = instr_desc(128, PF);
-    // B^T has landed, or (reported) the limit has run out; the copy still lands before the block ends
-    if (mbar_wait(bar_bt, 0, err, 15, wait_limit) || mbar_wait(bar_bt, 0, err, 15, wait_limit)) {
+    if (mbar_wait(bar_bt, 0, err, 15, wait_limit)) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
       for (int t = 0; t < NTILES; t++)
@@ -444,15 +445,21 @@ ssd_first_chunk_kernel(const __grid_constant__ CUtensorMap map_bt, const __nv_bf
                  smem_desc(sm0 + L_::XW + s * L_::X_SLAB + kk * 32), idesc, (s > 0 || kk > 0) ? 1u : 0u);
       umma_commit(bar_s);
     } else {
+      *absent = 1;                                      // no products, and nothing is stored
       mbar_arrive(bar_s);
+      // (the copy is still on its way into this block's memory: it gets the default limit before the block may end)
+      mbar_wait(bar_bt, 0, err, 15, last_limit);
     }
   }
   __syncwarp();
-  mbar_wait(bar_s, 0, err, 16, wait_limit);
+  // A wait that ran out is reported (the host raises) and its warp stores nothing; the products get the default limit once
+  // more before tensor memory is given back under them.
+  bool done = mbar_wait(bar_s, 0, err, 16, wait_limit);
+  if (!done) mbar_wait(bar_s, 0, err, 16, last_limit);
+  done = __all_sync(0xffffffffu, done && *absent == 0);
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  __syncwarp();
   const int tile = NTILES == 1 ? 0 : (warp >> 2), quarter = warp & 3;
-  if (NTILES == 2 || warp < 4) {
+  if (done && (NTILES == 2 || warp < 4)) {
     float* slot = state + (((size_t)slots[b] * Hs + h) * P + p0) * N + 128 * tile + 32 * quarter + lane;
 #pragma unroll
     for (int c = 0; c < PF / 32; c++) {
