@@ -1,15 +1,16 @@
-"""The row-by-row scan fetches eight rows at a time."""
+"""The row-by-row scan fetches four rows at a time, into two buffers in turn."""
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
 
+@pytest.mark.parametrize("aligned", [True, False])
 @pytest.mark.parametrize("N,P", [(3, 5), (32, 16), (68, 20), (130, 12), (256, 64)])
 @pytest.mark.parametrize("lens", [(1,), (7, 8, 9), (23, 1, 16)])
-def test_scan_rows_staged_in_batches(lens, N, P):
-    """Sequences that end before, at and after a batch, rows that are laid out in 16-byte pieces and rows that are not;
-    against the recurrence in 64 bits."""
+def test_scan_rows_staged_in_batches(lens, N, P, aligned):
+    """Sequences that end before, at and after a batch, rows that are laid out in 16-byte pieces and rows that are not,
+    states that start on a 16-byte boundary or 4 bytes past one; against the recurrence in 64 bits."""
     from tinyllama_c_b200 import ops
     g = torch.Generator().manual_seed(sum(lens) * 31 + N)
     Hs, G = 4, 2
@@ -29,7 +30,9 @@ def test_scan_rows_staged_in_batches(lens, N, P):
             S = S * dA[t].double()[:, None, None] + (x * dt[t].double()[:, None])[..., None] * Bm[:, None]
             y_ref[t] = ((S * Cm[:, None]).sum(-1) + x * D.double()[:, None]).reshape(-1)
         S_ref[b] = S
-    y, st = torch.empty(T, Di, device="cuda"), state.cuda()
+    y, off = torch.empty(T, Di, device="cuda"), 0 if aligned else 1
+    st = torch.empty(state.numel() + off, device="cuda")[off:].view(state.shape)
+    st.copy_(state)
     ops.ssm_scan(xbc.cuda(), dt.cuda(), dA.cuda(), D.cuda(), st, cu.cuda(), torch.arange(B, dtype=torch.int32).cuda(), start.cuda(), y, Hs, P, N, G)
     torch.cuda.synchronize()
     # products and sums of N terms in 32 bits over at most 23 rows

@@ -337,7 +337,7 @@ __device__ __forceinline__ void scan_copy16(float* dst, const float* src, bool o
 __device__ __forceinline__ void scan_copy4(float* dst, const float* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
-template <int NPL, int RP>
+template <int NPL, int RP, bool VEC>
 __global__ void __launch_bounds__(128, 7)
 ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dt, const float* __restrict__ dA,
                 const float* __restrict__ Dskip, float* __restrict__ state, float* __restrict__ chunk_state,
@@ -370,9 +370,8 @@ ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dt, con
   else if (mode == SCAN_CHUNK_STATE) S_final = S_chunk;
   else if (seg + 1 == seq_seg_start[b + 1]) S_final = S_slot;        // the sequence's last chunk
   const bool want_y = mode != SCAN_CHUNK_STATE;
-  // A lane owns the columns lane, lane + 32, ... of its rows, or (VEC: more than 64 columns, a multiple of 4)
-  // four consecutive columns 4 lane + 128 jj, which it loads and stores 16 bytes at a time.
-  const bool VEC = NPL % 4 == 0 && N % 4 == 0;
+  // A lane owns the columns lane, lane + 32, ... of its rows, or (VEC: more than 64 columns, a multiple of 4, in states that
+  // start on 16-byte boundaries) four consecutive columns 4 lane + 128 jj, which it loads and stores 16 bytes at a time.
   auto col = [&](int j) { return VEC ? 4 * lane + 128 * (j >> 2) + (j & 3) : lane + 32 * j; };
   float s[RP][NPL];
 #pragma unroll
@@ -600,9 +599,16 @@ static int launch_scan(const float* xbc, const float* dt, const float* dA, const
   constexpr int RP = 4;
   dim3 grid(n_seg, Hs, (P + 4 * RP - 1) / (4 * RP));
   const size_t smem = (size_t)2 * SCAN_TT * (2 * N + 4 * RP + 4) * sizeof(float);
-  tlc_launch(ssm_scan_kernel<NPL, RP>, dim3(grid), dim3(128), smem, stream, xbc, dt, dA, Dskip, state, chunk_state, seg_start, seg_seq,
-                                                        seq_seg_start, slots, start_pos, y, chunk_decay, mode, Hs, P, N, G,
-                                                        Cd);
+  auto run = [&](auto kernel) {
+    tlc_launch(kernel, dim3(grid), dim3(128), smem, stream, xbc, dt, dA, Dskip, state, chunk_state, seg_start, seg_seq, seq_seg_start,
+               slots, start_pos, y, chunk_decay, mode, Hs, P, N, G, Cd);
+  };
+  if constexpr (NPL % 4 == 0) {
+    if (N % 4 == 0 && (((uintptr_t)state | (uintptr_t)chunk_state) & 15) == 0) run(ssm_scan_kernel<NPL, RP, true>);
+    else run(ssm_scan_kernel<NPL, RP, false>);
+  } else {
+    run(ssm_scan_kernel<NPL, RP, false>);
+  }
   TLC_CHECK_LAUNCH("ssm_scan");
   return 0;
 }
