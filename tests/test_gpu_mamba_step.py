@@ -80,3 +80,41 @@ def test_step_whose_waits_run_out_leaves_whole_states():
                 ops.check_errors()
     finally:
         ops.wait_limit_cycles(0)
+
+
+def test_a_mixer_whose_convolution_weights_lie_at_any_address():
+    """Weights bound as slices of one flat buffer, 4 bytes past a 16-byte boundary: a prompt, then one-token steps, give the
+    bits of a mixer with weights of their own (the two kernels take the steps)."""
+    from tinyllama_c_b200 import ops
+    from tinyllama_c_b200.cache import Cache
+    from tinyllama_c_b200.engine.step import StepEntry, pack
+    from tinyllama_c_b200.parts.mixers.mamba2 import Mamba2Mixer
+    g = torch.Generator().manual_seed(5)
+    got = []
+    for off in (None, 1):
+        mixer = Mamba2Mixer(64, 64, 4, 16, 1, 128, 4, "", 1e-5)
+        tensors = {spec.name: torch.randn(spec.shape, generator=g).cuda() * 0.2 for spec in mixer.weight_specs()}
+        if off is not None:
+            tensors = first                        # the same values
+            for name in ("conv1d.weight", "conv1d.bias"):
+                flat = torch.empty(tensors[name].numel() + off, device="cuda")[off:]
+                tensors[name] = flat.view(tensors[name].shape).copy_(tensors[name])
+        first = dict(tensors)
+        mixer.bind(tensors, torch.float32, torch.device("cuda"))
+        cache = Cache({0: mixer.cache_requests()}, 64, 3, torch.float32, "cuda")
+        assert (mixer.conv_w.data_ptr() % 16 == 0) == (off is None)
+        slots, outs = [cache.acquire() for _ in range(2)], []
+        for lens in ((5, 3), (1, 1), (1, 1)):
+            entries = [StepEntry(s, [0] * n) for s, n in zip(slots, lens)]
+            step, _, _ = pack(entries, [cache.reserve(s, n) for s, n in zip(slots, lens)], 1, torch.device("cuda"))
+            x = torch.randn(sum(lens), 64, generator=torch.Generator().manual_seed(sum(lens))).cuda()
+            out = torch.zeros(sum(lens), 64, device="cuda")
+            mixer.forward(x, step, cache.layer_view(0), out)
+            outs.append(out)
+            for s, n in zip(slots, lens):
+                cache.commit(s, n)
+        torch.cuda.synchronize()
+        ops.check_errors()
+        got.append(outs + [grp.data for grp in cache.state_groups])
+    for a, b in zip(*got):
+        assert torch.equal(a, b)

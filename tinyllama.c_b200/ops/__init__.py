@@ -905,10 +905,12 @@ def mamba_conv(proj: torch.Tensor, xbc_off: int, dt_off: int, w: torch.Tensor, b
           int(bool(all_fresh)), _stream())
 
 
-def mamba_step_ok(proj: torch.Tensor, xbc_off: int, Hs: int, P: int, N: int, G: int, K: int) -> bool:
-    """Whether mamba_step takes this projection and these sizes."""
+def mamba_step_ok(proj: torch.Tensor, xbc_off: int, Hs: int, P: int, N: int, G: int, K: int, *operands: Optional[torch.Tensor]) -> bool:
+    """Whether mamba_step takes this projection, these sizes and, where given, these weights, biases and states, which it
+    moves in pieces of 16 bytes."""
     return bool(proj.is_cuda and proj.dtype == torch.float32 and proj.stride(0) % 4 == 0 and xbc_off % 4 == 0
-                and proj.data_ptr() % 16 == 0 and library().tlc_mamba_step_ok(Hs, P, N, G, Hs * P + 2 * G * N, K))
+                and proj.data_ptr() % 16 == 0 and all(t is None or t.data_ptr() % 16 == 0 for t in operands)
+                and library().tlc_mamba_step_ok(Hs, P, N, G, Hs * P + 2 * G * N, K))
 
 
 def mamba_step(proj: torch.Tensor, xbc_off: int, dt_off: int, w: torch.Tensor, bias: Optional[torch.Tensor],

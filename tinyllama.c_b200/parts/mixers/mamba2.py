@@ -151,8 +151,8 @@ class Mamba2Mixer(Part):
         ssm_state = cache.state[self.cache_key + ".ssm"]
         new = lambda tag, shape, dtype: scratch_buf(f"mamba2.{self.cache_key}.{tag}", shape, dtype, proj.device)   # (two mixers of a layer have two keys)
         y = new("y", (T, self.Di), f32)
-        if step.max_new == 1 and T == step.n_seqs and conv_state.data_ptr() % 16 == 0 and ssm_state.data_ptr() % 16 == 0 \
-                and ops.mamba_step_ok(proj, self.Di, self.Hs, self.P, self.N, self.G, self.K):
+        if step.max_new == 1 and T == step.n_seqs and ops.mamba_step_ok(proj, self.Di, self.Hs, self.P, self.N, self.G, self.K,
+                                                                        self.conv_w, self.conv_b, conv_state, ssm_state):
             # one token per sequence: convolution and scan in one kernel
             ops.mamba_step(proj, self.Di, self.Di + self.Cd, self.conv_w, self.conv_b, self.dt_bias, self.A, self.D, conv_state,
                            ssm_state, step.slots, step.start_pos, y, self.Hs, self.P, self.N, self.G, self.dtype == torch.bfloat16)
