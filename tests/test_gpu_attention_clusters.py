@@ -51,3 +51,32 @@ def test_attention_splits_that_meet_in_a_cluster_or_through_scratch(n_splits, T)
                 assert (out[t].cpu().double() - ref).abs().max().item() <= 2.0 ** -8 * (ref.abs().max().item() + vv.abs().max().item() * 2.0 ** -1), (t, sink)
     finally:
         ops.attention_decode_fused_passes(0)
+
+
+@pytest.mark.parametrize("T", [1, 9])
+@pytest.mark.parametrize("n_splits", [1, 3])
+@pytest.mark.parametrize("what", ["one key", "every key of a split"])
+def test_a_nan_among_the_scores_reaches_the_result_by_every_route(n_splits, T, what):
+    """One block a (row, head), a cluster (T 1) and scratch (T 9): the heads whose keys hold a NaN are NaN in the row that sees
+    them, everything else is finite."""
+    from tinyllama_c_b200 import ops
+    g = torch.Generator().manual_seed(3)
+    H, KV, hd, n = 6, 2, 64, 128 * n_splits
+    table = (1 + torch.arange(T * 2 * n_splits, dtype=torch.int32)).view(T, 2 * n_splits)
+    k, v = (torch.randn(1 + T * 2 * n_splits, KV, 64, hd, generator=g).bfloat16() for _ in range(2))
+    if what == "one key":
+        k[table[0, 0], 1, 17, 3] = float("nan")
+    else:
+        k[table[0, :2].long(), 1] = float("nan")
+    qkv = torch.randn(T, (H + 2 * KV) * hd, generator=g).cuda()
+    pos, ar = torch.full((T,), n - 1, dtype=torch.int32).cuda(), torch.arange(T, dtype=torch.int32).cuda()
+    kd, vd, out, table = k.cuda(), v.cuda(), torch.empty(T, H * hd, device="cuda", dtype=torch.bfloat16), table.cuda()
+    try:
+        ops.attention_decode_fused_passes(1)
+        ops.attention_decode_fused(qkv, 0, H * hd, (H + KV) * hd, kd, vd, torch.zeros(0).cuda(), True, table, pos, ar, ar, out, H, KV, hd, 0.125,
+                                   0, n, ops.new_arrival_counters(torch.device("cuda")))
+        torch.cuda.synchronize()
+    finally:
+        ops.attention_decode_fused_passes(0)
+    bad = out.float().isnan().view(T, H, hd)
+    assert bad[0, 3:].all() and not bad[0, :3].any() and not bad[1:].any()

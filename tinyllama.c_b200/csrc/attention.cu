@@ -571,12 +571,12 @@ __global__ void attention_decode_merge_kernel(const float* __restrict__ part_o, 
   float m = sink ? sv : -INFINITY;            // (a sink is one more split: its score the maximum, sum 1, no values)
   for (int s = 0; s < n_splits; s++) m = fmaxf(m, ml[2 * s]);
   float l = sink ? expf(sv - m) : 0.f;
-  for (int s = 0; s < n_splits; s++) if (ml[2 * s + 1] > 0.f) l += ml[2 * s + 1] * expf(ml[2 * s] - m);
+  for (int s = 0; s < n_splits; s++) if (ml[2 * s + 1] != 0.f) l += ml[2 * s + 1] * expf(ml[2 * s] - m);
   const float inv = tlc_head_gate(head_gate, gate_ld, (int)(th / H), (int)(th % H)) / l;
   for (int d = threadIdx.x; d < hd; d += blockDim.x) {
     float acc = 0.f;
     for (int s = 0; s < n_splits; s++)
-      if (ml[2 * s + 1] > 0.f) acc = fmaf(part_o[(th * n_splits + s) * hd + d], expf(ml[2 * s] - m), acc);
+      if (ml[2 * s + 1] != 0.f) acc = fmaf(part_o[(th * n_splits + s) * hd + d], expf(ml[2 * s] - m), acc);
     orow[d] = from_f32<T>(acc * inv);
   }
 }

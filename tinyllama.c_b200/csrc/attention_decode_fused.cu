@@ -351,9 +351,10 @@ attention_decode_fused_kernel(const float* __restrict__ qkv, int ld, int q_off, 
 #pragma unroll
       for (int x = 0; x < FM_NW; x++) {
         const float mw = m_s[x * 8 + hg];
-        if (mw > -INFINITY) {
-          const float e = expf(mw - M);
-          l = fmaf(l_s[x * 8 + hg], e, l);
+        const float lw = l_s[x * 8 + hg];
+        if (lw != 0.f) {                                    // 0: a warp without keys; NaN goes on into the result, also from a warp
+          const float e = expf(mw - M);                     // whose keys all score NaN and leave no maximum
+          l = fmaf(lw, e, l);
           o = fmaf(reinterpret_cast<const float*>(smraw + (size_t)x * L::WARP)[hg * HD + d], e, o);
         }
       }
@@ -403,7 +404,7 @@ attention_decode_fused_kernel(const float* __restrict__ qkv, int ld, int q_off, 
       float e[8], x[8];
 #pragma unroll
       for (int q = 0; q < 8; q++) {
-        e[q] = st[q].y > 0.f ? expf(st[q].x - M) : 0.f;                // (a block without keys has left no outputs)
+        e[q] = st[q].y != 0.f ? expf(st[q].x - M) : 0.f;               // (a block without keys has left no outputs)
         x[q] = __fmul_rn(st[q].y, e[q]);
       }
       float l = ((x[0] + x[4]) + (x[2] + x[6])) + ((x[1] + x[5]) + (x[3] + x[7]));

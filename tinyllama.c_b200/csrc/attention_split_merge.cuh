@@ -7,7 +7,7 @@
 
 // part_o [T, H, n_splits, HD], part_ml [T, H, n_splits, 2]; out: rows of out_ld elements, head h at h * HD;
 // sh: the block's dynamic shared memory of smem_floats floats (free by now); NT threads.  All threads of
-// the block call it.  head_gate: see tlc_head_gate.  sink: one more split of maximum 0 (or sink_values[head]) and sum 1 that carries no values.
+// the block call it.  A split without keys has a sum of 0 and no outputs; any other sum counts, NaN among them.  head_gate: see tlc_head_gate.  sink: one more split of maximum 0 (or sink_values[head]) and sum 1 that carries no values.
 template <int HD, int NT>
 __device__ __forceinline__ void attention_merge_splits(const float* part_o, const float* part_ml, __nv_bfloat16* out,
                                                        float* sh, int smem_floats, int t, int g, int G, int H,
@@ -34,11 +34,11 @@ __device__ __forceinline__ void attention_merge_splits(const float* part_o, cons
       const float sv = (sink && sink_values) ? sink_values[g * G + hg] : 0.f;    // the sink's score: 0, or the head's own
       if (sink) m = fmaxf(m, sv);
       float l = 0.f;
-      for (int s = lane; s < n_splits; s += 32) if (e[2 * s + 1] > 0.f) l += e[2 * s + 1] * expf(e[2 * s] - m);
+      for (int s = lane; s < n_splits; s += 32) if (e[2 * s + 1] != 0.f) l += e[2 * s + 1] * expf(e[2 * s] - m);
       l = warp_sum(l);
       if (sink) l += expf(sv - m);
       const float inv = tlc_head_gate(head_gate, gate_ld, t, g * G + hg) / l;
-      for (int s = lane; s < n_splits; s += 32) e[2 * s] = e[2 * s + 1] > 0.f ? expf(e[2 * s] - m) * inv : 0.f;
+      for (int s = lane; s < n_splits; s += 32) e[2 * s] = e[2 * s + 1] != 0.f ? expf(e[2 * s] - m) * inv : 0.f;
     }
     __syncthreads();
     // four outputs of a thread at a time, eight splits of each: 32 loads in flight, all unconditional (past the last split or
@@ -88,13 +88,13 @@ __device__ __forceinline__ void attention_merge_splits(const float* part_o, cons
     float l = sink ? expf(sv - m) : 0.f;
     for (int s = 0; s < n_splits; s++) {
       const float ls = __ldcg(mlh + 2 * s + 1);
-      if (ls > 0.f) l += ls * expf(__ldcg(mlh + 2 * s) - m);
+      if (ls != 0.f) l += ls * expf(__ldcg(mlh + 2 * s) - m);
     }
     const float inv = tlc_head_gate(head_gate, gate_ld, t, g * G + hg) / l;
     for (int d = tid; d < HD; d += NT) {
       float acc = 0.f;
       for (int s = 0; s < n_splits; s++)
-        if (__ldcg(mlh + 2 * s + 1) > 0.f)
+        if (__ldcg(mlh + 2 * s + 1) != 0.f)
           acc = fmaf(__ldcg(part_o + (th * n_splits + s) * HD + d), expf(__ldcg(mlh + 2 * s) - m), acc);
       out[(size_t)t * out_ld + ((size_t)g * G + hg) * HD + d] = __float2bfloat16_rn(acc * inv);
     }
