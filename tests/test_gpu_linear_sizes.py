@@ -74,3 +74,29 @@ def test_linear_with_16_or_32_rows_on_the_narrow_side_and_a_fixed_split(M, N, K,
             ops.check_errors()
     finally:
         ops.linear_few_rows(True, 0)
+
+
+_WITHOUT_SET_UP = """
+import ctypes, sys, torch
+from tinyllama_c_b200 import ops
+from tinyllama_c_b200.csrc import build
+lib = build.load()
+lib.tlc_linear.restype, lib.tlc_linear.argtypes = ops._SIGNATURES["tlc_linear"]
+lib.tlc_last_error.restype = ctypes.c_char_p
+a, w, out = torch.randn(64, 64).cuda(), torch.randn(64, 64).cuda(), torch.empty(64, 64, device="cuda")
+rc = lib.tlc_linear(a.data_ptr(), 0, 64, w.data_ptr(), 0, 64, out.data_ptr(), 0, 64, None, None, 0, 64, 64, 64, 33, None)
+torch.cuda.synchronize()
+assert rc == 0, lib.tlc_last_error()
+assert (out.double() - a.double() @ w.double().T).abs().max().item() < 72 * 2.0 ** -24 * 64 * 16
+"""
+
+
+def test_32_bit_products_without_the_set_up_of_the_tensor_core_kernels():
+    """A process that has not called tlc_linear_init: the 32-bit products need none (the tile with K in four parts takes more
+    shared memory than a kernel has unasked)."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    run = subprocess.run([sys.executable, "-c", _WITHOUT_SET_UP], cwd=root, capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, run.stderr[-2000:]

@@ -358,16 +358,22 @@ gemm_tiled_f32x4_kernel(const float* __restrict__ a, int lda, const float* __res
 constexpr int ft_smem(int CT, int KG) { return KG * 2 * FT_K * (FT_M + 16 * CT + 2 * FT_LD) * 4; }
 static_assert(ft_smem(4, 4) >= 3 * 8 * 4 * 128 * 4 && ft_smem(8, 1) <= 48 * 1024, "the other groups' sums reuse the operands' memory");
 
-// Kernels that ask for more than 48 KB of shared memory, prepared outside any stream capture.
+// Kernels that ask for more than 48 KB of shared memory: once a device, ahead of any stream capture where the library is set up
+// first (tlc_linear_init), else with the first product that takes one of them.
 int tlc_linear_simt_init() {
+  static bool ready[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && ready[dev]) return 0;
   if (cudaFuncSetAttribute(gemm_tiled_f32x4_kernel<float, 4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, ft_smem(4, 4)) != cudaSuccess ||
       cudaFuncSetAttribute(gemm_tiled_f32x4_kernel<__nv_bfloat16, 4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, ft_smem(4, 4)) != cudaSuccess)
     return tlc_fail(-2, "linear(32 bits): cannot reserve %d bytes of shared memory", ft_smem(4, 4));
+  if (dev >= 0 && dev < 64) ready[dev] = true;
   return 0;
 }
 
 template <typename TO>
-static void launch_simt_f32x4(const float* a, int lda, const float* w, int ldw, TO* out, int ldo, const float* colscale,
+static int launch_simt_f32x4(const float* a, int lda, const float* w, int ldw, TO* out, int ldo, const float* colscale,
                               const float* colbias, TlcEpi accumulate, int M, int N, int K, cudaStream_t stream) {
   static int sms = 0;
   if (sms == 0) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
@@ -377,10 +383,13 @@ static void launch_simt_f32x4(const float* a, int lda, const float* w, int ldw, 
     if ((long long)my * ((N + 127) / 128) >= 2 * sms)
       tlc_launch(gemm_tiled_f32x4_kernel<TO, 8, 1>, dim3((N + 127) / 128, my), dim3(128), ft_smem(8, 1), stream, a, lda, w, ldw, out, ldo, colscale,
                  colbias, accumulate, M, N, K);
-    else
+    else {
+      if (int rc = tlc_linear_simt_init()) return rc;
       tlc_launch(gemm_tiled_f32x4_kernel<TO, 4, 4>, dim3((N + 63) / 64, my), dim3(512), ft_smem(4, 4), stream, a, lda, w, ldw, out, ldo, colscale,
                  colbias, accumulate, M, N, K);
-    return;
+    }
+    TLC_CHECK_LAUNCH("linear(simt)");
+    return 0;
   }
   // A warp's columns share its activations: a read of them costs as much as one of the weights, so up to 2 rows take two
   // columns and more rows four, where that still makes two blocks an SM.
@@ -395,6 +404,8 @@ static void launch_simt_f32x4(const float* a, int lda, const float* w, int ldw, 
     else { if (two) TLC_SK4(8, 4, 2); else TLC_SK4(8, 2, 2); }
   }
 #undef TLC_SK4
+  TLC_CHECK_LAUNCH("linear(simt)");
+  return 0;
 }
 
 template <typename TA, typename TW, typename TO>
@@ -402,11 +413,8 @@ static int launch_simt(const void* a, int lda, const void* w, int ldw, void* out
                        const float* colbias, TlcEpi accumulate, int M, int N, int K, cudaStream_t stream) {
   constexpr int MT = 8;
   if constexpr (std::is_same<TA, float>::value && std::is_same<TW, float>::value) {
-    if (K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)a % 16 == 0) && ((uintptr_t)w % 16 == 0)) {
-      launch_simt_f32x4<TO>((const float*)a, lda, (const float*)w, ldw, (TO*)out, ldo, colscale, colbias, accumulate, M, N, K, stream);
-      TLC_CHECK_LAUNCH("linear(simt)");
-      return 0;
-    }
+    if (K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)a % 16 == 0) && ((uintptr_t)w % 16 == 0))
+      return launch_simt_f32x4<TO>((const float*)a, lda, (const float*)w, ldw, (TO*)out, ldo, colscale, colbias, accumulate, M, N, K, stream);
   }
   if (M <= 16) {
     const bool vec = std::is_same<TA, __nv_bfloat16>::value && std::is_same<TW, __nv_bfloat16>::value && (K % 8 == 0) &&
