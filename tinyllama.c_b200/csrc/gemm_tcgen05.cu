@@ -482,6 +482,7 @@ typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, v
                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 EncodeTiled g_encode = nullptr;
 int g_sms = 148;
+int g_err_device = -1;          // the device that g_err_dev lies on
 ErrWords* g_err_dev = nullptr;   // device memory: the flag kernels read + where its host-visible copy lives
 int* g_err_host = nullptr;       // host-mapped word, written by a kernel on failure only
 std::mutex g_mu;
@@ -581,6 +582,7 @@ int init_once() {
       cudaMemset(g_part_arrivals, 0, SPLIT_SLOTS * SPLIT_SLOT_COUNTERS * sizeof(unsigned)) != cudaSuccess)
     return tlc_fail(-3, "linear: cannot allocate the scratch of split products");
   *g_err_host = 0;
+  cudaGetDevice(&g_err_device);
   ErrWords init{0, host_dev_view, TLC_WAIT_LIMIT_CYCLES};
   if (cudaMemcpy(g_err_dev, &init, sizeof(init), cudaMemcpyHostToDevice) != cudaSuccess)
     return tlc_fail(-3, "linear: cannot initialise the error words");
@@ -738,6 +740,10 @@ int launch_pairs(const CUtensorMap& ma, const CUtensorMap& mb, void* out, int ld
 // Error word of the tensor-core kernels: 0, or which bounded wait ran out
 // (1 loader, 2 MMA issuer, 3 epilogue, 4 drain).  Reading it does not synchronise.
 ErrWords* tlc_error_words() { return g_err_dev; }
+ErrWords* tlc_error_words_here() {
+  int dev = -1;
+  return g_err_dev && cudaGetDevice(&dev) == cudaSuccess && dev == g_err_device ? g_err_dev : nullptr;
+}
 
 extern "C" int tlc_linear_error() { return g_err_host ? *(volatile int*)g_err_host : 0; }
 extern "C" void tlc_linear_error_clear() {

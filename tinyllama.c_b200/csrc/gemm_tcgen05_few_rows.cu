@@ -393,7 +393,7 @@ int few_rows_ok(int a_dtype, int lda, const void* a, int w_dtype, int ldw, const
   static int sms = 0;
   if (sms == 0) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
   if (!g_few_rows || a_dtype != TLC_BF16 || w_dtype != TLC_BF16 || M > g_max_rows || K % 8 != 0 || lda % 8 != 0 || ldw % 8 != 0 ||
-      (uintptr_t)a % 16 != 0 || (uintptr_t)w % 16 != 0 || tlc_error_words() == nullptr)
+      (uintptr_t)a % 16 != 0 || (uintptr_t)w % 16 != 0 || tlc_error_words_here() == nullptr)
     return 0;
   const int tiles = (N + WM - 1) / WM;
   if (g_force_split > 0) return M > 8 && N >= WM;

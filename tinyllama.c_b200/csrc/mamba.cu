@@ -822,9 +822,9 @@ mamba_step_kernel(const float* __restrict__ proj, int ld, int xbc_off, int dt_of
 constexpr int STEP_BLOCKS = 4096;
 
 // Whether mamba_step_kernel takes these sizes: 65..256 state columns and the other sizes in pieces of 16 bytes (smaller
-// states leave lanes idle: they keep the two kernels), 2 to 4 taps.
+// states leave lanes idle: they keep the two kernels), 2 to 4 taps, on the device that the library is set up on.
 extern "C" int tlc_mamba_step_ok(int Hs, int P, int N, int G, int Cd, int K) {
-  return N > 64 && N <= 256 && N % 4 == 0 && P % 4 == 0 && Cd % 4 == 0 && K >= 2 && K <= 4 && G > 0 && Hs % G == 0 && Hs <= 65535 && Hs * P + 2 * G * N == Cd;
+  return N > 64 && N <= 256 && N % 4 == 0 && P % 4 == 0 && Cd % 4 == 0 && K >= 2 && K <= 4 && G > 0 && Hs % G == 0 && Hs <= 65535 && Hs * P + 2 * G * N == Cd && tlc_error_words_here() != nullptr;
 }
 
 extern "C" int tlc_mamba_step(const float* proj, int ld, int xbc_off, int dt_off, const float* w, const float* bias,
@@ -832,11 +832,11 @@ extern "C" int tlc_mamba_step(const float* proj, int ld, int xbc_off, int dt_off
                               const int* slots, const int* start_pos, float* y, int B, int Hs, int P, int N, int G, int Cd, int K,
                               int bf16_run, cudaStream_t stream) {
   if (B == 0) return 0;
+  TLC_REQUIRE(tlc_error_words_here() != nullptr, "mamba_step: the library is not set up on this device (tlc_linear_init)");
   TLC_REQUIRE(tlc_mamba_step_ok(Hs, P, N, G, Cd, K), "mamba_step: %d heads of %d, state %d, %d groups, %d taps are outside the kernel's range", Hs, P, N, G, K);
   const void* aligned[] = {proj, w, bias, conv_state, state};
   for (const void* p : aligned) TLC_REQUIRE(((uintptr_t)p & 15) == 0, "mamba_step: operands must start on 16-byte boundaries");
   TLC_REQUIRE(ld % 4 == 0 && xbc_off % 4 == 0, "mamba_step: rows of the projection must start on 16-byte boundaries");
-  TLC_REQUIRE(tlc_error_words() != nullptr, "mamba_step: the library is not set up (tlc_linear_init)");
   // 16 rows a block (18.6 KB of shared memory), and 32 where that still makes STEP_BLOCKS blocks: then the convolution that every
   // block makes for itself counts, and the kernels beside this one no longer do.  A step of the 1.5B sizes at batch 64 (6,144 blocks
   // of 32 rows): 2.96 ms, with 16 rows 3.12; of the 7B sizes at batch 32 (3,072): 7.17 and 7.03; of 1.5B at batch 8 (768): 1.51 and

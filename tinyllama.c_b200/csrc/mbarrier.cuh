@@ -48,5 +48,7 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-// The error words of the library (set up by tlc_linear_init); nullptr before that.
+// The error words of the library (set up by tlc_linear_init); nullptr before that.  They lie in the memory of one device:
+// where a kernel without bounded waits can do the work, the other form says nullptr on every other device.
 ErrWords* tlc_error_words();
+ErrWords* tlc_error_words_here();

@@ -253,8 +253,9 @@ int tlc_mamba_conv(const void* proj, int dtype, int ld, int xbc_off, int dt_off,
                    void* xbc_out, int xbc_dtype, float* dt_out, float* dA_out, int T, int B, int Cd, int K,
                    int Hs, int single_rows, int quick, int all_fresh, cudaStream_t stream);
 /* Steps in which every sequence brings one row (row b is sequence b's): tlc_mamba_conv and tlc_ssm_scan in one kernel, for
- * 32-bit projections and the sizes of tlc_mamba_step_ok.  The windows of the B and C channels stay as they were: the
- * kernel that follows, tlc_gated_rmsnorm_step, advances them. */
+ * 32-bit projections and the sizes of tlc_mamba_step_ok (which also says no on a device that the library is not set up
+ * on).  The windows of the B and C channels stay as they were: the kernel that follows, tlc_gated_rmsnorm_step,
+ * advances them. */
 int tlc_mamba_step_ok(int Hs, int P, int N, int G, int Cd, int K);
 int tlc_mamba_step(const float* proj, int ld, int xbc_off, int dt_off, const float* w, const float* bias,
                    const float* dt_bias, const float* A, const float* Dskip, float* conv_state, float* state,
