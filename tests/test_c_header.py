@@ -64,6 +64,11 @@ def test_every_declared_function_is_loaded_with_matching_types():
         assert got == kinds, f"{name}: header {kinds}\n table {got}"
 
 
+def test_functions_that_programs_were_built_against_keep_their_arguments():
+    """A C program passes as many arguments as the header had when it was built."""
+    assert parse_header()["tlc_linear_few_rows_ok"] == ("int", ["int", "int", "pointer"] * 2 + ["int"] * 3)
+
+
 def test_every_definition_is_declared():
     """No .cu file exports a tlc_ function that the header does not declare."""
     protos = parse_header()

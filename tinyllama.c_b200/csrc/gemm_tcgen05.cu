@@ -28,6 +28,7 @@
 
 int tlc_linear_simt_init();      // gemm_simt.cu
 // gemm_tcgen05_few_rows.cu
+int tlc_linear_few_rows_takes(int a_dtype, int lda, const void* a, int w_dtype, int ldw, const void* w, int M, int N, int K, bool plain32);
 int tlc_linear_few_rows_run(const void* a, int lda, const void* w, int ldw, void* out, int out_dtype, int ldo,
                             const float* colscale, const float* colbias, TlcEpi accumulate, int M, int N, int K,
                             cudaStream_t stream);
@@ -820,7 +821,7 @@ extern "C" int tlc_linear_swiglu(const void* a, int a_dtype, int lda, const void
   TLC_REQUIRE(K > 0 && lda >= K && ldw >= K && ldo >= N / 2, "linear: bad sizes M=%d N=%d K=%d lda=%d ldw=%d ldo=%d", M, N, K,
               lda, ldw, ldo);
   if (out_dtype != TLC_F32 && out_dtype != TLC_BF16) return tlc_fail(-1, "linear: unknown output dtype %d", out_dtype);
-  if (min_rows_for_tensor_cores <= 128 && tlc_linear_few_rows_ok(a_dtype, lda, a, w_dtype, ldw, w, M, N, K, 0)) {
+  if (min_rows_for_tensor_cores <= 128 && tlc_linear_few_rows_ok(a_dtype, lda, a, w_dtype, ldw, w, M, N, K)) {
     if (int rc = init_once()) return rc;
     return tlc_linear_few_rows_swiglu(a, lda, w, ldw, out, out_dtype, ldo, colscale, colbias, M, N, K, act, stream);
   }
@@ -860,7 +861,7 @@ extern "C" int tlc_linear(const void* a, int a_dtype, int lda, const void* w, in
   // few tiles to keep the GPU busy (narrow outputs) and too few K-steps to share among blocks.
   // (a threshold above 128 rows keeps every tensor-core kernel out, this one too)
   if (min_rows_for_tensor_cores <= 128 && (out_dtype == TLC_F32 || out_dtype == TLC_BF16) &&
-      tlc_linear_few_rows_ok(a_dtype, lda, a, w_dtype, ldw, w, M, N, K, out_dtype == TLC_F32 && !accumulate)) {
+      tlc_linear_few_rows_takes(a_dtype, lda, a, w_dtype, ldw, w, M, N, K, out_dtype == TLC_F32 && !accumulate)) {
     TLC_REQUIRE(K > 0 && lda >= K && ldw >= K && ldo >= N, "linear: bad sizes M=%d N=%d K=%d lda=%d ldw=%d ldo=%d", M, N, K,
                 lda, ldw, ldo);
     if (int rc = init_once()) return rc;

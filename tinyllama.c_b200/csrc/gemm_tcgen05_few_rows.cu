@@ -410,9 +410,11 @@ extern "C" void tlc_linear_few_rows_min_tiles(int tiles) { g_min_tiles = tiles; 
 extern "C" void tlc_linear_few_rows_max_rows(int rows) { g_max_rows = rows; }
 
 // plain32: the output is 32-bit and overwritten, not added to.
-extern "C" int tlc_linear_few_rows_ok(int a_dtype, int lda, const void* a, int w_dtype, int ldw, const void* w, int M, int N, int K,
-                                      int plain32) {
-  return few_rows_ok(a_dtype, lda, a, w_dtype, ldw, w, M, N, K, plain32 != 0);
+int tlc_linear_few_rows_takes(int a_dtype, int lda, const void* a, int w_dtype, int ldw, const void* w, int M, int N, int K, bool plain32) {
+  return few_rows_ok(a_dtype, lda, a, w_dtype, ldw, w, M, N, K, plain32);
+}
+extern "C" int tlc_linear_few_rows_ok(int a_dtype, int lda, const void* a, int w_dtype, int ldw, const void* w, int M, int N, int K) {
+  return few_rows_ok(a_dtype, lda, a, w_dtype, ldw, w, M, N, K, false);
 }
 
 int tlc_linear_few_rows_run(const void* a, int lda, const void* w, int ldw, void* out, int out_dtype, int ldo,

@@ -156,12 +156,12 @@ int tlc_linear_swiglu(const void* a, int a_dtype, int lda, const void* w, int w_
 int tlc_linear_simt(const void* a, int a_dtype, int lda, const void* w, int w_dtype, int ldw, void* out,
                     int out_dtype, int ldo, const float* colscale, const float* colbias, int accumulate,
                     int M, int N, int K, cudaStream_t stream);
-// The product for 17..64 rows (weights on the 128-row side of tcgen05.mma, K shared among the blocks of a cluster).
+// The product for up to 128 rows (weights on the 128-row side of tcgen05.mma, K shared among the blocks of a cluster).
 void tlc_linear_few_rows(int on);          // 0: never this kernel (for comparisons)
 void tlc_linear_few_rows_split(int split); // 0: the number of blocks per tile is chosen; 1, 2, 4, 8: fixed (for tests)
 void tlc_linear_few_rows_min_tiles(int tiles);   // outputs of fewer tiles of 128 weight rows stay with the other kernels (0: 16 tiles with more than 32 rows, else 32)
 void tlc_linear_few_rows_max_rows(int rows);     // products of more rows go to the tiles of the prompt product (128; for comparisons)
-int tlc_linear_few_rows_ok(int a_dtype, int lda, const void* a, int w_dtype, int ldw, const void* w, int M, int N, int K, int plain32);
+int tlc_linear_few_rows_ok(int a_dtype, int lda, const void* a, int w_dtype, int ldw, const void* w, int M, int N, int K);   // whatever the output is
 void tlc_linear_tma_out(int on);        // 0: the tensor-core product's 32-bit outputs never leave through the copy engine (for comparisons)
 void tlc_linear_skinny_pairs(int on);   // 0: the skinny product never splits K over a pair of blocks (for comparisons)
 int tlc_linear_skinny_ok(int a_dtype, int lda, const void* a, int w_dtype, int ldw, const void* w, int M, int K);

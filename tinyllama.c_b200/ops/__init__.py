@@ -65,7 +65,7 @@ _SIGNATURES = {
     "tlc_linear_few_rows_split": (None, [_i]),
     "tlc_linear_few_rows_min_tiles": (None, [_i]),
     "tlc_linear_few_rows_max_rows": (None, [_i]),
-    "tlc_linear_few_rows_ok": (_i, [_i, _i, _vp, _i, _i, _vp, _i, _i, _i, _i]),
+    "tlc_linear_few_rows_ok": (_i, [_i, _i, _vp, _i, _i, _vp, _i, _i, _i]),
     "tlc_linear_pairs": (_i, []),
     "tlc_rope_kv_store": (_i, [_vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i,
                                _i, _i, _vp]),
@@ -557,7 +557,7 @@ def linear_pair_override(mode: int) -> None:
 
 
 def linear_few_rows(on: bool, split: int = 0) -> None:
-    """Whether products of 17..64 rows take the tensor-core kernel that puts the weights on the 128-row side and
+    """Whether products of up to 128 rows may take the tensor-core kernel that puts the weights on the 128-row side and
     shares a tile's K-steps among the blocks of a cluster; split fixes the number of blocks per tile (1, 2, 4, 8;
     0: chosen from the sizes).  For tests and comparisons."""
     library().tlc_linear_few_rows(int(bool(on)))
