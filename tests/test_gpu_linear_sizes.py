@@ -100,3 +100,18 @@ def test_32_bit_products_without_the_set_up_of_the_tensor_core_kernels():
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     run = subprocess.run([sys.executable, "-c", _WITHOUT_SET_UP], cwd=root, capture_output=True, text=True, timeout=300)
     assert run.returncode == 0, run.stderr[-2000:]
+
+
+@pytest.mark.parametrize("M", [1, 4, 8, 9, 16, 17, 100])
+def test_32_bit_products_of_what_the_kernel_before_them_writes(M):
+    """w comes from the kernel in front of the product (here a norm's rows): the product reads it after that kernel's end."""
+    from tinyllama_c_b200 import ops
+    g = torch.Generator().manual_seed(M)
+    N, K = 4100, 1028
+    a, x, gain = torch.randn(M, K, generator=g).cuda(), torch.randn(N, K, generator=g).cuda(), torch.ones(K, device="cuda")
+    w, out = torch.full((N, K), float("nan"), device="cuda"), torch.empty(M, N, device="cuda")
+    torch.cuda.synchronize()
+    ops.rmsnorm(x, gain, 1e-5, w)
+    ops.linear(a, w, out)
+    torch.cuda.synchronize()
+    _check(out, a, w, None, None, None)

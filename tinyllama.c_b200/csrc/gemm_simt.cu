@@ -18,7 +18,7 @@ __global__ void __launch_bounds__(256)
 gemm_tiled_kernel(const TA* __restrict__ a, int lda, const TW* __restrict__ w, int ldw, TO* __restrict__ out, int ldo,
                   const float* __restrict__ colscale, const float* __restrict__ colbias, TlcEpi accumulate, int M, int N,
                   int K) {
-  tlc_pdl(a, out);
+  tlc_pdl(a, w, out);
   __shared__ float As[BK][BM + 4];
   __shared__ float Ws[BK][BN + 4];
   const int tid = threadIdx.x;
@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(256)
 gemm_skinny_kernel(const TA* __restrict__ a, int lda, const TW* __restrict__ w, int ldw, TO* __restrict__ out, int ldo,
                    const float* __restrict__ colscale, const float* __restrict__ colbias, TlcEpi accumulate, int M, int N,
                    int K, int m_base) {
-  tlc_pdl(a, out);
+  tlc_pdl(a, w, out);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n = blockIdx.x * (blockDim.x >> 5) + warp;
   if (n >= N) return;
@@ -159,15 +159,16 @@ __device__ __forceinline__ float4 load_once(const float4* p) {
   return v;
 }
 
-// Few rows: a warp takes COLS output columns and reads their weight rows 512 bytes at a time, U pieces a column in flight
-// (the first ones before the wait on the previous kernel); an activation piece serves COLS columns.
-// 2 rows, 2048 -> 8240 (67 MB): 90 -> 12.7 us, 4096 -> 2048 (34 MB): 95 -> 12.4 us; 8 rows 216 -> 19 and 237 -> 50 us.
+// Few rows: a warp takes COLS output columns and reads their weight rows 512 bytes at a time, U pieces a column in flight; an
+// activation piece serves COLS columns.  Nothing is read before the wait on the previous kernel: in this arithmetic w may be
+// what that kernel wrote (weights asked for ahead of the wait: 2 rows 13.4 us and not 14.1, 8 rows 44.9 and not 42.1).
+// 2 rows, 2048 -> 8240 (67 MB): 90 -> 14.1 us, 4096 -> 2048 (34 MB): 95 -> 13.0 us; 8 rows 216 -> 20.6 and 237 -> 42 us.
 template <typename TO, int MT, int COLS, int U>
 __global__ void __launch_bounds__(256)
 gemm_skinny_f32x4_kernel(const float* __restrict__ a, int lda, const float* __restrict__ w, int ldw, TO* __restrict__ out,
                          int ldo, const float* __restrict__ colscale, const float* __restrict__ colbias, TlcEpi accumulate,
                          int M, int N, int K, int m_base) {
-  asm volatile("griddepcontrol.launch_dependents;");
+  tlc_pdl(a, w, out);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n0 = (blockIdx.x * 8 + warp) * COLS;
   const int K4 = K >> 2;
@@ -185,7 +186,6 @@ gemm_skinny_f32x4_kernel(const float* __restrict__ a, int lda, const float* __re
     for (int u = 0; u < U; u++)
 #pragma unroll
       for (int c = 0; c < COLS; c++) wv[c][u] = i0 + 32 * u < K4 ? load_once(wr[c] + i0 + 32 * u) : make_float4(0.f, 0.f, 0.f, 0.f);
-    if (i0 == lane) tlc_wait(a, out);
 #pragma unroll
     for (int u = 0; u < U; u++) {
       if (i0 + 32 * u < K4) {
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(128 * KG)
 gemm_tiled_f32x4_kernel(const float* __restrict__ a, int lda, const float* __restrict__ w, int ldw, TO* __restrict__ out,
                         int ldo, const float* __restrict__ colscale, const float* __restrict__ colbias, TlcEpi accumulate,
                         int M, int N, int K) {
-  tlc_pdl(a, out);
+  tlc_pdl(a, w, out);
   constexpr int TN = 16 * CT, LA = FT_M + FT_LD, LW = TN + FT_LD;
   constexpr int PA = FT_M * FT_K / 4 / 128, PW = TN * FT_K / 4 / 128;   // 16-byte pieces a thread brings of each operand
   extern __shared__ __align__(16) float ft_sm[];

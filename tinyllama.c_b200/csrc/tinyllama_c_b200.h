@@ -142,7 +142,10 @@ int tlc_rmsnorm_add(const float* parts, int n_parts, const float* extra, const f
  * out[m, n] (+)= (sum_k a[m, k] w[n, k]) * colscale[n] + colbias[n];  a [M, K], w [N, K], 32-bit sums.
  * tlc_linear chooses: bfloat16 operands go to the tcgen05 kernel (TMA -> shared memory -> tensor memory)
  * from min_rows_for_tensor_cores rows on, to the weight-streaming mma.sync kernel below that; float
- * operands run on the CUDA cores in true 32-bit arithmetic (tlc_linear_simt). */
+ * operands run on the CUDA cores in true 32-bit arithmetic (tlc_linear_simt).
+ * With programmatic launches (tlc_set_pdl) a bfloat16 w is fetched while the kernel before the product may still run: it must
+ * not be what a kernel writes that was launched on the stream since the last step boundary (see tlc_embed).  a, out and
+ * a float w may. */
 int tlc_linear(const void* a, int a_dtype, int lda, const void* w, int w_dtype, int ldw, void* out,
                int out_dtype, int ldo, const float* colscale, const float* colbias, int accumulate, int M,
                int N, int K, int min_rows_for_tensor_cores, cudaStream_t stream);

@@ -639,7 +639,8 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, colscale: Option
     """out[m, n] (+)= (sum_k a[m, k] w[n, k]) * colscale[n] + colbias[n].
 
     a [M, K] and out [M, N] may be row-strided views; w is [N, K].  Accumulation is
-    32-bit.  float32 operands run on the CUDA cores in true 32-bit arithmetic."""
+    32-bit.  float32 operands run on the CUDA cores in true 32-bit arithmetic.  bfloat16 weights are fetched while the
+    kernel before may still run: w must not be the output of a kernel of the same step (a float32 w may)."""
     _gpu(a, w, out, colscale, colbias)
     M, K = a.shape
     N = w.shape[0]
