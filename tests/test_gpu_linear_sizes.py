@@ -44,7 +44,15 @@ def _run(M, N, K, dtype, pad=4):
 @pytest.mark.parametrize("N,K", [(1, 4), (67, 36), (130, 1028), (4740, 132), (2048, 68)])
 def test_linear_of_32_bit_rows_in_pieces_of_16_bytes(M, N, K):
     """Few rows (one or two columns a warp, two or four from five rows on; more than eight rows in two launches), then
-    tiles of 64 x 128 or of 64 x 64 with K in four parts: K shorter than a step, parts without a step, edges in M and N."""
+    tiles of 64 x 64 with K in four parts: K shorter than a step, parts without a step, edges in M and N."""
+    _run(M, N, K, torch.float32)
+
+
+@pytest.mark.parametrize("M,N,K", [(449, 4740, 132), (1211, 2050, 36), (577, 4096, 4), (2368, 1028, 68)])
+def test_linear_of_32_bit_rows_in_tiles_of_64_by_128(M, N, K):
+    """As many tiles as two an SM (296 on 148 SMs): one K-step or several, the last one shorter, edges in M and N or none."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert -(-M // 64) * -(-N // 128) >= 2 * min(sms, 148)
     _run(M, N, K, torch.float32)
 
 

@@ -7,11 +7,14 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("bf16_run", [False, True])
 @pytest.mark.parametrize("Hs,P,N,G,K,bias", [(4, 16, 68, 1, 4, True), (2, 20, 128, 2, 3, False), (6, 4, 132, 3, 2, True), (3, 64, 256, 1, 4, True),
-                                             (8, 36, 72, 4, 4, False), (120, 36, 72, 4, 4, False), (64, 64, 256, 1, 4, True)])
+                                             (8, 36, 72, 4, 4, False), (120, 36, 72, 4, 4, False), (64, 64, 256, 1, 4, True),
+                                             (416, 36, 72, 4, 4, False), (416, 64, 128, 1, 3, True), (820, 4, 68, 2, 2, True),
+                                             (280, 68, 132, 4, 4, True), (416, 64, 256, 1, 3, False), (210, 100, 136, 3, 2, True)])
 def test_step_kernel_against_convolution_and_scan(Hs, P, N, G, K, bias, bf16_run):
-    """State columns that fill a warp's loads or not, rows of a head that end inside a block (of 16 rows, with many heads
-    of 32), several groups, sequences at position 0 (zero window, zero state) beside ones that continue, slots in any
-    order; y, the states and, after the norm that follows, all windows."""
+    """State columns that fill a warp's loads or not, rows of a head that end inside a block (of 16 rows; in the last
+    six sets, 4,096 blocks and more, of 32), several groups, sequences at position 0 (zero window, zero state) beside ones
+    that continue, slots in any order; y, the states and, after the norm that follows, all windows.  In 32 bits the
+    recurrence in 64 bits too."""
     from tinyllama_c_b200 import ops
     g = torch.Generator().manual_seed(Hs * 1009 + N)
     B, Di = 5, Hs * P
@@ -44,6 +47,31 @@ def test_step_kernel_against_convolution_and_scan(Hs, P, N, G, K, bias, bf16_run
         got.append((y, state, conv, out))
     for a, b, name in zip(got[0], got[1], ("y", "states", "windows", "gated output")):
         assert torch.equal(a, b), name
+    if bf16_run:
+        return
+    # the convolution of the last K - 1 stored rows and the new one, the time step, one step of the recurrence, with bounds on
+    # the magnitudes that the roundings of a convolution, a SiLU of slope at most 1.1 and a sum of N terms are relative to
+    live, at = start > 0, slots.long()
+    ulp = 2.0 ** -24
+    taps = torch.cat([conv0[at].double() * live[:, None, None], proj[:, None, Di:Di + Cd].double()], 1)      # [B, K, Cd]
+    u, mag = (taps * w.double().T).sum(1), (taps.abs() * w.double().abs().T).sum(1)
+    if bias:
+        u, mag = u + cb.double(), mag + cb.double().abs()
+    v = torch.nn.functional.silu(u)
+    x, Bm, Cm = v[:, :Di].view(B, Hs, P), v[:, Di:Di + G * N], v[:, Di + G * N:]
+    xm, bm, cm = (1.1 * mag[:, :Di]).view(B, Hs, P), 1.1 * mag[:, Di:Di + G * N], 1.1 * mag[:, Di + G * N:]
+    by_head = lambda t: t.reshape(B, G, N).repeat_interleave(Hs // G, 1)[:, :, None]  # noqa: E731
+    dt = torch.nn.functional.softplus(proj[:, Di + Cd:Di + Cd + Hs].double() + dt_bias.double())[:, :, None, None]
+    dA = torch.exp(dt * A.double()[:, None, None])
+    S0 = state0[at].double() * live[:, None, None, None] * dA
+    S = S0 + x[..., None] * dt * by_head(Bm)
+    size = S0.abs() + xm[..., None] * dt * by_head(bm)
+    y = (S * by_head(Cm)).sum(-1) + x * D.double()[:, None]
+    y_size = (size * by_head(cm)).sum(-1) + xm * D.double().abs()[:, None]
+    # (the decay's exponent, of up to 4 |dt A| units, and a dozen products and functions of a few units each)
+    steps = 64 + 4 * float((dt * A.double()[:, None, None]).abs().max())
+    assert ((got[1][1][at].double() - S).abs() <= steps * ulp * size + 1e-30).all(), "states against 64 bits"
+    assert ((got[1][0].view(B, Hs, P).double() - y).abs() <= (N + steps) * ulp * y_size + 1e-30).all(), "y against 64 bits"
 
 
 def test_step_whose_waits_run_out_leaves_whole_states():
