@@ -19,10 +19,13 @@
 // Where the grid is small (CLUSTER_BLOCKS) the splits of a (row, key/value head), up to 8, are one thread-block cluster: each
 // block leaves its outputs and statistics in its own shared memory, the cluster meets at a barrier, and block r merges
 // its share of the outputs from all of them, read through distributed shared memory in the order of the splits.  Through
-// scratch and an arrival counter the merge is five trips to memory one after the other: one sequence of 128 tokens, a
-// step of the 1.5B sizes 1036 us, as a cluster 924.  More blocks go through scratch: a cluster's blocks start together and stay
-// until the last has read, and beside another mixer's kernel that costs more than it saves (8 sequences, 128 blocks: a step
-// 1280 us through scratch, 1322 as clusters).
+// scratch and an arrival counter the merge is five trips to memory one after the other.  More blocks go through scratch: a
+// cluster's blocks start together and stay until the last has read, and beside another mixer's kernel that can cost more than
+// it saves.  A step of the 1.5B sizes (two key/value heads) through scratch and as clusters, microseconds: contexts of up to
+// 512 in 4 splits, 1 sequence (8 blocks) 1013 and 921, 2 (16) 1030 and 939, 3 (24) 1054 and 960, 4 (32) 1080 and 988, 8 (64)
+// 1171 and 1183; of up to 1,024 in 8 splits, 1 (16) 1016 and 925, 2 (32) 1033 and 946, 3 (48) 1060 and 973, 4 (64) 1086 and
+// 1047, 8 (128) 1252 and 1287.  The line at 32 blocks is below every size that loses; 48 blocks, and 64 in clusters of eight,
+// would gain too.
 //
 // Arrival counting: every block of a (row, kv head) adds one to arrivals[row * KV + kv head] with
 // atomicInc modulo the number of splits, so the counter is back at zero when the kernel ends and needs
@@ -436,7 +439,7 @@ attention_decode_fused_kernel(const float* __restrict__ qkv, int ld, int q_off, 
   attention_merge_splits<HD, FM_NT>(part_o, part_ml, out, reinterpret_cast<float*>(smraw), smem_floats, t, g, G, H, n_splits, out_ld, sink, sink_values, head_gate, gate_ld);
 }
 
-constexpr int CLUSTER_BLOCKS = 32;
+constexpr int CLUSTER_BLOCKS = 32;        // (both sides measured: see the head of this file)
 int g_fused_passes = 0;       // > 0: rounds a block takes, for tests (0: chosen from the grid)
 
 template <int HD, int CK, int STAGES, bool CLUSTER, typename... Args>

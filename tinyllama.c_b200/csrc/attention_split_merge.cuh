@@ -43,6 +43,7 @@ __device__ __forceinline__ void attention_merge_splits(const float* part_o, cons
     __syncthreads();
     // four outputs of a thread at a time, eight splits of each: 32 loads in flight, all unconditional (past the last split or
     // output they read the last one, with weight 0); one output after the other, 32 splits were 16 trips to memory in a row
+    // (a step of the 1.5B sizes after 3,700 tokens: one sequence 1108 -> 1090 us, two 1161 -> 1131, four 1186 -> 1160)
     constexpr int NI = 4, NS = 8;
     for (int base = tid; base < G * HD; base += NI * NT) {
       const float* po[NI];

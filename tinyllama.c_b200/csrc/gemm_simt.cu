@@ -2,10 +2,12 @@
 //
 // y[r] = sum_c W[r,c] x[c] with W stored [out, in] is the reference's matmul
 // (cpu_op.c:121-189 for one row, 253-328 for a batch).  These kernels are the true
-// 32-bit path (FFMA, 32-bit accumulation in k order, no tensor cores, no reduced
-// matrix mode) and the fall-back for bfloat16 shapes the tensor-core kernel refuses.
-// Two shapes: a 64x64 tile kernel for many rows and a warp-per-column kernel for the
-// few rows of a decode step, where the weight matrix is streamed once.
+// 32-bit path (FFMA, 32-bit accumulation, no tensor cores, no reduced matrix mode) and the
+// fall-back for bfloat16 shapes the tensor-core kernel refuses.
+// Two shapes: tiles for many rows, and a warp for one to four columns for the few rows of a
+// decode step, where the weight matrix is streamed once.  The order of a sum follows from the
+// kernel, and so from M, N and K: a lane's shares of K in order and then the lanes, K in order,
+// or K in four parts that are each in order and then added.
 #include "common.cuh"
 
 // ---- tiled kernel ---------------------------------------------------------------------
@@ -232,7 +234,10 @@ __device__ __forceinline__ void fma_pair(float2& d, float2 a, float2 b) {
 // Many rows: a tile of 64 rows x 16 CT columns, 128 threads with 8 x CT results each (CT 8 or 4); two K-steps of 16 in
 // shared memory, the next one in registers.  With KG = 4 four groups of 128 threads take a quarter of K each and the
 // first adds the others' sums to its own: outputs of few columns have too few tiles to keep an SM's schedulers busy.
-// 310 rows: 2048 -> 8192: 595 -> 311 us (33 TFLOP/s), 4096 -> 2048: 920 -> 270 us; 1,200 rows 1633 -> 878 and 1185 -> 626 us.
+// 310 rows: 2048 -> 8192: 595 -> 313 us (33 TFLOP/s), 4096 -> 2048: 920 -> 264 us; 1,200 rows 1633 -> 879 and 1185 -> 622 us.
+// What bounds them: 310 rows of 2048 -> 8192 are 320 blocks of four warps, 0.7 of what the SMs hold at three blocks each (143
+// registers), so that a scheduler has one or two warps and waits for the pipes' latency; with K in four parts the warps wait for
+// shared memory (stalls per issue: short scoreboard 3.8 of 9) in blocks of which an SM holds one.
 constexpr int FT_M = 64, FT_K = 16, FT_LD = 4;
 template <typename TO, int CT, int KG>
 __global__ void __launch_bounds__(128 * KG)
@@ -378,7 +383,10 @@ static int launch_simt_f32x4(const float* a, int lda, const float* w, int ldw, T
   static int sms = 0;
   if (sms == 0) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
   if (M > 16) {
-    // 128 columns a tile where that still makes two blocks an SM, else 64 columns and K in four parts
+    // 128 columns a tile where that still makes two blocks an SM, else 64 columns and K in four parts: 310 rows, 2048 -> 8192
+    // (320 tiles of 128 columns) 313 us, in the other form 339, 600 rows 501 and 605; 200 rows (256 tiles) 294 and 267, 310 rows
+    // of 4096 -> 2048 (80) 322 and 264.  From 17 rows on tiles: 17 rows of 2048 -> 8192 66 us, 32 rows 67, 64 rows 70; three or
+    // four launches of the other kernel would take 46 and 66 (of 4096 -> 2048: 125 and 127 us, 87 and 151).
     const unsigned my = (unsigned)((M + FT_M - 1) / FT_M);
     if ((long long)my * ((N + 127) / 128) >= 2 * sms)
       tlc_launch(gemm_tiled_f32x4_kernel<TO, 8, 1>, dim3((N + 127) / 128, my), dim3(128), ft_smem(8, 1), stream, a, lda, w, ldw, out, ldo, colscale,
@@ -392,7 +400,8 @@ static int launch_simt_f32x4(const float* a, int lda, const float* w, int ldw, T
     return 0;
   }
   // A warp's columns share its activations: a read of them costs as much as one of the weights, so up to 2 rows take two
-  // columns and more rows four, where that still makes two blocks an SM.
+  // columns and more rows four, where that still makes two blocks an SM.  9 to 16 rows are two launches, each of which reads the
+  // weights: 12 rows of 2048 -> 8240 40 us, of 4096 -> 2048 62 us; as tiles 66 and 126.
   auto blocks_of = [&](int cols) { return (unsigned)((N + 8 * cols - 1) / (8 * cols)); };
 #define TLC_SK4(MT_, C_, U_) tlc_launch(gemm_skinny_f32x4_kernel<TO, MT_, C_, U_>, dim3(blocks_of(C_)), dim3(256), 0, stream, a, lda, w, ldw, out, ldo, \
                                         colscale, colbias, accumulate, M, N, K, mb)

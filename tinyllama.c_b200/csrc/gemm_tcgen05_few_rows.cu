@@ -14,15 +14,16 @@
 // shared memory, the cluster meets at a barrier, and block r adds up its share of the rows of all blocks' sums,
 // read through distributed shared memory in the order of the ranks (so the result does not depend on
 // timing), applies the epilogue and stores: a warp a row, a lane four weight rows in 16-byte pieces (a thread a weight
-// row instead, with 4-byte reads: 64 x 2048 x 8240 12.6 us, so 10.6).  What the sums are added to is asked for while the
+// row instead, with 4-byte reads: 64 rows of 2048 -> 8240 11.5 us, so 10.8).  What the sums are added to is asked for while the
 // products run.  A second barrier keeps every block's shared memory alive until all have read it.  A block that has the
 // whole of K writes from tensor memory.  With SWIGLU the weight rows come in groups of 16 = 8 gate rows and their
 // 8 up rows, and the block writes silu(gate) * up ([M, N / 2]).
 //
 // What bounds it: the stream of the weights; a copy loop of the same boxes without products takes 26.7 us for 24576 x 3072
-// (151 MB), the product of 64 rows 34.9 (40.3 with four stages for every width and the 4-byte reads).  Where a block has few K-steps, the chain from the wait on the
-// kernel before to the last store (activations, products, the meeting of the sums: 3 to 4 us) counts as much as the
-// stream: 64 rows, 4096 -> 2048 8.2 us (9.7 before), of which the 17 MB are 2.6.
+// (151 MB), the product of 64 rows 28.7 (34.2 before the 16-byte reads and the unshared tiles' own way out).  Where a block has
+// few K-steps, the chain from the wait on the kernel before to the last store (activations, products, the meeting of the
+// sums: 3 to 4 us) counts as much as the stream: 64 rows of 4096 -> 2048 added to what is there 8.4 us (10.0), of which the
+// 17 MB are 2.6.
 //
 // Every mbarrier wait is bounded (codes 31-33 of the error word); a block whose wait ran out still goes to both
 // cluster barriers, so that no block of its cluster waits for it.
@@ -344,11 +345,15 @@ int launch_few(const CUtensorMap& mw, const CUtensorMap& mx, void* out, int ldo,
   return 0;
 }
 
-// Stages of a block's ring: as many as leave room for a second block on the SM (113 KB each).
+// Stages of a block's ring.  Two blocks fit on an SM up to 113 KB each, which five stages of 32 rows (102 KB) would still do; but
+// what runs beside a layer's products (attention, the scan of the other mixer) then finds no room there: a step of the 7B sizes
+// at batch 32 7.29 ms with four, 7.85 with five.  So 32, 64 and 128 rows stay below 98 KB (82, 98 and 98).  16 rows come from
+// vocabularies alone, beside which nothing runs: six (110 KB).
 constexpr int fr_stages(int NB) { return NB == 16 ? 6 : NB <= 64 ? 4 : 3; }
 
 // How many blocks share a tile's K-steps: as many (2, 4, 8) as bring the grid closest to two blocks an SM (what
-// fits beside one another) without passing it, each with at least 4 K-steps.
+// fits beside one another) without passing it, each with at least 4 K-steps.  (64 rows of 2048 -> 8240, 65 tiles, four blocks
+// each: 10.8 us.)
 int pick_split(int N, int K, int NB, int sms) {
   const int tiles = (N + WM - 1) / WM, num_k = (K + FBK - 1) / FBK;
   int split = 1;
@@ -379,11 +384,11 @@ int run_few(const void* a, int lda, const void* w, int ldw, void* out, int out_d
 // loop over operand sets larger than the L2):
 //   * from 17 rows on, an output that is wide enough, 32 tiles of 128 weight rows, 16 with more than 32 rows, and not more
 //     tiles than two an SM (96 rows, 3072 -> 130048: 141 with the tiles of the product for prompts, 149 here).  At 64 rows
-//     2048 -> 8240 10.6, 4096 -> 2048 8.2, 2560 -> 16384 with SwiGLU 20.7, 3072 -> 24576 34.9;
+//     2048 -> 8240 10.8, 4096 -> 2048 8.4, 2560 -> 16384 18.7, 3072 -> 24576 28.7;
 //   * up to 32 rows, a plain 32-bit output of 128 tiles or more, a vocabulary: there the weight-streaming mma.sync kernel
 //     re-reads the activations for every 16 columns, and its rounds of K (2,048; from 9 rows on 1,024) may end in a part
-//     of one (32 rows, 3072 -> 130048: 221 with that kernel, 126 here; 16 rows, 2560 -> 65536: 68 and 53; 8 rows, 3072 ->
-//     130048 141 and 120; 1 row 138 and 117).  Up to 4 rows with full rounds it is as quick (2048 -> 65536: 40.9 and 42.1)
+//     of one (32 rows, 3072 -> 130048: 240 with that kernel, 129 here; 16 rows, 2560 -> 65536: 67 and 53; 8 rows, 3072 ->
+//     130048 143 and 120; 1 row 125 and 117).  Up to 4 rows with full rounds it is as quick (2048 -> 65536: 40.9 and 42.1)
 //     and keeps them.
 // Narrower outputs of up to 32 rows would gain as well (32 rows, 12288 -> 3072: 31.6 and 15.9), but their sums would be made
 // in another order, and what a layer rounds to 16 bits after them would move the tokens that a model picks; a logit is

@@ -396,8 +396,10 @@ ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dt, con
   if (mode == SCAN_PLAIN) tlc_wait(xbc, dt, dA, y);
   // Shared staging: per row  B[N] | C[N] | x[rows_per_block] | dt | dA, the rows SCAN_TT at a time, in two buffers: the
   // copies of a batch, in pieces of 16 bytes where the rows are laid out in them, are on their way while the batch
-  // before it is worked on, so that a row costs its arithmetic and not a trip to memory (a loop over the rows, each with
-  // its own loads, made a row of a 23-token prompt take 2 us).
+  // before it is worked on, so that a row costs its arithmetic and not a trip to memory.  Eight rows at a time in one
+  // buffer, each row's loads in a loop of their own, before: 23 rows of the 1.5B sizes (48 heads of 64, 256 columns) 56.7 us,
+  // so 46.8; eight sequences of 10 rows 53.0 and 38.6, one of 32 77.3 and 64.1, a single row 5.3 and 4.8.  A prompt of 23
+  // tokens is bound by the host and takes what it took.  Seven blocks an SM (72 registers, no spills) as before.
   const int per_tok = 2 * N + rows_per_block + 4;            // (a multiple of 4 where N is one)
   const float Dh = Dskip[h];
   const bool quads = N % 4 == 0 && P % 4 == 0 && Cd % 4 == 0 && ((uintptr_t)xbc & 15) == 0;
@@ -665,13 +667,15 @@ extern "C" int tlc_ssm_scan_chunked(const float* xbc, const float* dt, const flo
 // stored windows of the channels that the block needs and the convolution's weights do not depend on the kernel before
 // this one and are asked for ahead of the wait on it; after it come the row's projection, the convolution of the
 // block's channels (B and C of the head's group, a thread four channels; x of its rows, the fifth warp), dt and the decay.
-// B and C are convolved by every block of the group: 512 channels of L2 reads beside up to 64 KB of state, instead of a
+// B and C are convolved by every block of the group: 512 channels of L2 reads beside 16 or 32 KB of state, instead of a
 // kernel of their own (2 to 5 us a layer) and a trip through memory.
 //
 // The windows of the x channels are the block's own to advance.  Those of B and C are read by all the blocks of (sequence,
 // group), so the mixer's next kernel advances them (tlc_gated_rmsnorm_step).
-// What bounds it: the state, read and written once.  A step of the 1.5B sizes at batch 64 (403 MB of states a layer) takes 2.97 ms, with the two
-// kernels 3.45; at batch 8 1.18 and 1.27; of the 3B sizes at batch 16 3.29 and 3.41; of the 7B sizes at batch 32 7.01 and 7.27.
+// What bounds it: at batch 64 of the 1.5B sizes the state, 201 MB of a layer read and 201 MB written in 63 us (6.4 TB/s, the
+// copy bandwidth measured here is 6.5); at batch 8 (25 + 25 MB in 13 us) the trip to memory and back of 1.5 waves of blocks.
+// A step of the 1.5B sizes at batch 64 takes 2.97 ms, with the two kernels 3.45; at batch 8 and contexts of up to 512 1.18 and
+// 1.27; of the 3B sizes at batch 16 3.29 and 3.41; of the 7B sizes at batch 32 7.01 and 7.27.
 template <int NPL, int ROWS>
 struct StepSmem {
   static constexpr int STATE = ROWS * 32 * NPL * 4;                       // at most
@@ -821,8 +825,11 @@ mamba_step_kernel(const float* __restrict__ proj, int ld, int xbc_off, int dt_of
 
 constexpr int STEP_BLOCKS = 4096;
 
-// Whether mamba_step_kernel takes these sizes: 65..256 state columns and the other sizes in pieces of 16 bytes (smaller
-// states leave lanes idle: they keep the two kernels), 2 to 4 taps, on the device that the library is set up on.
+// Whether mamba_step_kernel takes these sizes: 65..256 state columns and the other sizes in pieces of 16 bytes, 2 to 4 taps, on the
+// device that the library is set up on.  Smaller states keep the two kernels, although measured the one would be about as
+// quick or quicker there too (with the norm behind them, 48 heads of 64: 64 columns, batch 1 / 8 / 64 5.6 / 9.2 / 36.9 us with
+// the two, 4.5 / 9.0 / 30.3 with the one; 16 columns 5.3 / 8.4 / 31.1 and 4.4 / 8.5 / 27.0); at 128 columns 6.2 / 11.2 / 49.3
+// and 4.6 / 10.4 / 39.5, at 256 7.7 / 16.7 / 77.1 and 5.2 / 13.5 / 70.3.
 extern "C" int tlc_mamba_step_ok(int Hs, int P, int N, int G, int Cd, int K) {
   return N > 64 && N <= 256 && N % 4 == 0 && P % 4 == 0 && Cd % 4 == 0 && K >= 2 && K <= 4 && G > 0 && Hs % G == 0 && Hs <= 65535 && Hs * P + 2 * G * N == Cd && tlc_error_words_here() != nullptr;
 }

@@ -354,8 +354,12 @@ ssd_walk_tc_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_const
 // From a zero state a chunk leaves S^T = B^T (w x) and adds nothing to the outputs: no C, no copy of the state, no
 // accumulator of outputs, and no chunk before it to wait for.  So it needs 80 KB of shared memory instead of the walk's
 // 211, and two blocks share an SM, each with a head's 64 (or 32) rows p.  The products are the walk's, in its order, on an
-// accumulator that starts at zero: the same bits.  What bounds it: the states that it writes.  64 prompts of 16 to 128
-// tokens (1.5B sizes, 201 MB of states a layer): 18.76 -> 16.97 ms; 32 prompts of 24 to 100 (7B) 30.8 -> 29.2 (with twelve and ten steps after them: 57.6 -> 55.6, 101.9 -> 101.0).
+// accumulator that starts at zero: the same bits.  64 prompts of 16 to 128 tokens (1.5B sizes): 18.76 -> 16.97 ms; 32 prompts of
+// 24 to 100 (7B) 30.8 -> 29.2 (with twelve and ten steps after them: 57.6 -> 55.6, 101.9 -> 101.0).
+// What bounds it: a block's chain, not the 201 MB of states that the 64 prompts leave a layer (96 us under the profiler, 2.7
+// TB/s of memory traffic, a third of the peak): loads of w and x, (w x)^T into shared memory in 2-byte stores, B^T, the
+// products, tensor memory, 4-byte stores of the state, with two blocks an SM to overlap them (stalls per issue: 13 cycles of 23
+// on global loads, 4 on the queue of the stores).
 template <int NTILES, int PF>
 struct FirstSmem {
   static constexpr int N = 128 * NTILES;

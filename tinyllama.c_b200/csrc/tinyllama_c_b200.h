@@ -54,7 +54,9 @@ int tlc_linear_init(void);
 int tlc_attention_prefill_init(void);
 int tlc_ssd_init(void);
 /* Error word of kernels whose waits are bounded: 0, or the code of the wait that ran out (1 loader,
- * 2 issuer, 3 epilogue, 4 drain, 5 accumulator of the tcgen05 product; 9 the self-test).  Reading does
+ * 2 issuer, 3 epilogue, 4 drain, 5 accumulator of the tcgen05 product; 9 the self-test; 11-14 the walk of the scan
+ * of prompts, 15 operands and 16 products of its first chunks; 21-29 attention of prompts; 31 loader, 32 issuer, 33
+ * epilogue, 34 drain of the product of few rows; 41 the state of a one-token Mamba2 step).  Reading does
  * not synchronise; clear sets it back to 0. */
 int tlc_linear_error(void);
 void tlc_linear_error_clear(void);

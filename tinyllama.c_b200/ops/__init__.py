@@ -616,7 +616,9 @@ def check_errors() -> None:
     if code:
         library().tlc_linear_error_clear()
         raise KernelError(f"a kernel gave up on a bounded wait (code {code}: 1 loader, 2 issuer, 3 epilogue, 4 drain, "
-                          f"5 accumulator of the tensor-core product; 9 the self-test); its output is incomplete")
+                          f"5 accumulator of the tensor-core product; 9 the self-test; 11-16 the scan of prompts; 21-29 "
+                          f"attention of prompts; 31-34 the product of few rows; 41 the state of a one-token Mamba2 step); "
+                          f"its output is incomplete")
 
 
 def wait_limit_cycles(cycles: int) -> None:
