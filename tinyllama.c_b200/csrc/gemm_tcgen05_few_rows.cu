@@ -384,7 +384,7 @@ int run_few(const void* a, int lda, const void* w, int ldw, void* out, int out_d
 // loop over operand sets larger than the L2):
 //   * from 17 rows on, an output that is wide enough, 32 tiles of 128 weight rows, 16 with more than 32 rows, and not more
 //     tiles than two an SM (96 rows, 3072 -> 130048: 141 with the tiles of the product for prompts, 149 here).  At 64 rows
-//     2048 -> 8240 10.8, 4096 -> 2048 8.4, 2560 -> 16384 18.7, 3072 -> 24576 28.7;
+//     2048 -> 8240 10.8, 4096 -> 2048 8.4, 2560 -> 16384 18.7 (with SwiGLU 20.7), 3072 -> 24576 28.7 (34.9);
 //   * up to 32 rows, a plain 32-bit output of 128 tiles or more, a vocabulary: there the weight-streaming mma.sync kernel
 //     re-reads the activations for every 16 columns, and its rounds of K (2,048; from 9 rows on 1,024) may end in a part
 //     of one (32 rows, 3072 -> 130048: 240 with that kernel, 129 here; 16 rows, 2560 -> 65536: 67 and 53; 8 rows, 3072 ->
