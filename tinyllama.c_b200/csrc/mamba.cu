@@ -334,11 +334,14 @@ extern "C" int tlc_mamba_conv(const void* proj, int dtype, int ld, int xbc_off, 
 __device__ __forceinline__ void scan_copy16(float* dst, const float* src, bool on) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(on ? 16 : 0) : "memory");   // (0: zeros)
 }
-__device__ __forceinline__ void scan_copy4(float* dst, const float* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+__device__ __forceinline__ void scan_copy4(float* dst, const float* src, bool on = true) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(on ? 4 : 0) : "memory");
 }
+// Blocks an SM: the registers that the state needs leave room for these, and what the compiler takes beyond them costs more than it
+// gives (seven for every size: 64 sequences of one row, 48 heads of 64, 32 columns 26.7 us and not 24.1, 64 columns 31.5 and
+// 28.2; a prompt of 1,500 rows in chunks, 128 columns 659 and 523, 130 columns 1215 and 878).
 template <int NPL, int RP, bool VEC>
-__global__ void __launch_bounds__(128, 7)
+__global__ void __launch_bounds__(128, NPL == 1 ? 11 : NPL == 2 ? 9 : NPL == 4 ? 8 : VEC ? 7 : 6)
 ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dt, const float* __restrict__ dA,
                 const float* __restrict__ Dskip, float* __restrict__ state, float* __restrict__ chunk_state,
                 const int* __restrict__ seg_start, const int* __restrict__ seg_seq,
@@ -398,8 +401,9 @@ ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dt, con
   // copies of a batch, in pieces of 16 bytes where the rows are laid out in them, are on their way while the batch
   // before it is worked on, so that a row costs its arithmetic and not a trip to memory.  Eight rows at a time in one
   // buffer, each row's loads in a loop of their own, before: 23 rows of the 1.5B sizes (48 heads of 64, 256 columns) 56.7 us,
-  // so 46.8; eight sequences of 10 rows 53.0 and 38.6, one of 32 77.3 and 64.1, a single row 5.3 and 4.8.  A prompt of 23
-  // tokens is bound by the host and takes what it took.  Seven blocks an SM (72 registers, no spills) as before.
+  // so 46.8; eight sequences of 10 rows 53.0 and 38.5, one of 32 77.3 and 64.1, a single row 5.3 and 4.7; rows that are not in
+  // pieces of 16 bytes (130 columns) 34.0 and 29.0, 36.4 and 34.6.  A prompt of 23 tokens is bound by the host and takes what
+  // it took.
   const int per_tok = 2 * N + rows_per_block + 4;            // (a multiple of 4 where N is one)
   const float Dh = Dskip[h];
   const bool quads = N % 4 == 0 && P % 4 == 0 && Cd % 4 == 0 && ((uintptr_t)xbc & 15) == 0;
@@ -419,15 +423,20 @@ ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dt, con
         scan_copy16(buf + (size_t)k * per_tok + 4 * q, src, on);
       }
     } else {
-#pragma unroll 4
-      for (int idx = threadIdx.x; idx < nt * (per_tok - 4); idx += 128) {
-        const int k = idx / (per_tok - 4), e = idx - k * (per_tok - 4);
+#pragma unroll 1
+      for (int k = 0; k < nt; k++) {
         const float* row = xbc + (size_t)(t0 + tt0 + k) * Cd;
-        float v = 0.f;
-        if (e < N) v = row[Di + (size_t)g * N + e];
-        else if (e < 2 * N) { if (want_y) v = row[Di + (size_t)G * N + (size_t)g * N + (e - N)]; }
-        else if (p_blk + e - 2 * N < P) v = row[(size_t)h * P + p_blk + (e - 2 * N)];
-        buf[(size_t)k * per_tok + e] = v;
+        const float* Bg = row + Di + (size_t)g * N;
+        float* dst = buf + (size_t)k * per_tok;
+#pragma unroll 1
+        for (int e = threadIdx.x; e < N; e += 128) {
+          scan_copy4(dst + e, Bg + e);
+          scan_copy4(dst + N + e, Bg + (size_t)G * N + e, want_y);
+        }
+        if (threadIdx.x < rows_per_block) {
+          const bool on = p_blk + threadIdx.x < P;
+          scan_copy4(dst + 2 * N + threadIdx.x, on ? row + (size_t)h * P + p_blk + threadIdx.x : row, on);
+        }
       }
     }
     if (threadIdx.x < 2 * SCAN_TT && (threadIdx.x >> 1) < nt)
