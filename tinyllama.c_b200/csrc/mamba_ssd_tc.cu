@@ -545,8 +545,12 @@ int tlc_ssd_tc_run(const __nv_bfloat16* xbc, const float* row_w, const float* ro
   CUtensorMap mc, mbt;
   if (int rc = tlc_tensor_map_bf16(xbc, T, Cd, Cd, 64, Q, &mc)) return rc;
   if (int rc = tlc_tensor_map_bf16(bt, (long long)n_seg * G * N, Q, Q, 64, N, &mbt)) return rc;
-  // first chunks apart where most sequences have no second one (eight prompts of four chunks: as long either way)
-  const bool fresh = g_first_chunks != 1 && (n_seg < 2 * B || g_first_chunks == 2);
+  // First chunks apart where most sequences have no second one (eight prompts of four chunks: as long either way), in blocks of
+  // 32 rows, which gain less, two in three (64 heads of 32, the whole scan, apart and in the walk: prompts of 100, 300, 90 and 60
+  // tokens, 6 chunks of 4 sequences, 32.1 us and 30.8; 30 of 60 and one of 900, 38 of 31, 81.6 and 91.9; 8 of 100 28.5 and 32.9.
+  // 24 heads of 128: 39.2 and 39.4, 107.7 and 140.8, 33.7 and 45.7).
+  const bool few_more = P % 64 == 0 ? n_seg < 2 * B : 2 * n_seg < 3 * B;
+  const bool fresh = g_first_chunks != 1 && (few_more || g_first_chunks == 2);
   if (N == 128) return launch<1>(mc, mbt, xbc, row_w, row_e, seg_decay, state, seg_start, seq_seg_start, slots, start_pos, y, add_to_y, B, Hs, P, G, Cd, fresh, stream);
   return launch<2>(mc, mbt, xbc, row_w, row_e, seg_decay, state, seg_start, seq_seg_start, slots, start_pos, y, add_to_y, B, Hs, P, G, Cd, fresh, stream);
 }
