@@ -1,0 +1,128 @@
+"""Layers whose calls are made again from the first one's (models/repeat.py)."""
+import ctypes
+import random
+
+import pytest
+import torch
+
+import tinyllama_c_b200 as tlc
+from tinyllama_c_b200 import ops
+from tinyllama_c_b200.config import config_from_dict
+from tinyllama_c_b200.engine import StepEntry
+from tinyllama_c_b200.models.repeat import RepeatedLayers
+from tinyllama_c_b200.weights import build_model
+
+import configs
+
+# the kernels of long prompts, of short ones and the general ones; more than two layers
+SIZES = {"tensor cores": dict(configs.TINY_D, num_hidden_layers=4, mamba_d_head=64, mamba_d_ssm=128, mamba_d_state=128),
+         "odd": dict(configs.TINY_C, num_hidden_layers=3), "small": dict(configs.TINY_A, num_hidden_layers=5)}
+
+
+def _model(name, dtype, device):
+    model = build_model(config_from_dict(dict(SIZES[name])))
+    g = torch.Generator().manual_seed(3)
+    tensors = {}
+    for s in model.weight_specs():
+        t = torch.randn(s.shape, generator=g) * 0.2
+        tensors[s.name] = 1.0 + t if s.init == "ones" else t.abs() if s.init == "a_log" else t
+        if s.init == "normal":
+            tensors[s.name] = tensors[s.name].bfloat16()
+    model.bind({k: v.to(device) for k, v in tensors.items()}, dtype, torch.device(device))
+    return model
+
+
+@pytest.mark.parametrize("name", list(SIZES))
+def test_like_layers_are_found_and_an_edit_is_noticed(name):
+    model = _model(name, torch.bfloat16, "cpu")
+    found = RepeatedLayers.of(model.layers, model.schedule)
+    assert found is not None and found.stands() and len(found.layers) == SIZES[name]["num_hidden_layers"]
+    assert len({len(t) for t in found.tensors}) == 1
+    # one layer's constant, one layer's weight type, one layer's shape: each makes the layers unlike
+    last = model.layers[-1]
+    for part, attribute, value in ((last.mixers[1], "eps", 0.5), (last.ffn.down, "weight", last.ffn.down.weight.float()),
+                                   (last.mixer_norm, "weight", last.mixer_norm.weight[:-4]), (last.mixers[0], "window", 7)):
+        before = getattr(part, attribute)
+        setattr(part, attribute, value)
+        assert not found.stands() and RepeatedLayers.of(model.layers, model.schedule) is None, attribute
+        setattr(part, attribute, before)
+        found = RepeatedLayers.of(model.layers, model.schedule)
+        assert found is not None and found.stands()
+
+
+def test_parts_that_say_nothing_are_not_repeated():
+    model = _model("small", torch.float32, "cpu")
+
+    class Own(type(model.layers[1].ffn)):
+        pass
+
+    model.layers[1].ffn.__class__ = Own
+    assert RepeatedLayers.of(model.layers, model.schedule) is None
+
+
+def test_the_table_of_calls_is_checked_before_the_first_call():
+    lib = ops.library()
+    assert lib.tlc_replay_index(b"tlc_linear") >= 0 and lib.tlc_replay_index(b"tlc_argmax") == -1
+    words = (ctypes.c_ulonglong * 4)()
+    for functions, n_words in (([lib.tlc_replay_index(b"tlc_event_record")], 4), ([99], 4), ([-1], 0)):
+        fns = (ctypes.c_int * len(functions))(*functions)
+        assert lib.tlc_replay(fns, words, n_words, len(functions), 1) < 0 and b"replay" in lib.tlc_last_error()
+    assert lib.tlc_replay(None, None, 0, 0, 3) == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("name", list(SIZES))
+def test_repeated_layers_give_the_same_bits_as_layers_one_by_one(name, dtype):
+    """Prompts in batches (row by row, in chunks, longer than a chunk), a further turn, single tokens without a captured
+    step: logits and the whole cache, on the default stream and on another."""
+    model = _model(name, getattr(torch, dtype), "cuda:0")
+    assert model.repeated is not None
+    V, r = SIZES[name]["vocab_size"], random.Random(5)
+    ids = lambda n: [r.randrange(V) for _ in range(n)]  # noqa: E731
+    steps = [[ids(n) for n in lens] for lens in ((5, 1, 3), (40, 150, 20), (1, 1, 1), (33, 1, 260))]
+    got, calls = [], []
+    for repeated in (model.repeated, None):
+        for stream in (torch.cuda.current_stream(), torch.cuda.Stream()):
+            model.repeated = repeated
+            llm = tlc.LLM(model, dtype=dtype, max_tokens=64 * 32, max_seqs=3)
+            slots = [llm.cache.acquire() for _ in range(3)]
+            before = ops.launch_count()
+            torch.cuda.synchronize()
+            with torch.cuda.stream(stream):
+                out = [llm.step([StepEntry(s, t, (len(t) - 1,)) for s, t in zip(slots, step)]) for step in steps]
+            torch.cuda.synchronize()
+            calls.append(ops.launch_count() - before)
+            got.append([t.clone() for t in out] + [g.k.clone() for g in llm.cache.kv_groups] + [g.v.clone() for g in llm.cache.kv_groups]
+                       + [g.data.clone() for g in llm.cache.state_groups])
+    assert len(set(calls)) == 1
+    for other in got[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(got[0], other))
+
+
+@pytest.mark.gpu
+def test_every_layer_of_a_repeated_step_goes_through_the_library_once():
+    """The first layer's calls through Python, the others' from the table; tensors that change their place between steps are
+    found again."""
+    model = _model("tensor cores", torch.bfloat16, "cuda:0")
+    llm = tlc.LLM(model, dtype="bfloat16", max_tokens=64 * 8, max_seqs=2)
+    table, times = ops.replay, []
+    ops.replay = lambda functions, words, n: (times.append(n), table(functions, words, n))
+    try:
+        tokens = list(range(1, 60))
+
+        def logits():
+            slot = llm.cache.acquire()
+            out = llm.step([StepEntry(slot, tokens, (58,))]).clone()
+            llm.cache.release(slot)
+            return out
+
+        first = logits()
+        assert times == [3]
+        w = model.layers[2].ffn.down
+        w.weight = w.weight.clone()                     # an edit: found alike again, at the new place
+        assert torch.equal(first, logits()) and times == [3, 3]
+        w.weight = w.weight.t().contiguous().t()        # other strides in one layer: one by one
+        assert torch.equal(first, logits()) and times == [3, 3]
+    finally:
+        ops.replay = table

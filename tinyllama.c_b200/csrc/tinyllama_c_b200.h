@@ -47,6 +47,15 @@ const char* tlc_last_error(void);
  * predecessor drains); 0: plain stream order.  The embedding kernel never carries it: it is the boundary
  * between steps (see tlc_embed). */
 void tlc_set_pdl(int on);
+/* Calls made again from a table: `times` rounds of n_calls calls, the functions of a round by their index
+ * (tlc_replay_index: -1 for a function that is not among those that can be) and the arguments of all rounds one after the other
+ * as 64-bit words (pointers and integers by value, floats by their bits; n_words in all; both arrays host).  Stops at the
+ * first call that fails and returns its code. */
+int tlc_replay_index(const char* name);
+int tlc_replay(const int* functions, const unsigned long long* words, long long n_words, int n_calls, int times);
+/* An event (cudaEvent_t) recorded on a stream; a stream that waits for one. */
+int tlc_event_record(void* event, cudaStream_t stream);
+int tlc_event_wait(void* event, cudaStream_t stream);
 /* Set-up of the tensor-core products, of prompt attention and of the chunked scan (shared-memory
  * attributes, the driver's tensor-map encoder, the error words, scratch).  Once per process, before any
  * stream capture. */

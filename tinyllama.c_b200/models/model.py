@@ -18,6 +18,7 @@ from ..parts.base import (ChunkRequest, KVRequest, LayerCache, LayerRun, LayerSp
 from ..parts.block import Block
 from ..parts.feed_forward import MoEFeedForward
 from ..parts.linear import StackedLinear, matrix_dtype
+from .repeat import RepeatedLayers
 
 
 class Model:
@@ -73,6 +74,7 @@ class Model:
         self.by_table: List[MoEFeedForward] = []
         self.dtype: Optional[torch.dtype] = None
         self.device: Optional[torch.device] = None
+        self.repeated: Optional[RepeatedLayers] = None      # the run order's layers, where they are all alike
 
     # ---- declarations ----------------------------------------------------------------------
     def weight_specs(self) -> List[WeightSpec]:
@@ -124,6 +126,7 @@ class Model:
             self.head.bind({self.embed_name: self.embed_table}, dtype, device)     # shares the table's storage
         else:
             self.head.bind(tensors, dtype, device)
+        self.repeated = RepeatedLayers.of(self.layers, self.schedule) if self.device.type == "cuda" else None
 
     # ---- forward ------------------------------------------------------------------------------
     def forward(self, step: StepInfo, cache, want_rows: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
@@ -138,8 +141,14 @@ class Model:
         if self.by_table:                              # experts that token ids choose: all layers' routing at once
             MoEFeedForward.route_step(self.by_table, self.expert_tables, step)
         with step_scratch(step):                       # the layers share the step's temporaries
-            ready = False                              # whether a layer left the next one's input (Block.entry)
-            for r, run in enumerate(self.schedule):
+            ready, done = False, 0                     # whether a layer left the next one's input (Block.entry)
+            if self.repeated is not None and not torch.cuda.is_current_stream_capturing():
+                if not self.repeated.stands():
+                    self.repeated = RepeatedLayers.of(self.layers, self.schedule)
+                if self.repeated is not None:
+                    done, ready = self.repeated.run(x, step, cache)
+            for r in range(done, len(self.schedule)):
+                run = self.schedule[r]
                 if run.add is not None:            # a learned row joins the stream before this entry (a pass of a repeated range)
                     ops.add_row(x, self.rows_of[run.add[0]][run.add[1]])
                     ready = False

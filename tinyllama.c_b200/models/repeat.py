@@ -1,0 +1,157 @@
+"""The calls of one layer made again for the layers that are like it.
+
+CodeClaper/tinyllama.c walks a static list of nodes for every step (graph.c:1278-1302).  Here a layer's forward() is
+Python that checks its operands and makes a dozen calls of the kernel library, and for prompts of up to a few hundred
+tokens that is slower than the kernels: 24 layers of the 1.5B sizes took the host 4 ms, 13 us a call, where the GPU
+needs 1 to 2.5.  Where all layers of the run order are alike (the same parts of the same sizes and constants, tensors of the same
+types, shapes and strides), the first one runs as ever and its calls are noted; the others' are the same calls with their
+own weights and their own part of the cache in place of the first one's, and are made by the library in one go.
+
+Nothing is kept from one step for the next but the description of the layers, which an edit of any of their parts makes
+void; the tensors' addresses, types, shapes and strides are read in every step.  A pointer that is neither one of the
+first layer's tensors nor something that all layers share (the stream of rows, the step's tables and temporaries) ends the
+attempt: the layers then run one by one, as they do under capture, on other devices and with parts that do not
+say that they can be repeated.
+"""
+from __future__ import annotations
+
+from operator import attrgetter
+from typing import List, Optional, Tuple
+
+import numpy as np
+import torch
+
+from .. import ops
+from ..parts.base import Editable, LayerCache, StepInfo
+
+
+class _Unlike(Exception):
+    pass
+
+
+_PLAIN = (type(None), bool, int, float, str, torch.dtype, torch.device)
+_edits = attrgetter("edits")
+_ptr, _size, _stride, _dtype = torch.Tensor.data_ptr, torch.Tensor.size, torch.Tensor.stride, attrgetter("dtype")
+
+
+def _describe(obj, tensors: List[torch.Tensor], parts: List[Editable]):
+    """A value that is equal for two objects whose calls differ in their tensors' addresses alone; collects the tensors, in
+    the order in which they come up, and the parts whose edits would change it."""
+    if isinstance(obj, _PLAIN):
+        return type(obj), obj
+    if isinstance(obj, torch.Tensor):
+        tensors.append(obj)
+        return "tensor", obj.dtype, tuple(obj.shape), obj.stride(), obj.device
+    if isinstance(obj, (list, tuple)):
+        return type(obj), tuple(_describe(o, tensors, parts) for o in obj)
+    if isinstance(obj, dict):
+        return dict, tuple((k, _describe(v, tensors, parts)) for k, v in sorted(obj.items()))
+    if isinstance(obj, Editable):
+        aside = obj.repeats()
+        if aside is None or "repeats" not in type(obj).__dict__:      # (a class derived from such a part speaks for itself)
+            raise _Unlike
+        parts.append(obj)
+        return type(obj), tuple((k, _describe(v, tensors, parts)) for k, v in sorted(vars(obj).items())
+                                if k not in aside and k != "edits")
+    raise _Unlike
+
+
+def _of_cache(view: LayerCache) -> Tuple[tuple, List[torch.Tensor]]:
+    """(what must be equal, tensors) of a layer's part of the cache."""
+    tensors = []
+    for kv in view.kv.values():
+        tensors += [kv.k_pages, kv.block_table] if kv.v_pages is None else [kv.k_pages, kv.block_table, kv.v_pages]
+    tensors += view.state.values()
+    return (view.writes, view.kv_writes, [(k, kv.window, kv.v_pages is None) for k, kv in view.kv.items()], list(view.state)), tensors
+
+
+class RepeatedLayers:
+    """The layers of a run order that are alike."""
+
+    @staticmethod
+    def of(layers, schedule) -> Optional["RepeatedLayers"]:
+        """None where the run order is more than one pass of like layers, each with a cache of its own."""
+        if len(schedule) < 3 or any(r.cache is not None or r.kv_cache is not None or r.add is not None or r.add_embedding for r in schedule):
+            return None
+        self = RepeatedLayers()
+        self.layers = [layers[r.layer] for r in schedule]
+        self.tensors, self.parts, first = [], [], None
+        try:
+            for layer in self.layers:
+                mine: List[torch.Tensor] = []
+                form = _describe(layer, mine, self.parts)
+                if first is None:
+                    first = form
+                elif form != first:
+                    return None
+                self.tensors.append(mine)
+        except _Unlike:
+            return None
+        self.edits = list(map(_edits, self.parts))
+        return self
+
+    def run(self, x: torch.Tensor, step: StepInfo, cache) -> Tuple[int, bool]:
+        """Runs the first layer, and the others if they can be repeated; (how many entries of the run order have run,
+        whether the last of them has left the next one's input)."""
+        views = [cache.layer_view(r, True, None) for r in range(len(self.layers))]
+        with ops.noting() as notes:
+            left = self.layers[0].forward(x, step, views[0], False, self.layers[1].entry)
+        if left or not notes.complete:
+            return 1, left
+        form, mine = _of_cache(views[0])
+        firsts = self.tensors[0] + mine
+        at = {}                                            # address -> which of the first layer's tensors
+        addresses = list(map(_ptr, firsts))
+        for i, p in enumerate(addresses):
+            if p:
+                at.setdefault(p, i)
+        common = self._shared(x, step, notes)
+        shared = notes.handles.union((0,), map(_ptr, common))
+        ranges = None
+        places, which = [], []                             # words to replace, and by which tensor's address
+        for w, (word, pointer) in enumerate(zip(notes.words, notes.is_pointer)):
+            if not pointer or word in shared:
+                continue
+            i = at.get(word)
+            if i is not None:
+                places.append(w)
+                which.append(i)
+                continue
+            if ranges is None:
+                ranges = [(_ptr(t), _ptr(t) + t.untyped_storage().nbytes() - t.storage_offset() * t.element_size()) for t in common]
+            if not any(lo <= word < hi for lo, hi in ranges):
+                return 1, left
+        used = sorted(set(which))
+        rank = {i: n for n, i in enumerate(used)}
+        like = self._meta([firsts[i] for i in used])
+        table = np.empty((len(self.layers) - 1, len(used)), dtype=np.uint64)
+        for r in range(1, len(self.layers)):
+            other, theirs = _of_cache(views[r])
+            theirs = self.tensors[r] + theirs
+            row = [theirs[i] for i in used]
+            if other != form or self._meta(row) != like:
+                return 1, left
+            table[r - 1] = list(map(_ptr, row))
+        base = np.array([addresses[i] for i in used], dtype=np.uint64)
+        if ((table ^ base) & np.uint64(15)).any() or not table.all():
+            return 1, left                                 # (the calls may choose by how their operands are aligned)
+        words = np.tile(np.array(notes.words, dtype=np.uint64), (len(self.layers) - 1, 1))
+        words[:, places] = table[:, [rank[i] for i in which]]
+        ops.replay(np.array(notes.functions, dtype=np.int32), words, len(self.layers) - 1)
+        return len(self.layers), False
+
+    def stands(self) -> bool:
+        """Whether no part has been edited since the layers were found alike."""
+        return list(map(_edits, self.parts)) == self.edits
+
+    @staticmethod
+    def _meta(tensors):
+        return list(map(_size, tensors)), list(map(_stride, tensors)), list(map(_dtype, tensors))
+
+    @staticmethod
+    def _shared(x: torch.Tensor, step: StepInfo, notes) -> List[torch.Tensor]:
+        """What all layers of the step read or write alike."""
+        out = [x, step.tokens, step.positions, step.row_seq, step.cu_seqlens, step.slots, step.start_pos]
+        for table in step.chunks.values():
+            out += table or ()
+        return out + [t for t in list(step.scratch.values()) + notes.owned if isinstance(t, torch.Tensor)]

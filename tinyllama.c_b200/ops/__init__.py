@@ -10,6 +10,8 @@ from __future__ import annotations
 
 import ctypes
 import os
+import struct
+import threading
 from typing import Optional
 
 import torch
@@ -33,6 +35,10 @@ _vp, _i, _f, _ll = ctypes.c_void_p, ctypes.c_int, ctypes.c_float, ctypes.c_longl
 _SIGNATURES = {
     "tlc_last_error": (ctypes.c_char_p, []),
     "tlc_set_pdl": (None, [_i]),
+    "tlc_replay_index": (_i, [ctypes.c_char_p]),
+    "tlc_replay": (_i, [_vp, _vp, _ll, _i, _i]),
+    "tlc_event_record": (_i, [_vp, _vp]),
+    "tlc_event_wait": (_i, [_vp, _vp]),
     "tlc_linear_init": (_i, []),
     "tlc_attention_prefill_init": (_i, []),
     "tlc_ssd_init": (_i, []),
@@ -200,6 +206,114 @@ def _call(name: str, *args) -> None:
     rc = getattr(lib, name)(*args)
     if rc != 0:
         raise KernelError(f"{name}: {lib.tlc_last_error().decode()}")
+    notes = _notes.calls
+    if notes is not None:
+        notes.add(name, args)
+
+
+# ---- calls made again --------------------------------------------------------------------
+# A step makes the same calls for every layer of a model whose layers are alike, with other weights and another part of
+# the cache, and each takes a dozen microseconds on its way through the checks here.  Inside `noting()` the calls of this
+# thread are noted beside being made; replay() then makes them again, many rounds in one call of the library, with the
+# arguments that the caller has put in their places (models/repeat.py).
+class NotedCalls:
+    """Calls in the order they were made.  words: the arguments as 64-bit words; is_pointer marks those that are pointers.
+    owned: what the calls were given that no argument keeps alive (scratch, numbers on the host that a call writes).
+    handles: streams and events that the calls name.  complete: False once a call was made that cannot be made again."""
+
+    def __init__(self):
+        self.functions, self.words, self.is_pointer = [], [], []
+        self.owned, self.handles, self.complete = [], set(), True
+
+    def add(self, name: str, args) -> None:
+        index, kinds = _replayable(name)
+        if index < 0:
+            self.complete = False
+            return
+        self.functions.append(index)
+        for a, pointer in zip(args, kinds):
+            if pointer is None:                            # a float, by its bits
+                self.words.append(_F32_BITS.unpack(_F32_PACK.pack(a))[0])
+                self.is_pointer.append(False)
+                continue
+            if a is None:
+                a = 0
+            elif not isinstance(a, int):                   # ctypes.byref of a number on the host
+                a = a._obj
+                self.owned.append(a)
+                a = ctypes.addressof(a)
+                self.handles.add(a)
+            self.words.append(a & 0xFFFFFFFFFFFFFFFF)
+            self.is_pointer.append(pointer)
+        if name not in ("tlc_event_record", "tlc_event_wait"):
+            self.handles.add(args[-1])                     # the stream
+
+
+_F32_PACK, _F32_BITS = struct.Struct("<f"), struct.Struct("<I")
+
+
+class _Notes(threading.local):
+    calls: Optional[NotedCalls] = None
+
+
+_notes = _Notes()
+_replay_kinds: dict = {}
+
+
+def _replayable(name: str):
+    """(index of the function in the library's table, or -1; per argument: True a pointer, False an integer, None a float)."""
+    hit = _replay_kinds.get(name)
+    if hit is None:
+        kinds = tuple(None if t is _f else t is _vp for t in _SIGNATURES[name][1])
+        hit = _replay_kinds[name] = (library().tlc_replay_index(name.encode()), kinds)
+    return hit
+
+
+class noting:
+    """Context manager: notes the calls that this thread makes inside; a NotedCalls."""
+
+    def __enter__(self) -> NotedCalls:
+        self.before, _notes.calls = _notes.calls, NotedCalls()
+        return _notes.calls
+
+    def __exit__(self, *exc):
+        _notes.calls = self.before
+        return False
+
+
+def _note_owned(*tensors) -> None:
+    """Scratch of a call that is given back when the call has been made: kept while calls are being noted."""
+    if _notes.calls is not None:
+        _notes.calls.owned += [t for t in tensors if t is not None]
+
+
+def replay(functions, words, times: int) -> None:
+    """Makes the calls of `functions` (int32 array of indices) `times` times; words: the arguments of all rounds (uint64 array)."""
+    global _launches
+    lib = library()
+    rc = lib.tlc_replay(functions.ctypes.data, words.ctypes.data, words.size, functions.size, int(times))
+    if rc != 0:
+        raise KernelError(f"tlc_replay: {lib.tlc_last_error().decode()}")
+    _launches += int(times) * int((functions >= _event_functions()).sum())
+
+
+def _event_functions() -> int:
+    """The first entries of the library's table are the events, which launch nothing."""
+    return max(_replayable("tlc_event_record")[0], _replayable("tlc_event_wait")[0]) + 1
+
+
+def record_event(event: "torch.cuda.Event", stream: "torch.cuda.Stream") -> None:
+    event.record(stream)
+    if _notes.calls is not None:
+        _notes.calls.handles |= {event.cuda_event, stream.cuda_stream}
+        _notes.calls.add("tlc_event_record", (event.cuda_event, stream.cuda_stream))
+
+
+def wait_event(stream: "torch.cuda.Stream", event: "torch.cuda.Event") -> None:
+    stream.wait_event(event)
+    if _notes.calls is not None:
+        _notes.calls.handles |= {event.cuda_event, stream.cuda_stream}
+        _notes.calls.add("tlc_event_wait", (event.cuda_event, stream.cuda_stream))
 
 
 # The current stream's handle is asked for by every call; torch.cuda.current_stream() builds a Stream object each
@@ -598,16 +712,20 @@ def linear_swiglu(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, colscale:
     global _launches
     lib = library()
     _launches += 1
-    rc = lib.tlc_linear_swiglu(a.data_ptr(), dtype_code(a.dtype), _rows(a, "linear input"), w.data_ptr(), dtype_code(w.dtype),
-                               _rows(w, "linear weight"), out.data_ptr(), dtype_code(out.dtype), N // 2, _p(colscale),
-                               _p(colbias), M, N, K, TENSOR_CORE_MIN_ROWS, DENSE_ACTS[act], float(limit), float(alpha), _stream())
+    args = (a.data_ptr(), dtype_code(a.dtype), _rows(a, "linear input"), w.data_ptr(), dtype_code(w.dtype),
+            _rows(w, "linear weight"), out.data_ptr(), dtype_code(out.dtype), N // 2, _p(colscale),
+            _p(colbias), M, N, K, TENSOR_CORE_MIN_ROWS, DENSE_ACTS[act], float(limit), float(alpha), _stream())
+    rc = lib.tlc_linear_swiglu(*args)
     if rc == 1:                                   # no fused kernel for these operands
         _launches -= 1
         gu = torch.empty((M, N), dtype=torch.float32, device=a.device)
+        _note_owned(gu)
         linear(a, w, gu, colscale, colbias)
         glu(gu, out, act, interleaved=True, limit=limit, alpha=alpha)
     elif rc != 0:
         raise KernelError(f"tlc_linear_swiglu: {lib.tlc_last_error().decode()}")
+    elif _notes.calls is not None:
+        _notes.calls.add("tlc_linear_swiglu", args)
 
 
 def check_errors() -> None:
@@ -746,6 +864,7 @@ def attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, blo
         n_splits = (decode_max_keys + 127) // 128
         part_o = torch.empty((T, H, n_splits, hd), dtype=torch.float32, device=q.device)
         part_ml = torch.empty((T, H, n_splits, 2), dtype=torch.float32, device=q.device)
+        _note_owned(part_o, part_ml)
         _call("tlc_attention_decode", q.data_ptr(), dtype_code(q.dtype), k_pages.data_ptr(), v_pages.data_ptr(),
               block_table.data_ptr(), block_table.shape[1], positions.data_ptr(), row_seq.data_ptr(),
               slots.data_ptr(), out.data_ptr(), part_o.data_ptr(), part_ml.data_ptr(), T, H, KV, hd, float(scale),
@@ -765,6 +884,7 @@ def attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, blo
         if n_split > 1:
             part_o = torch.empty((T, H, n_split, hd), dtype=torch.float32, device=q.device)
             part_ml = torch.empty((T, H, n_split, 2), dtype=torch.float32, device=q.device)
+            _note_owned(part_o, part_ml)
         _call("tlc_attention_prefill_tc", q.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(), k_pages.shape[0],
               block_table.data_ptr(), block_table.shape[1], cu_seqlens.data_ptr(), slots.data_ptr(), start_pos.data_ptr(),
               out.data_ptr(), B, T // 128 + B, H, KV, hd, float(scale), int(window or 0), int(max_keys), T,
@@ -781,6 +901,7 @@ def attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, blo
         if n_chunks > 1:
             part_o = torch.empty((T, H, n_chunks, hd), dtype=torch.float32, device=q.device)
             part_ml = torch.empty((T, H, n_chunks, 2), dtype=torch.float32, device=q.device)
+            _note_owned(part_o, part_ml)
         _call("tlc_attention_prefill", q.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(), block_table.data_ptr(),
               block_table.shape[1], cu_seqlens.data_ptr(), slots.data_ptr(), start_pos.data_ptr(), out.data_ptr(), B,
               n_tiles, H, KV, hd, float(scale), int(window or 0), (int(max_keys) + 63) // 64 if n_chunks > 1 else 0,
@@ -845,6 +966,7 @@ def attention_decode_fused(qkv: torch.Tensor, q_off: int, k_off: int, v_off: int
     n_splits = (max_keys + 127) // 128
     part_o = torch.empty((T, H, n_splits, hd), dtype=torch.float32, device=qkv.device)
     part_ml = torch.empty((T, H, n_splits, 2), dtype=torch.float32, device=qkv.device)
+    _note_owned(part_o, part_ml)
     _gpu(arrivals)
     _i32(arrivals, "arrival counters")
     if arrivals.numel() < T * KV:
@@ -1020,16 +1142,20 @@ def ssm_scan(xbc: torch.Tensor, dt: torch.Tensor, dA: torch.Tensor, Dskip: torch
         if matrix_form:
             _f32vec(A, Hs, "A")
             scratch = torch.empty(lib.tlc_ssd_scratch_floats(n_seg, T, Hs, P, N, G), dtype=torch.float32, device=xbc.device)
+            _note_owned(scratch)
             if y_part is not None and (y_part.dtype != torch.float32 or not y_part.is_contiguous() or y_part.shape != y.shape):
                 raise KernelError("ssm_scan: y_part must be contiguous float32 of y's shape")
             used = ctypes.c_int(0)
             aux = _aux_stream(xbc.device).cuda_stream if y_part is not None and not torch.cuda.is_current_stream_capturing() else None
+            if aux is not None and _notes.calls is not None:
+                _notes.calls.handles.add(aux)
             _call("tlc_ssm_scan_ssd", xbc.data_ptr(), dt.data_ptr(), A.data_ptr(), Dskip.data_ptr(), state.data_ptr(),
                   scratch.data_ptr(), seg_start.data_ptr(), seg_seq.data_ptr(), seq_seg_start.data_ptr(),
                   slots.data_ptr(), start_pos.data_ptr(), y.data_ptr(), _p(y_part), ctypes.byref(used), slots.numel(), n_seg,
                   T, Hs, P, N, G, Cd, _stream(), aux)
             return bool(used.value)
         scratch = torch.empty(n_seg * Hs * (P * N + 1), dtype=torch.float32, device=xbc.device)
+        _note_owned(scratch)
         _call("tlc_ssm_scan_chunked", xbc.data_ptr(), dt.data_ptr(), dA.data_ptr(), Dskip.data_ptr(), state.data_ptr(),
               scratch.data_ptr(), seg_start.data_ptr(), seg_seq.data_ptr(), seq_seg_start.data_ptr(), slots.data_ptr(),
               start_pos.data_ptr(), y.data_ptr(), slots.numel(), n_seg, Hs, P, N, G, Cd, _stream())

@@ -124,7 +124,23 @@ class LayerCache:
     kv_writes: bool = True   # False: the keys/values here are another entry's (LayerRun.kv_cache); the state is this entry's own
 
 
-class Part:
+class Editable:
+    """Counts how often its attributes are set, so that what was found out about it (models/repeat.py) can be dropped."""
+    edits = 0
+    passing = frozenset()        # attributes that a forward() sets for itself
+
+    def __setattr__(self, name, value):
+        object.__setattr__(self, name, value)
+        if name not in self.passing:
+            object.__setattr__(self, "edits", self.edits + 1)
+
+    def repeats(self) -> Optional[frozenset]:
+        """For a part whose forward() makes the same calls of the kernel library (and no other GPU work) whatever it is
+        named: the attributes that make no difference to them.  None: unknown.  A class that says so defines it itself."""
+        return None
+
+
+class Part(Editable):
     """Base of norms, position encodings, mixers and feed-forwards."""
 
     def weight_specs(self) -> List[WeightSpec]:

@@ -15,6 +15,7 @@ from typing import Dict, List, Optional
 
 import torch
 
+from .. import ops
 from .base import LayerCache, LayerSpec, Part, StepInfo, WeightSpec, current_stream, scratch_buf, scratch_is_shared
 from .linear import StackedLinear
 from .norm import RMSNorm
@@ -50,6 +51,13 @@ PARALLEL_FFN_PROMPTS = bool(int(os.environ.get("TLC_PARALLEL_FFN_PROMPTS", "0"))
 
 
 class Block(Part):
+    passing = frozenset(("_copied", "_side", "_fork", "_done", "_ffn_side", "_ffn_fork", "_ffn_done"))
+
+    def repeats(self):
+        """A plain layer: norm, mixers whose results are added into the stream, norm, feed-forward."""
+        plain = self.mixer_join is None and self.mixer_out_norm is None and self.ffn_out_norm is None and not self.parallel_ffn
+        return self.passing | {"spec"} if plain else None
+
     def __init__(self, spec: LayerSpec, act_dtype_of=None):
         self.spec = spec
         self.mixer_norm = spec.mixer_norm.build()
@@ -138,7 +146,7 @@ class Block(Part):
         lengths = [int(getattr(m, "single_token_launches", 1)) for m in self.mixers]
         here = _MAIN_MIXER if _MAIN_MIXER is not None else lengths.index(max(lengths))
         fork = self._fork
-        fork.record(main)
+        ops.record_event(fork, main)
         acts, done = [None] * len(self.mixers), [None] * len(self.mixers)
         joint, views = self._joint_activations(x32)
         sides = iter(self._side)
@@ -146,13 +154,13 @@ class Block(Part):
             if i == here:
                 continue
             side = next(sides)
-            side.wait_event(fork)
+            ops.wait_event(side, fork)
             torch.cuda.set_stream(side)              # (the context manager asks for the current stream again: 10 us)
             try:
                 bound = PROMPT_SIDE_BLOCKS if step.max_new > 1 and getattr(m, "mix_takes_max_blocks", False) else 0
                 acts[i] = self._mix(i, part, step, cache, views[i], max_blocks=bound)
                 done[i] = self._done[i]
-                done[i].record(side)
+                ops.record_event(done[i], side)
             finally:
                 torch.cuda.set_stream(main)
         # The wait for the side streams breaks the chain of programmatic launches on this stream.  A mixer that
@@ -164,7 +172,7 @@ class Block(Part):
                 joined.append(True)
                 for ev in done:
                     if ev is not None:
-                        main.wait_event(ev)
+                        ops.wait_event(main, ev)
 
         early = getattr(self.mixers[here], "mix_takes_join", False)
         acts[here] = self._mix(here, parts[here], step, cache, views[here], join if early else None)

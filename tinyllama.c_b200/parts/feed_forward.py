@@ -66,6 +66,9 @@ class SwiGLU(Part):
             if self.gate_up.colbias is not None:
                 self.gate_up.colbias = self.gate_up.colbias[idx].contiguous()
 
+    def repeats(self):
+        return frozenset()
+
     def forward(self, normed: torch.Tensor, residual: torch.Tensor, accumulate: bool = True) -> None:
         """Adds the result into `residual` (float32 [T, D]), or overwrites it with accumulate False."""
         T = normed.shape[0]

@@ -15,7 +15,7 @@ from typing import Dict, List, Optional, Sequence
 import torch
 
 from .. import ops
-from .base import WeightSpec
+from .base import Editable, WeightSpec
 
 
 def matrix_dtype(stored: torch.dtype, run: torch.dtype) -> torch.dtype:
@@ -26,7 +26,7 @@ def matrix_dtype(stored: torch.dtype, run: torch.dtype) -> torch.dtype:
     return torch.bfloat16
 
 
-class StackedLinear:
+class StackedLinear(Editable):
     """Rows of several named weights (and optional biases) stacked into one projection."""
 
     def __init__(self, in_features: int, in_heads: Optional[tuple] = None):
@@ -139,6 +139,9 @@ class StackedLinear:
                 any_scale = True
         self.colscale = scale.to(torch.float32).to(device) if any_scale else None
         self.colbias = bias.to(torch.float32).to(device) if any_bias else None
+
+    def repeats(self):
+        return frozenset(("segments",))
 
     def forward(self, x: torch.Tensor, out: torch.Tensor, accumulate: bool = False) -> torch.Tensor:
         # a part of a product fused along K keeps its weight as a column range of the fused matrix; used on

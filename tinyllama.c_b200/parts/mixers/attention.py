@@ -264,6 +264,11 @@ class AttentionMixer(Part):
         full[:, :self.qk_dim] = w.reshape(heads, self.qk_dim)
         return full.reshape(-1).contiguous()
 
+    def repeats(self):
+        """One map, no convolution (whose values a later layer may read), a position part that is a rotation."""
+        plain = self.maps == 1 and not self.conv_taps and not self.v_mix and self.position.rotation_table() is not None
+        return frozenset(("prefix", "sink_name")) if plain else None
+
     def input_projection(self) -> StackedLinear:
         """What this mixer computes from the normed input before anything else (a block may stack
         the input projections of its mixers into one product)."""

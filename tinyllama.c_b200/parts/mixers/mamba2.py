@@ -117,6 +117,9 @@ class Mamba2Mixer(Part):
         self.norm_w = to_vec(tensors[p + nm["norm"]], device) if self.rms_norm else None
 
     # ---- one step --------------------------------------------------------------------------
+    def repeats(self):
+        return frozenset(("prefix",))
+
     def input_projection(self) -> StackedLinear:
         return self.in_proj
 

@@ -37,6 +37,9 @@ class RMSNorm(Part):
         if self.scale != 1.0:
             self.weight = (self.weight * self.scale).contiguous()
 
+    def repeats(self):
+        return frozenset(("weight_name",))
+
     def forward(self, x32: torch.Tensor, out: torch.Tensor, rows: Optional[torch.Tensor] = None) -> torch.Tensor:
         ops.rmsnorm(x32, self.weight, self.eps, out, rows)
         return out

@@ -51,6 +51,9 @@ class RotaryNeox(Position):
         self.theta = float(theta)
         self.inv_freq: Optional[torch.Tensor] = None
 
+    def repeats(self):
+        return frozenset()
+
     def bind(self, tensors, dtype, device) -> None:
         i = torch.arange(self.rope_dim // 2, dtype=torch.float64)
         inv = 1.0 / torch.pow(torch.tensor(self.theta, dtype=torch.float64), 2.0 * i / self.rope_dim)
