@@ -123,3 +123,32 @@ def test_32_bit_products_of_what_the_kernel_before_them_writes(M):
     ops.linear(a, w, out)
     torch.cuda.synchronize()
     _check(out, a, w, None, None, None)
+
+
+@pytest.mark.parametrize("M", [1, 5, 8])
+@pytest.mark.parametrize("N,K", [(4752, 2048), (8240, 2048), (8244, 1032), (9472, 2040), (4768, 1160)])
+def test_products_of_up_to_8_rows_with_two_tiles_a_block(M, N, K):
+    """297, 515 and 516 tiles (an odd number, a part of one), 592; K of a whole round and of parts of one: the bits of a tile a
+    block, and the oracle's values."""
+    from tinyllama_c_b200 import ops
+    g = torch.Generator().manual_seed(N + K + M)
+    a, w = torch.randn(M, K, generator=g).bfloat16().cuda(), torch.randn(N, K, generator=g).bfloat16().cuda()
+    scale, bias, before = torch.randn(N, generator=g).cuda(), torch.randn(N, generator=g).cuda(), torch.randn(M, N, generator=g).cuda()
+    got = []
+    for two in (True, False):
+        ops.linear_skinny_two(two)
+        try:
+            out = [before.clone(), before.clone(), torch.full((M, N), float("nan"), device="cuda").bfloat16()]
+            ops.linear(a, w, out[0], scale, bias, True)
+            ops.linear(a, w, out[1])
+            ops.linear(a, w, out[2], scale)
+            if N % 16 == 0:
+                out.append(torch.full((M, N // 2), float("nan"), device="cuda").bfloat16())
+                ops.linear_swiglu(a, w, out[3], scale, bias)
+            torch.cuda.synchronize()
+        finally:
+            ops.linear_skinny_two(True)
+        got.append(out)
+    assert all(torch.equal(x, y) for x, y in zip(got[0][1:], got[1][1:]))
+    _check(got[0][0], a.float(), w.float(), scale, bias, before)         # (the compiler may round scale, bias and sum as one or as two)
+    _check(got[0][1], a.float(), w.float(), None, None, None)

@@ -363,19 +363,7 @@ gemm_tiled_f32x4_kernel(const float* __restrict__ a, int lda, const float* __res
 constexpr int ft_smem(int CT, int KG) { return KG * 2 * FT_K * (FT_M + 16 * CT + 2 * FT_LD) * 4; }
 static_assert(ft_smem(4, 4) >= 3 * 8 * 4 * 128 * 4 && ft_smem(8, 1) <= 48 * 1024, "the other groups' sums reuse the operands' memory");
 
-// Kernels that ask for more than 48 KB of shared memory: once a device, ahead of any stream capture where the library is set up
-// first (tlc_linear_init), else with the first product that takes one of them.
-int tlc_linear_simt_init() {
-  static bool ready[64] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 64 && ready[dev]) return 0;
-  if (cudaFuncSetAttribute(gemm_tiled_f32x4_kernel<float, 4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, ft_smem(4, 4)) != cudaSuccess ||
-      cudaFuncSetAttribute(gemm_tiled_f32x4_kernel<__nv_bfloat16, 4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, ft_smem(4, 4)) != cudaSuccess)
-    return tlc_fail(-2, "linear(32 bits): cannot reserve %d bytes of shared memory", ft_smem(4, 4));
-  if (dev >= 0 && dev < 64) ready[dev] = true;
-  return 0;
-}
+int tlc_linear_simt_init();
 
 template <typename TO>
 static int launch_simt_f32x4(const float* a, int lda, const float* w, int ldw, TO* out, int ldo, const float* colscale,
@@ -613,6 +601,132 @@ gemm_skinny_mma_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_
   }
 }
 
+// Up to 8 rows, K of one round, and more tiles than the SMs hold blocks but not more than twice as many: two tiles of 16 columns a
+// block, so that all of the matrix is on its way before the wait on the previous kernel.  (With a tile a block, the blocks past
+// the first two of an SM ask for their weights when others have gone through the wait, the products and the sums: the
+// 33.7 MB of 2048 -> 8240 took 7.6 us behind the wait where the two narrow products of a layer, all of whose blocks are resident
+// at once, take 4.4.)  The second tile's weights come by cp.async into shared memory, every thread its own pieces, and take
+// neither registers nor lines of the first-level cache while they travel, which is what bounds the first tile's; the sums
+// are those of a tile a block, in the same order.  A captured step of the 1.5B sizes, contexts of up to 512, microseconds,
+// a tile a block and two: batch 1 925 and 855, 2 941 and 880, 4 998 and 931, 8 1186 and 1105.
+template <typename TO, bool SWIGLU>
+__global__ void __launch_bounds__(SK_WARPS * 32, 2)
+gemm_skinny_two_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfloat16* __restrict__ w, int ldw,
+                       TO* __restrict__ out, int ldo, const float* __restrict__ colscale, const float* __restrict__ colbias,
+                       TlcEpi accumulate, int M, int N, int K) {
+  asm volatile("griddepcontrol.launch_dependents;");
+  constexpr int U = 4, NT = SK_WARPS * 32;
+  extern __shared__ __align__(16) uint4 second[];                    // [U][2][NT]
+  __shared__ float red[2][SK_WARPS][32][4];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, t = lane & 3;
+  const int K8 = K >> 3, n_steps = (K8 + 3) >> 2;
+  const int tiles[2] = {(int)blockIdx.x * 16, (int)(blockIdx.x + gridDim.x) * 16};
+  const bool two = tiles[1] < N;
+  const uint4* rows[2][2];
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    rows[i][0] = reinterpret_cast<const uint4*>(w + (size_t)min(tiles[i] + g, N - 1) * ldw);         // clamped rows are never stored
+    rows[i][1] = reinterpret_cast<const uint4*>(w + (size_t)min(tiles[i] + g + 8, N - 1) * ldw);
+  }
+  if (two) {
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int c = (warp * U + u) * 4 + t;
+      const bool in = warp * U + u < n_steps && c < K8;
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+        const unsigned dst = (unsigned)__cvta_generic_to_shared(second + (u * 2 + r) * NT + threadIdx.x);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(rows[1][r] + (in ? c : 0)), "r"(in ? 16 : 0) : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  uint4 wv[U][2];
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    const int c = (warp * U + u) * 4 + t;
+    const bool in = warp * U + u < n_steps && c < K8;
+#pragma unroll
+    for (int r = 0; r < 2; r++) wv[u][r] = in ? __ldg(rows[0][r] + c) : make_uint4(0, 0, 0, 0);
+  }
+  tlc_wait(a, out);
+  uint4 xq[U];
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    const int c = (warp * U + u) * 4 + t;
+    const bool in = warp * U + u < n_steps && c < K8;
+    xq[u] = (in && g < M) ? *(reinterpret_cast<const uint4*>(a + (size_t)g * lda) + c) : make_uint4(0, 0, 0, 0);
+  }
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    if (i == 1) {
+      if (!two) break;
+      asm volatile("cp.async.wait_all;" ::: "memory");               // (a thread reads its own pieces alone)
+    }
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const uint4 p = i == 0 ? wv[u][0] : second[(u * 2) * NT + threadIdx.x], q = i == 0 ? wv[u][1] : second[(u * 2 + 1) * NT + threadIdx.x];
+      mma_bf16_16816(acc, p.x, q.x, p.y, q.y, xq[u].x, xq[u].y);
+      mma_bf16_16816(acc, p.z, q.z, p.w, q.w, xq[u].z, xq[u].w);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) red[i][warp][lane][j] = acc[j];
+  }
+  __syncthreads();
+  // one thread per output value: the warps' sums in their order, epilogue, store
+  constexpr int PER = SWIGLU ? 64 : 128;
+  if ((int)threadIdx.x < (two ? 2 : 1) * PER) {
+    const int i = (int)threadIdx.x / PER, idx = (int)threadIdx.x % PER, n0 = i ? tiles[1] : tiles[0];
+    if (SWIGLU) {
+      const int ln = idx >> 1, j = idx & 1;
+      float vg = 0.f, vu = 0.f;
+#pragma unroll
+      for (int ww = 0; ww < SK_WARPS; ww++) { vg += red[i][ww][ln][j]; vu += red[i][ww][ln][j + 2]; }
+      const int ng = n0 + (ln >> 2), nu = ng + 8, m = 2 * (ln & 3) + j;
+      if (nu < N && m < M) {
+        if (colscale) { vg *= colscale[ng]; vu *= colscale[nu]; }
+        if (colbias) { vg += colbias[ng]; vu += colbias[nu]; }
+        out[(size_t)m * ldo + (n0 >> 1) + (ln >> 2)] = from_f32<TO>(glu_epilogue<false>(accumulate, vg, vu));   // (the activation's code)
+      }
+    } else {
+      const int ln = idx >> 2, j = idx & 3;
+      float v = 0.f;
+#pragma unroll
+      for (int ww = 0; ww < SK_WARPS; ww++) v += red[i][ww][ln][j];
+      const int n = n0 + (ln >> 2) + (j >= 2 ? 8 : 0), m = 2 * (ln & 3) + (j & 1);
+      if (n < N && m < M) {
+        if (colscale) v *= colscale[n];
+        if (colbias) v += colbias[n];
+        TO* o = out + (size_t)m * ldo + n;
+        if (accumulate) v += to_f32(*o);
+        *o = from_f32<TO>(v);
+      }
+    }
+  }
+}
+constexpr int SK_TWO_SMEM = 4 * 2 * SK_WARPS * 32 * (int)sizeof(uint4);
+static int g_skinny_two = 1;          // 0: never two tiles a block (for comparisons)
+
+// Kernels that ask for more than 48 KB of shared memory: once a device, ahead of any stream capture where the library is set up
+// first (tlc_linear_init), else with the first product that takes one of them.
+template <typename TO> static bool simt_reserve() {
+  const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  return cudaFuncSetAttribute(gemm_tiled_f32x4_kernel<TO, 4, 4>, attr, ft_smem(4, 4)) == cudaSuccess &&
+         cudaFuncSetAttribute(gemm_skinny_two_kernel<TO, false>, attr, SK_TWO_SMEM) == cudaSuccess &&
+         cudaFuncSetAttribute(gemm_skinny_two_kernel<TO, true>, attr, SK_TWO_SMEM) == cudaSuccess;
+}
+int tlc_linear_simt_init() {
+  static bool ready[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && ready[dev]) return 0;
+  if (!simt_reserve<float>() || !simt_reserve<__nv_bfloat16>()) return tlc_fail(-2, "linear: cannot reserve %d and %d bytes of shared memory", ft_smem(4, 4), SK_TWO_SMEM);
+  if (dev >= 0 && dev < 64) ready[dev] = true;
+  return 0;
+}
+
 template <typename TO, int MG, bool SWIGLU>
 static void launch_skinny_mg(const __nv_bfloat16* a, int lda, const __nv_bfloat16* w, int ldw, TO* out, int ldo,
                              const float* colscale, const float* colbias, TlcEpi accumulate, int M, int N, int K,
@@ -643,6 +757,16 @@ static void launch_skinny_mg(const __nv_bfloat16* a, int lda, const __nv_bfloat1
         cudaLaunchKernelEx(&cfg, gemm_skinny_mma_kernel<TO, MG, 2, false, true>, a, lda, w, ldw, out, ldo, colscale, colbias, accumulate, M, N, K);
       else
         cudaLaunchKernelEx(&cfg, gemm_skinny_mma_kernel<TO, MG, 4, false, true>, a, lda, w, ldw, out, ldo, colscale, colbias, accumulate, M, N, K);
+      return;
+    }
+  }
+  if constexpr (MG == 1) {
+    static int sms = 0;
+    if (sms == 0) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
+    if (g_skinny_two && n_steps > SK_WARPS * 2 && n_steps <= SK_WARPS * 4 && (int)blocks > 2 * sms && (int)blocks <= 4 * sms &&
+        tlc_linear_simt_init() == 0) {
+      tlc_launch(gemm_skinny_two_kernel<TO, SWIGLU>, dim3((blocks + 1) / 2), dim3(SK_WARPS * 32), SK_TWO_SMEM, stream, a, lda, w, ldw, out, ldo, colscale,
+                 colbias, accumulate, M, N, K);
       return;
     }
   }
@@ -686,6 +810,7 @@ extern "C" int tlc_linear_skinny(const void* a, int lda, const void* w, int ldw,
 }
 
 extern "C" void tlc_linear_skinny_pairs(int on) { g_skinny_pairs = on; }
+extern "C" void tlc_linear_skinny_two(int on) { g_skinny_two = on; }
 
 extern "C" int tlc_linear_skinny_swiglu(const void* a, int lda, const void* w, int ldw, void* out, int out_dtype, int ldo,
                                         const float* colscale, const float* colbias, int M, int N, int K, int act_code,

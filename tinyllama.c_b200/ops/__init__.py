@@ -66,6 +66,7 @@ _SIGNATURES = {
     "tlc_linear_split_override": (None, [_i]),
     "tlc_linear_pair_override": (None, [_i]),
     "tlc_linear_skinny_pairs": (None, [_i]),
+    "tlc_linear_skinny_two": (None, [_i]),
     "tlc_linear_tma_out": (None, [_i]),
     "tlc_linear_few_rows": (None, [_i]),
     "tlc_linear_few_rows_split": (None, [_i]),
@@ -688,6 +689,11 @@ def linear_skinny_pairs(on: bool) -> None:
     """Whether the few-row product may give a tile of 16 columns to two blocks of a cluster, each with one half
     of K (it does where the matrix has fewer tiles than the GPU has SMs); for tests and comparisons."""
     library().tlc_linear_skinny_pairs(int(bool(on)))
+
+
+def linear_skinny_two(on: bool) -> None:
+    """Whether the product of up to 8 rows may take two tiles a block (for comparisons)."""
+    library().tlc_linear_skinny_two(int(bool(on)))
 
 
 def linear_pairs() -> int:
