@@ -16,7 +16,7 @@ import configs
 
 # the kernels of long prompts, of short ones and the general ones; more than two layers
 SIZES = {"tensor cores": dict(configs.TINY_D, num_hidden_layers=4, mamba_d_head=64, mamba_d_ssm=128, mamba_d_state=128),
-         "odd": dict(configs.TINY_C, num_hidden_layers=3), "small": dict(configs.TINY_A, num_hidden_layers=5)}
+         "odd": dict(configs.TINY_C, num_hidden_layers=3), "small": dict(configs.TINY_A, num_hidden_layers=8)}
 
 
 def _model(name, dtype, device):
@@ -80,12 +80,12 @@ def test_repeated_layers_give_the_same_bits_as_layers_one_by_one(name, dtype):
     assert model.repeated is not None
     V, r = SIZES[name]["vocab_size"], random.Random(5)
     ids = lambda n: [r.randrange(V) for _ in range(n)]  # noqa: E731
-    steps = [[ids(n) for n in lens] for lens in ((5, 1, 3), (40, 150, 20), (1, 1, 1), (33, 1, 260))]
+    steps = [[ids(n) for n in lens] for lens in ((5, 1, 3), (40, 150, 20), (1, 1, 1), (33, 1, 260), (500, 30, 600))]
     got, calls = [], []
     for repeated in (model.repeated, None):
         for stream in (torch.cuda.current_stream(), torch.cuda.Stream()):
             model.repeated = repeated
-            llm = tlc.LLM(model, dtype=dtype, max_tokens=64 * 32, max_seqs=3)
+            llm = tlc.LLM(model, dtype=dtype, max_tokens=64 * 64, max_seqs=3)
             slots = [llm.cache.acquire() for _ in range(3)]
             before = ops.launch_count()
             torch.cuda.synchronize()
@@ -118,11 +118,11 @@ def test_every_layer_of_a_repeated_step_goes_through_the_library_once():
             return out
 
         first = logits()
-        assert times == [3]
+        assert times == [1, 1, 1]
         w = model.layers[2].ffn.down
         w.weight = w.weight.clone()                     # an edit: found alike again, at the new place
-        assert torch.equal(first, logits()) and times == [3, 3]
+        assert torch.equal(first, logits()) and times == [1, 1, 1] * 2
         w.weight = w.weight.t().contiguous().t()        # other strides in one layer: one by one
-        assert torch.equal(first, logits()) and times == [3, 3]
+        assert torch.equal(first, logits()) and times == [1, 1, 1] * 2
     finally:
         ops.replay = table

@@ -220,11 +220,12 @@ def _call(name: str, *args) -> None:
 class NotedCalls:
     """Calls in the order they were made.  words: the arguments as 64-bit words; is_pointer marks those that are pointers.
     owned: what the calls were given that no argument keeps alive (scratch, numbers on the host that a call writes).
-    handles: streams and events that the calls name.  complete: False once a call was made that cannot be made again."""
+    handles: streams and events that the calls name.  complete: False once a call was made that cannot be made again.
+    forks: whether an event was recorded."""
 
     def __init__(self):
         self.functions, self.words, self.is_pointer = [], [], []
-        self.owned, self.handles, self.complete = [], set(), True
+        self.owned, self.handles, self.complete, self.forks = [], set(), True, False
 
     def add(self, name: str, args) -> None:
         index, kinds = _replayable(name)
@@ -306,6 +307,7 @@ def _event_functions() -> int:
 def record_event(event: "torch.cuda.Event", stream: "torch.cuda.Stream") -> None:
     event.record(stream)
     if _notes.calls is not None:
+        _notes.calls.forks = True
         _notes.calls.handles |= {event.cuda_event, stream.cuda_stream}
         _notes.calls.add("tlc_event_record", (event.cuda_event, stream.cuda_stream))
 

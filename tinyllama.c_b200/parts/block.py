@@ -128,6 +128,24 @@ class Block(Part):
                     self.out_offsets.append((off, pr.in_features))
                     off += pr.in_features
 
+    def _make_sides(self, device) -> None:
+        if not hasattr(self, "_side"):
+            self._side = [torch.cuda.Stream(device=device) for _ in self.mixers[1:]]
+            # events are made once: a record overwrites the event's last state, and every wait of this block follows
+            # its record in program order
+            self._fork = torch.cuda.Event()
+            self._done = [torch.cuda.Event() for _ in self.mixers]
+
+    def handles(self, device) -> List[int]:
+        """This layer's own streams and events, made and once recorded if they are not there yet (an event has no handle
+        before that): a layer that is run by another one's calls (models/repeat.py) keeps to its own."""
+        self._make_sides(device)
+        main = current_stream(device)
+        for event in [self._fork] + self._done:
+            if not event.cuda_event:
+                event.record(main)
+        return [s.cuda_stream for s in self._side] + [e.cuda_event for e in [self._fork] + self._done]
+
     def _mix_in_parallel(self, parts, step: StepInfo, cache: LayerCache, x32: torch.Tensor, outs: Optional[torch.Tensor] = None) -> None:
         """One mixer runs on the current stream, every other on a side stream that starts after the
         shared input projection.  Output projections add into the residual stream one after the
@@ -135,12 +153,7 @@ class Block(Part):
         side streams become parallel branches of the graph.)  outs [T, n, D]: every mixer's output projection is written
         to its own rows outs[:, i] instead (a layer that joins its mixers' results by something else than their sum)."""
         main = current_stream(x32.device)
-        if not hasattr(self, "_side"):
-            self._side = [torch.cuda.Stream(device=x32.device) for _ in self.mixers[1:]]
-            # events are made once: a record overwrites the event's last state, and every wait of this block follows
-            # its record in program order
-            self._fork = torch.cuda.Event()
-            self._done = [torch.cuda.Event() for _ in self.mixers]
+        self._make_sides(x32.device)
         # the mixer with the longest chain of kernels stays on the current stream, where every
         # kernel follows its predecessor by a programmatic edge
         lengths = [int(getattr(m, "single_token_launches", 1)) for m in self.mixers]
