@@ -38,3 +38,34 @@ def test_scan_rows_staged_in_batches(lens, N, P, aligned):
     # products and sums of N terms in 32 bits over at most 23 rows
     assert (y.cpu().double() - y_ref).abs().max().item() <= (N + 40) * 2.0 ** -23 * 16 * N ** 0.5 * 4
     assert (st.cpu().double() - S_ref).abs().max().item() <= 60 * 2.0 ** -23 * S_ref.abs().max().item()
+
+
+@pytest.mark.parametrize("N,P", [(68, 4), (128, 20), (132, 64), (256, 12)])
+@pytest.mark.parametrize("lens,chunk", [((1,), 0), ((4, 5, 1), 0), ((23, 8), 0), ((1, 70, 33), 32)])
+def test_rows_in_16_byte_pieces_give_the_general_kernels_bits(N, P, lens, chunk):
+    """The same outputs and states, row by row; in chunks the general kernel multiplies a chunk's decays in another order."""
+    from tinyllama_c_b200 import ops
+    g = torch.Generator().manual_seed(sum(lens) + N)
+    Hs, G = 6, 2
+    T, B, Di = sum(lens), len(lens), Hs * P
+    xbc, dt, dA = torch.randn(T, Di + 2 * G * N, generator=g).cuda(), torch.rand(T, Hs, generator=g).cuda(), torch.rand(T, Hs, generator=g).cuda()
+    D, state = torch.randn(Hs, generator=g).cuda(), torch.randn(B, Hs, P, N, generator=g).cuda()
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    cu = [sum(lens[:b]) for b in range(B + 1)]
+    chunks = None
+    if chunk:
+        firsts = [[c for c in range(cu[b], cu[b + 1], chunk)] for b in range(B)]
+        chunks = (i32(sum(firsts, []) + [T]), i32([b for b in range(B) for _ in firsts[b]]),
+                  i32([sum(len(f) for f in firsts[:b]) for b in range(B + 1)]))
+    got = []
+    for own in (True, False):
+        ops.ssm_scan_rows(own)
+        try:
+            y, st = torch.full((T, Di), float("nan"), device="cuda"), state.clone()
+            ops.ssm_scan(xbc, dt, dA, D, st, i32(cu), i32(range(B)), i32([3 if b % 2 else 0 for b in range(B)]), y, Hs, P, N, G, chunks)
+            torch.cuda.synchronize()
+        finally:
+            ops.ssm_scan_rows(True)
+        got.append((y, st))
+    for a, b in zip(*got):
+        assert torch.equal(a, b) if not chunk else (a - b).abs().max() <= 70 * 2.0 ** -23 * b.abs().max()

@@ -515,6 +515,169 @@ ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dt, con
   }
 }
 
+// The same for states of more than 64 columns where everything lies in pieces of 16 bytes (columns and head rows multiples of 4,
+// xbc, its rows and the states on 16-byte boundaries): the state's values and the order of every sum are those of the kernel
+// above, a row costs less.  What a row cost there: four sums over a warp of five shuffles each, one after the other, B and C
+// read value by value with a stride of four (bank conflicts), and a division and an address from scratch for every piece that
+// is copied.  Here the sums of SCAN_TT rows x RP head rows, which every lane holds a share of, go through the same tree together:
+// at each of the first steps a lane hands half of its values to its partner and keeps the other half (16 values: 16 shuffles
+// and not 80), which leaves every pair of lanes with one value to store; B and C are read 16 bytes at a time; a thread copies the
+// same pieces of every row and only moves its pointers on.  48 heads of 64, 256 columns, before and now, microseconds: one row 4.4
+// and 3.7, 23 rows 30.3 and 13.0, eight sequences of 10 rows 40.0 and 23.4; in chunks (three passes) 310 rows of 128 353 and 188,
+// of 32 212 and 140.  (Two head rows a warp, twice the warps: 23 rows 14.8, eight of 10 29.1.)
+template <int NPL>
+__global__ void __launch_bounds__(128, NPL == 4 ? 6 : 5)
+ssm_scan_rows_kernel(const float* __restrict__ xbc, const float* __restrict__ dt, const float* __restrict__ dA,
+                     const float* __restrict__ Dskip, float* __restrict__ state, float* __restrict__ chunk_state,
+                     const int* __restrict__ seg_start, const int* __restrict__ seg_seq,
+                     const int* __restrict__ seq_seg_start, const int* __restrict__ slots,
+                     const int* __restrict__ start_pos, float* __restrict__ y, float* __restrict__ chunk_decay, int mode,
+                     int Hs, int P, int N, int G, int Cd) {
+  asm volatile("griddepcontrol.launch_dependents;");
+  if (mode != SCAN_PLAIN) tlc_wait(xbc, dt, dA, state, chunk_state, y, chunk_decay);
+  static_assert(NPL % 4 == 0, "four columns a lane at a time");
+  constexpr int RP = 4, TT = SCAN_TT, PB = 4 * RP, V = TT * RP, NQ = NPL / 4;
+  extern __shared__ __align__(16) float sm[];
+  const int seg = blockIdx.x, h = blockIdx.y;
+  const int b = seg_seq ? seg_seq[seg] : seg;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int p_blk = blockIdx.z * PB, p_base = p_blk + warp * RP;
+  const int Di = Hs * P, g = h / (Hs / G);
+  const int t0 = seg_start[seg], n_tok = seg_start[seg + 1] - t0;
+  if (n_tok == 0) return;
+  float* S_slot = state + (((size_t)slots[b] * Hs + h) * P) * N;
+  float* S_chunk = chunk_state ? chunk_state + (((size_t)seg * Hs + h) * P) * N : nullptr;
+  const float* S_init = mode == SCAN_PLAIN ? (start_pos[b] > 0 ? S_slot : nullptr) : mode == SCAN_CHUNK_OUT ? S_chunk : nullptr;
+  float* S_final = mode == SCAN_PLAIN ? S_slot : mode == SCAN_CHUNK_STATE ? S_chunk : seg + 1 == seq_seg_start[b + 1] ? S_slot : nullptr;
+  const bool want_y = mode != SCAN_CHUNK_STATE;
+  float4 s[RP][NQ];                                          // columns 4 lane + 128 jj of the warp's head rows
+#pragma unroll
+  for (int r = 0; r < RP; r++)
+#pragma unroll
+    for (int jj = 0; jj < NQ; jj++) {
+      const int n = 4 * lane + 128 * jj;
+      s[r][jj] = S_init && p_base + r < P && n < N ? *reinterpret_cast<const float4*>(S_init + (size_t)(p_base + r) * N + n)
+                                                    : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  if (mode == SCAN_PLAIN) tlc_wait(xbc, dt, dA, y);
+  // a row in shared memory: B[N] | C[N] | x[PB] | dt | dA
+  const int per_tok = 2 * N + PB + 4, nq = N >> 2, row_q = 2 * nq + RP;
+  const float Dh = Dskip[h];
+  // this thread's pieces of a row: where they come from (of the segment's first row), and whether they are copied at all
+  const float* src[2];
+  bool on[2];
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    const int q = tid + 128 * i, p = p_blk + 4 * (q - 2 * nq);
+    const float* row = xbc + (size_t)t0 * Cd;
+    src[i] = row;
+    on[i] = true;
+    if (q < nq) src[i] = row + Di + (size_t)g * N + 4 * q;
+    else if (q < 2 * nq) { src[i] = row + Di + (size_t)G * N + (size_t)g * N + 4 * (q - nq); on[i] = want_y; }
+    else { on[i] = p < P; if (on[i]) src[i] = row + (size_t)h * P + p; }
+  }
+  const float* src_dt = ((tid & 1) ? dA : dt) + (size_t)(t0 + (tid >> 1)) * Hs + h;      // (threads 0 .. 2 TT - 1)
+  auto fetch = [&](int tt0, float* buf) {
+    const int nt = min(TT, n_tok - tt0);
+#pragma unroll
+    for (int k = 0; k < TT; k++) {
+      if (k < nt) {
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+          if (tid + 128 * i < row_q) {
+            scan_copy16(buf + k * per_tok + 4 * (tid + 128 * i), src[i], on[i]);
+            src[i] += Cd;
+          }
+      }
+    }
+    if (tid < 2 * TT && (tid >> 1) < nt) scan_copy4(buf + (tid >> 1) * per_tok + 2 * N + PB + (tid & 1), src_dt + (size_t)tt0 * Hs);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fetch(0, sm);
+#pragma unroll 1
+  for (int tt0 = 0, turn = 0; tt0 < n_tok; tt0 += TT, turn ^= 1) {
+    const int nt = min(TT, n_tok - tt0);
+    const float* smb = sm + turn * TT * per_tok;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                                         // this batch is here, and every warp is done with the one before it
+    if (tt0 + TT < n_tok) fetch(tt0 + TT, sm + (turn ^ 1) * TT * per_tok);
+    float v[V];
+#pragma unroll
+    for (int k = 0; k < TT; k++) {
+      if (k < nt) {
+        const float* tk = smb + k * per_tok;
+        const float2 dd = *reinterpret_cast<const float2*>(tk + 2 * N + PB);
+        float x[RP];
+#pragma unroll
+        for (int r = 0; r < RP; r += 2) {
+          const float2 u = *reinterpret_cast<const float2*>(tk + 2 * N + warp * RP + r);
+          x[r] = u.x * dd.x;
+          x[r + 1] = u.y * dd.x;
+        }
+#pragma unroll
+        for (int r = 0; r < RP; r++) v[k * RP + r] = 0.f;
+#pragma unroll
+        for (int jj = 0; jj < NQ; jj++) {
+          const int n = 4 * lane + 128 * jj;
+          const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+          const float4 B = n < N ? *reinterpret_cast<const float4*>(tk + n) : z;
+          const float4 C = want_y && n < N ? *reinterpret_cast<const float4*>(tk + N + n) : z;
+#pragma unroll
+          for (int r = 0; r < RP; r++) {
+            float4& u = s[r][jj];
+            float& a = v[k * RP + r];
+            u.x = fmaf(u.x, dd.y, B.x * x[r]); a = fmaf(u.x, C.x, a);
+            u.y = fmaf(u.y, dd.y, B.y * x[r]); a = fmaf(u.y, C.y, a);
+            u.z = fmaf(u.z, dd.y, B.z * x[r]); a = fmaf(u.z, C.z, a);
+            u.w = fmaf(u.w, dd.y, B.w * x[r]); a = fmaf(u.w, C.w, a);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < RP; r++) v[k * RP + r] = 0.f;
+      }
+    }
+    if (want_y) {
+      // the tree of warp_sum for all values at once; bit by bit a lane keeps the half that its number names
+#pragma unroll
+      for (int o = 16, m = V / 2; o > 0; o >>= 1, m >>= 1) {
+        if (m > 0) {
+          const bool upper = lane & o;
+#pragma unroll
+          for (int i = 0; i < m; i++) {
+            const float mine = upper ? v[i + m] : v[i], theirs = upper ? v[i] : v[i + m];
+            v[i] = mine + __shfl_xor_sync(0xffffffffu, theirs, o);
+          }
+        } else {
+          v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        }
+      }
+      constexpr int SPARE = 32 / V;                          // lanes that hold the same value
+      const int idx = lane / SPARE, k = idx / RP, r = idx % RP, p = p_base + r;
+      if (lane % SPARE == 0 && k < nt && p < P)
+        y[(size_t)(t0 + tt0 + k) * Di + (size_t)h * P + p] = v[0] + smb[k * per_tok + 2 * N + warp * RP + r] * Dh;
+    }
+  }
+  if (mode == SCAN_CHUNK_STATE && blockIdx.z == 0 && warp == 0) {
+    float d = 1.f;                         // decay of the whole chunk: the product of its rows' decays
+    for (int k = lane; k < n_tok; k += 32) d *= dA[(size_t)(t0 + k) * Hs + h];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) d *= __shfl_xor_sync(0xffffffffu, d, o);
+    if (lane == 0) chunk_decay[(size_t)seg * Hs + h] = d;
+  }
+  if (S_final) {
+#pragma unroll
+    for (int r = 0; r < RP; r++)
+#pragma unroll
+      for (int jj = 0; jj < NQ; jj++) {
+        const int n = 4 * lane + 128 * jj;
+        if (p_base + r < P && n < N) *reinterpret_cast<float4*>(S_final + (size_t)(p_base + r) * N + n) = s[r][jj];
+      }
+  }
+}
+static int g_scan_rows = 1;                // test hook: 0 = the general kernel everywhere
+extern "C" void tlc_ssm_scan_rows(int on) { g_scan_rows = on; }
+
 // Pass 2: carries the state through a sequence's chunks.  chunk_state[c] holds the chunk's own
 // contribution on entry and the state *before* the chunk on exit.  grid (B, Hs, blocks over P*N).
 // With write_final the state after the last chunk goes to the sequence's slot.
@@ -608,6 +771,14 @@ static int launch_scan(const float* xbc, const float* dt, const float* dA, const
                        const int* slots, const int* start_pos, float* y, float* chunk_decay, int mode, int n_seg, int Hs,
                        int P, int N, int G, int Cd, cudaStream_t stream) {
   constexpr int RP = 4;
+  if constexpr (NPL % 4 == 0) {
+    if (g_scan_rows && N % 4 == 0 && P % 4 == 0 && Cd % 4 == 0 && (((uintptr_t)state | (uintptr_t)chunk_state | (uintptr_t)xbc) & 15) == 0) {
+      tlc_launch(ssm_scan_rows_kernel<NPL>, dim3(n_seg, Hs, (P + 15) / 16), dim3(128), (size_t)2 * SCAN_TT * (2 * N + 20) * sizeof(float), stream,
+                 xbc, dt, dA, Dskip, state, chunk_state, seg_start, seg_seq, seq_seg_start, slots, start_pos, y, chunk_decay, mode, Hs, P, N, G, Cd);
+      TLC_CHECK_LAUNCH("ssm_scan");
+      return 0;
+    }
+  }
   dim3 grid(n_seg, Hs, (P + 4 * RP - 1) / (4 * RP));
   const size_t smem = (size_t)2 * SCAN_TT * (2 * N + 4 * RP + 4) * sizeof(float);
   auto run = [&](auto kernel) {

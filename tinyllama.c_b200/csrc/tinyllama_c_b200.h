@@ -276,6 +276,7 @@ int tlc_mamba_step(const float* proj, int ld, int xbc_off, int dt_off, const flo
                    const float* dt_bias, const float* A, const float* Dskip, float* conv_state, float* state,
                    const int* slots, const int* start_pos, float* y, int B, int Hs, int P, int N, int G, int Cd, int K,
                    int bf16_run, cudaStream_t stream);
+void tlc_ssm_scan_rows(int on);         // 0: the row-by-row scan takes the general kernel everywhere (for comparisons)
 /* S = S * dA + B (x dt), y = S.C + x D, row by row from each slot's state [n_slots, Hs, P, N] (zero at
  * position 0), which is updated in place. */
 int tlc_ssm_scan(const float* xbc, const float* dt, const float* dA, const float* Dskip, float* state,

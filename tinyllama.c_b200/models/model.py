@@ -51,16 +51,7 @@ class Model:
                         or self.schedule[run.kv_cache].kv_cache is not None:
                     raise ValueError(f"run-order entry {r} reads the keys and values of entry {run.kv_cache}, which must be "
                                      f"an earlier entry that stores its own")
-        # chunk lengths that parts want the step function to cut sequences into (one table each, every step)
-        # as (rows, from how many rows of a sequence the table is wanted): the smallest threshold asked for a length
-        asked: Dict[int, int] = {}
-        for layer in self.layers:
-            for q in layer.step_requests():
-                if isinstance(q, ChunkRequest):
-                    start = q.rows if q.from_rows is None else min(q.rows, q.from_rows)
-                    asked[q.rows] = min(asked.get(q.rows, start), start)
-        self.chunk_rows = tuple(sorted(asked))
-        self.chunk_from = dict(asked)               # chunk length -> rows a sequence must exceed for the table to be made
+        self._collect_chunks()
         self.final_norm = final_norm.build()
         self.embed_name, self.head_name = embed_name, head_name            # head_name None: tied (core.c:1246-1249)
         self.embed_scale = float(embed_scale)
@@ -75,6 +66,19 @@ class Model:
         self.dtype: Optional[torch.dtype] = None
         self.device: Optional[torch.device] = None
         self.repeated: Optional[RepeatedLayers] = None      # the run order's layers, where they are all alike
+
+    def _collect_chunks(self) -> None:
+        """What the layers ask the step function for."""
+        # chunk lengths that parts want the step function to cut sequences into (one table each, every step)
+        # as (rows, from how many rows of a sequence the table is wanted): the smallest threshold asked for a length
+        asked: Dict[int, int] = {}
+        for layer in self.layers:
+            for q in layer.step_requests():
+                if isinstance(q, ChunkRequest):
+                    start = q.rows if q.from_rows is None else min(q.rows, q.from_rows)
+                    asked[q.rows] = min(asked.get(q.rows, start), start)
+        self.chunk_rows = tuple(sorted(asked))
+        self.chunk_from = dict(asked)               # chunk length -> rows a sequence must exceed for the table to be made
 
     # ---- declarations ----------------------------------------------------------------------
     def weight_specs(self) -> List[WeightSpec]:
@@ -115,6 +119,7 @@ class Model:
         self.dtype, self.device = dtype, torch.device(device)
         for layer in self.layers:
             layer.bind(tensors, dtype, device)
+        self._collect_chunks()
         self.final_norm.bind(tensors, dtype, device)
         self.by_table = [l.ffn for l in self.layers if isinstance(l.ffn, MoEFeedForward) and l.ffn.table is not None] \
             if self.device.type == "cuda" else []

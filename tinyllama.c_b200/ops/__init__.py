@@ -98,6 +98,7 @@ _SIGNATURES = {
                             _i, _vp]),
     "tlc_gated_rmsnorm_step": (_i, [_vp, _vp, _i, _vp, _f, _i, _i, _i, _i, _vp, _i, _i, _f, _vp, _i, _i, _vp, _vp, _vp, _i, _i, _i,
                                     _i, _vp]),
+    "tlc_ssm_scan_rows": (None, [_i]),
     "tlc_ssm_scan": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp]),
     "tlc_ssm_scan_chunked": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i,
                                   _vp]),
@@ -1076,6 +1077,11 @@ def mamba_step(proj: torch.Tensor, xbc_off: int, dt_off: int, w: torch.Tensor, b
     _call("tlc_mamba_step", proj.data_ptr(), _rows(proj, "proj"), xbc_off, dt_off, w.data_ptr(), _p(bias), dt_bias.data_ptr(),
           A.data_ptr(), Dskip.data_ptr(), conv_state.data_ptr(), state.data_ptr(), slots.data_ptr(), start_pos.data_ptr(),
           y.data_ptr(), T, Hs, P, N, G, Cd, K, int(bool(bf16_run)), _stream())
+
+
+def ssm_scan_rows(on: bool) -> None:
+    """Whether the row-by-row scan may take its kernel for rows and states in 16-byte pieces (for comparisons)."""
+    library().tlc_ssm_scan_rows(int(bool(on)))
 
 
 def ssd_first_chunks(mode: int) -> None:

@@ -100,8 +100,16 @@ class Mamba2Mixer(Part):
     CHUNKS_FROM_ROWS = 8
     CHUNKS_WORTH_ROWS, CHUNKS_WORTH_STEP = 32, 128
 
+    # In 32 bits the chunks run row by row, one beside the other, and a chunk's rows are what a step of few rows waits for: steps
+    # of up to SHORT_CHUNKS_STEP rows are cut into chunks of SHORT_CHUNK (48 heads of 64, 256 columns, chunks of 128 / 32 rows, the
+    # three passes: 120 rows 91 / 79 us, 310 rows 188 / 140, 600 281 / 252, 1,000 418 / 417).  More rows fill the GPU with
+    # chunks of any length, and every chunk costs a state of scratch.
+    SHORT_CHUNK, SHORT_CHUNKS_STEP = 32, 1024
+
     def step_requests(self) -> list:
-        return [ChunkRequest(self.scan_chunk, min(self.scan_chunk, self.CHUNKS_FROM_ROWS))]
+        """(asked for again once the run's type is known)"""
+        rows = [self.scan_chunk] + ([self.SHORT_CHUNK] if self.dtype == torch.float32 and self.SHORT_CHUNK < self.scan_chunk else [])
+        return [ChunkRequest(n, min(n, self.CHUNKS_FROM_ROWS)) for n in rows]
 
     def bind(self, tensors: Dict[str, torch.Tensor], dtype, device) -> None:
         p = self.prefix
@@ -163,7 +171,8 @@ class Mamba2Mixer(Part):
                               (proj, self.Di, conv_state, step.slots, step.start_pos, self.Di, self.Cd - self.Di))
         # prompts cut into chunks of a bfloat16 run: the scan in matrix form, whose operands x|B|C the convolution
         # writes in bfloat16 at once; everything else scans 32-bit values
-        chunks = step.chunks.get(self.scan_chunk)
+        short = self.dtype == torch.float32 and step.n_rows <= self.SHORT_CHUNKS_STEP
+        chunks = step.chunks.get(self.SHORT_CHUNK if short and self.SHORT_CHUNK in step.chunks else self.scan_chunk)
         if chunks is not None and step.max_new <= self.CHUNKS_WORTH_ROWS and step.n_rows < self.CHUNKS_WORTH_STEP:
             chunks = None
         matrix_form = chunks is not None and self.dtype == torch.bfloat16 and self.scan_chunk <= ops.SSD_CHUNK \
