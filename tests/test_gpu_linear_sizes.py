@@ -149,6 +149,32 @@ def test_products_of_up_to_8_rows_with_two_tiles_a_block(M, N, K):
         finally:
             ops.linear_skinny_two(True)
         got.append(out)
-    assert all(torch.equal(x, y) for x, y in zip(got[0][1:], got[1][1:]))
-    _check(got[0][0], a.float(), w.float(), scale, bias, before)         # (the compiler may round scale, bias and sum as one or as two)
+    assert all(torch.equal(x, y) for x, y in zip(*got))
     _check(got[0][1], a.float(), w.float(), None, None, None)
+
+
+@pytest.mark.parametrize("M", [17, 24, 31, 32])
+@pytest.mark.parametrize("N,K", [(2384, 4096), (2572, 5384), (3072, 12288), (4092, 4104)])
+def test_products_of_17_to_32_rows_shared_among_clusters_of_four(M, N, K):
+    """149, 161, 192 and 256 tiles of 16 columns (an odd number, a part of one), whole rounds of K and parts of one: the bits of the
+    kernel with a tile a block, and the oracle's values."""
+    from tinyllama_c_b200 import ops
+    g = torch.Generator().manual_seed(N + K + M)
+    a, w = torch.randn(M, K, generator=g).bfloat16().cuda(), torch.randn(N, K, generator=g).bfloat16().cuda()
+    scale, bias, before = torch.randn(N, generator=g).cuda(), torch.randn(N, generator=g).cuda(), torch.randn(M, N + 4, generator=g).cuda()
+    got = []
+    for ring in (True, False):
+        ops.linear_skinny_ring(ring)
+        try:
+            out = [before.clone() for _ in range(3)] + [torch.full((M, N), float("nan"), device="cuda").bfloat16()]
+            ops.linear(a, w, out[0][:, :N], scale, bias, True)
+            ops.linear(a, w, out[1][:, :N], scale, None, True)
+            ops.linear(a, w, out[2][:, :N])
+            ops.linear(a, w, out[3], None, bias)
+            torch.cuda.synchronize()
+        finally:
+            ops.linear_skinny_ring(True)
+        got.append(out)
+    assert all(torch.equal(x, y) for x, y in zip(*got))
+    assert torch.equal(got[0][0][:, N:], before[:, N:])
+    _check(got[0][2][:, :N], a.float(), w.float(), None, None, None)

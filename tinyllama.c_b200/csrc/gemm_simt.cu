@@ -465,6 +465,22 @@ __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], uint32_t a0, uint3
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// A sum on its way out: scaled, with its bias, added to what is there.  The products that fuse into a sum are named, so that
+// every kernel of this file that makes a value rounds it alike.
+__device__ __forceinline__ float skinny_scaled(float v, int n, const float* __restrict__ colscale, const float* __restrict__ colbias) {
+  if (colbias) return colscale ? fmaf(v, colscale[n], colbias[n]) : v + colbias[n];
+  return colscale ? v * colscale[n] : v;
+}
+template <typename TO>
+__device__ __forceinline__ void skinny_store(float v, int n, TO* o, const float* __restrict__ colscale, const float* __restrict__ colbias, bool accumulate) {
+  if (accumulate && colscale && !colbias) v = fmaf(v, colscale[n], to_f32(*o));
+  else {
+    v = skinny_scaled(v, n, colscale, colbias);
+    if (accumulate) v += to_f32(*o);
+  }
+  *o = from_f32<TO>(v);
+}
+
 constexpr int SK_WARPS = 16;          // warps per block, each with its own slices of K
 static int g_skinny_pairs = 1;        // 0: never two blocks a tile (for comparisons)
 
@@ -558,8 +574,8 @@ gemm_skinny_mma_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_
         const int ng = n0 + (ln >> 2), nu = ng + 8;
         const int m = (g0 + mg) * 8 + 2 * (ln & 3) + j;
         if (nu < N && m < M) {
-          if (colscale) { vg *= colscale[ng]; vu *= colscale[nu]; }
-          if (colbias) { vg += colbias[ng]; vu += colbias[nu]; }
+          vg = skinny_scaled(vg, ng, colscale, colbias);
+          vu = skinny_scaled(vu, nu, colscale, colbias);
           out[(size_t)m * ldo + (n0 >> 1) + (ln >> 2)] = from_f32<TO>(glu_epilogue<false>(accumulate, vg, vu));   // (the activation's code)
         }
       }
@@ -591,11 +607,7 @@ gemm_skinny_mma_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_
       const int n = n0 + (ln >> 2) + (j >= 2 ? 8 : 0);
       const int m = (g0 + mg) * 8 + 2 * (ln & 3) + (j & 1);
       if (n < N && m < M) {
-        if (colscale) v *= colscale[n];
-        if (colbias) v += colbias[n];
-        TO* o = out + (size_t)m * ldo + n;
-        if (accumulate) v += to_f32(*o);
-        *o = from_f32<TO>(v);
+        skinny_store(v, n, out + (size_t)m * ldo + n, colscale, colbias, accumulate);
       }
     }
   }
@@ -686,8 +698,8 @@ gemm_skinny_two_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_
       for (int ww = 0; ww < SK_WARPS; ww++) { vg += red[i][ww][ln][j]; vu += red[i][ww][ln][j + 2]; }
       const int ng = n0 + (ln >> 2), nu = ng + 8, m = 2 * (ln & 3) + j;
       if (nu < N && m < M) {
-        if (colscale) { vg *= colscale[ng]; vu *= colscale[nu]; }
-        if (colbias) { vg += colbias[ng]; vu += colbias[nu]; }
+        vg = skinny_scaled(vg, ng, colscale, colbias);
+        vu = skinny_scaled(vu, nu, colscale, colbias);
         out[(size_t)m * ldo + (n0 >> 1) + (ln >> 2)] = from_f32<TO>(glu_epilogue<false>(accumulate, vg, vu));   // (the activation's code)
       }
     } else {
@@ -697,15 +709,137 @@ gemm_skinny_two_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_
       for (int ww = 0; ww < SK_WARPS; ww++) v += red[i][ww][ln][j];
       const int n = n0 + (ln >> 2) + (j >= 2 ? 8 : 0), m = 2 * (ln & 3) + (j & 1);
       if (n < N && m < M) {
-        if (colscale) v *= colscale[n];
-        if (colbias) v += colbias[n];
-        TO* o = out + (size_t)m * ldo + n;
-        if (accumulate) v += to_f32(*o);
-        *o = from_f32<TO>(v);
+        skinny_store(v, n, out + (size_t)m * ldo + n, colscale, colbias, accumulate);
       }
     }
   }
 }
+// 17 to 32 rows: the same sums on another division of the work.  The kernel above holds a round of weights and activations in
+// registers, which leaves one block of 17 and more rows an SM and 64 KB on their way (32 rows, 12288 -> 3072: 75 MB in 33 us).
+// Here a block is four of the 16 warps' shares of K of two tiles of 16 columns, and the blocks of a cluster of four are the 16: a
+// warp's weights and activations come by cp.async into a ring of its own, every thread its own pieces, so that nothing but
+// the copies' arrival holds a warp up, and an activation serves two tiles.  The 16 shares are added in their order by
+// the block whose values they are, read from the others' shared memory: the bits of the kernel above.
+struct RingSmem {
+  static constexpr int MG = 4, U = 4;                                // groups of 8 rows; steps of a share in a round, as above
+  static constexpr int TILES = 2, WARPS = 4;
+  static constexpr int D = 4;                                        // steps of a warp on their way
+  static constexpr int STAGE = (2 * TILES + MG) * 32;                // 16-byte pieces of a step: two rows a tile, MG groups of activation rows
+  static constexpr int SUMS = TILES * MG * 128;                      // a warp's sums (floats), in its ring when it is through
+  static constexpr int BYTES = WARPS * D * STAGE * 16;
+  static_assert(SUMS * 4 <= D * STAGE * 16, "the sums reuse the ring");
+};
+template <typename TO>
+__global__ void __launch_bounds__(128, 3)
+gemm_skinny_ring_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv_bfloat16* __restrict__ w, int ldw,
+                        TO* __restrict__ out, int ldo, const float* __restrict__ colscale, const float* __restrict__ colbias,
+                        TlcEpi accumulate, int M, int N, int K) {
+  asm volatile("griddepcontrol.launch_dependents;");
+  using S = RingSmem;
+  constexpr int D = S::D, MG = S::MG, U = S::U;
+  extern __shared__ __align__(16) uint4 ring_sm[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int rank = (int)(blockIdx.x & 3), n0 = (int)(blockIdx.x >> 2) * 32;    // clusters are runs of four blocks
+  const int share = rank * 4 + warp;                                 // which of the 16 shares of K
+  const int K8 = K >> 3, n_steps = (K8 + 3) >> 2;
+  uint4* ring = ring_sm + warp * D * S::STAGE + lane;
+  const uint4* wr[2 * S::TILES];
+#pragma unroll
+  for (int i = 0; i < 2 * S::TILES; i++) wr[i] = reinterpret_cast<const uint4*>(w + (size_t)min(n0 + 8 * i + g, N - 1) * ldw);   // clamped rows are never stored
+  // step i of this share; past its end the copies bring zeros to nobody
+  auto chunk_of = [&](int i) { return ((i / U) * SK_WARPS * U + share * U + i % U) * 4 + t; };
+  auto copy = [&](uint4* dst, const uint4* src, bool in) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
+  };
+  auto fetch_w = [&](int i) {
+    const int c = chunk_of(i);
+    const bool in = c < K8;
+#pragma unroll
+    for (int q = 0; q < 2 * S::TILES; q++) copy(ring + (i % D) * S::STAGE + q * 32, wr[q] + (in ? c : 0), in);
+  };
+  auto fetch_x = [&](int i) {
+    const int c = chunk_of(i);
+#pragma unroll
+    for (int mg = 0; mg < MG; mg++) {
+      const int row = mg * 8 + g;
+      const bool in = c < K8 && row < M;
+      copy(ring + (i % D) * S::STAGE + (2 * S::TILES + mg) * 32, reinterpret_cast<const uint4*>(a + (size_t)(in ? row : 0) * lda) + (in ? c : 0), in);
+    }
+  };
+  const int rounds = (n_steps + SK_WARPS * U - 1) / (SK_WARPS * U), last = n_steps - (rounds - 1) * SK_WARPS * U - share * U;
+  const int mine = (rounds - 1) * U + min(max(last, 0), U);          // this share's steps
+#pragma unroll
+  for (int i = 0; i < D; i++) if (i < mine) fetch_w(i);
+  tlc_wait(a, out);
+#pragma unroll
+  for (int i = 0; i < D; i++) {
+    if (i < mine) fetch_x(i);
+    asm volatile("cp.async.commit_group;" ::: "memory");             // (the weights of all of them go with the first)
+  }
+  float acc[S::TILES][MG][4];
+#pragma unroll
+  for (int i = 0; i < S::TILES; i++)
+#pragma unroll
+    for (int mg = 0; mg < MG; mg++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) acc[i][mg][j] = 0.f;
+#pragma unroll 1
+  for (int i = 0; i < mine; i++) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(D - 1) : "memory"); // (a thread reads its own pieces alone)
+    const uint4* st = ring + (i % D) * S::STAGE;
+    uint4 wv[2 * S::TILES];
+#pragma unroll
+    for (int q = 0; q < 2 * S::TILES; q++) wv[q] = st[q * 32];
+#pragma unroll
+    for (int mg = 0; mg < MG; mg++) {
+      const uint4 x = st[(2 * S::TILES + mg) * 32];
+#pragma unroll
+      for (int q = 0; q < S::TILES; q++) {
+        mma_bf16_16816(acc[q][mg], wv[2 * q].x, wv[2 * q + 1].x, wv[2 * q].y, wv[2 * q + 1].y, x.x, x.y);
+        mma_bf16_16816(acc[q][mg], wv[2 * q].z, wv[2 * q + 1].z, wv[2 * q].w, wv[2 * q + 1].w, x.z, x.w);
+      }
+    }
+    if (i + D < mine) { fetch_w(i + D); fetch_x(i + D); }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncwarp();
+  float* sums = reinterpret_cast<float*>(ring_sm + warp * D * S::STAGE);   // [tile][mg][lane][4]
+#pragma unroll
+  for (int q = 0; q < S::TILES; q++)
+#pragma unroll
+    for (int mg = 0; mg < MG; mg++)
+      *reinterpret_cast<float4*>(sums + ((q * MG + mg) * 32 + lane) * 4) = make_float4(acc[q][mg][0], acc[q][mg][1], acc[q][mg][2], acc[q][mg][3]);
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  const float* from[4];
+#pragma unroll
+  for (int r = 0; r < 4; r++) {
+    unsigned long long at;                                           // the same word in the block of rank r, for ordinary loads
+    asm("mapa.u64 %0, %1, %2;" : "=l"(at) : "l"((unsigned long long)(uintptr_t)ring_sm), "r"(r));
+    from[r] = reinterpret_cast<const float*>((uintptr_t)at);
+  }
+  // this block's quarter of the values
+  for (int idx = rank * (S::SUMS / 4) + threadIdx.x; idx < (rank + 1) * (S::SUMS / 4); idx += 128) {
+    const int j = idx & 3, ln = (idx >> 2) & 31, qm = idx >> 7;
+    float part[SK_WARPS];
+#pragma unroll
+    for (int ww = 0; ww < SK_WARPS; ww++) part[ww] = from[ww >> 2][(ww & 3) * D * S::STAGE * 4 + idx];
+    float v = 0.f;
+#pragma unroll
+    for (int ww = 0; ww < SK_WARPS; ww++) v += part[ww];
+    const int n = n0 + 16 * (qm / MG) + (ln >> 2) + (j >= 2 ? 8 : 0), m = qm % MG * 8 + 2 * (ln & 3) + (j & 1);
+    if (n < N && m < M) {
+      skinny_store(v, n, out + (size_t)m * ldo + n, colscale, colbias, accumulate);
+    }
+  }
+  // no block leaves while another may still read its sums
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+static int g_skinny_ring = 1;         // 0: never that division of the work (for comparisons)
+
 constexpr int SK_TWO_SMEM = 4 * 2 * SK_WARPS * 32 * (int)sizeof(uint4);
 static int g_skinny_two = 1;          // 0: never two tiles a block (for comparisons)
 
@@ -714,6 +848,7 @@ static int g_skinny_two = 1;          // 0: never two tiles a block (for compari
 template <typename TO> static bool simt_reserve() {
   const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
   return cudaFuncSetAttribute(gemm_tiled_f32x4_kernel<TO, 4, 4>, attr, ft_smem(4, 4)) == cudaSuccess &&
+         cudaFuncSetAttribute(gemm_skinny_ring_kernel<TO>, attr, RingSmem::BYTES) == cudaSuccess &&
          cudaFuncSetAttribute(gemm_skinny_two_kernel<TO, false>, attr, SK_TWO_SMEM) == cudaSuccess &&
          cudaFuncSetAttribute(gemm_skinny_two_kernel<TO, true>, attr, SK_TWO_SMEM) == cudaSuccess;
 }
@@ -770,6 +905,33 @@ static void launch_skinny_mg(const __nv_bfloat16* a, int lda, const __nv_bfloat1
       return;
     }
   }
+  if constexpr (MG == 4 && !SWIGLU) {
+    // Narrow outputs of a long K, all of whose blocks are resident at once.  Microseconds, the kernel below and the ring: 17 / 32
+    // rows of 5376 -> 2560 16.2 / 17.8 and 11.5 / 12.0, 8192 -> 2560 21.1 / 23.2 and 14.0 / 14.6, 4608 -> 3072 15.8 / 17.4 and 11.6 /
+    // 12.0, 12288 -> 3072 30.2 / 32.7 and 19.6 / 21.1, but 4096 -> 2048 (128 tiles) 7.3 / 7.9 and 9.0 / 9.2.  A captured step of the 3B
+    // sizes at batch 24 4057 and 3610, of the 7B sizes at batch 32 7041 and 5970.  (9 to 16 rows gained up to a tenth alone and
+    // lost in a step, beside kernels that want another split of the SM's memory: 3B at batch 16 3253 and 3728.)
+    static int sms = 0;
+    if (sms == 0) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
+    if (g_skinny_ring && (int)blocks > sms && (int)blocks <= 2 * sms && n_steps >= 128 && tlc_linear_simt_init() == 0) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((blocks + 1) / 2 * 4);
+      cfg.blockDim = dim3(128);
+      cfg.dynamicSmemBytes = RingSmem::BYTES;
+      cfg.stream = stream;
+      cudaLaunchAttribute attr[2];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = 4;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[1].val.programmaticStreamSerializationAllowed = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = g_tlc_pdl ? 2 : 1;
+      cudaLaunchKernelEx(&cfg, gemm_skinny_ring_kernel<TO>, a, lda, w, ldw, out, ldo, colscale, colbias, accumulate, M, N, K);
+      return;
+    }
+  }
   // U steps per warp and round: with one row group and U <= 4, or two and U = 2, two blocks fit on an SM
   // (a warp holds the weights and the activations of a round in registers)
   if (MG == 4 && blocks > 296)      // 17..32 rows, many row tiles: one step a round keeps two blocks on an SM
@@ -811,6 +973,7 @@ extern "C" int tlc_linear_skinny(const void* a, int lda, const void* w, int ldw,
 
 extern "C" void tlc_linear_skinny_pairs(int on) { g_skinny_pairs = on; }
 extern "C" void tlc_linear_skinny_two(int on) { g_skinny_two = on; }
+extern "C" void tlc_linear_skinny_ring(int on) { g_skinny_ring = on; }
 
 extern "C" int tlc_linear_skinny_swiglu(const void* a, int lda, const void* w, int ldw, void* out, int out_dtype, int ldo,
                                         const float* colscale, const float* colbias, int M, int N, int K, int act_code,

@@ -67,6 +67,7 @@ _SIGNATURES = {
     "tlc_linear_pair_override": (None, [_i]),
     "tlc_linear_skinny_pairs": (None, [_i]),
     "tlc_linear_skinny_two": (None, [_i]),
+    "tlc_linear_skinny_ring": (None, [_i]),
     "tlc_linear_tma_out": (None, [_i]),
     "tlc_linear_few_rows": (None, [_i]),
     "tlc_linear_few_rows_split": (None, [_i]),
@@ -697,6 +698,11 @@ def linear_skinny_pairs(on: bool) -> None:
 def linear_skinny_two(on: bool) -> None:
     """Whether the product of up to 8 rows may take two tiles a block (for comparisons)."""
     library().tlc_linear_skinny_two(int(bool(on)))
+
+
+def linear_skinny_ring(on: bool) -> None:
+    """Whether the product of 17 to 32 rows may share two tiles' K among a cluster of four blocks (for comparisons)."""
+    library().tlc_linear_skinny_ring(int(bool(on)))
 
 
 def linear_pairs() -> int:
