@@ -100,7 +100,7 @@ assert (out.double() - a.double() @ w.double().T).abs().max().item() < 72 * 2.0 
 
 
 def test_32_bit_products_without_the_set_up_of_the_tensor_core_kernels():
-    """A process that has not called tlc_linear_init: the 32-bit products need none (the tile with K in four parts takes more
+    """A process that has not called tlc_linear_init: the 32-bit products need none (tiles with shared K-steps take more
     shared memory than a kernel has unasked)."""
     import os
     import subprocess
@@ -178,3 +178,27 @@ def test_products_of_17_to_32_rows_shared_among_clusters_of_four(M, N, K):
     assert all(torch.equal(x, y) for x, y in zip(*got))
     assert torch.equal(got[0][0][:, N:], before[:, N:])
     _check(got[0][2][:, :N], a.float(), w.float(), None, None, None)
+
+
+@pytest.mark.parametrize("rows,split", [(32, 1), (32, 2), (32, 8), (64, 0), (64, 1), (64, 4), (64, 8)])
+@pytest.mark.parametrize("M,N,K", [(17, 132, 36), (33, 516, 260), (70, 1030, 132), (129, 257, 1028)])
+def test_32_bit_tiles_with_their_k_steps_shared(M, N, K, rows, split):
+    """Every tile with one block, some and eight (fewer K-steps than blocks, too), edges in part in both directions; sums added into
+    the output, overwritten, in 16 bits, into rows that are not on 16-byte boundaries."""
+    from tinyllama_c_b200 import ops
+    g = torch.Generator().manual_seed(M + N + K)
+    a, w = torch.randn(M, K, generator=g).cuda(), torch.randn(N, K, generator=g).cuda()
+    scale, bias, before = torch.randn(N, generator=g).cuda(), torch.randn(N, generator=g).cuda(), torch.randn(M + 1, N + 3, generator=g).cuda()
+    ops.linear_f32_tiles(rows, split)
+    try:
+        out, once, half = before.clone(), torch.full((M, N), float("nan"), device="cuda"), torch.full((M, N), float("nan"), device="cuda").bfloat16()
+        ops.linear(a, w, out[:M, :N], scale, bias, True)
+        ops.linear(a, w, once)
+        ops.linear(a, w, half, scale)
+        torch.cuda.synchronize()
+    finally:
+        ops.linear_f32_tiles(0)
+    _check(out[:M, :N], a, w, scale, bias, before[:M, :N])
+    _check(once, a, w, None, None, None)
+    _check(half, a, w, scale, None, None, True)
+    assert torch.equal(out[M], before[M]) and torch.equal(out[:, N:], before[:, N:])

@@ -231,30 +231,22 @@ __device__ __forceinline__ void fma_pair(float2& d, float2 a, float2 b) {
       : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
 }
 
-// Many rows: a tile of 64 rows x 16 CT columns, 128 threads with 8 x CT results each (CT 8 or 4); two K-steps of 16 in
-// shared memory, the next one in registers.  With KG = 4 four groups of 128 threads take a quarter of K each and the
-// first adds the others' sums to its own: outputs of few columns have too few tiles to keep an SM's schedulers busy.
-// 310 rows: 2048 -> 8192: 595 -> 313 us (33 TFLOP/s), 4096 -> 2048: 920 -> 264 us; 1,200 rows 1633 -> 879 and 1185 -> 622 us.
-// What bounds them: 310 rows of 2048 -> 8192 are 320 blocks of four warps, 0.7 of what the SMs hold at three blocks each (143
-// registers), so that a scheduler has one or two warps and waits for the pipes' latency; with K in four parts the warps wait for
-// shared memory (stalls per issue: short scoreboard 3.8 of 9) in blocks of which an SM holds one.
+// A tile of 64 rows x 128 columns, 128 threads with 8 x 8 results each; two K-steps of 16 in shared memory, the next one in
+// registers.  For outputs of many tiles: 600 rows of 2048 -> 8192 500 us (41 TFLOP/s), 1,200 879 us (46).
 constexpr int FT_M = 64, FT_K = 16, FT_LD = 4;
-template <typename TO, int CT, int KG>
-__global__ void __launch_bounds__(128 * KG)
+template <typename TO>
+__global__ void __launch_bounds__(128)
 gemm_tiled_f32x4_kernel(const float* __restrict__ a, int lda, const float* __restrict__ w, int ldw, TO* __restrict__ out,
                         int ldo, const float* __restrict__ colscale, const float* __restrict__ colbias, TlcEpi accumulate,
                         int M, int N, int K) {
   tlc_pdl(a, w, out);
-  constexpr int TN = 16 * CT, LA = FT_M + FT_LD, LW = TN + FT_LD;
+  constexpr int CT = 8, TN = 16 * CT, LA = FT_M + FT_LD, LW = TN + FT_LD;
   constexpr int PA = FT_M * FT_K / 4 / 128, PW = TN * FT_K / 4 / 128;   // 16-byte pieces a thread brings of each operand
-  extern __shared__ __align__(16) float ft_sm[];
-  const int grp = threadIdx.x >> 7, tid = threadIdx.x & 127;
-  float* As = ft_sm + grp * 2 * FT_K * (LA + LW);            // [2][FT_K][LA]
-  float* Ws = As + 2 * FT_K * LA;                            // [2][FT_K][LW]
+  __shared__ __align__(16) float As[2 * FT_K * LA], Ws[2 * FT_K * LW];    // [2][FT_K][LA], [2][FT_K][LW]
+  const int tid = threadIdx.x;
   const int m0 = blockIdx.y * FT_M, n0 = blockIdx.x * TN;
   const int tx = tid & 15, ty = tid >> 4;
-  const int steps = (K + FT_K - 1) / FT_K, per = (steps + KG - 1) / KG;
-  const int s_begin = min(steps, grp * per), s_end = min(steps, s_begin + per);
+  const int steps = (K + FT_K - 1) / FT_K;
   float4 ra[PA], rw[PW];
   auto load = [&](int s) {
 #pragma unroll
@@ -287,14 +279,14 @@ gemm_tiled_f32x4_kernel(const float* __restrict__ a, int lda, const float* __res
   for (int i = 0; i < 8; i++)
 #pragma unroll
     for (int j = 0; j < CT / 2; j++) acc[i][j] = make_float2(0.f, 0.f);
-  // all groups go through the same number of barriers
-  if (s_begin < s_end) { load(s_begin); store(0); }
+  load(0);
+  store(0);
   __syncthreads();
 #pragma unroll 1
-  for (int i = 0; i < per; i++) {
-    const int s = s_begin + i, buf = i & 1;
-    if (s + 1 < s_end) load(s + 1);
-    if (s < s_end) {
+  for (int s = 0; s < steps; s++) {
+    const int buf = s & 1;
+    if (s + 1 < steps) load(s + 1);
+    {
       const float* Ab = As + buf * FT_K * LA + ty * 8;
       const float* Wb = Ws + buf * FT_K * LW + tx * 4;
 #pragma unroll
@@ -314,34 +306,8 @@ gemm_tiled_f32x4_kernel(const float* __restrict__ a, int lda, const float* __res
           for (int j = 0; j < CT / 2; j++) fma_pair(acc[r][j], make_float2(av[r], av[r]), wv[j]);
       }
     }
-    if (s + 1 < s_end) store(buf ^ 1);
+    if (s + 1 < steps) store(buf ^ 1);
     __syncthreads();
-  }
-  if constexpr (KG > 1) {
-    float* part = ft_sm;                                     // the other groups' sums, [KG - 1][8 * CT][128]
-    if (grp > 0) {
-      float* mine = part + (grp - 1) * 8 * CT * 128 + tid;
-#pragma unroll
-      for (int i = 0; i < 8; i++)
-#pragma unroll
-        for (int j = 0; j < CT / 2; j++) {
-          mine[((i * CT) + 2 * j) * 128] = acc[i][j].x;
-          mine[((i * CT) + 2 * j + 1) * 128] = acc[i][j].y;
-        }
-    }
-    __syncthreads();
-    if (grp > 0) return;
-#pragma unroll
-    for (int q = 0; q < KG - 1; q++) {                       // in the order of K
-      const float* other = part + q * 8 * CT * 128 + tid;
-#pragma unroll
-      for (int i = 0; i < 8; i++)
-#pragma unroll
-        for (int j = 0; j < CT / 2; j++) {
-          acc[i][j].x += other[((i * CT) + 2 * j) * 128];
-          acc[i][j].y += other[((i * CT) + 2 * j + 1) * 128];
-        }
-    }
   }
 #pragma unroll
   for (int i = 0; i < 8; i++) {
@@ -360,8 +326,210 @@ gemm_tiled_f32x4_kernel(const float* __restrict__ a, int lda, const float* __res
     }
   }
 }
-constexpr int ft_smem(int CT, int KG) { return KG * 2 * FT_K * (FT_M + 16 * CT + 2 * FT_LD) * 4; }
-static_assert(ft_smem(4, 4) >= 3 * 8 * 4 * 128 * 4 && ft_smem(8, 1) <= 48 * 1024, "the other groups' sums reuse the operands' memory");
+// The same where the tiles are too few for the SMs, or fill their last round badly: a tile of 8 TM rows x 64 NC columns, 128 threads
+// with TM x 4 NC results each, K-steps of KS.  Rows of both operands lie turned by 32 / (KS / 4) values for every four of K,
+// which keeps the stores of the transposed pieces clear of bank conflicts.  `split` blocks of a thread-block cluster share a tile's
+// K-steps: each leaves its sums in its own shared memory, the cluster meets, and block r adds up its share of the rows over
+// all ranks, in their order, through distributed shared memory (the order follows from M, N and K alone).  K in four parts
+// within a block of 64 x 64 (or the tiles of 64 x 128), before, and this, microseconds: 4096 -> 2048 at 17 / 64 / 128 / 200 / 310 / 600 /
+// 1,200 rows 125 / 134 / 135 / 136 / 263 / 392 / 621 and 47 / 60 / 71 / 116 / 180 / 306 / 533, 2048 -> 8192 at 17 / 64 / 128 / 200 / 310
+// rows 66 / 71 / 138 / 267 / 313 and 40 / 67 / 119 / 240 / 296.  What bounds all of these tiles is a rate of about 42 TFLOP/s of the 74 that the FP32 lanes have: more
+// warps an SM (sixteen, 64 x 128), more results a thread (8 x 16) and operands stored twice so that no register
+// has to be doubled all came to 38 to 42.
+template <int TM, int NC, int KS> constexpr int fs_smem(int split) {
+  constexpr int FS_N = 64 * NC;
+  return (int)sizeof(float) * (split > 1 && 8 * TM * FS_N > 2 * KS * (8 * TM + FS_N) ? 8 * TM * FS_N : 2 * KS * (8 * TM + FS_N));   // (the sums reuse the operands' memory)
+}
+template <typename TO, int TM, int NC, int KS>
+__global__ void __launch_bounds__(128, TM == 8 ? 2 : 4)
+gemm_split_f32x4_kernel(const float* __restrict__ a, int lda, const float* __restrict__ w, int ldw, TO* __restrict__ out,
+                        int ldo, const float* __restrict__ colscale, const float* __restrict__ colbias, TlcEpi accumulate,
+                        int M, int N, int K, int split) {
+  tlc_pdl(a, w, out);
+  constexpr int FS_N = 64 * NC, ROWS = 8 * TM, PK = KS / 4, PW = FS_N * PK / 128;   // 16-byte pieces of a row; of the weights, a thread (of the activations one)
+  extern __shared__ __align__(16) float fs_sm[];
+  float* As = fs_sm;                                         // [2][KS][ROWS]
+  float* Ws = fs_sm + 2 * KS * ROWS;                       // [2][KS][FS_N]
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int rank = (int)blockIdx.x % split;                  // clusters are runs of `split` consecutive blocks
+  const int m0 = blockIdx.y * ROWS, n0 = (int)blockIdx.x / split * FS_N;
+  const int steps = (K + KS - 1) / KS;
+  const int s_begin = (int)((long long)steps * rank / split), s_end = (int)((long long)steps * (rank + 1) / split);
+  // this thread's pieces: rows past the matrices are clamped (what they make is not stored), K past its end reads as zero
+  static_assert(ROWS * PK == 128, "one piece of the activations a thread");
+  constexpr int TURN = 32 / PK;                              // by how much rows are turned for every four of K
+  const int q = tid / PK, kq = tid % PK * 4;
+  const float* pa = a + (size_t)min(m0 + q, M - 1) * lda + kq;
+  const float* pw[PW];
+#pragma unroll
+  for (int i = 0; i < PW; i++) pw[i] = w + (size_t)min(n0 + q + 128 / PK * i, N - 1) * ldw + kq;
+  float4 ra, rw[PW];
+  auto load = [&](int s) {
+    const bool in = s * KS + kq < K;                       // (K is a multiple of 4)
+    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    ra = in ? *reinterpret_cast<const float4*>(pa + s * KS) : z;
+#pragma unroll
+    for (int i = 0; i < PW; i++) rw[i] = in ? *reinterpret_cast<const float4*>(pw[i] + s * KS) : z;
+  };
+  auto store = [&](int buf) {
+    float* d = As + buf * KS * ROWS + kq * ROWS + ((q + TURN * (kq / 4)) & (ROWS - 1));
+    d[0] = ra.x; d[ROWS] = ra.y; d[2 * ROWS] = ra.z; d[3 * ROWS] = ra.w;
+#pragma unroll
+    for (int i = 0; i < PW; i++) {
+      const int c = q + 128 / PK * i;
+      d = Ws + buf * KS * FS_N + kq * FS_N + (c & ~63) + ((c + TURN * (kq / 4)) & 63);
+      d[0] = rw[i].x; d[FS_N] = rw[i].y; d[2 * FS_N] = rw[i].z; d[3 * FS_N] = rw[i].w;
+    }
+  };
+  float2 acc[TM][2 * NC];
+#pragma unroll
+  for (int i = 0; i < TM; i++)
+#pragma unroll
+    for (int j = 0; j < 2 * NC; j++) acc[i][j] = make_float2(0.f, 0.f);
+  if (s_begin < s_end) { load(s_begin); store(0); }
+  __syncthreads();
+#pragma unroll 1
+  for (int s = s_begin; s < s_end; s++) {
+    const int buf = (s - s_begin) & 1;
+    if (s + 1 < s_end) load(s + 1);
+#pragma unroll
+    for (int k = 0; k < KS; k++) {
+      const int turn = TURN * (k >> 2);
+      const float* Ab = As + (buf * KS + k) * ROWS + ((TM * ty + turn) & (ROWS - 1));
+      const float* Wb = Ws + (buf * KS + k) * FS_N + ((4 * tx + turn) & 63);
+      float av[TM];
+#pragma unroll
+      for (int h = 0; h < TM / 4; h++) {
+        const float4 v = *reinterpret_cast<const float4*>(Ab + 4 * h);
+        av[4 * h] = v.x; av[4 * h + 1] = v.y; av[4 * h + 2] = v.z; av[4 * h + 3] = v.w;
+      }
+#pragma unroll
+      for (int h = 0; h < NC; h++) {
+        const float4 v = *reinterpret_cast<const float4*>(Wb + 64 * h);
+#pragma unroll
+        for (int r = 0; r < TM; r++) {
+          fma_pair(acc[r][2 * h], make_float2(av[r], av[r]), make_float2(v.x, v.y));
+          fma_pair(acc[r][2 * h + 1], make_float2(av[r], av[r]), make_float2(v.z, v.w));
+        }
+      }
+    }
+    if (s + 1 < s_end) store(buf ^ 1);
+    __syncthreads();
+  }
+  // four columns of a row from their sum to the output
+  const bool vec = ldo % 4 == 0 && (uintptr_t)out % (4 * sizeof(TO)) == 0;
+  auto finish = [&](int m, int n, float4 v) {
+    const float x[4] = {v.x, v.y, v.z, v.w};
+    float y[4];
+    TO* o = out + (size_t)m * ldo + n;
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      y[c] = x[c];
+      if (n + c < N) {
+        if (colscale) y[c] *= colscale[n + c];
+        if (colbias) y[c] += colbias[n + c];
+        if (accumulate) y[c] += to_f32(o[c]);
+      }
+    }
+    if (std::is_same<TO, float>::value && vec && n + 4 <= N) {
+      *reinterpret_cast<float4*>(o) = make_float4(y[0], y[1], y[2], y[3]);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 4; c++)
+        if (n + c < N) o[c] = from_f32<TO>(y[c]);
+    }
+  };
+  if (split == 1) {
+#pragma unroll
+    for (int i = 0; i < TM; i++) {
+      const int m = m0 + ty * TM + i;
+      if (m >= M) break;
+#pragma unroll
+      for (int h = 0; h < NC; h++)
+        finish(m, n0 + 4 * tx + 64 * h, make_float4(acc[i][2 * h].x, acc[i][2 * h].y, acc[i][2 * h + 1].x, acc[i][2 * h + 1].y));
+    }
+    return;
+  }
+  // (the last barrier of the loop is behind every read of the operands)
+#pragma unroll
+  for (int i = 0; i < TM; i++)
+#pragma unroll
+    for (int h = 0; h < NC; h++)
+      *reinterpret_cast<float4*>(fs_sm + (ty * TM + i) * FS_N + 4 * tx + 64 * h) =
+          make_float4(acc[i][2 * h].x, acc[i][2 * h].y, acc[i][2 * h + 1].x, acc[i][2 * h + 1].y);
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  const int rows_per = ROWS / split, lane4 = (tid & 31) * 4;
+  const float* src[8];
+#pragma unroll
+  for (int r = 0; r < 8; r++) {
+    unsigned long long at;                                   // the same word in the block of rank r, for ordinary loads
+    asm("mapa.u64 %0, %1, %2;" : "=l"(at) : "l"((unsigned long long)(uintptr_t)fs_sm), "r"(min(r, split - 1)));
+    src[r] = reinterpret_cast<const float*>((uintptr_t)at);
+  }
+#pragma unroll 1
+  for (int i = tid >> 5; i < NC / 2 * rows_per; i += 4) {    // (128 columns of a row a warp)
+    const int row = rank * rows_per + i / (NC / 2), col = 128 * (i % (NC / 2)) + lane4;
+    if (m0 + row >= M) break;
+    float4 x[8];
+#pragma unroll
+    for (int r = 0; r < 8; r++)
+      x[r] = r < split ? *reinterpret_cast<const float4*>(src[r] + row * FS_N + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 v = x[0];
+#pragma unroll
+    for (int r = 1; r < 8; r++) { v.x += x[r].x; v.y += x[r].y; v.z += x[r].z; v.w += x[r].w; }   // absent ranks add zero
+    finish(m0 + row, n0 + col, v);
+  }
+  // no block leaves while another may still read its sums
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+static int g_f32_tile_rows = 0, g_f32_split = 0;             // test hooks: rows of a tile (32 or 64), blocks a tile; 0: chosen
+extern "C" void tlc_linear_f32_tiles(int rows, int split) { g_f32_tile_rows = rows; g_f32_split = split; }
+
+template <typename TO, int TM, int NC, int KS>
+static void launch_split_f32x4(const float* a, int lda, const float* w, int ldw, TO* out, int ldo, const float* colscale, const float* colbias,
+                               TlcEpi accumulate, int M, int N, int K, int split, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((N + 64 * NC - 1) / (64 * NC) * split, (M + 8 * TM - 1) / (8 * TM));
+  cfg.blockDim = dim3(128);
+  cfg.dynamicSmemBytes = fs_smem<TM, NC, KS>(split);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = g_tlc_pdl ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = split;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = split > 1 ? 2 : 1;
+  cudaLaunchKernelEx(&cfg, gemm_split_f32x4_kernel<TO, TM, NC, KS>, a, lda, w, ldw, out, ldo, colscale, colbias, accumulate, M, N, K, split);
+}
+
+// Which tiles 17 and more rows take.  In units of the time that a block of 64 x 256 columns with all of K takes beside a second one
+// on its SM: n blocks on the fullest SM cost 1, 1, 1.6, 2, 2.6, ... (a block alone is no quicker than two: the schedulers wait), a
+// cluster 0.012 for each of its blocks, and the tiles of 64 x 128, at two and more blocks an SM, 0.71, 0.935, 1.16, ... for 3,
+// 4, 5, ... on the fullest SM (fitted to 17 to 1,200 rows of 2048 -> 8192 and 4096 -> 2048).  No split below four: a block's
+// sums would be longer, and further off, than those of K in four parts were.  Tiles of 32 rows, eight blocks each, where
+// that makes no more than four blocks an SM.
+struct F32Plan { int rows, split; };                         // split 0: the tiles of 64 x 128
+static F32Plan f32_plan(int M, int N, int sms) {
+  if (g_f32_tile_rows) return F32Plan{g_f32_tile_rows == 32 ? 32 : 64, g_f32_split};
+  auto over = [](long long x, long long y) { return (x + y - 1) / y; };
+  if (over(N, 128) * over(M, 32) * 8 <= 4 * sms) return F32Plan{32, 8};
+  const long long whole = over(N, 128) * over(M, 64);
+  double cost = whole >= 2 * sms ? 0.225 * over(whole, sms) + 0.035 : 1e30;
+  F32Plan best{64, 0};
+  for (int split = 4; split <= 8; split *= 2) {
+    const long long f = over(over(N, 256) * over(M, 64) * split, sms);
+    const double c = (f <= 2 ? 1.0 : f / 2 + (f & 1 ? 0.6 : 0.0)) / split + 0.012 * split;
+    if (c < cost) { cost = c; best.split = split; }
+  }
+  return best;
+}
 
 int tlc_linear_simt_init();
 
@@ -371,19 +539,14 @@ static int launch_simt_f32x4(const float* a, int lda, const float* w, int ldw, T
   static int sms = 0;
   if (sms == 0) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
   if (M > 16) {
-    // 128 columns a tile where that still makes two blocks an SM, else 64 columns and K in four parts: 310 rows, 2048 -> 8192
-    // (320 tiles of 128 columns) 313 us, in the other form 339, 600 rows 501 and 605; 200 rows (256 tiles) 294 and 267, 310 rows
-    // of 4096 -> 2048 (80) 322 and 264.  From 17 rows on tiles: 17 rows of 2048 -> 8192 66 us, 32 rows 67, 64 rows 70; three or
-    // four launches of the other kernel would take 46 and 66 (of 4096 -> 2048: 125 and 127 us, 87 and 151).
-    const unsigned my = (unsigned)((M + FT_M - 1) / FT_M);
-    if ((long long)my * ((N + 127) / 128) >= 2 * sms)
-      tlc_launch(gemm_tiled_f32x4_kernel<TO, 8, 1>, dim3((N + 127) / 128, my), dim3(128), ft_smem(8, 1), stream, a, lda, w, ldw, out, ldo, colscale,
-                 colbias, accumulate, M, N, K);
-    else {
-      if (int rc = tlc_linear_simt_init()) return rc;
-      tlc_launch(gemm_tiled_f32x4_kernel<TO, 4, 4>, dim3((N + 63) / 64, my), dim3(512), ft_smem(4, 4), stream, a, lda, w, ldw, out, ldo, colscale,
-                 colbias, accumulate, M, N, K);
-    }
+    if (int rc = tlc_linear_simt_init()) return rc;
+    const F32Plan plan = f32_plan(M, N, sms);
+#define TLC_FS(TM_, NC_, KS_) launch_split_f32x4<TO, TM_, NC_, KS_>(a, lda, w, ldw, out, ldo, colscale, colbias, accumulate, M, N, K, plan.split, stream)
+    if (plan.rows == 32) TLC_FS(4, 2, 16);
+    else if (plan.split) TLC_FS(8, 4, 8);
+    else
+      tlc_launch(gemm_tiled_f32x4_kernel<TO>, dim3((N + 127) / 128, (M + 63) / 64), dim3(128), 0, stream, a, lda, w, ldw, out, ldo, colscale, colbias, accumulate, M, N, K);
+#undef TLC_FS
     TLC_CHECK_LAUNCH("linear(simt)");
     return 0;
   }
@@ -847,7 +1010,7 @@ static int g_skinny_two = 1;          // 0: never two tiles a block (for compari
 // first (tlc_linear_init), else with the first product that takes one of them.
 template <typename TO> static bool simt_reserve() {
   const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  return cudaFuncSetAttribute(gemm_tiled_f32x4_kernel<TO, 4, 4>, attr, ft_smem(4, 4)) == cudaSuccess &&
+  return cudaFuncSetAttribute(gemm_split_f32x4_kernel<TO, 8, 4, 8>, attr, fs_smem<8, 4, 8>(2)) == cudaSuccess &&
          cudaFuncSetAttribute(gemm_skinny_ring_kernel<TO>, attr, RingSmem::BYTES) == cudaSuccess &&
          cudaFuncSetAttribute(gemm_skinny_two_kernel<TO, false>, attr, SK_TWO_SMEM) == cudaSuccess &&
          cudaFuncSetAttribute(gemm_skinny_two_kernel<TO, true>, attr, SK_TWO_SMEM) == cudaSuccess;
@@ -857,7 +1020,7 @@ int tlc_linear_simt_init() {
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && ready[dev]) return 0;
-  if (!simt_reserve<float>() || !simt_reserve<__nv_bfloat16>()) return tlc_fail(-2, "linear: cannot reserve %d and %d bytes of shared memory", ft_smem(4, 4), SK_TWO_SMEM);
+  if (!simt_reserve<float>() || !simt_reserve<__nv_bfloat16>()) return tlc_fail(-2, "linear: cannot reserve %d and %d bytes of shared memory", fs_smem<8, 4, 8>(2), SK_TWO_SMEM);
   if (dev >= 0 && dev < 64) ready[dev] = true;
   return 0;
 }

@@ -74,6 +74,7 @@ _SIGNATURES = {
     "tlc_linear_few_rows_min_tiles": (None, [_i]),
     "tlc_linear_few_rows_max_rows": (None, [_i]),
     "tlc_linear_few_rows_ok": (_i, [_i, _i, _vp, _i, _i, _vp, _i, _i, _i]),
+    "tlc_linear_f32_tiles": (None, [_i, _i]),
     "tlc_linear_pairs": (_i, []),
     "tlc_rope_kv_store": (_i, [_vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i,
                                _i, _i, _vp]),
@@ -703,6 +704,12 @@ def linear_skinny_two(on: bool) -> None:
 def linear_skinny_ring(on: bool) -> None:
     """Whether the product of 17 to 32 rows may share two tiles' K among a cluster of four blocks (for comparisons)."""
     library().tlc_linear_skinny_ring(int(bool(on)))
+
+
+def linear_f32_tiles(rows: int, split: int = 0) -> None:
+    """32-bit products of more than 16 rows: tiles of 32 or 64 rows, `split` blocks a tile (64 and 0: the tiles of 64 x 128); 0: chosen
+    (for tests)."""
+    library().tlc_linear_f32_tiles(int(rows), int(split))
 
 
 def linear_pairs() -> int:
