@@ -1,6 +1,7 @@
 """Layers whose calls are made again from the first one's (models/repeat.py)."""
 import ctypes
 import random
+from types import SimpleNamespace
 
 import pytest
 import torch
@@ -10,6 +11,7 @@ from tinyllama_c_b200 import ops
 from tinyllama_c_b200.config import config_from_dict
 from tinyllama_c_b200.engine import StepEntry
 from tinyllama_c_b200.models.repeat import RepeatedLayers
+from tinyllama_c_b200.parts.base import Editable, LayerCache, LayerRun, StepInfo
 from tinyllama_c_b200.weights import build_model
 
 import configs
@@ -68,6 +70,79 @@ def test_the_table_of_calls_is_checked_before_the_first_call():
         fns = (ctypes.c_int * len(functions))(*functions)
         assert lib.tlc_replay(fns, words, n_words, len(functions), 1) < 0 and b"replay" in lib.tlc_last_error()
     assert lib.tlc_replay(None, None, 0, 0, 3) == 0
+
+
+class _Forks(Editable):
+    """A layer of four calls on the host: one on the caller's stream, one on a stream of its own between two events."""
+    entry = None
+
+    def __init__(self, number):
+        self.weight, self.gain = torch.ones(8), torch.ones(8)
+        self.side, self.fork, self.done = [0x1000 * (number + 1) + 0x100 * i for i in range(3)]
+
+    def repeats(self):
+        return frozenset(("side", "fork", "done"))
+
+    def handles(self, device):
+        return [self.side, self.fork, self.done]
+
+    def forward(self, x, step, cache, ready, wanted):
+        stream = lambda h: SimpleNamespace(cuda_stream=h)  # noqa: E731
+        event = lambda h: SimpleNamespace(cuda_event=h, record=lambda s: None)  # noqa: E731
+        waiting = lambda h: SimpleNamespace(cuda_stream=h, wait_event=lambda e: None)  # noqa: E731
+        norm = lambda w, h: ops._notes.calls.add("tlc_rmsnorm", (x.data_ptr(), 8, None, w.data_ptr(), 1e-5, 1, 8, x.data_ptr(), 0, h))  # noqa: E731
+        norm(self.weight, ops.stream_handle())
+        ops.record_event(event(self.fork), stream(ops.stream_handle()))
+        ops.wait_event(waiting(self.side), event(self.fork))
+        norm(self.gain, self.side)
+        ops.record_event(event(self.done), stream(self.side))
+        ops.wait_event(waiting(ops.stream_handle()), event(self.done))
+        return False
+
+
+def _run_on_the_host(monkeypatch, layers, stream):
+    """(entries that ran, [stream of every norm call made again]) of a step on a stream of that handle, and the words."""
+    got = []
+    monkeypatch.setattr(ops, "stream_handle", lambda: stream)
+    monkeypatch.setattr(ops, "replay", lambda functions, words, times: got.append((functions.copy(), words.copy())))
+    found = RepeatedLayers.of(layers, [LayerRun(i) for i in range(len(layers))])
+    i32 = torch.zeros(4, dtype=torch.int32)
+    step = StepInfo(1, 1, i32, i32, i32, i32, i32, i32)
+    done, left = found.run(torch.zeros(1, 8), step, SimpleNamespace(layer_view=lambda r, writes, kv: LayerCache()))
+    rows = [row for _, words in got for row in words.tolist()]
+    return done, rows
+
+
+def test_the_callers_stream_is_never_taken_for_a_layers_own(monkeypatch):
+    """torch hands out 32 streams in turn, and the layers have some of them: a step may run on a layer's own stream."""
+    layers = [_Forks(i) for i in range(4)]
+    norm_words, event_words = 10, 2
+    first, second = norm_words - 1, 2 * norm_words + 2 * event_words - 1     # where the streams of the two norm calls stand
+    for stream in (0, 0x77, layers[2].side):
+        done, rows = _run_on_the_host(monkeypatch, layers, stream)
+        assert done == 4 and [row[first] for row in rows] == [stream] * 3
+        assert [row[second] for row in rows] == [layer.side for layer in layers[1:]]
+    # the first layer's own: the words do not say which of the two is meant, so the layers run one by one
+    done, rows = _run_on_the_host(monkeypatch, layers, layers[0].side)
+    assert (done, rows) == (1, [])
+
+
+@pytest.mark.gpu
+def test_a_step_on_a_layers_own_stream_gives_the_same_bits():
+    model = _model("tensor cores", torch.bfloat16, "cuda:0")
+    r = random.Random(6)
+    tokens = [[r.randrange(SIZES["tensor cores"]["vocab_size"]) for _ in range(n)] for n in (40, 150, 20)]
+    got = []
+    for stream in (lambda: torch.cuda.current_stream(), lambda: model.layers[0]._side[0], lambda: model.layers[2]._side[0]):
+        llm = tlc.LLM(model, dtype="bfloat16", max_tokens=64 * 16, max_seqs=3)
+        slots = [llm.cache.acquire() for _ in tokens]
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream()):
+            out = [llm.step([StepEntry(s, t, (len(t) - 1,)) for s, t in zip(slots, tokens)]) for _ in range(2)]
+        torch.cuda.synchronize()
+        got.append([t.clone() for t in out] + [g.data.clone() for g in llm.cache.state_groups])
+    for other in got[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(got[0], other))
 
 
 @pytest.mark.gpu

@@ -10,8 +10,8 @@ own weights and their own part of the cache in place of the first one's, and are
 Nothing is kept from one step for the next but the description of the layers, which an edit of any of their parts makes
 void; the tensors' addresses, types, shapes and strides are read in every step.  A pointer that is neither one of the
 first layer's tensors nor something that all layers share (the stream of rows, the step's tables and temporaries) ends the
-attempt: the layers then run one by one, as they do under capture, on other devices and with parts that do not
-say that they can be repeated.
+attempt, and so does a caller's stream that is one of the first layer's own: the layers then run one by one, as they do under
+capture, on other devices and with parts that do not say that they can be repeated.
 """
 from __future__ import annotations
 
@@ -116,6 +116,8 @@ class RepeatedLayers:
             if p:
                 at.setdefault(p, i)
         handles = [layer.handles(x.device) if notes.forks else () for layer in self.layers]
+        if notes.forks and ops.stream_handle() in handles[0]:
+            return done, left       # the caller's stream (one of the few that torch hands out) is the first layer's own: a word cannot say which is meant
         for i, p in enumerate(handles[0]):
             at[p] = len(firsts) + i
         common = self._shared(x, step, notes)

@@ -335,6 +335,11 @@ def _stream() -> int:
     return torch.cuda.current_stream().cuda_stream
 
 
+def stream_handle() -> int:
+    """The handle of the stream that calls are made on."""
+    return _stream()
+
+
 def dtype_code(dt: torch.dtype) -> int:
     if dt == torch.float32:
         return F32
