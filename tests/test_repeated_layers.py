@@ -8,6 +8,7 @@ import torch
 
 import tinyllama_c_b200 as tlc
 from tinyllama_c_b200 import ops
+from tinyllama_c_b200.models import repeat
 from tinyllama_c_b200.config import config_from_dict
 from tinyllama_c_b200.engine import StepEntry
 from tinyllama_c_b200.models.repeat import RepeatedLayers
@@ -86,7 +87,7 @@ class _Forks(Editable):
     def handles(self, device):
         return [self.side, self.fork, self.done]
 
-    def forward(self, x, step, cache, ready, wanted):
+    def forward(self, x, step, cache, ready, wanted, scratch=()):
         stream = lambda h: SimpleNamespace(cuda_stream=h)  # noqa: E731
         event = lambda h: SimpleNamespace(cuda_event=h, record=lambda s: None)  # noqa: E731
         waiting = lambda h: SimpleNamespace(cuda_stream=h, wait_event=lambda e: None)  # noqa: E731
@@ -94,6 +95,7 @@ class _Forks(Editable):
         norm(self.weight, ops.stream_handle())
         ops.record_event(event(self.fork), stream(ops.stream_handle()))
         ops.wait_event(waiting(self.side), event(self.fork))
+        ops._note_owned(*scratch)
         norm(self.gain, self.side)
         ops.record_event(event(self.done), stream(self.side))
         ops.wait_event(waiting(ops.stream_handle()), event(self.done))
@@ -125,6 +127,30 @@ def test_the_callers_stream_is_never_taken_for_a_layers_own(monkeypatch):
     # the first layer's own: the words do not say which of the two is meant, so the layers run one by one
     done, rows = _run_on_the_host(monkeypatch, layers, layers[0].side)
     assert (done, rows) == (1, [])
+
+
+def test_scratch_of_repeated_calls_is_kept_until_the_callers_stream_is_through(monkeypatch):
+    """It was allocated on the first layer's own stream, where others may be handed it, and every layer's stream uses it."""
+    seen = []
+
+    class OnGpu(torch.Tensor):
+        is_cuda = True
+
+        def record_stream(self, stream):
+            seen.append((self.data_ptr(), stream))
+
+    scratch = torch.zeros(8).as_subclass(OnGpu)
+
+    class Layer(_Forks):
+        def repeats(self):
+            return super().repeats()
+
+        def forward(self, *args):
+            return super().forward(*args, scratch=(scratch,))
+
+    monkeypatch.setattr(repeat, "current_stream", lambda device: "the caller's")
+    done, rows = _run_on_the_host(monkeypatch, [Layer(i) for i in range(3)], 0x77)
+    assert done == 3 and len(rows) == 2 and seen == [(scratch.data_ptr(), "the caller's")]
 
 
 @pytest.mark.gpu

@@ -22,7 +22,7 @@ import numpy as np
 import torch
 
 from .. import ops
-from ..parts.base import Editable, LayerCache, StepInfo
+from ..parts.base import Editable, LayerCache, StepInfo, current_stream, used_on
 
 
 class _Unlike(Exception):
@@ -142,6 +142,9 @@ class RepeatedLayers:
         like = self._meta([firsts[i] for i in tensors])
         base = np.array([addresses[i] for i in tensors], dtype=np.uint64)
         first, functions = np.array(notes.words, dtype=np.uint64), np.array(notes.functions, dtype=np.int32)
+        # The calls' own scratch came from the stream that the first layer made them on; the others use it on theirs.
+        if notes.owned:
+            used_on(current_stream(x.device), notes.owned)
         columns = [rank[i] for i in which]
         # the next layer at once, so that the GPU has work while the others' addresses are gathered, then a few, then the rest
         # (all 23 in one go: 0.35 ms of a prompt of 2,048 tokens in which the GPU waits)

@@ -338,6 +338,14 @@ def current_stream(device) -> "torch.cuda.Stream":
     return hit
 
 
+def used_on(stream: "torch.cuda.Stream", tensors) -> None:
+    """Buffers that were allocated while another stream was current, and whose every use is over once `stream` has come to where
+    they are let go: the allocator hands them out again only then (it asks the stream they were allocated on alone, unasked)."""
+    for t in tensors:
+        if isinstance(t, torch.Tensor) and t.is_cuda:
+            t.record_stream(stream)
+
+
 class SideStream:
     """A stream of its own for work that runs beside what its caller launches next: run(f) starts after everything launched on
     the current stream so far, join() makes the current stream wait for it.  (Under stream capture: a branch of the graph.)"""
