@@ -241,3 +241,31 @@ def test_a_steps_temporaries_are_shared_inside_the_step_only():
         assert scratch_buf("a", (2, 3), torch.float32, "cpu") is a
     assert len(step.scratch) == 4 and len(other.scratch) == 1
     assert scratch_buf("a", (2, 3), torch.float32, "cpu") is not a
+
+
+def test_a_temporary_that_a_side_stream_asks_for_first_is_kept_for_the_models_stream(monkeypatch):
+    """It comes from the side stream's pool, whose next taker need not wait for the layers that used it."""
+    import types
+    from tinyllama_c_b200.parts import base
+    seen, streams = [], ["main"]
+
+    class OnGpu(torch.Tensor):
+        is_cuda = True
+
+        def record_stream(self, stream):
+            seen.append((self.numel(), stream))
+
+    empty = torch.empty
+    monkeypatch.setattr(base, "current_stream", lambda device: streams[-1])
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: streams[0] == "captured")
+    monkeypatch.setattr(torch, "empty", lambda shape, dtype, device: empty(shape, dtype=dtype).as_subclass(OnGpu))
+    for streams[0] in ("main", "captured"):
+        step = types.SimpleNamespace(scratch={}, tokens=types.SimpleNamespace(device=torch.device("cuda:0")))
+        with base.step_scratch(step):
+            base.scratch_buf("a", (1,), torch.float32, "cuda:0")
+            streams.append("side")
+            for _ in range(2):
+                base.scratch_buf("b", (2,), torch.float32, "cuda:0")
+            streams.pop()
+            base.scratch_buf("b", (2,), torch.float32, "cuda:0")
+    assert seen == [(2, "main")]          # (a captured step keeps its temporaries for as long as its graph lives)

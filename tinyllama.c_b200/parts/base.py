@@ -280,23 +280,28 @@ def act_empty(shape, like: torch.Tensor, dtype: Optional[torch.dtype] = None) ->
 # waited for before the layer's output projection), and a kernel writes only after its wait on its predecessor.
 # Two buffers that are alive at the same time carry different tags.  The buffers go when the step's StepInfo
 # goes (a captured step keeps its StepInfo, and so its buffers, for as long as the graph lives).
+# A buffer that is first asked for while a layer's side stream is current comes from that stream's pool, and the other layers use it
+# on their own: it is marked as used on the model's stream (used_on).
 _scratch: Optional[dict] = None
+_scratch_stream: Optional["torch.cuda.Stream"] = None       # the model's stream (None: on the host, or under capture)
 
 
 class step_scratch:
     """Context manager: temporaries asked for inside come from (and stay in) `step.scratch`."""
 
     def __init__(self, step: "StepInfo"):
-        self.store = step.scratch
+        self.store, self.device = step.scratch, step.tokens.device
 
     def __enter__(self):
-        global _scratch
-        self.before, _scratch = _scratch, self.store
+        global _scratch, _scratch_stream
+        self.before = _scratch, _scratch_stream
+        eager = self.device.type == "cuda" and not torch.cuda.is_current_stream_capturing()
+        _scratch, _scratch_stream = self.store, current_stream(self.device) if eager else None
         return self
 
     def __exit__(self, *exc):
-        global _scratch
-        _scratch = self.before
+        global _scratch, _scratch_stream
+        _scratch, _scratch_stream = self.before
         return False
 
 
@@ -314,6 +319,8 @@ def scratch_buf(tag: str, shape, dtype: torch.dtype, device) -> torch.Tensor:
     t = _scratch.get(key)
     if t is None:
         t = _scratch[key] = torch.empty(shape, dtype=dtype, device=device)
+        if _scratch_stream is not None and current_stream(t.device) != _scratch_stream:
+            used_on(_scratch_stream, (t,))
     return t
 
 
