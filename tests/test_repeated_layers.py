@@ -153,6 +153,25 @@ def test_scratch_of_repeated_calls_is_kept_until_the_callers_stream_is_through(m
     assert done == 3 and len(rows) == 2 and seen == [(scratch.data_ptr(), "the caller's")]
 
 
+def test_tensors_that_share_an_address_in_one_layer_only(monkeypatch):
+    """Two weights of the first layer that are one tensor: its calls do not say which is meant."""
+    tied = [_Forks(i) for i in range(4)]
+    for layer in tied:
+        layer.gain = layer.weight
+    done, rows = _run_on_the_host(monkeypatch, tied, 0x77)
+    assert done == 4 and [(row[3], row[17]) for row in rows] == [(l.weight.data_ptr(),) * 2 for l in tied[1:]]
+    others = [_Forks(i) for i in range(4)]
+    others[2].gain = others[2].weight                    # (its own words say so)
+    done, rows = _run_on_the_host(monkeypatch, others, 0x77)
+    assert done == 4 and [(row[3], row[17]) for row in rows] == [(l.weight.data_ptr(), l.gain.data_ptr()) for l in others[1:]]
+    first = [_Forks(i) for i in range(4)]
+    first[0].gain = first[0].weight
+    assert _run_on_the_host(monkeypatch, first, 0x77) == (1, [])
+    tied[3].gain = torch.ones(8)                         # the last one's are two: the layers before it are repeated
+    done, rows = _run_on_the_host(monkeypatch, tied, 0x77)
+    assert done == 1 + len(rows) <= 3
+
+
 @pytest.mark.gpu
 def test_a_step_on_a_layers_own_stream_gives_the_same_bits():
     model = _model("tensor cores", torch.bfloat16, "cuda:0")

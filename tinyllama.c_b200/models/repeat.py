@@ -110,11 +110,11 @@ class RepeatedLayers:
                 return done, left
         form, mine = _of_cache(views[0])
         firsts = self.tensors[0] + mine
-        at = {}                                            # address -> which of the first layer's tensors
+        at, also = {}, {}                                  # address -> which of the first layer's tensors; which others start there
         addresses = list(map(_ptr, firsts))
         for i, p in enumerate(addresses):
-            if p:
-                at.setdefault(p, i)
+            if p and at.setdefault(p, i) != i:
+                also.setdefault(p, []).append(i)
         handles = [layer.handles(x.device) if notes.forks else () for layer in self.layers]
         if notes.forks and ops.stream_handle() in handles[0]:
             return done, left       # the caller's stream (one of the few that torch hands out) is the first layer's own: a word cannot say which is meant
@@ -136,8 +136,11 @@ class RepeatedLayers:
                 ranges = [(_ptr(t), _ptr(t) + t.untyped_storage().nbytes() - t.storage_offset() * t.element_size()) for t in common]
             if not any(lo <= word < hi for lo, hi in ranges):
                 return done, left
-        used = sorted(set(which))
+        # a word says which address is meant, not which of the tensors that start there: they have to in every layer
+        ties = [(i, j) for i in set(which) if i < len(firsts) for j in also.get(addresses[i], ())]
+        used = sorted(set(which).union(j for _, j in ties))
         rank = {i: n for n, i in enumerate(used)}
+        tied = [[rank[i] for i, _ in ties], [rank[j] for _, j in ties]]
         tensors = [i for i in used if i < len(firsts)]      # (the layers' own streams and events come behind them)
         like = self._meta([firsts[i] for i in tensors])
         base = np.array([addresses[i] for i in tensors], dtype=np.uint64)
@@ -160,6 +163,8 @@ class RepeatedLayers:
                 table[r - done] = list(map(_ptr, row)) + [handles[r][i - len(firsts)] for i in used[len(tensors):]]
             if ((table[:, :len(tensors)] ^ base) & np.uint64(15)).any() or not table.all():
                 return done, left                          # (the calls may choose by how their operands are aligned)
+            if (table[:, tied[0]] != table[:, tied[1]]).any():
+                return done, left
             words = np.tile(first, (end - done, 1))
             words[:, places] = table[:, columns]
             ops.replay(functions, words, end - done)
