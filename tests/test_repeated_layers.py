@@ -53,6 +53,63 @@ def test_like_layers_are_found_and_an_edit_is_noticed(name):
         assert found is not None and found.stands()
 
 
+def test_edits_in_lists_are_noticed_and_one_that_is_undone_stands_again():
+    model, other = _model("small", torch.bfloat16, "cpu"), _model("small", torch.bfloat16, "cpu")
+    layers, block = model.layers, model.layers[2]
+    look = lambda: RepeatedLayers(model.layers, model.schedule)  # noqa: E731
+    stands = lambda found: found.stands(model.layers, model.schedule)  # noqa: E731
+    # a list (or the model's attribute), what is put in its place, and whether the layers are alike then
+    for where, at, new, alike in ((layers, 2, other.layers[2], True), (block.mixers, 0, other.layers[2].mixers[0], True),
+                                  (block.out_scales, 1, 0.5, False), (block.out_offsets, 0, (8, 64), False),
+                                  (model.schedule, 1, LayerRun(1, cache=0), False)):
+        found, before = look(), where[at]
+        assert found.alike and stands(found)
+        where[at] = new
+        assert not stands(found) and look().alike == alike
+        edited = look()
+        where[at] = before
+        assert not stands(edited) and look().alike
+    found = look()
+    model.layers = list(layers)
+    assert not stands(found) and look().alike
+    found = look()
+    model.layers.append(model.layers.pop())
+    assert stands(found)                                  # (the same again)
+    model.layers.append(other.layers[0])
+    assert not stands(found) and look().alike
+    found = look()
+    del block.ffn.limit
+    assert not stands(found) and not look().alike
+
+
+@pytest.mark.gpu
+def test_a_step_runs_the_layers_and_mixers_that_are_there_now():
+    """A layer and a mixer put in another's place count from the next prompt on, and so does taking them back."""
+    model = _model("tensor cores", torch.bfloat16, "cuda:0")
+    other = _model("tensor cores", torch.bfloat16, "cuda:0")
+    for layer in other.layers:
+        layer.ffn.down.weight = layer.ffn.down.weight * 0.5
+        layer.mixers[1].D = layer.mixers[1].D + 1.0
+    llm = tlc.LLM(model, dtype="bfloat16", max_tokens=64 * 8, max_seqs=2)
+
+    def logits():
+        slot = llm.cache.acquire()
+        out = llm.step([StepEntry(slot, list(range(1, 60)), (58,))]).clone()
+        llm.cache.release(slot)
+        return out
+
+    first = logits()
+    for where, at, new in ((model.layers, 2, other.layers[2]), (model.layers[1].mixers, 1, other.layers[1].mixers[1])):
+        before, where[at] = where[at], new
+        changed = logits()
+        repeated, model.repeated = model.repeated, None
+        one_by_one = logits()
+        model.repeated = repeated
+        assert torch.equal(changed, one_by_one) and not torch.equal(changed, first)
+        where[at] = before
+        assert torch.equal(logits(), first) and model.repeated.alike
+
+
 def test_parts_that_say_nothing_are_not_repeated():
     model = _model("small", torch.float32, "cpu")
 

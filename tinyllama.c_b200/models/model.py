@@ -65,7 +65,7 @@ class Model:
         self.by_table: List[MoEFeedForward] = []
         self.dtype: Optional[torch.dtype] = None
         self.device: Optional[torch.device] = None
-        self.repeated: Optional[RepeatedLayers] = None      # the run order's layers, where they are all alike
+        self.repeated: Optional[RepeatedLayers] = None      # the run order's layers, where they were all alike when bound
 
     def _collect_chunks(self) -> None:
         """What the layers ask the step function for."""
@@ -147,11 +147,12 @@ class Model:
             MoEFeedForward.route_step(self.by_table, self.expert_tables, step)
         with step_scratch(step):                       # the layers share the step's temporaries
             ready, done = False, 0                     # whether a layer left the next one's input (Block.entry)
-            if self.repeated is not None and not torch.cuda.is_current_stream_capturing():
-                if not self.repeated.stands():
-                    self.repeated = RepeatedLayers.of(self.layers, self.schedule)
-                if self.repeated is not None:
-                    done, ready = self.repeated.run(x, step, cache)
+            repeated = self.repeated
+            if repeated is not None and not torch.cuda.is_current_stream_capturing():
+                if not repeated.stands(self.layers, self.schedule):
+                    repeated = self.repeated = RepeatedLayers(self.layers, self.schedule)
+                if repeated.alike:
+                    done, ready = repeated.run(x, step, cache)
             for r in range(done, len(self.schedule)):
                 run = self.schedule[r]
                 if run.add is not None:            # a learned row joins the stream before this entry (a pass of a repeated range)

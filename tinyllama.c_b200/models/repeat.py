@@ -7,11 +7,12 @@ needs 1 to 2.5.  Where all layers of the run order are alike (the same parts of 
 types, shapes and strides), the first one runs as ever and its calls are noted; the others' are the same calls with their
 own weights and their own part of the cache in place of the first one's, and are made by the library in one go.
 
-Nothing is kept from one step for the next but the description of the layers, which an edit of any of their parts makes
-void; the tensors' addresses, types, shapes and strides are read in every step.  A pointer that is neither one of the
-first layer's tensors nor something that all layers share (the stream of rows, the step's tables and temporaries) ends the
-attempt, and so does a caller's stream that is one of the first layer's own: the layers then run one by one, as they do under
-capture, on other devices and with parts that do not say that they can be repeated.
+Nothing is kept from one step for the next but the description of the layers, which is made anew when a part of theirs, a list
+of parts or numbers, or the list of the layers itself has been edited; the tensors' addresses, types, shapes and strides are
+read in every step.  A pointer that is neither one of the first layer's tensors nor something that all layers share (the
+stream of rows, the step's tables and temporaries) ends the attempt, and so does a caller's stream that is one of the first
+layer's own: the layers then run one by one, as they do under capture, on other devices and with parts that do not say that
+they can be repeated.
 """
 from __future__ import annotations
 
@@ -25,35 +26,46 @@ from .. import ops
 from ..parts.base import Editable, LayerCache, StepInfo, current_stream, used_on
 
 
-class _Unlike(Exception):
-    pass
-
-
 _PLAIN = (type(None), bool, int, float, str, torch.dtype, torch.device)
 _edits = attrgetter("edits")
 _ptr, _size, _stride, _dtype = torch.Tensor.data_ptr, torch.Tensor.size, torch.Tensor.stride, attrgetter("dtype")
 
 
-def _describe(obj, tensors: List[torch.Tensor], parts: List[Editable]):
-    """A value that is equal for two objects whose calls differ in their tensors' addresses alone; collects the tensors, in
-    the order in which they come up, and the parts whose edits would change it."""
-    if isinstance(obj, _PLAIN):
-        return type(obj), obj
-    if isinstance(obj, torch.Tensor):
-        tensors.append(obj)
-        return "tensor", obj.dtype, tuple(obj.shape), obj.stride(), obj.device
-    if isinstance(obj, (list, tuple)):
-        return type(obj), tuple(_describe(o, tensors, parts) for o in obj)
-    if isinstance(obj, dict):
-        return dict, tuple((k, _describe(v, tensors, parts)) for k, v in sorted(obj.items()))
-    if isinstance(obj, Editable):
-        aside = obj.repeats()
-        if aside is None or "repeats" not in type(obj).__dict__:      # (a class derived from such a part speaks for itself)
-            raise _Unlike
-        parts.append(obj)
-        return type(obj), tuple((k, _describe(v, tensors, parts)) for k, v in sorted(vars(obj).items())
-                                if k not in aside and k != "edits")
-    raise _Unlike
+class _Description:
+    """What a layer is made of: a form that is equal for two layers whose calls differ in their tensors' addresses alone, the
+    tensors in the order in which they come up, and what an edit goes through: the parts (their attributes) and the lists."""
+
+    def __init__(self, layer, parts: List[Editable], lists: list):
+        self.tensors: List[torch.Tensor] = []
+        self.parts, self.lists = parts, lists
+        self.known, self.inside = True, set()            # known: whether every part says that it can be repeated
+        self.form = self._of(layer)
+
+    def _of(self, obj):
+        if isinstance(obj, _PLAIN):
+            return type(obj), obj
+        if isinstance(obj, torch.Tensor):
+            self.tensors.append(obj)
+            return "tensor", obj.dtype, tuple(obj.shape), obj.stride(), obj.device
+        if id(obj) in self.inside or not isinstance(obj, (list, tuple, dict, Editable)):
+            self.known = False
+            return type(obj), id(obj)
+        self.inside.add(id(obj))
+        try:
+            if not isinstance(obj, Editable):
+                items = list(obj.values() if isinstance(obj, dict) else obj)
+                if any(isinstance(v, torch.Tensor) for v in items):
+                    self.known = False                    # (compared with a list of old, a tensor compares its values)
+                elif not isinstance(obj, tuple):
+                    self.lists.append(obj)
+                return type(obj), tuple(obj) if isinstance(obj, dict) else None, tuple(map(self._of, items))
+            self.parts.append(obj)
+            aside = obj.repeats()
+            if aside is None or "repeats" not in type(obj).__dict__:      # (a class derived from such a part speaks for itself)
+                self.known, aside = False, ()
+            return type(obj), tuple((k, self._of(v)) for k, v in sorted(vars(obj).items()) if k not in aside and k != "edits")
+        finally:
+            self.inside.remove(id(obj))
 
 
 def _of_cache(view: LayerCache) -> Tuple[tuple, List[torch.Tensor]]:
@@ -75,24 +87,18 @@ class RepeatedLayers:
     @staticmethod
     def of(layers, schedule) -> Optional["RepeatedLayers"]:
         """None where the run order is more than one pass of like layers, each with a cache of its own."""
-        if len(schedule) < 3 or any(r.cache is not None or r.kv_cache is not None or r.add is not None or r.add_embedding for r in schedule):
-            return None
-        self = RepeatedLayers()
+        found = RepeatedLayers(layers, schedule)
+        return found if found.alike else None
+
+    def __init__(self, layers, schedule):
+        self.order = layers, schedule
+        self.parts, self.lists = [], [layers, schedule]
         self.layers = [layers[r.layer] for r in schedule]
-        self.tensors, self.parts, first = [], [], None
-        try:
-            for layer in self.layers:
-                mine: List[torch.Tensor] = []
-                form = _describe(layer, mine, self.parts)
-                if first is None:
-                    first = form
-                elif form != first:
-                    return None
-                self.tensors.append(mine)
-        except _Unlike:
-            return None
-        self.edits = list(map(_edits, self.parts))
-        return self
+        found = [_Description(layer, self.parts, self.lists) for layer in self.layers]
+        self.tensors = [d.tensors for d in found]
+        self.alike = len(found) >= 3 and all(d.known and d.form == found[0].form for d in found) \
+            and not any(r.cache is not None or r.kv_cache is not None or r.add is not None or r.add_embedding for r in schedule)
+        self.edits, self.copies = list(map(_edits, self.parts)), [l if isinstance(l, tuple) else l.copy() for l in self.lists]
 
     def run(self, x: torch.Tensor, step: StepInfo, cache) -> Tuple[int, bool]:
         """Runs the first layer, and the others if they can be repeated; (how many entries of the run order have run,
@@ -171,9 +177,11 @@ class RepeatedLayers:
             done = end
         return n, False
 
-    def stands(self) -> bool:
-        """Whether no part has been edited since the layers were found alike."""
-        return list(map(_edits, self.parts)) == self.edits
+    def stands(self, layers=None, schedule=None) -> bool:
+        """Whether nothing has been edited since the layers were looked at: no attribute of a part, no list or what is in it, and
+        these (where given) are the lists that were looked at."""
+        return (layers is None or layers is self.order[0]) and (schedule is None or schedule is self.order[1]) \
+            and list(map(_edits, self.parts)) == self.edits and self.lists == self.copies
 
     @staticmethod
     def _meta(tensors):

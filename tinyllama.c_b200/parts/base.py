@@ -125,7 +125,7 @@ class LayerCache:
 
 
 class Editable:
-    """Counts how often its attributes are set, so that what was found out about it (models/repeat.py) can be dropped."""
+    """Counts how often its attributes are set or deleted, so that what was found out about it (models/repeat.py) can be dropped."""
     edits = 0
     passing = frozenset()        # attributes that a forward() sets for itself
 
@@ -133,6 +133,10 @@ class Editable:
         object.__setattr__(self, name, value)
         if name not in self.passing:
             object.__setattr__(self, "edits", self.edits + 1)
+
+    def __delattr__(self, name):
+        object.__delattr__(self, name)
+        object.__setattr__(self, "edits", self.edits + 1)
 
     def repeats(self) -> Optional[frozenset]:
         """For a part whose forward() makes the same calls of the kernel library (and no other GPU work) whatever it is
