@@ -110,6 +110,31 @@ def test_a_step_runs_the_layers_and_mixers_that_are_there_now():
         assert torch.equal(logits(), first) and model.repeated.alike
 
 
+def test_a_copy_that_torch_makes_ends_the_attempt(monkeypatch):
+    """A weight that is multiplied by as a dense copy: the copy's address stands for nothing in the other layers."""
+    monkeypatch.setattr(ops, "linear", lambda *args: None)
+    down = _model("small", torch.bfloat16, "cpu").layers[0].ffn.down
+    for weight, complete in ((down.weight, True), (down.weight.t().contiguous().t(), False)):
+        down.weight = weight
+        with ops.noting() as notes:
+            down.forward(None, None)
+        assert notes.complete == complete
+
+
+@pytest.mark.gpu
+def test_layers_whose_weights_are_all_laid_out_otherwise_run_one_by_one():
+    model, got = _model("tensor cores", torch.bfloat16, "cuda:0"), []
+    repeated = model.repeated
+    for turned in (False, True):
+        for layer in model.layers if turned else ():
+            layer.ffn.down.weight = layer.ffn.down.weight.t().contiguous().t()
+        for model.repeated in (model.repeated, None):
+            llm = tlc.LLM(model, dtype="bfloat16", max_tokens=64 * 8, max_seqs=2)
+            got.append(llm.step([StepEntry(llm.cache.acquire(), list(range(1, 60)), (58,))]).clone())
+        model.repeated = repeated
+    assert all(torch.equal(got[0], other) for other in got[1:])
+
+
 def test_parts_that_say_nothing_are_not_repeated():
     model = _model("small", torch.float32, "cpu")
 

@@ -292,6 +292,13 @@ def _note_owned(*tensors) -> None:
         _notes.calls.owned += [t for t in tensors if t is not None]
 
 
+def cannot_repeat() -> None:
+    """Said by whoever gives the GPU work that is no call of the library (a copy that torch makes, into memory that is given back
+    when the call is made): the calls noted so far do not stand for all of it."""
+    if _notes.calls is not None:
+        _notes.calls.complete = False
+
+
 def replay(functions, words, times: int) -> None:
     """Makes the calls of `functions` (int32 array of indices) `times` times; words: the arguments of all rounds (uint64 array)."""
     global _launches

@@ -146,7 +146,10 @@ class StackedLinear(Editable):
     def forward(self, x: torch.Tensor, out: torch.Tensor, accumulate: bool = False) -> torch.Tensor:
         # a part of a product fused along K keeps its weight as a column range of the fused matrix; used on
         # its own (a mixer outside its block) it multiplies by a dense copy
-        w = self.weight if self.weight.is_contiguous() else self.weight.contiguous()
+        w = self.weight
+        if not w.is_contiguous():
+            w = w.contiguous()
+            ops.cannot_repeat()
         ops.linear(x, w, out, self.colscale, self.colbias, accumulate)
         return out
 
