@@ -12,7 +12,7 @@ from tinyllama_c_b200.models import repeat
 from tinyllama_c_b200.config import config_from_dict
 from tinyllama_c_b200.engine import StepEntry
 from tinyllama_c_b200.models.repeat import RepeatedLayers
-from tinyllama_c_b200.parts.base import Editable, LayerCache, LayerRun, StepInfo
+from tinyllama_c_b200.parts.base import Editable, LayerCache, LayerRun, StepInfo, step_scratch
 from tinyllama_c_b200.weights import build_model
 
 import configs
@@ -119,6 +119,18 @@ def test_a_copy_that_torch_makes_ends_the_attempt(monkeypatch):
         with ops.noting() as notes:
             down.forward(None, None)
         assert notes.complete == complete
+
+
+def test_a_mixers_own_projection_lives_as_long_as_the_step(monkeypatch):
+    """A mixer that is the only one of its layer projects for itself; its calls are made again for the other layers."""
+    mixer = next(m for m in _model("small", torch.float32, "cpu").layers[0].mixers if type(m).__name__ == "Mamba2Mixer")
+    i32, seen = torch.zeros(4, dtype=torch.int32), []
+    step = StepInfo(3, 1, i32, i32, i32, i32, i32, i32)
+    monkeypatch.setattr(ops, "linear", lambda x, w, out, *args: seen.append(out))
+    monkeypatch.setattr(type(mixer), "forward_projected", lambda self, proj, *args: seen.append(proj))
+    with step_scratch(step):
+        mixer.forward(torch.zeros(3, mixer.in_proj.in_features), step, None, None)
+    assert len(seen) == 2 and all(any(t is held for held in step.scratch.values()) for t in seen)
 
 
 @pytest.mark.gpu

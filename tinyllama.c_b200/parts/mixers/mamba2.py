@@ -18,7 +18,7 @@ from typing import Callable, Dict, List, Optional, Sequence
 import torch
 
 from ... import ops
-from ..base import ChunkRequest, LayerCache, Part, StateRequest, StepInfo, WeightSpec, act_empty, register_mixer, scratch_buf, to_vec
+from ..base import ChunkRequest, LayerCache, Part, StateRequest, StepInfo, WeightSpec, register_mixer, scratch_buf, to_vec
 from ..linear import StackedLinear
 
 
@@ -132,7 +132,7 @@ class Mamba2Mixer(Part):
         return self.in_proj
 
     def forward(self, normed: torch.Tensor, step: StepInfo, cache: LayerCache, residual: torch.Tensor) -> None:
-        proj = act_empty((step.n_rows, self.in_proj.out_features), normed, torch.float32)
+        proj = scratch_buf(f"mamba2.{self.cache_key}.proj", (step.n_rows, self.in_proj.out_features), torch.float32, normed.device)
         self.in_proj.forward(normed, proj)
         self.forward_projected(proj, step, cache, residual)
 
