@@ -1,6 +1,7 @@
 """Layers whose calls are made again from the first one's (models/repeat.py)."""
 import ctypes
 import random
+import weakref
 from types import SimpleNamespace
 
 import pytest
@@ -145,6 +146,28 @@ def test_layers_whose_weights_are_all_laid_out_otherwise_run_one_by_one():
             got.append(llm.step([StepEntry(llm.cache.acquire(), list(range(1, 60)), (58,))]).clone())
         model.repeated = repeated
     assert all(torch.equal(got[0], other) for other in got[1:])
+
+
+def test_no_weight_is_held_beside_the_layer_that_has_it():
+    """A model that is bound again, or whose weights a program sets to something else, has room for one set of weights."""
+    model = _model("small", torch.bfloat16, "cpu")
+    found = RepeatedLayers.of(model.layers, model.schedule)
+    part = model.layers[1].ffn.down
+    old = weakref.ref(part.weight)
+    part.weight = part.weight.clone()
+    assert old() is None and not found.stands()
+    old = [weakref.ref(l.ffn.down.weight) for l in model.layers]
+    alive = []
+
+    class Tensors(dict):
+        def __getitem__(self, name):
+            alive.append(sum(w() is not None for w in old))
+            return super().__getitem__(name)
+
+    specs = model.weight_specs()
+    model.repeated = found
+    model.bind(Tensors({s.name: torch.ones(s.shape) for s in specs}), torch.bfloat16, torch.device("cpu"))
+    assert alive[0] == len(old) and alive[-1] == 0
 
 
 def test_parts_that_say_nothing_are_not_repeated():

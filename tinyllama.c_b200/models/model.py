@@ -117,6 +117,7 @@ class Model:
 
     def bind(self, tensors: Dict[str, torch.Tensor], dtype: torch.dtype, device) -> None:
         self.dtype, self.device = dtype, torch.device(device)
+        self.repeated = None
         for layer in self.layers:
             layer.bind(tensors, dtype, device)
         self._collect_chunks()

@@ -32,11 +32,12 @@ _ptr, _size, _stride, _dtype = torch.Tensor.data_ptr, torch.Tensor.size, torch.T
 
 
 class _Description:
-    """What a layer is made of: a form that is equal for two layers whose calls differ in their tensors' addresses alone, the
-    tensors in the order in which they come up, and what an edit goes through: the parts (their attributes) and the lists."""
+    """What a layer is made of: a form that is equal for two layers whose calls differ in their tensors' addresses alone, where
+    its tensors are (a part's attributes and the name, in the order in which they come up: none is held here), and what an
+    edit goes through: the parts (their attributes) and the lists."""
 
     def __init__(self, layer, parts: List[Editable], lists: list):
-        self.tensors: List[torch.Tensor] = []
+        self.tensors: List[Tuple[dict, str]] = []
         self.parts, self.lists = parts, lists
         self.known, self.inside = True, set()            # known: whether every part says that it can be repeated
         self.form = self._of(layer)
@@ -45,7 +46,6 @@ class _Description:
         if isinstance(obj, _PLAIN):
             return type(obj), obj
         if isinstance(obj, torch.Tensor):
-            self.tensors.append(obj)
             return "tensor", obj.dtype, tuple(obj.shape), obj.stride(), obj.device
         if id(obj) in self.inside or not isinstance(obj, (list, tuple, dict, Editable)):
             self.known = False
@@ -63,7 +63,9 @@ class _Description:
             aside = obj.repeats()
             if aside is None or "repeats" not in type(obj).__dict__:      # (a class derived from such a part speaks for itself)
                 self.known, aside = False, ()
-            return type(obj), tuple((k, self._of(v)) for k, v in sorted(vars(obj).items()) if k not in aside and k != "edits")
+            names = [k for k in sorted(vars(obj)) if k not in aside and k != "edits"]
+            self.tensors += [(vars(obj), k) for k in names if isinstance(vars(obj)[k], torch.Tensor)]
+            return type(obj), tuple((k, self._of(vars(obj)[k])) for k in names)
         finally:
             self.inside.remove(id(obj))
 
@@ -115,7 +117,8 @@ class RepeatedLayers:
             if left:
                 return done, left
         form, mine = _of_cache(views[0])
-        firsts = self.tensors[0] + mine
+        n_own = len(self.tensors[0])
+        firsts = [attributes[name] for attributes, name in self.tensors[0]] + mine
         at, also = {}, {}                                  # address -> which of the first layer's tensors; which others start there
         addresses = list(map(_ptr, firsts))
         for i, p in enumerate(addresses):
@@ -162,8 +165,8 @@ class RepeatedLayers:
             table = np.empty((end - done, len(used)), dtype=np.uint64)
             for r in range(done, end):
                 other, theirs = _of_cache(views[r])
-                theirs = self.tensors[r] + theirs
-                row = [theirs[i] for i in tensors]
+                row = [self.tensors[r][i] for i in tensors if i < n_own]
+                row = [attributes[name] for attributes, name in row] + [theirs[i - n_own] for i in tensors[len(row):]]
                 if other != form or self._meta(row) != like:
                     return done, left
                 table[r - done] = list(map(_ptr, row)) + [handles[r][i - len(firsts)] for i in used[len(tensors):]]
