@@ -170,6 +170,38 @@ def test_no_weight_is_held_beside_the_layer_that_has_it():
     assert alive[0] == len(old) and alive[-1] == 0
 
 
+def test_functions_put_around_a_layers_methods_or_the_kernels_wrappers_are_noticed(monkeypatch):
+    model = _model("small", torch.bfloat16, "cpu")
+    found = RepeatedLayers.of(model.layers, model.schedule)
+    layer = model.layers[0]
+    assert found.untouched()
+    for owner, name in ((type(layer), "forward"), (type(layer.ffn), "forward"), (type(layer.mixers[0]), "mix"),
+                        (type(layer), "entry"), (ops, "linear"), (ops, "attention"), (ops, "_call")):
+        with monkeypatch.context() as m:
+            old = getattr(owner, name)
+            m.setattr(owner, name, lambda *args: old(*args))
+            assert not found.untouched(), name
+        assert found.untouched() and found.stands()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("where", ["a layer", "a kernel"])
+def test_a_function_put_around_the_layers_is_called_for_every_one(monkeypatch, where):
+    model = _model("small", torch.bfloat16, "cuda:0")
+    llm = tlc.LLM(model, dtype="bfloat16", max_tokens=64 * 8, max_seqs=2)
+    calls, got = [], []
+    owner, name, times = (type(model.layers[0]), "forward", 1) if where == "a layer" else (ops, "linear_swiglu", 1)
+    old = getattr(owner, name)
+    for traced in (False, True, False):
+        with monkeypatch.context() as m:
+            if traced:
+                m.setattr(owner, name, lambda *args, **more: (calls.append(1), old(*args, **more))[1])
+            slot = llm.cache.acquire()
+            got.append(llm.step([StepEntry(slot, list(range(1, 60)), (58,))]).clone())
+            llm.cache.release(slot)
+    assert len(calls) == times * len(model.layers) and torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+
+
 def test_parts_that_say_nothing_are_not_repeated():
     model = _model("small", torch.float32, "cpu")
 

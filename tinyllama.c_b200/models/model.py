@@ -152,7 +152,7 @@ class Model:
             if repeated is not None and not torch.cuda.is_current_stream_capturing():
                 if not repeated.stands(self.layers, self.schedule):
                     repeated = self.repeated = RepeatedLayers(self.layers, self.schedule)
-                if repeated.alike:
+                if repeated.alike and repeated.untouched():
                     done, ready = repeated.run(x, step, cache)
             for r in range(done, len(self.schedule)):
                 run = self.schedule[r]

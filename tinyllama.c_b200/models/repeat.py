@@ -17,6 +17,7 @@ they can be repeated.
 from __future__ import annotations
 
 from operator import attrgetter
+from types import FunctionType
 from typing import List, Optional, Tuple
 
 import numpy as np
@@ -31,14 +32,18 @@ _edits = attrgetter("edits")
 _ptr, _size, _stride, _dtype = torch.Tensor.data_ptr, torch.Tensor.size, torch.Tensor.stride, attrgetter("dtype")
 
 
+# The wrappers of the kernel library as they are defined.  (ops.replay is what this module itself calls.)
+_OPS = {k: f for k, f in vars(ops).items() if isinstance(f, FunctionType) and k != "replay"}
+
+
 class _Description:
     """What a layer is made of: a form that is equal for two layers whose calls differ in their tensors' addresses alone, where
     its tensors are (a part's attributes and the name, in the order in which they come up: none is held here), and what an
     edit goes through: the parts (their attributes) and the lists."""
 
-    def __init__(self, layer, parts: List[Editable], lists: list):
+    def __init__(self, layer, parts: List[Editable], lists: list, classes: set):
         self.tensors: List[Tuple[dict, str]] = []
-        self.parts, self.lists = parts, lists
+        self.parts, self.lists, self.classes = parts, lists, classes
         self.known, self.inside = True, set()            # known: whether every part says that it can be repeated
         self.form = self._of(layer)
 
@@ -60,6 +65,7 @@ class _Description:
                     self.lists.append(obj)
                 return type(obj), tuple(obj) if isinstance(obj, dict) else None, tuple(map(self._of, items))
             self.parts.append(obj)
+            self.classes.update(c for c in type(obj).__mro__ if issubclass(c, Editable))
             aside = obj.repeats()
             if aside is None or "repeats" not in type(obj).__dict__:      # (a class derived from such a part speaks for itself)
                 self.known, aside = False, ()
@@ -96,7 +102,9 @@ class RepeatedLayers:
         self.order = layers, schedule
         self.parts, self.lists = [], [layers, schedule]
         self.layers = [layers[r.layer] for r in schedule]
-        found = [_Description(layer, self.parts, self.lists) for layer in self.layers]
+        classes = set()
+        found = [_Description(layer, self.parts, self.lists, classes) for layer in self.layers]
+        self.written = [(vars(ops), list(_OPS), list(_OPS.values()))] + [(vars(c), list(c.as_written), list(c.as_written.values())) for c in classes]
         self.tensors = [d.tensors for d in found]
         self.alike = len(found) >= 3 and all(d.known and d.form == found[0].form for d in found) \
             and not any(r.cache is not None or r.kv_cache is not None or r.add is not None or r.add_embedding for r in schedule)
@@ -185,6 +193,11 @@ class RepeatedLayers:
         these (where given) are the lists that were looked at."""
         return (layers is None or layers is self.order[0]) and (schedule is None or schedule is self.order[1]) \
             and list(map(_edits, self.parts)) == self.edits and self.lists == self.copies
+
+    def untouched(self) -> bool:
+        """Whether the layers' methods and the wrappers of the kernel library are those that the source has.  A function that a
+        program puts around one of them (to trace, to time, to gather statistics) is called for every layer."""
+        return all(list(map(holder.get, names)) == functions for holder, names, functions in self.written)
 
     @staticmethod
     def _meta(tensors):

@@ -128,6 +128,11 @@ class Editable:
     """Counts how often its attributes are set or deleted, so that what was found out about it (models/repeat.py) can be dropped."""
     edits = 0
     passing = frozenset()        # attributes that a forward() sets for itself
+    as_written: Dict[str, Any] = {}     # every class's methods, as its definition has them
+
+    def __init_subclass__(cls, **kwargs):
+        super().__init_subclass__(**kwargs)
+        cls.as_written = {k: f for k, f in vars(cls).items() if callable(f) or isinstance(f, (property, staticmethod, classmethod))}
 
     def __setattr__(self, name, value):
         object.__setattr__(self, name, value)
