@@ -487,7 +487,12 @@ gemm_split_f32x4_kernel(const float* __restrict__ a, int lda, const float* __res
 }
 
 static int g_f32_tile_rows = 0, g_f32_split = 0;             // test hooks: rows of a tile (32 or 64), blocks a tile; 0: chosen
-extern "C" void tlc_linear_f32_tiles(int rows, int split) { g_f32_tile_rows = rows; g_f32_split = split; }
+extern "C" void tlc_linear_f32_tiles(int rows, int split) {
+  // (a cluster adds up to eight blocks' sums, each a whole share of the rows; tiles of 64 x 128 have one block)
+  const bool there = (rows == 32 || rows == 64) && (split == 1 || split == 2 || split == 4 || split == 8 || (split == 0 && rows == 64));
+  g_f32_tile_rows = there ? rows : 0;
+  g_f32_split = there ? split : 0;
+}
 
 template <typename TO, int TM, int NC, int KS>
 static void launch_split_f32x4(const float* a, int lda, const float* w, int ldw, TO* out, int ldo, const float* colscale, const float* colbias,
@@ -529,6 +534,11 @@ static F32Plan f32_plan(int M, int N, int sms) {
     if (c < cost) { cost = c; best.split = split; }
   }
   return best;
+}
+
+extern "C" int tlc_linear_f32_plan(int M, int N, int sms) {
+  const F32Plan plan = f32_plan(M, N, sms);
+  return plan.rows * 16 + plan.split;
 }
 
 int tlc_linear_simt_init();
