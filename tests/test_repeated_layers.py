@@ -202,6 +202,27 @@ def test_a_function_put_around_the_layers_is_called_for_every_one(monkeypatch, w
     assert len(calls) == times * len(model.layers) and torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
 
 
+def test_steps_that_wait_for_the_gpu_run_layer_by_layer(monkeypatch):
+    """From a number of rows on that falls with the size of a layer's matrices, and with their type's rate."""
+    layers = [_Forks(i) for i in range(4)]
+    assert _run_on_the_host(monkeypatch, layers, 0x77, 1023)[0] == 4
+    assert _run_on_the_host(monkeypatch, layers, 0x77, 1024) == (0, [])
+    first = {}
+    for dtype in (torch.float32, torch.bfloat16):
+        for n in (2048, 4096):
+            for layer in layers:
+                layer.weight = torch.empty(n, n, dtype=dtype)
+                layer.gain = layer.weight[:n // 2]              # (rows of the same matrix: counted once)
+            found = RepeatedLayers.of(layers, [LayerRun(i) for i in range(len(layers))])
+            first[dtype, n] = next(rows for rows in range(1, 1025) if found.is_long(rows))
+    rows = first[torch.float32, 4096]
+    assert rows < first[torch.float32, 2048] < first[torch.bfloat16, 4096] <= first[torch.bfloat16, 2048] == 1024
+    for layer in layers:
+        layer.weight = layer.gain = torch.empty(4096, 4096)
+    assert _run_on_the_host(monkeypatch, layers, 0x77, rows - 1)[0] == 4
+    assert _run_on_the_host(monkeypatch, layers, 0x77, rows) == (0, [])
+
+
 def test_parts_that_say_nothing_are_not_repeated():
     model = _model("small", torch.float32, "cpu")
 
@@ -251,7 +272,7 @@ class _Forks(Editable):
         return False
 
 
-def _run_on_the_host(monkeypatch, layers, stream):
+def _run_on_the_host(monkeypatch, layers, stream, rows=1):
     """(entries that ran, [stream of every norm call made again]) of a step on a stream of that handle, and the words."""
     got = []
     monkeypatch.setattr(ops, "stream_handle", lambda: stream)
@@ -259,7 +280,7 @@ def _run_on_the_host(monkeypatch, layers, stream):
     found = RepeatedLayers.of(layers, [LayerRun(i) for i in range(len(layers))])
     i32 = torch.zeros(4, dtype=torch.int32)
     step = StepInfo(1, 1, i32, i32, i32, i32, i32, i32)
-    done, left = found.run(torch.zeros(1, 8), step, SimpleNamespace(layer_view=lambda r, writes, kv: LayerCache()))
+    done, left = found.run(torch.zeros(rows, 8), step, SimpleNamespace(layer_view=lambda r, writes, kv: LayerCache()))
     rows = [row for _, words in got for row in words.tolist()]
     return done, rows
 

@@ -88,9 +88,14 @@ def _of_cache(view: LayerCache) -> Tuple[tuple, List[torch.Tensor]]:
 class RepeatedLayers:
     """The layers of a run order that are alike."""
 
-    # From how many rows on the second layer runs like the first one: its kernels take the GPU longer than the host takes to
-    # look through the first one's calls (2,048 rows: 8.23 ms without it, 8.06 with every layer on its own).
-    LONG_STEP = 1024
+    # Where a layer keeps the GPU longer than Python takes for one (0.22 ms), the layers run one by one: while the first one's calls
+    # are looked through the GPU waits for 0.3 ms, which pays where the GPU would wait for every layer.  That is so up to the
+    # rows that make a layer's products take LONG_LAYER at the rates below (the norms, the scan and attention come on top) and up
+    # to LONG_STEP rows at most.  Milliseconds a prompt, repeated and one by one: 1.5B sizes, 600 / 700 / 1,000 / 2,048 rows 5.13 / 5.28 /
+    # 5.55 / 8.2 and 5.35 / 5.30 / 5.27 / 8.0; 3B, 250 / 270 / 700 6.54 / 7.54 / 8.7 and 6.75 / 7.14 / 8.4; 7B, 125 / 140 / 333 7.7 /
+    # 9.60 / 11.3 and 9.1 / 9.52 / 11.0; 1.5B in 32 bits, 5 / 10 / 20 4.25 / 6.27 / 5.71 and 4.78 / 6.02 / 5.44.
+    LONG_STEP, LONG_LAYER = 1024, 87e-6
+    READ_RATE, RATE_16, RATE_32 = 6.5e12, 1e15, 1.4e13        # bytes, operations of 16-bit and of few-row 32-bit products a second
 
     @staticmethod
     def of(layers, schedule) -> Optional["RepeatedLayers"]:
@@ -106,6 +111,16 @@ class RepeatedLayers:
         found = [_Description(layer, self.parts, self.lists, classes) for layer in self.layers]
         self.written = [(vars(ops), list(_OPS), list(_OPS.values()))] + [(vars(c), list(c.as_written), list(c.as_written.values())) for c in classes]
         self.tensors = [d.tensors for d in found]
+        self.read_s = self.row_s = 0.0                     # a layer's matrices read once, and what every row adds, in seconds
+        spans, end = [], 0
+        for t in (attributes[name] for attributes, name in self.tensors[0]) if self.tensors else ():
+            if t.dim() == 2 and t.numel():
+                n = 1 + sum((size - 1) * stride for size, stride in zip(t.shape, t.stride()))
+                spans.append((t.data_ptr(), t.data_ptr() + n * t.element_size(), t.dtype))
+        for lo, hi, dtype in sorted(spans, key=lambda s: s[:2]):
+            n, end = max(0, hi - max(lo, end)), max(hi, end)      # (a product's parts keep ranges of its matrix)
+            self.read_s += n / self.READ_RATE
+            self.row_s += 2 * n / 4 / self.RATE_32 if dtype == torch.float32 else 2 * n / 2 / self.RATE_16
         self.alike = len(found) >= 3 and all(d.known and d.form == found[0].form for d in found) \
             and not any(r.cache is not None or r.kv_cache is not None or r.add is not None or r.add_embedding for r in schedule)
         self.edits, self.copies = list(map(_edits, self.parts)), [l if isinstance(l, tuple) else l.copy() for l in self.lists]
@@ -113,17 +128,14 @@ class RepeatedLayers:
     def run(self, x: torch.Tensor, step: StepInfo, cache) -> Tuple[int, bool]:
         """Runs the first layer, and the others if they can be repeated; (how many entries of the run order have run,
         whether the last of them has left the next one's input)."""
+        if self.is_long(x.shape[0]):
+            return 0, False
         views = [cache.layer_view(r, True, None) for r in range(len(self.layers))]
         with ops.noting() as notes:
             left = self.layers[0].forward(x, step, views[0], False, self.layers[1].entry)
         if left or not notes.complete:
             return 1, left
         done, n = 1, len(self.layers)
-        if x.shape[0] >= self.LONG_STEP:                   # work for the GPU while the calls are looked through
-            left = self.layers[1].forward(x, step, views[1], False, self.layers[2].entry if n > 2 else None)
-            done = 2
-            if left:
-                return done, left
         form, mine = _of_cache(views[0])
         n_own = len(self.tensors[0])
         firsts = [attributes[name] for attributes, name in self.tensors[0]] + mine
@@ -167,7 +179,6 @@ class RepeatedLayers:
             used_on(current_stream(x.device), notes.owned)
         columns = [rank[i] for i in which]
         # the next layer at once, so that the GPU has work while the others' addresses are gathered, then a few, then the rest
-        # (all 23 in one go: 0.35 ms of a prompt of 2,048 tokens in which the GPU waits)
         while done < n:
             end = min(n, done + (1 if done < 3 else 4 if done < 6 else n))
             table = np.empty((end - done, len(used)), dtype=np.uint64)
@@ -187,6 +198,10 @@ class RepeatedLayers:
             ops.replay(functions, words, end - done)
             done = end
         return n, False
+
+    def is_long(self, rows: int) -> bool:
+        """Whether a step of that many rows waits for the GPU and not for the host."""
+        return rows >= self.LONG_STEP or self.read_s + rows * self.row_s >= self.LONG_LAYER
 
     def stands(self, layers=None, schedule=None) -> bool:
         """Whether nothing has been edited since the layers were looked at: no attribute of a part, no list or what is in it, and
