@@ -202,3 +202,25 @@ def test_32_bit_tiles_with_their_k_steps_shared(M, N, K, rows, split):
     _check(once, a, w, None, None, None)
     _check(half, a, w, scale, None, None, True)
     assert torch.equal(out[M], before[M]) and torch.equal(out[:, N:], before[:, N:])
+
+
+@pytest.mark.parametrize("M,N,K", [(17, 60, 4), (33, 132, 36), (70, 1030, 132), (129, 257, 1028)])
+def test_32_bit_tiles_with_k_in_four_parts(M, N, K):
+    """Fewer K-steps than parts, parts of unequal length, edges in part; sums added into the output, overwritten, in 16 bits."""
+    from tinyllama_c_b200 import ops
+    g = torch.Generator().manual_seed(M + N + K)
+    a, w = torch.randn(M, K, generator=g).cuda(), torch.randn(N, K, generator=g).cuda()
+    scale, bias, before = torch.randn(N, generator=g).cuda(), torch.randn(N, generator=g).cuda(), torch.randn(M + 1, N + 3, generator=g).cuda()
+    ops.linear_f32_tiles(64, -4)
+    try:
+        out, once, half = before.clone(), torch.full((M, N), float("nan"), device="cuda"), torch.full((M, N), float("nan"), device="cuda").bfloat16()
+        ops.linear(a, w, out[:M, :N], scale, bias, True)
+        ops.linear(a, w, once)
+        ops.linear(a, w, half, scale)
+        torch.cuda.synchronize()
+    finally:
+        ops.linear_f32_tiles(0)
+    _check(out[:M, :N], a, w, scale, bias, before[:M, :N])
+    _check(once, a, w, None, None, None)
+    _check(half, a, w, scale, None, None, True)
+    assert torch.equal(out[M], before[M]) and torch.equal(out[:, N:], before[:, N:])

@@ -6,16 +6,30 @@ from tinyllama_c_b200 import ops
 
 def test_tiles_that_do_not_exist_cannot_be_asked_for():
     """Shares of a tile's rows that are no whole numbers would leave rows out, more blocks than eight their sums."""
-    chosen = ops.linear_f32_plan(310, 2048, 148)
+    chosen = ops.linear_f32_plan(310, 2048, 2048, 148)
     try:
-        for rows, split in ((32, 1), (32, 8), (64, 0), (64, 2), (64, 8)):
+        for rows, split in ((32, 1), (32, 8), (64, 0), (64, -4), (64, 2), (64, 8)):
             ops.linear_f32_tiles(rows, split)
-            assert ops.linear_f32_plan(310, 2048, 148) == (rows, split)
+            assert ops.linear_f32_plan(310, 2048, 2048, 148) == (rows, split)
         for rows, split in ((32, 0), (32, 3), (64, 5), (64, 16), (64, -1), (48, 4), (0, 4)):
             with pytest.raises(ops.KernelError, match="no 32-bit tiles"):
                 ops.linear_f32_tiles(rows, split)
             ops.library().tlc_linear_f32_tiles(rows, split)          # the library's own entry: as if nothing had been asked for
-            assert ops.linear_f32_plan(310, 2048, 148) == chosen
+            assert ops.linear_f32_plan(310, 2048, 2048, 148) == chosen
     finally:
         ops.linear_f32_tiles(0)
-    assert ops.linear_f32_plan(310, 2048, 148) == chosen
+    assert ops.linear_f32_plan(310, 2048, 2048, 148) == chosen
+
+
+@pytest.mark.parametrize("K,N,M,plan", [
+    # one block a tile where K is short: what a cluster costs is more than what it brings (microseconds, one block and the cluster)
+    (32, 2048, 1200, (64, 0)), (256, 2048, 1200, (64, 0)), (128, 8192, 310, (64, 0)),          # 9.4 / 39.5, 43.1 / 58.6, 24.1 / 49.2
+    (32, 512, 310, (64, -4)), (64, 2048, 48, (64, -4)), (256, 8192, 48, (64, -4)),             # 4.2 / 6.8, 5.0 / 6.2, 12.0 / 14.7
+    # and where the output has no use for tiles of 256 columns, however long K is
+    (1024, 64, 3000, (64, -4)), (12288, 64, 3000, (64, -4)),                                    # 36 / 56
+    # clusters elsewhere, as the kernels were fitted
+    (128, 64, 17, (32, 8)), (512, 2048, 17, (32, 8)), (1024, 2048, 48, (32, 8)),                # 6.6 / 3.3, 18.7 / 10.6, 35.3 / 19.7
+    (1024, 2048, 130, (64, 8)), (2048, 2048, 310, (64, 8)), (4096, 2048, 310, (64, 8)),         # 36.6 / 34.5, 134 / 93, 264 / 179
+    (2048, 8192, 17, (32, 8)), (2048, 8192, 130, (64, 4)), (2048, 8192, 1200, (64, 0)), (4096, 2048, 17, (32, 8))])
+def test_tiles_of_32_bit_products_by_their_sizes(K, N, M, plan):
+    assert ops.linear_f32_plan(M, N, K, 148) == plan

@@ -231,22 +231,27 @@ __device__ __forceinline__ void fma_pair(float2& d, float2 a, float2 b) {
       : "l"(reinterpret_cast<const unsigned long long&>(a)), "l"(reinterpret_cast<const unsigned long long&>(b)));
 }
 
-// A tile of 64 rows x 128 columns, 128 threads with 8 x 8 results each; two K-steps of 16 in shared memory, the next one in
-// registers.  For outputs of many tiles: 600 rows of 2048 -> 8192 500 us (41 TFLOP/s), 1,200 879 us (46).
+// A tile of 64 rows x 16 CT columns, 128 threads with 8 x CT results each; two K-steps of 16 in shared memory, the next one in
+// registers.  CT = 8 for outputs of many tiles: 600 rows of 2048 -> 8192 500 us (41 TFLOP/s), 1,200 879 us (46).  CT = 4 with KG = 4,
+// four groups of 128 threads that take a quarter of K each, for outputs of few tiles and a K so short that the meetings of a
+// cluster (below) would cost more than its blocks bring: f32_plan has both sides.
 constexpr int FT_M = 64, FT_K = 16, FT_LD = 4;
-template <typename TO>
-__global__ void __launch_bounds__(128)
+template <typename TO, int CT, int KG>
+__global__ void __launch_bounds__(128 * KG)
 gemm_tiled_f32x4_kernel(const float* __restrict__ a, int lda, const float* __restrict__ w, int ldw, TO* __restrict__ out,
                         int ldo, const float* __restrict__ colscale, const float* __restrict__ colbias, TlcEpi accumulate,
                         int M, int N, int K) {
   tlc_pdl(a, w, out);
-  constexpr int CT = 8, TN = 16 * CT, LA = FT_M + FT_LD, LW = TN + FT_LD;
+  constexpr int TN = 16 * CT, LA = FT_M + FT_LD, LW = TN + FT_LD;
   constexpr int PA = FT_M * FT_K / 4 / 128, PW = TN * FT_K / 4 / 128;   // 16-byte pieces a thread brings of each operand
-  __shared__ __align__(16) float As[2 * FT_K * LA], Ws[2 * FT_K * LW];    // [2][FT_K][LA], [2][FT_K][LW]
-  const int tid = threadIdx.x;
+  extern __shared__ __align__(16) float ft_sm[];
+  const int grp = threadIdx.x >> 7, tid = threadIdx.x & 127;
+  float* As = ft_sm + grp * 2 * FT_K * (LA + LW);            // [2][FT_K][LA]
+  float* Ws = As + 2 * FT_K * LA;                            // [2][FT_K][LW]
   const int m0 = blockIdx.y * FT_M, n0 = blockIdx.x * TN;
   const int tx = tid & 15, ty = tid >> 4;
-  const int steps = (K + FT_K - 1) / FT_K;
+  const int steps = (K + FT_K - 1) / FT_K, per = (steps + KG - 1) / KG;
+  const int s_begin = min(steps, grp * per), s_end = min(steps, s_begin + per);
   float4 ra[PA], rw[PW];
   auto load = [&](int s) {
 #pragma unroll
@@ -279,14 +284,14 @@ gemm_tiled_f32x4_kernel(const float* __restrict__ a, int lda, const float* __res
   for (int i = 0; i < 8; i++)
 #pragma unroll
     for (int j = 0; j < CT / 2; j++) acc[i][j] = make_float2(0.f, 0.f);
-  load(0);
-  store(0);
+  // all groups go through the same number of barriers
+  if (s_begin < s_end) { load(s_begin); store(0); }
   __syncthreads();
 #pragma unroll 1
-  for (int s = 0; s < steps; s++) {
-    const int buf = s & 1;
-    if (s + 1 < steps) load(s + 1);
-    {
+  for (int i = 0; i < per; i++) {
+    const int s = s_begin + i, buf = i & 1;
+    if (s + 1 < s_end) load(s + 1);
+    if (s < s_end) {
       const float* Ab = As + buf * FT_K * LA + ty * 8;
       const float* Wb = Ws + buf * FT_K * LW + tx * 4;
 #pragma unroll
@@ -306,8 +311,34 @@ gemm_tiled_f32x4_kernel(const float* __restrict__ a, int lda, const float* __res
           for (int j = 0; j < CT / 2; j++) fma_pair(acc[r][j], make_float2(av[r], av[r]), wv[j]);
       }
     }
-    if (s + 1 < steps) store(buf ^ 1);
+    if (s + 1 < s_end) store(buf ^ 1);
     __syncthreads();
+  }
+  if constexpr (KG > 1) {
+    float* part = ft_sm;                                     // the other groups' sums, [KG - 1][8 * CT][128]
+    if (grp > 0) {
+      float* mine = part + (grp - 1) * 8 * CT * 128 + tid;
+#pragma unroll
+      for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int j = 0; j < CT / 2; j++) {
+          mine[((i * CT) + 2 * j) * 128] = acc[i][j].x;
+          mine[((i * CT) + 2 * j + 1) * 128] = acc[i][j].y;
+        }
+    }
+    __syncthreads();
+    if (grp > 0) return;
+#pragma unroll
+    for (int q = 0; q < KG - 1; q++) {                       // in the order of K
+      const float* other = part + q * 8 * CT * 128 + tid;
+#pragma unroll
+      for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int j = 0; j < CT / 2; j++) {
+          acc[i][j].x += other[((i * CT) + 2 * j) * 128];
+          acc[i][j].y += other[((i * CT) + 2 * j + 1) * 128];
+        }
+    }
   }
 #pragma unroll
   for (int i = 0; i < 8; i++) {
@@ -326,7 +357,10 @@ gemm_tiled_f32x4_kernel(const float* __restrict__ a, int lda, const float* __res
     }
   }
 }
-// The same where the tiles are too few for the SMs, or fill their last round badly: a tile of 8 TM rows x 64 NC columns, 128 threads
+constexpr int ft_smem(int CT, int KG) { return KG * 2 * FT_K * (FT_M + 16 * CT + 2 * FT_LD) * 4; }
+static_assert(ft_smem(4, 4) >= 3 * 8 * 4 * 128 * 4 && ft_smem(8, 1) <= 48 * 1024, "the other groups' sums reuse the operands' memory");
+
+// The same where the tiles are too few for the SMs, or fill their last round badly, and K is long enough: a tile of 8 TM rows x 64 NC columns, 128 threads
 // with TM x 4 NC results each, K-steps of KS.  Rows of both operands lie turned by 32 / (KS / 4) values for every four of K,
 // which keeps the stores of the transposed pieces clear of bank conflicts.  `split` blocks of a thread-block cluster share a tile's
 // K-steps: each leaves its sums in its own shared memory, the cluster meets, and block r adds up its share of the rows over
@@ -488,8 +522,8 @@ gemm_split_f32x4_kernel(const float* __restrict__ a, int lda, const float* __res
 
 static int g_f32_tile_rows = 0, g_f32_split = 0;             // test hooks: rows of a tile (32 or 64), blocks a tile; 0: chosen
 extern "C" void tlc_linear_f32_tiles(int rows, int split) {
-  // (a cluster adds up to eight blocks' sums, each a whole share of the rows; tiles of 64 x 128 have one block)
-  const bool there = (rows == 32 || rows == 64) && (split == 1 || split == 2 || split == 4 || split == 8 || (split == 0 && rows == 64));
+  // (a cluster adds up to eight blocks' sums, each a whole share of the rows; the other two kinds of tiles have one block)
+  const bool there = (rows == 32 || rows == 64) && (split == 1 || split == 2 || split == 4 || split == 8 || (rows == 64 && (split == 0 || split == -4)));
   g_f32_tile_rows = there ? rows : 0;
   g_f32_split = there ? split : 0;
 }
@@ -514,31 +548,63 @@ static void launch_split_f32x4(const float* a, int lda, const float* w, int ldw,
   cudaLaunchKernelEx(&cfg, gemm_split_f32x4_kernel<TO, TM, NC, KS>, a, lda, w, ldw, out, ldo, colscale, colbias, accumulate, M, N, K, split);
 }
 
-// Which tiles 17 and more rows take.  In units of the time that a block of 64 x 256 columns with all of K takes beside a second one
-// on its SM: n blocks on the fullest SM cost 1, 1, 1.6, 2, 2.6, ... (a block alone is no quicker than two: the schedulers wait), a
+// Which tiles 17 and more rows take, by how much work lands on the fullest SM (so the order of a sum follows from the sizes and
+// the number of SMs).  For a K of some thousand, in units of the time that a block of 64 x 256 columns with all of K takes beside a
+// second one on its SM: n blocks cost 1, 1, 1.6, 2, 2.6, ... (a block alone is no quicker than two: the schedulers wait), a
 // cluster 0.012 for each of its blocks, and the tiles of 64 x 128, at two and more blocks an SM, 0.71, 0.935, 1.16, ... for 3,
-// 4, 5, ... on the fullest SM (fitted to 17 to 1,200 rows of 2048 -> 8192 and 4096 -> 2048).  No split below four: a block's
-// sums would be longer, and further off, than those of K in four parts were.  Tiles of 32 rows, eight blocks each, where
+// 4, 5, ... (fitted to 17 to 1,200 rows of 2048 -> 8192 and 4096 -> 2048).  No split below four: a block's
+// sums would be longer, and further off, than those of K in four parts are.  Tiles of 32 rows, eight blocks each, where
 // that makes no more than four blocks an SM.
-struct F32Plan { int rows, split; };                         // split 0: the tiles of 64 x 128
-static F32Plan f32_plan(int M, int N, int sms) {
+//
+// What a cluster costs whatever K is (its meetings, and a tile's sums through shared memory) is more than it brings where K is
+// short, and tiles of 256 columns are where the output has 64: there one block a tile, of 64 x 128 or with K in four parts
+// within the block.  f32_us is a time in microseconds of each kind, fitted to 905 products of K 32 to 12288, N 64 to 16384 and
+// 17 to 3,000 rows; of the two candidates the better one by it is within 6 % of the better one as measured in all but 7 of them
+// (15 % at most).  Cluster and one block a tile, microseconds: 1,200 rows of 32 -> 2048 39.5 and 9.4, of 256 -> 2048 58.6
+// and 43.1, of 1024 -> 2048 153 and 159; 310 rows of 128 -> 8192 49.2 and 24.1, of 1024 -> 8192 162 and 159; 48 rows of 64 -> 2048 6.2
+// and 5.0, of 128 -> 2048 6.3 and 7.0, of 1024 -> 2048 19.7 and 35.3; 3,000 rows of 1024 -> 64 56 and 36.
+struct F32Plan { int rows, split; };                         // split 0: the tiles of 64 x 128; -4: of 64 x 64, K in four parts
+static int f32_blocks(int rows, int cols, int split, int M, int N, int sms) {   // on the fullest SM
+  const long long tiles = (long long)((M + rows - 1) / rows) * ((N + cols - 1) / cols);
+  return (int)((tiles * split + sms - 1) / sms);
+}
+static double f32_pairs(int f) { return f <= 2 ? 1.0 : f / 2 + (f & 1 ? 0.6 : 0.0); }   // f blocks of 64 x 256 columns
+static double f32_us(F32Plan p, int M, int N, int K, int sms) {
+  if (p.rows == 32) {
+    const int f = f32_blocks(32, 128, p.split, M, N, sms);
+    return 3.0 + f + K * (0.0031 + 0.003 * f);
+  }
+  if (p.split > 0) {
+    const int f = f32_blocks(64, 256, p.split, M, N, sms);
+    return 1.2 + 4.5 * f + 0.162 * K / p.split * f32_pairs(f);
+  }
+  if (p.split == 0) {
+    const int f = f32_blocks(64, 128, 1, M, N, sms);
+    return 2.5 + 0.85 * f + K * (0.0126 + 0.0458 * (f < 3 ? 3 : f));
+  }
+  return 1.1 + f32_blocks(64, 64, 1, M, N, sms) * (2.44 + 0.0315 * K);
+}
+static F32Plan f32_plan(int M, int N, int K, int sms) {
   if (g_f32_tile_rows) return F32Plan{g_f32_tile_rows == 32 ? 32 : 64, g_f32_split};
   auto over = [](long long x, long long y) { return (x + y - 1) / y; };
-  if (over(N, 128) * over(M, 32) * 8 <= 4 * sms) return F32Plan{32, 8};
   const long long whole = over(N, 128) * over(M, 64);
-  double cost = whole >= 2 * sms ? 0.225 * over(whole, sms) + 0.035 : 1e30;
-  F32Plan best{64, 0};
-  for (int split = 4; split <= 8; split *= 2) {
-    const long long f = over(over(N, 256) * over(M, 64) * split, sms);
-    const double c = (f <= 2 ? 1.0 : f / 2 + (f & 1 ? 0.6 : 0.0)) / split + 0.012 * split;
-    if (c < cost) { cost = c; best.split = split; }
+  const F32Plan alone{64, whole >= 2 * sms ? 0 : -4};
+  F32Plan best = alone;
+  if (over(N, 128) * over(M, 32) * 8 <= 4 * sms) {
+    best = F32Plan{32, 8};
+  } else {
+    double cost = whole >= 2 * sms ? 0.225 * over(whole, sms) + 0.035 : 1e30;
+    for (int split = 4; split <= 8; split *= 2) {
+      const double c = f32_pairs(f32_blocks(64, 256, split, M, N, sms)) / split + 0.012 * split;
+      if (c < cost) { cost = c; best = F32Plan{64, split}; }
+    }
   }
-  return best;
+  return best.split > 0 && f32_us(alone, M, N, K, sms) < f32_us(best, M, N, K, sms) ? alone : best;
 }
-
-extern "C" int tlc_linear_f32_plan(int M, int N, int sms) {
-  const F32Plan plan = f32_plan(M, N, sms);
-  return plan.rows * 16 + plan.split;
+// 256 * rows + split (its low byte)
+extern "C" int tlc_linear_f32_plan(int M, int N, int K, int sms) {
+  const F32Plan plan = f32_plan(M, N, K, sms);
+  return plan.rows * 256 + (plan.split & 255);
 }
 
 int tlc_linear_simt_init();
@@ -550,12 +616,14 @@ static int launch_simt_f32x4(const float* a, int lda, const float* w, int ldw, T
   if (sms == 0) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
   if (M > 16) {
     if (int rc = tlc_linear_simt_init()) return rc;
-    const F32Plan plan = f32_plan(M, N, sms);
+    const F32Plan plan = f32_plan(M, N, K, sms);
 #define TLC_FS(TM_, NC_, KS_) launch_split_f32x4<TO, TM_, NC_, KS_>(a, lda, w, ldw, out, ldo, colscale, colbias, accumulate, M, N, K, plan.split, stream)
     if (plan.rows == 32) TLC_FS(4, 2, 16);
-    else if (plan.split) TLC_FS(8, 4, 8);
+    else if (plan.split > 0) TLC_FS(8, 4, 8);
+    else if (plan.split == 0)
+      tlc_launch(gemm_tiled_f32x4_kernel<TO, 8, 1>, dim3((N + 127) / 128, (M + 63) / 64), dim3(128), ft_smem(8, 1), stream, a, lda, w, ldw, out, ldo, colscale, colbias, accumulate, M, N, K);
     else
-      tlc_launch(gemm_tiled_f32x4_kernel<TO>, dim3((N + 127) / 128, (M + 63) / 64), dim3(128), 0, stream, a, lda, w, ldw, out, ldo, colscale, colbias, accumulate, M, N, K);
+      tlc_launch(gemm_tiled_f32x4_kernel<TO, 4, 4>, dim3((N + 63) / 64, (M + 63) / 64), dim3(512), ft_smem(4, 4), stream, a, lda, w, ldw, out, ldo, colscale, colbias, accumulate, M, N, K);
 #undef TLC_FS
     TLC_CHECK_LAUNCH("linear(simt)");
     return 0;
@@ -1020,7 +1088,8 @@ static int g_skinny_two = 1;          // 0: never two tiles a block (for compari
 // first (tlc_linear_init), else with the first product that takes one of them.
 template <typename TO> static bool simt_reserve() {
   const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  return cudaFuncSetAttribute(gemm_split_f32x4_kernel<TO, 8, 4, 8>, attr, fs_smem<8, 4, 8>(2)) == cudaSuccess &&
+  return cudaFuncSetAttribute(gemm_tiled_f32x4_kernel<TO, 4, 4>, attr, ft_smem(4, 4)) == cudaSuccess &&
+         cudaFuncSetAttribute(gemm_split_f32x4_kernel<TO, 8, 4, 8>, attr, fs_smem<8, 4, 8>(2)) == cudaSuccess &&
          cudaFuncSetAttribute(gemm_skinny_ring_kernel<TO>, attr, RingSmem::BYTES) == cudaSuccess &&
          cudaFuncSetAttribute(gemm_skinny_two_kernel<TO, false>, attr, SK_TWO_SMEM) == cudaSuccess &&
          cudaFuncSetAttribute(gemm_skinny_two_kernel<TO, true>, attr, SK_TWO_SMEM) == cudaSuccess;
@@ -1030,7 +1099,7 @@ int tlc_linear_simt_init() {
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && ready[dev]) return 0;
-  if (!simt_reserve<float>() || !simt_reserve<__nv_bfloat16>()) return tlc_fail(-2, "linear: cannot reserve %d and %d bytes of shared memory", fs_smem<8, 4, 8>(2), SK_TWO_SMEM);
+  if (!simt_reserve<float>() || !simt_reserve<__nv_bfloat16>()) return tlc_fail(-2, "linear: cannot reserve %d bytes of shared memory", ft_smem(4, 4));
   if (dev >= 0 && dev < 64) ready[dev] = true;
   return 0;
 }

@@ -176,8 +176,8 @@ void tlc_linear_few_rows_split(int split); // 0: the number of blocks per tile i
 void tlc_linear_few_rows_min_tiles(int tiles);   // outputs of fewer tiles of 128 weight rows stay with the other kernels (0: 16 tiles with more than 32 rows, else 32)
 void tlc_linear_few_rows_max_rows(int rows);     // products of more rows go to the tiles of the prompt product (128; for comparisons)
 int tlc_linear_few_rows_ok(int a_dtype, int lda, const void* a, int w_dtype, int ldw, const void* w, int M, int N, int K);   // whatever the output is
-void tlc_linear_f32_tiles(int rows, int split);  // 32-bit products of more than 16 rows: 32: tiles of 32 x 128, 64: of 64 x 256 (split 0: of 64 x 128, one block each), 1, 2, 4 or 8 blocks a tile; anything else: chosen (for tests)
-int tlc_linear_f32_plan(int M, int N, int sms);  // which of these a product of M > 16 rows takes: 16 * rows + split
+void tlc_linear_f32_tiles(int rows, int split);  // 32-bit products of more than 16 rows: 32: tiles of 32 x 128, 64: of 64 x 256, 1, 2, 4 or 8 blocks a tile; 64 and 0: of 64 x 128, 64 and -4: of 64 x 64 with K in four parts, one block each; anything else: chosen (for tests)
+int tlc_linear_f32_plan(int M, int N, int K, int sms);   // which of these a product of M > 16 rows takes: 256 * rows + the low byte of split
 void tlc_linear_tma_out(int on);        // 0: the tensor-core product's 32-bit outputs never leave through the copy engine (for comparisons)
 void tlc_linear_skinny_pairs(int on);   // 0: the skinny product never splits K over a pair of blocks (for comparisons)
 void tlc_linear_skinny_two(int on);      // 0: the product of up to 8 rows never takes two tiles a block (for comparisons)

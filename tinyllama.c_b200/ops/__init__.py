@@ -75,7 +75,7 @@ _SIGNATURES = {
     "tlc_linear_few_rows_max_rows": (None, [_i]),
     "tlc_linear_few_rows_ok": (_i, [_i, _i, _vp, _i, _i, _vp, _i, _i, _i]),
     "tlc_linear_f32_tiles": (None, [_i, _i]),
-    "tlc_linear_f32_plan": (_i, [_i, _i, _i]),
+    "tlc_linear_f32_plan": (_i, [_i, _i, _i, _i]),
     "tlc_linear_pairs": (_i, []),
     "tlc_rope_kv_store": (_i, [_vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _i,
                                _i, _i, _vp]),
@@ -721,15 +721,16 @@ def linear_skinny_ring(on: bool) -> None:
 
 def linear_f32_tiles(rows: int, split: int = 0) -> None:
     """32-bit products of more than 16 rows: tiles of 32 or 64 rows, `split` blocks a tile (1, 2, 4 or 8; 64 and 0: the tiles of 64 x
-    128); linear_f32_tiles(0): chosen.  For tests."""
-    if (rows, split) != (0, 0) and not (rows in (32, 64) and split in (1, 2, 4, 8)) and (rows, split) != (64, 0):
+    128; 64 and -4: those of 64 x 64 with K in four parts); linear_f32_tiles(0): chosen.  For tests."""
+    if (rows, split) not in ((0, 0), (64, 0), (64, -4)) and not (rows in (32, 64) and split in (1, 2, 4, 8)):
         raise KernelError(f"linear: there are no 32-bit tiles of {rows} rows shared by {split} blocks")
     library().tlc_linear_f32_tiles(int(rows), int(split))
 
 
-def linear_f32_plan(M: int, N: int, sms: int) -> tuple:
+def linear_f32_plan(M: int, N: int, K: int, sms: int) -> tuple:
     """(rows of a tile, blocks a tile) of a 32-bit product of M > 16 rows, as linear_f32_tiles names them."""
-    return divmod(library().tlc_linear_f32_plan(int(M), int(N), int(sms)), 16)
+    rows, split = divmod(library().tlc_linear_f32_plan(int(M), int(N), int(K), int(sms)), 256)
+    return rows, split - 256 if split > 127 else split
 
 
 def linear_pairs() -> int:
