@@ -1,4 +1,4 @@
-"""Which tiles a 32-bit product takes: the rule and the test hook that overrides it, on the host."""
+"""Which kernels a product takes: the rules, and the test hooks that override them, on the host."""
 import pytest
 
 from tinyllama_c_b200 import ops
@@ -33,3 +33,12 @@ def test_tiles_that_do_not_exist_cannot_be_asked_for():
     (2048, 8192, 17, (32, 8)), (2048, 8192, 130, (64, 4)), (2048, 8192, 1200, (64, 0)), (4096, 2048, 17, (32, 8))])
 def test_tiles_of_32_bit_products_by_their_sizes(K, N, M, plan):
     assert ops.linear_f32_plan(M, N, K, 148) == plan
+
+
+@pytest.mark.parametrize("N,K,takes", [
+    (2368, 4096, False), (2384, 4096, True), (2384, 4064, False),               # 148 tiles and 149; a K of 127 steps
+    (3328, 4096, True), (3329, 4096, False), (3552, 5384, False),               # 208 tiles are 104 clusters, all at once; 209
+    (3552, 8192, True), (3553, 8192, False), (3552, 12288, True), (4064, 12288, False)])
+def test_rings_of_17_to_32_rows_where_all_clusters_run_at_once(N, K, takes):
+    """Beyond that a second round of clusters costs more than the ring brings, up to K = 8192 (figures beside the rule)."""
+    assert bool(ops.library().tlc_linear_skinny_ring_takes(N, K, 148, 104)) == takes

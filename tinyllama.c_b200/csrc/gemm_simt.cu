@@ -562,7 +562,7 @@ static void launch_split_f32x4(const float* a, int lda, const float* w, int ldw,
 // 17 to 3,000 rows; of the two candidates the better one by it is within 6 % of the better one as measured in all but 7 of them
 // (15 % at most).  Cluster and one block a tile, microseconds: 1,200 rows of 32 -> 2048 39.5 and 9.4, of 256 -> 2048 58.6
 // and 43.1, of 1024 -> 2048 153 and 159; 310 rows of 128 -> 8192 49.2 and 24.1, of 1024 -> 8192 162 and 159; 48 rows of 64 -> 2048 6.2
-// and 5.0, of 128 -> 2048 6.3 and 7.0, of 1024 -> 2048 19.7 and 35.3; 3,000 rows of 1024 -> 64 56 and 36.
+// and 5.0, of 128 -> 2048 6.3 and 7.0, of 1024 -> 2048 19.7 and 35.3; 3,000 rows of 1024 -> 64 57 and 37.
 struct F32Plan { int rows, split; };                         // split 0: the tiles of 64 x 128; -4: of 64 x 64, K in four parts
 static int f32_blocks(int rows, int cols, int split, int M, int N, int sms) {   // on the fullest SM
   const long long tiles = (long long)((M + rows - 1) / rows) * ((N + cols - 1) / cols);
@@ -1081,6 +1081,40 @@ gemm_skinny_ring_kernel(const __nv_bfloat16* __restrict__ a, int lda, const __nv
 }
 static int g_skinny_ring = 1;         // 0: never that division of the work (for comparisons)
 
+// The launch of gemm_skinny_ring_kernel for `tiles` tiles of 16 columns; how many of its clusters the GPU runs at once.
+static cudaLaunchConfig_t ring_config(unsigned tiles, cudaLaunchAttribute* attr) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((tiles + 1) / 2 * 4);
+  cfg.blockDim = dim3(128);
+  cfg.dynamicSmemBytes = RingSmem::BYTES;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 4;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = g_tlc_pdl ? 2 : 1;
+  return cfg;
+}
+template <typename TO> static int ring_clusters() {
+  static int n = -1;
+  if (n < 0) {
+    cudaLaunchAttribute attr[2];
+    cudaLaunchConfig_t cfg = ring_config(2, attr);
+    cfg.numAttrs = 1;
+    int got = 0;
+    n = cudaOccupancyMaxActiveClusters(&got, gemm_skinny_ring_kernel<TO>, &cfg) == cudaSuccess ? got : 0;
+    if (n == 0) cudaGetLastError();
+  }
+  return n;
+}
+// Whether an output of N columns is among those that the ring serves (where the rule's sides are measured: launch_skinny_mg).
+extern "C" int tlc_linear_skinny_ring_takes(int N, int K, int sms, int clusters) {
+  const int tiles = (N + 15) / 16, n_steps = ((K >> 3) + 3) >> 2;
+  return tiles > sms && n_steps >= 128 && ((tiles + 1) / 2 <= clusters || (n_steps >= 256 && tiles <= sms * 3 / 2));
+}
+
 constexpr int SK_TWO_SMEM = 4 * 2 * SK_WARPS * 32 * (int)sizeof(uint4);
 static int g_skinny_two = 1;          // 0: never two tiles a block (for comparisons)
 
@@ -1148,28 +1182,21 @@ static void launch_skinny_mg(const __nv_bfloat16* a, int lda, const __nv_bfloat1
     }
   }
   if constexpr (MG == 4 && !SWIGLU) {
-    // Narrow outputs of a long K, all of whose blocks are resident at once.  Microseconds, the kernel below and the ring: 17 / 32
-    // rows of 5376 -> 2560 16.2 / 17.8 and 11.5 / 12.0, 8192 -> 2560 21.1 / 23.2 and 14.0 / 14.6, 4608 -> 3072 15.8 / 17.4 and 11.6 /
-    // 12.0, 12288 -> 3072 30.2 / 32.7 and 19.6 / 21.1, but 4096 -> 2048 (128 tiles) 7.3 / 7.9 and 9.0 / 9.2.  A captured step of the 3B
-    // sizes at batch 24 4057 and 3610, of the 7B sizes at batch 32 7041 and 5970.  (9 to 16 rows gained up to a tenth alone and
-    // lost in a step, beside kernels that want another split of the SM's memory: 3B at batch 16 3253 and 3728.)
+    // Narrow outputs of a long K.  Microseconds, the kernel below and the ring: 17 / 32 rows of 5376 -> 2560 16.2 / 17.8 and 11.5 /
+    // 12.0, 8192 -> 2560 21.1 / 23.2 and 14.0 / 14.6, 4608 -> 3072 15.8 / 17.4 and 11.6 / 12.0, 12288 -> 3072 30.2 / 32.7 and 19.6 /
+    // 21.1, but 4096 -> 2048 (128 tiles) 7.3 / 7.9 and 9.0 / 9.2.  A captured step of the 3B sizes at batch 24 4057 and 3610, of the 7B
+    // sizes at batch 32 7041 and 5970.  (9 to 16 rows gained up to a tenth alone and lost in a step, beside kernels that want
+    // another split of the SM's memory: 3B at batch 16 3253 and 3728.)  It pays while all clusters are resident at once, 104
+    // here (208 tiles): 4096 -> 3328 13.7 / 15.1 and 10.2 / 10.7, 4096 -> 3360 13.7 / 15.1 and 14.8 / 15.4, 4096 -> 4064 14.1 /
+    // 15.4 and 16.3 / 17.8, 5384 -> 3552 19.2 / 22.1 and 21.6 / 24.4; from K = 8192 on up to 222 tiles: 8192 -> 3360 22.7 / 24.7 and 21.8 /
+    // 23.0, 12288 -> 3552 31.6 / 34.3 and 30.4 / 32.7, but 8192 -> 4064 23.5 / 25.5 and 24.7 / 25.2.  (Outputs of 4,096 and more
+    // are another kernel's.)
     static int sms = 0;
     if (sms == 0) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
-    if (g_skinny_ring && (int)blocks > sms && (int)blocks <= 2 * sms && n_steps >= 128 && tlc_linear_simt_init() == 0) {
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3((blocks + 1) / 2 * 4);
-      cfg.blockDim = dim3(128);
-      cfg.dynamicSmemBytes = RingSmem::BYTES;
-      cfg.stream = stream;
+    if (g_skinny_ring && (int)blocks > sms && tlc_linear_simt_init() == 0 && tlc_linear_skinny_ring_takes(N, K, sms, ring_clusters<TO>())) {
       cudaLaunchAttribute attr[2];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = 4;
-      attr[0].val.clusterDim.y = 1;
-      attr[0].val.clusterDim.z = 1;
-      attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-      attr[1].val.programmaticStreamSerializationAllowed = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = g_tlc_pdl ? 2 : 1;
+      cudaLaunchConfig_t cfg = ring_config(blocks, attr);
+      cfg.stream = stream;
       cudaLaunchKernelEx(&cfg, gemm_skinny_ring_kernel<TO>, a, lda, w, ldw, out, ldo, colscale, colbias, accumulate, M, N, K);
       return;
     }

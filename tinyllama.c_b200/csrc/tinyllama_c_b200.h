@@ -181,6 +181,7 @@ int tlc_linear_f32_plan(int M, int N, int K, int sms);   // which of these a pro
 void tlc_linear_tma_out(int on);        // 0: the tensor-core product's 32-bit outputs never leave through the copy engine (for comparisons)
 void tlc_linear_skinny_pairs(int on);   // 0: the skinny product never splits K over a pair of blocks (for comparisons)
 void tlc_linear_skinny_two(int on);      // 0: the product of up to 8 rows never takes two tiles a block (for comparisons)
+int tlc_linear_skinny_ring_takes(int N, int K, int sms, int clusters);   // whether it does, where `clusters` of them run at once on `sms` SMs
 void tlc_linear_skinny_ring(int on);     // 0: the product of 17 to 32 rows never shares a tile among a cluster of four (for comparisons)
 int tlc_linear_skinny_ok(int a_dtype, int lda, const void* a, int w_dtype, int ldw, const void* w, int M, int K);
 int tlc_linear_skinny(const void* a, int lda, const void* w, int ldw, void* out, int out_dtype, int ldo,
