@@ -42,3 +42,14 @@ def test_tiles_of_32_bit_products_by_their_sizes(K, N, M, plan):
 def test_rings_of_17_to_32_rows_where_all_clusters_run_at_once(N, K, takes):
     """Beyond that a second round of clusters costs more than the ring brings, up to K = 8192 (figures beside the rule)."""
     assert bool(ops.library().tlc_linear_skinny_ring_takes(N, K, 148, 104)) == takes
+
+
+@pytest.mark.parametrize("N,K,plain,activation", [
+    (4736, 2048, False, False), (4752, 2048, True, False), (9472, 2048, True, True), (9488, 2048, False, False),   # 296, 297, 592, 593 tiles
+    (8192, 1024, False, False), (8192, 1032, True, True), (8192, 2056, False, False),                              # one round of K
+    (4752, 1032, True, True), (4752, 1280, True, False), (5600, 1280, True, True), (5600, 1800, True, False), (6400, 1800, True, True),
+    (5600, 2048, True, False), (6400, 2048, True, True)])
+def test_two_tiles_a_block_where_that_is_quicker(N, K, plain, activation):
+    """With the gated activation a little later than without (figures beside the rule)."""
+    takes = ops.library().tlc_linear_skinny_two_takes
+    assert (bool(takes(N, K, 0, 148)), bool(takes(N, K, 1, 148))) == (plain, activation)

@@ -1117,6 +1117,16 @@ extern "C" int tlc_linear_skinny_ring_takes(int N, int K, int sms, int clusters)
 
 constexpr int SK_TWO_SMEM = 4 * 2 * SK_WARPS * 32 * (int)sizeof(uint4);
 static int g_skinny_two = 1;          // 0: never two tiles a block (for comparisons)
+// Whether two tiles a block serve an output of N columns: more tiles than the SMs hold blocks of one (two an SM), K of one round.
+// With the activation the second tile's share has to be a little larger, the more the longer K is (a tile a block, two; 1 / 8 rows):
+// 1280 -> 4752 4.07 / 4.17 and 4.14 / 4.53, -> 5600 4.71 / 4.71 and 4.41 / 4.70; 1800 -> 4752 5.01 / 5.65 and 5.55 / 6.29, -> 5600
+// 5.64 / 6.24 and 5.91 / 6.60, -> 6400 6.29 / 6.80 and 6.14 / 6.66; 2048 -> 5600 5.61 / 6.11 and 5.72 / 6.17, -> 6400 6.51 / 6.45 and 5.97 /
+// 6.35, -> 8192 7.47 / 7.65 and 6.55 / 6.91; without it 2048 -> 4752 5.49 / 5.91 and 5.25 / 5.71, 1032 -> 9472 5.48 / 5.94 and 4.71 / 5.19.
+extern "C" int tlc_linear_skinny_two_takes(int N, int K, int activation, int sms) {
+  const int tiles = (N + 15) / 16, n_steps = ((K >> 3) + 3) >> 2;
+  const int from = 2 * sms + (activation ? (n_steps - 33) * sms / 64 : 0);
+  return n_steps > SK_WARPS * 2 && n_steps <= SK_WARPS * 4 && tiles > from && tiles <= 4 * sms;
+}
 
 // Kernels that ask for more than 48 KB of shared memory: once a device, ahead of any stream capture where the library is set up
 // first (tlc_linear_init), else with the first product that takes one of them.
@@ -1174,8 +1184,7 @@ static void launch_skinny_mg(const __nv_bfloat16* a, int lda, const __nv_bfloat1
   if constexpr (MG == 1) {
     static int sms = 0;
     if (sms == 0) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
-    if (g_skinny_two && n_steps > SK_WARPS * 2 && n_steps <= SK_WARPS * 4 && (int)blocks > 2 * sms && (int)blocks <= 4 * sms &&
-        tlc_linear_simt_init() == 0) {
+    if (g_skinny_two && tlc_linear_skinny_two_takes(N, K, SWIGLU, sms) && tlc_linear_simt_init() == 0) {
       tlc_launch(gemm_skinny_two_kernel<TO, SWIGLU>, dim3((blocks + 1) / 2), dim3(SK_WARPS * 32), SK_TWO_SMEM, stream, a, lda, w, ldw, out, ldo, colscale,
                  colbias, accumulate, M, N, K);
       return;

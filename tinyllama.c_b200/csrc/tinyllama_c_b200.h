@@ -180,6 +180,7 @@ void tlc_linear_f32_tiles(int rows, int split);  // 32-bit products of more than
 int tlc_linear_f32_plan(int M, int N, int K, int sms);   // which of these a product of M > 16 rows takes: 256 * rows + the low byte of split
 void tlc_linear_tma_out(int on);        // 0: the tensor-core product's 32-bit outputs never leave through the copy engine (for comparisons)
 void tlc_linear_skinny_pairs(int on);   // 0: the skinny product never splits K over a pair of blocks (for comparisons)
+int tlc_linear_skinny_two_takes(int N, int K, int activation, int sms);   // whether it does, with or without the gated activation, on `sms` SMs
 void tlc_linear_skinny_two(int on);      // 0: the product of up to 8 rows never takes two tiles a block (for comparisons)
 int tlc_linear_skinny_ring_takes(int N, int K, int sms, int clusters);   // whether it does, where `clusters` of them run at once on `sms` SMs
 void tlc_linear_skinny_ring(int on);     // 0: the product of 17 to 32 rows never shares a tile among a cluster of four (for comparisons)

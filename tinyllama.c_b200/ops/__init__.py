@@ -68,6 +68,7 @@ _SIGNATURES = {
     "tlc_linear_skinny_pairs": (None, [_i]),
     "tlc_linear_skinny_two": (None, [_i]),
     "tlc_linear_skinny_ring": (None, [_i]),
+    "tlc_linear_skinny_two_takes": (_i, [_i, _i, _i, _i]),
     "tlc_linear_skinny_ring_takes": (_i, [_i, _i, _i, _i]),
     "tlc_linear_tma_out": (None, [_i]),
     "tlc_linear_few_rows": (None, [_i]),
