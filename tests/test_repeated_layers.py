@@ -202,25 +202,33 @@ def test_a_function_put_around_the_layers_is_called_for_every_one(monkeypatch, w
     assert len(calls) == times * len(model.layers) and torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
 
 
-def test_steps_that_wait_for_the_gpu_run_layer_by_layer(monkeypatch):
+def test_steps_that_wait_for_the_gpu_are_told_by_rows_and_weights():
     """From a number of rows on that falls with the size of a layer's matrices, and with their type's rate."""
     layers = [_Forks(i) for i in range(4)]
-    assert _run_on_the_host(monkeypatch, layers, 0x77, 1023)[0] == 4
-    assert _run_on_the_host(monkeypatch, layers, 0x77, 1024) == (0, [])
+    look = lambda: RepeatedLayers.of(layers, [LayerRun(i) for i in range(len(layers))])  # noqa: E731
+    assert not look().is_long(1023) and look().is_long(1024)
     first = {}
     for dtype in (torch.float32, torch.bfloat16):
         for n in (2048, 4096):
             for layer in layers:
                 layer.weight = torch.empty(n, n, dtype=dtype)
                 layer.gain = layer.weight[:n // 2]              # (rows of the same matrix: counted once)
-            found = RepeatedLayers.of(layers, [LayerRun(i) for i in range(len(layers))])
-            first[dtype, n] = next(rows for rows in range(1, 1025) if found.is_long(rows))
-    rows = first[torch.float32, 4096]
-    assert rows < first[torch.float32, 2048] < first[torch.bfloat16, 4096] <= first[torch.bfloat16, 2048] == 1024
-    for layer in layers:
-        layer.weight = layer.gain = torch.empty(4096, 4096)
-    assert _run_on_the_host(monkeypatch, layers, 0x77, rows - 1)[0] == 4
-    assert _run_on_the_host(monkeypatch, layers, 0x77, rows) == (0, [])
+            first[dtype, n] = next(rows for rows in range(1, 1025) if look().is_long(rows))
+    assert first[torch.float32, 4096] < first[torch.float32, 2048] < first[torch.bfloat16, 4096] <= first[torch.bfloat16, 2048] == 1024
+
+
+@pytest.mark.gpu
+def test_long_steps_run_layer_by_layer(monkeypatch):
+    model, got, times = _model("tensor cores", torch.bfloat16, "cuda:0"), [], []
+    table = ops.replay
+    monkeypatch.setattr(ops, "replay", lambda functions, words, n: (times.append(n), table(functions, words, n)))
+    for limit, repeated in ((1024, 3), (60, 3), (59, 0)):
+        model.repeated.LONG_STEP = limit
+        llm = tlc.LLM(model, dtype="bfloat16", max_tokens=64 * 8, max_seqs=2)
+        got.append(llm.step([StepEntry(llm.cache.acquire(), list(range(1, 60)), (58,))]).clone())
+        assert sum(times) == repeated
+        times.clear()
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
 
 
 def test_parts_that_say_nothing_are_not_repeated():
@@ -272,7 +280,7 @@ class _Forks(Editable):
         return False
 
 
-def _run_on_the_host(monkeypatch, layers, stream, rows=1):
+def _run_on_the_host(monkeypatch, layers, stream):
     """(entries that ran, [stream of every norm call made again]) of a step on a stream of that handle, and the words."""
     got = []
     monkeypatch.setattr(ops, "stream_handle", lambda: stream)
@@ -280,7 +288,7 @@ def _run_on_the_host(monkeypatch, layers, stream, rows=1):
     found = RepeatedLayers.of(layers, [LayerRun(i) for i in range(len(layers))])
     i32 = torch.zeros(4, dtype=torch.int32)
     step = StepInfo(1, 1, i32, i32, i32, i32, i32, i32)
-    done, left = found.run(torch.zeros(rows, 8), step, SimpleNamespace(layer_view=lambda r, writes, kv: LayerCache()))
+    done, left = found.run(torch.zeros(1, 8), step, SimpleNamespace(layer_view=lambda r, writes, kv: LayerCache()))
     rows = [row for _, words in got for row in words.tolist()]
     return done, rows
 

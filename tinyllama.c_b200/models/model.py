@@ -149,7 +149,7 @@ class Model:
         with step_scratch(step):                       # the layers share the step's temporaries
             ready, done = False, 0                     # whether a layer left the next one's input (Block.entry)
             repeated = self.repeated
-            if repeated is not None and not torch.cuda.is_current_stream_capturing():
+            if repeated is not None and not repeated.is_long(step.n_rows) and not torch.cuda.is_current_stream_capturing():
                 if not repeated.stands(self.layers, self.schedule):
                     repeated = self.repeated = RepeatedLayers(self.layers, self.schedule)
                 if repeated.alike and repeated.untouched():

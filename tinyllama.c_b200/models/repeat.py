@@ -128,8 +128,6 @@ class RepeatedLayers:
     def run(self, x: torch.Tensor, step: StepInfo, cache) -> Tuple[int, bool]:
         """Runs the first layer, and the others if they can be repeated; (how many entries of the run order have run,
         whether the last of them has left the next one's input)."""
-        if self.is_long(x.shape[0]):
-            return 0, False
         views = [cache.layer_view(r, True, None) for r in range(len(self.layers))]
         with ops.noting() as notes:
             left = self.layers[0].forward(x, step, views[0], False, self.layers[1].entry)
@@ -200,7 +198,8 @@ class RepeatedLayers:
         return n, False
 
     def is_long(self, rows: int) -> bool:
-        """Whether a step of that many rows waits for the GPU and not for the host."""
+        """Whether a step of that many rows waits for the GPU and not for the host (its layers run one by one, and nothing is
+        looked at)."""
         return rows >= self.LONG_STEP or self.read_s + rows * self.row_s >= self.LONG_LAYER
 
     def stands(self, layers=None, schedule=None) -> bool:
