@@ -97,3 +97,21 @@ def test_output_projections_as_one_product(cpu_kernels):
     rows = [1.0] * 12 + [2.0] * 12
     assert StackedLinear.fuse_bound_inputs([_bound(16, 24, 1.0, False, 1), _bound(40, 24, rows, False, 2)], [False, True]) is None
     assert StackedLinear.fuse_bound_inputs([_bound(16, 24, 1.0, False, 1), _bound(40, 32, 1.0, False, 2)], [True, True]) is None
+
+
+@pytest.mark.parametrize("lens,rows", [
+    ((30,), None), ((33,), 128), ((48,), 128), ((49,), 32), ((500,), 32), ((800,), 32), ((900,), 128), ((60,) * 4, 32), ((60,) * 11, 32),
+    ((60,) * 12, 128), ((100,) * 5, 32), ((100,) * 6, 128), ((200,) * 4, 32), ((200,) * 5, 128), ((33,) * 20, 128), ((600, 600), 128)])
+def test_chunks_of_32_bit_scans_by_how_many_there_are(lens, rows):
+    """Short ones where they are few (48 heads of 64: up to 22, or 28 where a sequence is cut by 128 too); a 16-bit run never takes them."""
+    from types import SimpleNamespace
+    from tinyllama_c_b200.engine.step import chunk_table
+    from tinyllama_c_b200.parts.mixers.mamba2 import Mamba2Mixer
+    mixer = Mamba2Mixer(64, 48 * 64, 48, 64, 1, 256, 4, "m.", 1e-5)
+    for dtype in (torch.float32, torch.bfloat16):
+        mixer.dtype = dtype
+        tables = {q.rows: chunk_table(lens, q.rows, q.from_rows) for q in mixer.step_requests()}
+        tables = {n: tuple(map(torch.tensor, t)) if t else None for n, t in tables.items()}
+        step = SimpleNamespace(chunks=tables, max_new=max(lens), n_rows=sum(lens))
+        want = None if rows is None else tables[rows if dtype == torch.float32 else 128]
+        assert mixer._chunks(step) is want

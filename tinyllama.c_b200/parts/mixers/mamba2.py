@@ -100,11 +100,28 @@ class Mamba2Mixer(Part):
     CHUNKS_FROM_ROWS = 8
     CHUNKS_WORTH_ROWS, CHUNKS_WORTH_STEP = 32, 128
 
-    # In 32 bits the chunks run row by row, one beside the other, and a chunk's rows are what a step of few rows waits for: steps
-    # of up to SHORT_CHUNKS_STEP rows are cut into chunks of SHORT_CHUNK (48 heads of 64, 256 columns, chunks of 128 / 32 rows, the
-    # three passes: 120 rows 91 / 79 us, 310 rows 188 / 140, 600 281 / 252, 1,000 418 / 417).  More rows fill the GPU with
-    # chunks of any length, and every chunk costs a state of scratch.
-    SHORT_CHUNK, SHORT_CHUNKS_STEP = 32, 1024
+    # In 32 bits the chunks run row by row, one beside the other, and a chunk's rows are what a step of few chunks waits for: such steps
+    # are cut into chunks of SHORT_CHUNK.  More chunks fill the GPU whatever their length, and every chunk costs a state of
+    # scratch that three passes read and write: the blocks of a pass (16 head rows of a head of a chunk each) may be as many as
+    # 22 chunks of 48 heads of 64 make, 28 where a sequence is cut by scan_chunk too, and sequences of no more than SHORT_ROWS gain
+    # nothing.  Microseconds for the three passes with 256 columns, chunks of 128 and of 32 rows: 60 rows 64 / 54, 128 115 / 75,
+    # 500 240 / 210, 800 (25 short chunks) 344 / 330, 900 (29) 370 / 376; sequences of 60 rows, 2 / 4 / 6 of them 101 / 145 / 187
+    # and 79 / 136 / 192; of 100 rows, 4 / 6 / 9 (16 / 24 / 36 short chunks) 217 / 275 / 403 and 198 / 293 / 470; of 200, 3 / 4 (21 / 28)
+    # 303 / 371 and 263 / 359; 20 of 33 (40) 399 / 511; 4 of 40 110 / 114.  (So the rounding of a sequence's rows in 32 bits depends
+    # on what else a step brings, as CHUNKS_WORTH_STEP lets it in any type.)
+    SHORT_CHUNK, SHORT_ROWS, SHORT_CHUNKS_STEP = 32, 48, 1024
+    SHORT_BLOCKS, SHORT_BLOCKS_CUT = 22 * 48 * 4, 28 * 48 * 4
+
+    def _chunks(self, step: StepInfo):
+        """The table that cuts this step's sequences into chunks (None: row by row)."""
+        if step.max_new <= self.CHUNKS_WORTH_ROWS and step.n_rows < self.CHUNKS_WORTH_STEP:
+            return None
+        short = step.chunks.get(self.SHORT_CHUNK) if self.dtype == torch.float32 and self.SHORT_CHUNK < self.scan_chunk else None
+        if short is not None and step.max_new > self.SHORT_ROWS and step.n_rows <= self.SHORT_CHUNKS_STEP:
+            blocks = short[1].numel() * self.Hs * ((self.P + 15) // 16)
+            if blocks <= (self.SHORT_BLOCKS_CUT if step.max_new > self.scan_chunk else self.SHORT_BLOCKS):
+                return short
+        return step.chunks.get(self.scan_chunk)
 
     def step_requests(self) -> list:
         """(asked for again once the run's type is known)"""
@@ -171,10 +188,7 @@ class Mamba2Mixer(Part):
                               (proj, self.Di, conv_state, step.slots, step.start_pos, self.Di, self.Cd - self.Di))
         # prompts cut into chunks of a bfloat16 run: the scan in matrix form, whose operands x|B|C the convolution
         # writes in bfloat16 at once; everything else scans 32-bit values
-        short = self.dtype == torch.float32 and step.n_rows <= self.SHORT_CHUNKS_STEP
-        chunks = step.chunks.get(self.SHORT_CHUNK if short and self.SHORT_CHUNK in step.chunks else self.scan_chunk)
-        if chunks is not None and step.max_new <= self.CHUNKS_WORTH_ROWS and step.n_rows < self.CHUNKS_WORTH_STEP:
-            chunks = None
+        chunks = self._chunks(step)
         matrix_form = chunks is not None and self.dtype == torch.bfloat16 and self.scan_chunk <= ops.SSD_CHUNK \
             and ops.ssd_ok(self.Hs, self.P, self.N, self.G)
         xbc = new("xbc", (T, self.Cd), torch.bfloat16 if matrix_form else f32)
