@@ -516,8 +516,9 @@ ssm_scan_kernel(const float* __restrict__ xbc, const float* __restrict__ dt, con
 }
 
 // The same for states of more than 64 columns where everything lies in pieces of 16 bytes (columns and head rows multiples of 4,
-// xbc, its rows and the states on 16-byte boundaries): the state's values and the order of every sum are those of the kernel
-// above, a row costs less.  What a row cost there: four sums over a warp of five shuffles each, one after the other, B and C
+// xbc, its rows and the states on 16-byte boundaries): row by row the state's values and the order of every sum are those of the
+// kernel above, a row costs less.  (In chunks the decays of a chunk's rows are multiplied in another order: a lane's rows first,
+// then the lanes.)  What a row cost there: four sums over a warp of five shuffles each, one after the other, B and C
 // read value by value with a stride of four (bank conflicts), and a division and an address from scratch for every piece that
 // is copied.  Here the sums of SCAN_TT rows x RP head rows, which every lane holds a share of, go through the same tree together:
 // at each of the first steps a lane hands half of its values to its partner and keeps the other half (16 values: 16 shuffles
