@@ -134,6 +134,15 @@ def test_a_mixers_own_projection_lives_as_long_as_the_step(monkeypatch):
     assert len(seen) == 2 and all(any(t is held for held in step.scratch.values()) for t in seen)
 
 
+def test_numbers_are_noted_as_the_library_gets_them():
+    """A number beyond the 32-bit range is infinite for the call (a clamp that is meant to be none), and so it is when noted."""
+    with ops.noting() as notes:
+        for v in (0.5, -0.0, 3, 1e39, -1e39, float("inf"), 1e-46):
+            notes.add("tlc_glu", (16, 0, 8, 1, 0, 32, 0, 4, 1, v, 1.0, 0))
+    got = [notes.words[12 * i + 9] for i in range(7)]
+    assert got == [0x3F000000, 0x80000000, 0x40400000, 0x7F800000, 0xFF800000, 0x7F800000, 0]
+
+
 @pytest.mark.gpu
 def test_layers_whose_weights_are_all_laid_out_otherwise_run_one_by_one():
     model, got = _model("tensor cores", torch.bfloat16, "cuda:0"), []

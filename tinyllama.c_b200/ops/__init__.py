@@ -241,7 +241,7 @@ class NotedCalls:
         self.functions.append(index)
         for a, pointer in zip(args, kinds):
             if pointer is None:                            # a float, by its bits
-                self.words.append(_F32_BITS.unpack(_F32_PACK.pack(a))[0])
+                self.words.append(_F32_BITS.unpack(_f(a))[0])
                 self.is_pointer.append(False)
                 continue
             if a is None:
@@ -257,7 +257,7 @@ class NotedCalls:
             self.handles.add(args[-1])                     # the stream
 
 
-_F32_PACK, _F32_BITS = struct.Struct("<f"), struct.Struct("<I")
+_F32_BITS = struct.Struct("<I")
 
 
 class _Notes(threading.local):
