@@ -1202,7 +1202,7 @@ static void launch_skinny_mg(const __nv_bfloat16* a, int lda, const __nv_bfloat1
     // are another kernel's.)
     static int sms = 0;
     if (sms == 0) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
-    if (g_skinny_ring && (int)blocks > sms && tlc_linear_simt_init() == 0 && tlc_linear_skinny_ring_takes(N, K, sms, ring_clusters<TO>())) {
+    if (g_skinny_ring && (int)blocks > sms && n_steps >= 128 && tlc_linear_simt_init() == 0 && tlc_linear_skinny_ring_takes(N, K, sms, ring_clusters<TO>())) {
       cudaLaunchAttribute attr[2];
       cudaLaunchConfig_t cfg = ring_config(blocks, attr);
       cfg.stream = stream;

@@ -16,7 +16,7 @@ they can be repeated.
 """
 from __future__ import annotations
 
-from operator import attrgetter
+from operator import attrgetter, getitem, itemgetter
 from types import FunctionType
 from typing import List, Optional, Tuple
 
@@ -28,12 +28,17 @@ from ..parts.base import Editable, LayerCache, StepInfo, current_stream, used_on
 
 
 _PLAIN = (type(None), bool, int, float, str, torch.dtype, torch.device)
+_LOW = np.uint64(15)
 _edits = attrgetter("edits")
 _ptr, _size, _stride, _dtype = torch.Tensor.data_ptr, torch.Tensor.size, torch.Tensor.stride, attrgetter("dtype")
 
 
-# The wrappers of the kernel library as they are defined.  (ops.replay is what this module itself calls.)
-_OPS = {k: f for k, f in vars(ops).items() if isinstance(f, FunctionType) and k != "replay"}
+# The wrappers of the kernel library as they are defined: the functions that make its calls.  (ops.replay is what this module itself calls.)
+_OPS = {k: f for k, f in vars(ops).items()
+        if isinstance(f, FunctionType) and k != "replay" and (k == "_call" or {"_call", "library"}.intersection(f.__code__.co_names))}
+# methods that a step has no use for
+_NOT_IN_A_STEP = {"__init__", "bind", "weight_specs", "cache_requests", "step_requests", "shapes_from", "parts", "repeats", "add", "fuse_bound",
+                  "fuse_bound_inputs", "out_features", "__setattr__", "__delattr__", "__init_subclass__"}
 
 
 class _Description:
@@ -76,6 +81,13 @@ class _Description:
             self.inside.remove(id(obj))
 
 
+def _items(places: List[int]):
+    """What takes the values at these places out of a list."""
+    if len(places) > 1:
+        return itemgetter(*places)
+    return (lambda values: (values[places[0]],)) if places else (lambda values: ())
+
+
 def _of_cache(view: LayerCache) -> Tuple[tuple, List[torch.Tensor]]:
     """(what must be equal, tensors) of a layer's part of the cache."""
     tensors = []
@@ -105,12 +117,18 @@ class RepeatedLayers:
 
     def __init__(self, layers, schedule):
         self.order = layers, schedule
+        self.all_edits = Editable.all_edits[0]            # (ahead of the look)
         self.parts, self.lists = [], [layers, schedule]
         self.layers = [layers[r.layer] for r in schedule]
         classes = set()
         found = [_Description(layer, self.parts, self.lists, classes) for layer in self.layers]
-        self.written = [(vars(ops), list(_OPS), list(_OPS.values()))] + [(vars(c), list(c.as_written), list(c.as_written.values())) for c in classes]
+        self.written = [(vars(ops), list(_OPS), list(_OPS.values()))]
+        for c in classes:
+            methods = {k: f for k, f in c.as_written.items() if k not in _NOT_IN_A_STEP}
+            if methods:
+                self.written.append((vars(c), list(methods), list(methods.values())))
         self.tensors = [d.tensors for d in found]
+        self.holders = [[attributes for attributes, _ in t] for t in self.tensors]
         self.read_s = self.row_s = 0.0                     # a layer's matrices read once, and what every row adds, in seconds
         spans, end = [], 0
         for t in (attributes[name] for attributes, name in self.tensors[0]) if self.tensors else ():
@@ -151,8 +169,9 @@ class RepeatedLayers:
         shared = notes.handles.difference(handles[0]).union((0,), map(_ptr, common))
         ranges = None
         places, which = [], []                             # words to replace, and by which tensor's address
-        for w, (word, pointer) in enumerate(zip(notes.words, notes.is_pointer)):
-            if not pointer or word in shared:
+        for w in notes.pointers:
+            word = notes.words[w]
+            if word in shared:
                 continue
             i = at.get(word)
             if i is not None:
@@ -164,34 +183,44 @@ class RepeatedLayers:
             if not any(lo <= word < hi for lo, hi in ranges):
                 return done, left
         # a word says which address is meant, not which of the tensors that start there: they have to in every layer
-        ties = [(i, j) for i in set(which) if i < len(firsts) for j in also.get(addresses[i], ())]
-        used = sorted(set(which).union(j for _, j in ties))
+        used = sorted(set(which))
         rank = {i: n for n, i in enumerate(used)}
-        tied = [[rank[i] for i, _ in ties], [rank[j] for _, j in ties]]
+        ties = [(rank[i], j) for i in used if i < len(firsts) for j in also.get(addresses[i], ())]
         tensors = [i for i in used if i < len(firsts)]      # (the layers' own streams and events come behind them)
         like = self._meta([firsts[i] for i in tensors])
+        place = self.tensors[0]
+        own, own_names = _items([i for i in tensors if i < n_own]), [place[i][1] for i in tensors if i < n_own]
+        cached = _items([i - n_own for i in tensors if i >= n_own])
+        tied, tied_names = _items([j for _, j in ties if j < n_own]), [place[j][1] for _, j in ties if j < n_own]
+        tied_cached = _items([j - n_own for _, j in ties if j >= n_own])
+        tied_to = _items([n for n, j in ties if j < n_own] + [n for n, j in ties if j >= n_own])
+        own_handles = _items([i - len(firsts) for i in used[len(tensors):]])
         base = np.array([addresses[i] for i in tensors], dtype=np.uint64)
         first, functions = np.array(notes.words, dtype=np.uint64), np.array(notes.functions, dtype=np.int32)
         # The calls' own scratch came from the stream that the first layer made them on; the others use it on theirs.
         if notes.owned:
             used_on(current_stream(x.device), notes.owned)
-        columns = [rank[i] for i in which]
+        columns, places = np.array([rank[i] for i in which], dtype=np.intp), np.array(places, dtype=np.intp)
         # the next layer at once, so that the GPU has work while the others' addresses are gathered, then a few, then the rest
         while done < n:
             end = min(n, done + (1 if done < 3 else 4 if done < 6 else n))
             table = np.empty((end - done, len(used)), dtype=np.uint64)
             for r in range(done, end):
                 other, theirs = _of_cache(views[r])
-                row = [self.tensors[r][i] for i in tensors if i < n_own]
-                row = [attributes[name] for attributes, name in row] + [theirs[i - n_own] for i in tensors[len(row):]]
+                holders = self.holders[r]
+                row = list(map(getitem, own(holders), own_names))
+                row += cached(theirs)
                 if other != form or self._meta(row) != like:
                     return done, left
-                table[r - done] = list(map(_ptr, row)) + [handles[r][i - len(firsts)] for i in used[len(tensors):]]
-            if ((table[:, :len(tensors)] ^ base) & np.uint64(15)).any() or not table.all():
+                row = list(map(_ptr, row))
+                if ties and tuple(map(_ptr, (*map(getitem, tied(holders), tied_names), *tied_cached(theirs)))) != tied_to(row):
+                    return done, left
+                row += own_handles(handles[r])
+                table[r - done] = row
+            if np.count_nonzero((table[:, :len(tensors)] ^ base) & _LOW) or np.count_nonzero(table) != table.size:
                 return done, left                          # (the calls may choose by how their operands are aligned)
-            if (table[:, tied[0]] != table[:, tied[1]]).any():
-                return done, left
-            words = np.tile(first, (end - done, 1))
+            words = np.empty((end - done, first.size), dtype=np.uint64)
+            words[:] = first
             words[:, places] = table[:, columns]
             ops.replay(functions, words, end - done)
             done = end
@@ -205,8 +234,14 @@ class RepeatedLayers:
     def stands(self, layers=None, schedule=None) -> bool:
         """Whether nothing has been edited since the layers were looked at: no attribute of a part, no list or what is in it, and
         these (where given) are the lists that were looked at."""
-        return (layers is None or layers is self.order[0]) and (schedule is None or schedule is self.order[1]) \
-            and list(map(_edits, self.parts)) == self.edits and self.lists == self.copies
+        if (layers is not None and layers is not self.order[0]) or (schedule is not None and schedule is not self.order[1]) or self.lists != self.copies:
+            return False
+        now = Editable.all_edits[0]
+        if now != self.all_edits:                          # a part of some model
+            if list(map(_edits, self.parts)) != self.edits:
+                return False
+            self.all_edits = now
+        return True
 
     def untouched(self) -> bool:
         """Whether the layers' methods and the wrappers of the kernel library are those that the source has.  A function that a

@@ -224,13 +224,13 @@ def _call(name: str, *args) -> None:
 # thread are noted beside being made; replay() then makes them again, many rounds in one call of the library, with the
 # arguments that the caller has put in their places (models/repeat.py).
 class NotedCalls:
-    """Calls in the order they were made.  words: the arguments as 64-bit words; is_pointer marks those that are pointers.
+    """Calls in the order they were made.  words: the arguments as 64-bit words; pointers: which of them are pointers.
     owned: what the calls were given that no argument keeps alive (scratch, numbers on the host that a call writes).
     handles: streams and events that the calls name.  complete: False once a call was made that cannot be made again.
     forks: whether an event was recorded."""
 
     def __init__(self):
-        self.functions, self.words, self.is_pointer = [], [], []
+        self.functions, self.words, self.pointers = [], [], []
         self.owned, self.handles, self.complete, self.forks = [], set(), True, False
 
     def add(self, name: str, args) -> None:
@@ -242,7 +242,6 @@ class NotedCalls:
         for a, pointer in zip(args, kinds):
             if pointer is None:                            # a float, by its bits
                 self.words.append(_F32_BITS.unpack(_f(a))[0])
-                self.is_pointer.append(False)
                 continue
             if a is None:
                 a = 0
@@ -251,8 +250,9 @@ class NotedCalls:
                 self.owned.append(a)
                 a = ctypes.addressof(a)
                 self.handles.add(a)
+            if pointer:
+                self.pointers.append(len(self.words))
             self.words.append(a & 0xFFFFFFFFFFFFFFFF)
-            self.is_pointer.append(pointer)
         if name not in ("tlc_event_record", "tlc_event_wait"):
             self.handles.add(args[-1])                     # the stream
 

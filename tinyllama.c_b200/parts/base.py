@@ -125,8 +125,11 @@ class LayerCache:
 
 
 class Editable:
-    """Counts how often its attributes are set or deleted, so that what was found out about it (models/repeat.py) can be dropped."""
+    """Counts how often its attributes are set or deleted, so that what was found out about it (models/repeat.py) can be dropped.
+    all_edits[0] changes with every edit of any part; it counts up after the attribute is set, so that whoever reads it and then the
+    parts has seen every edit that it stands for."""
     edits = 0
+    all_edits = [0]
     passing = frozenset()        # attributes that a forward() sets for itself
     as_written: Dict[str, Any] = {}     # every class's methods, as its definition has them
 
@@ -138,10 +141,12 @@ class Editable:
         object.__setattr__(self, name, value)
         if name not in self.passing:
             object.__setattr__(self, "edits", self.edits + 1)
+            self.all_edits[0] += 1
 
     def __delattr__(self, name):
         object.__delattr__(self, name)
         object.__setattr__(self, "edits", self.edits + 1)
+        self.all_edits[0] += 1
 
     def repeats(self) -> Optional[frozenset]:
         """For a part whose forward() makes the same calls of the kernel library (and no other GPU work) whatever it is
