@@ -69,3 +69,27 @@ def test_rows_in_16_byte_pieces_give_the_general_kernels_bits(N, P, lens, chunk)
         got.append((y, st))
     for a, b in zip(*got):
         assert torch.equal(a, b) if not chunk else (a - b).abs().max() <= 70 * 2.0 ** -23 * b.abs().max()
+
+
+@pytest.mark.parametrize("B,Hs,P,N", [(3, 4, 8, 72), (64, 8, 64, 72), (65, 8, 64, 128), (65, 8, 64, 132)])
+def test_one_row_a_sequence_gives_the_same_bits_by_either_kernel(B, Hs, P, N):
+    """12, 2,048 and 2,080 blocks of up to 128 columns, and more columns; steps of one row each, and the same number of rows otherwise
+    divided (two of one sequence, none of another)."""
+    from tinyllama_c_b200 import ops
+    g = torch.Generator().manual_seed(B + N)
+    Di = Hs * P
+    xbc, dt, dA = torch.randn(B, Di + 2 * N, generator=g).cuda(), torch.rand(B, Hs, generator=g).cuda(), torch.rand(B, Hs, generator=g).cuda()
+    D, state = torch.randn(Hs, generator=g).cuda(), torch.randn(B, Hs, P, N, generator=g).cuda()
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")  # noqa: E731
+    for cu in (list(range(B + 1)), [0, 2, 2] + list(range(3, B + 1))):
+        got = []
+        for own in (True, False):
+            ops.ssm_scan_rows(own)
+            try:
+                y, st = torch.full((B, Di), float("nan"), device="cuda"), state.clone()
+                ops.ssm_scan(xbc, dt, dA, D, st, i32(cu), i32(range(B)), i32([3 if b % 2 else 0 for b in range(B)]), y, Hs, P, N, 1, None)
+                torch.cuda.synchronize()
+            finally:
+                ops.ssm_scan_rows(True)
+            got.append((y, st))
+        assert all(torch.equal(a, b) for a, b in zip(*got))

@@ -770,10 +770,16 @@ template <int NPL>
 static int launch_scan(const float* xbc, const float* dt, const float* dA, const float* Dskip, float* state,
                        float* chunk_state, const int* seg_start, const int* seg_seq, const int* seq_seg_start,
                        const int* slots, const int* start_pos, float* y, float* chunk_decay, int mode, int n_seg, int Hs,
-                       int P, int N, int G, int Cd, cudaStream_t stream) {
+                       int P, int N, int G, int Cd, bool one_row, cudaStream_t stream) {
   constexpr int RP = 4;
   if constexpr (NPL % 4 == 0) {
-    if (g_scan_rows && N % 4 == 0 && P % 4 == 0 && Cd % 4 == 0 && (((uintptr_t)state | (uintptr_t)chunk_state | (uintptr_t)xbc) & 15) == 0) {
+    // A row a sequence, up to 128 columns and many blocks: states in and out are all there is, and the general kernel has eight blocks
+    // an SM for that and not six.  Microseconds, by rows in 16-byte pieces and by the general kernel: 64 sequences of 24 heads of 64
+    // and 128 columns (6,144 blocks) 20.3 and 19.1, of 80 heads 59.5 and 54.5, 16 of 48 heads and 68 columns (3,072) 10.8 and 10.0;
+    // but 16 of 24 heads and 128 columns (1,536) 6.9 and 7.6, one sequence 3.0 and 3.2, and with two rows each 64 of 24 heads 22.6
+    // and 25.6.
+    const bool short_rows = one_row && NPL == 4 && (long long)n_seg * Hs * ((P + 15) / 16) > 2048;
+    if (g_scan_rows && !short_rows && N % 4 == 0 && P % 4 == 0 && Cd % 4 == 0 && (((uintptr_t)state | (uintptr_t)chunk_state | (uintptr_t)xbc) & 15) == 0) {
       tlc_launch(ssm_scan_rows_kernel<NPL>, dim3(n_seg, Hs, (P + 15) / 16), dim3(128), (size_t)2 * SCAN_TT * (2 * N + 20) * sizeof(float), stream,
                  xbc, dt, dA, Dskip, state, chunk_state, seg_start, seg_seq, seq_seg_start, slots, start_pos, y, chunk_decay, mode, Hs, P, N, G, Cd);
       TLC_CHECK_LAUNCH("ssm_scan");
@@ -799,8 +805,8 @@ static int launch_scan(const float* xbc, const float* dt, const float* dA, const
 static int scan_dispatch(const float* xbc, const float* dt, const float* dA, const float* Dskip, float* state,
                          float* chunk_state, const int* seg_start, const int* seg_seq, const int* seq_seg_start,
                          const int* slots, const int* start_pos, float* y, float* chunk_decay, int mode, int n_seg,
-                         int Hs, int P, int N, int G, int Cd, cudaStream_t stream) {
-#define TLC_SCAN(NPL) launch_scan<NPL>(xbc, dt, dA, Dskip, state, chunk_state, seg_start, seg_seq, seq_seg_start, slots, start_pos, y, chunk_decay, mode, n_seg, Hs, P, N, G, Cd, stream)
+                         int Hs, int P, int N, int G, int Cd, cudaStream_t stream, bool one_row = false) {
+#define TLC_SCAN(NPL) launch_scan<NPL>(xbc, dt, dA, Dskip, state, chunk_state, seg_start, seg_seq, seq_seg_start, slots, start_pos, y, chunk_decay, mode, n_seg, Hs, P, N, G, Cd, one_row, stream)
   if (N <= 32) return TLC_SCAN(1);
   if (N <= 64) return TLC_SCAN(2);
   if (N <= 128) return TLC_SCAN(4);
@@ -822,6 +828,16 @@ extern "C" int tlc_ssm_scan(const float* xbc, const float* dt, const float* dA, 
   if (int rc = scan_checks(Hs, N, G)) return rc;
   return scan_dispatch(xbc, dt, dA, Dskip, state, nullptr, cu_seqlens, nullptr, nullptr, slots, start_pos, y, nullptr,
                        SCAN_PLAIN, B, Hs, P, N, G, Cd, stream);
+}
+
+// The same for a step that brings one row of every sequence (a hint: the result does not depend on it).
+extern "C" int tlc_ssm_scan_one_row(const float* xbc, const float* dt, const float* dA, const float* Dskip, float* state,
+                                    const int* cu_seqlens, const int* slots, const int* start_pos, float* y, int B, int Hs,
+                                    int P, int N, int G, int Cd, cudaStream_t stream) {
+  if (B == 0) return 0;
+  if (int rc = scan_checks(Hs, N, G)) return rc;
+  return scan_dispatch(xbc, dt, dA, Dskip, state, nullptr, cu_seqlens, nullptr, nullptr, slots, start_pos, y, nullptr,
+                       SCAN_PLAIN, B, Hs, P, N, G, Cd, stream, true);
 }
 
 // The same scan with every sequence cut into chunks that run in parallel.  seg_start [n_seg + 1]:

@@ -42,7 +42,7 @@ const Entry kEntries[] = {
     TLC_ENTRY(tlc_linear), TLC_ENTRY(tlc_linear_swiglu), TLC_ENTRY(tlc_glu),
     TLC_ENTRY(tlc_rope_kv_store), TLC_ENTRY(tlc_attention), TLC_ENTRY(tlc_attention_decode), TLC_ENTRY(tlc_attention_decode_fused),
     TLC_ENTRY(tlc_attention_prefill), TLC_ENTRY(tlc_attention_prefill_tc),
-    TLC_ENTRY(tlc_mamba_conv), TLC_ENTRY(tlc_mamba_step), TLC_ENTRY(tlc_ssm_scan), TLC_ENTRY(tlc_ssm_scan_chunked), TLC_ENTRY(tlc_ssm_scan_ssd),
+    TLC_ENTRY(tlc_mamba_conv), TLC_ENTRY(tlc_mamba_step), TLC_ENTRY(tlc_ssm_scan), TLC_ENTRY(tlc_ssm_scan_one_row), TLC_ENTRY(tlc_ssm_scan_chunked), TLC_ENTRY(tlc_ssm_scan_ssd),
 };
 #undef TLC_ENTRY
 constexpr int kCount = (int)(sizeof(kEntries) / sizeof(kEntries[0]));

@@ -287,6 +287,10 @@ void tlc_ssm_scan_rows(int on);         // 0: the row-by-row scan takes the gene
 int tlc_ssm_scan(const float* xbc, const float* dt, const float* dA, const float* Dskip, float* state,
                  const int* cu_seqlens, const int* slots, const int* start_pos, float* y, int B, int Hs, int P,
                  int N, int G, int Cd, cudaStream_t stream);
+/* The same where the step brings one row of every sequence (a hint: the result does not depend on it). */
+int tlc_ssm_scan_one_row(const float* xbc, const float* dt, const float* dA, const float* Dskip, float* state,
+                 const int* cu_seqlens, const int* slots, const int* start_pos, float* y, int B, int Hs, int P,
+                 int N, int G, int Cd, cudaStream_t stream);
 /* The same with sequences cut into chunks (seg_start [n_seg+1], seg_seq [n_seg], seq_seg_start [B+1]) that
  * run in parallel in three 32-bit passes; chunk_state: n_seg*Hs*(P*N+1) floats of scratch. */
 int tlc_ssm_scan_chunked(const float* xbc, const float* dt, const float* dA, const float* Dskip, float* state,
