@@ -184,6 +184,7 @@ def test_functions_put_around_a_layers_methods_or_the_kernels_wrappers_are_notic
     found = RepeatedLayers.of(model.layers, model.schedule)
     layer = model.layers[0]
     assert found.untouched()
+    assert {n for n in ops._SIGNATURES if ops.library().tlc_replay_index(n.encode()) >= 0} == ops.REPEATABLE
     for owner, name in ((type(layer), "forward"), (type(layer.ffn), "forward"), (type(layer.mixers[0]), "mix"),
                         (type(layer), "entry"), (ops, "linear"), (ops, "attention"), (ops, "_call")):
         with monkeypatch.context() as m:

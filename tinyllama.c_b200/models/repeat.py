@@ -31,11 +31,12 @@ _PLAIN = (type(None), bool, int, float, str, torch.dtype, torch.device)
 _LOW = np.uint64(15)
 _edits = attrgetter("edits")
 _ptr, _size, _stride, _dtype = torch.Tensor.data_ptr, torch.Tensor.size, torch.Tensor.stride, attrgetter("dtype")
+_dense = torch.Tensor.is_contiguous
 
 
-# The wrappers of the kernel library as they are defined: the functions that make its calls.  (ops.replay is what this module itself calls.)
-_OPS = {k: f for k, f in vars(ops).items()
-        if isinstance(f, FunctionType) and k != "replay" and (k == "_call" or {"_call", "library"}.intersection(f.__code__.co_names))}
+# The wrappers of the kernel library as they are defined: the functions that name one of its calls, and those that they go through.
+_OPS = {k: f for k, f in vars(ops).items() if isinstance(f, FunctionType) and
+        (k in ("_call", "record_event", "wait_event") or any(isinstance(c, str) and c in ops.REPEATABLE for c in f.__code__.co_consts))}
 # methods that a step has no use for
 _NOT_IN_A_STEP = {"__init__", "bind", "weight_specs", "cache_requests", "step_requests", "shapes_from", "parts", "repeats", "add", "fuse_bound",
                   "fuse_bound_inputs", "out_features", "__setattr__", "__delattr__", "__init_subclass__"}
@@ -250,7 +251,9 @@ class RepeatedLayers:
 
     @staticmethod
     def _meta(tensors):
-        return list(map(_size, tensors)), list(map(_stride, tensors)), list(map(_dtype, tensors))
+        """Sizes, types and strides (of dense tensors the sizes say them)."""
+        dense = list(map(_dense, tensors))
+        return list(map(_size, tensors)), list(map(_dtype, tensors)), dense, None if all(dense) else list(map(_stride, tensors))
 
     @staticmethod
     def _shared(x: torch.Tensor, step: StepInfo, notes) -> List[torch.Tensor]:

@@ -224,6 +224,13 @@ def _call(name: str, *args) -> None:
 # the cache, and each takes a dozen microseconds on its way through the checks here.  Inside `noting()` the calls of this
 # thread are noted beside being made; replay() then makes them again, many rounds in one call of the library, with the
 # arguments that the caller has put in their places (models/repeat.py).
+# The calls that the library makes from a table (csrc/replay.cu; a test compares the two).
+REPEATABLE = frozenset(("tlc_event_record", "tlc_event_wait", "tlc_rmsnorm", "tlc_gated_rmsnorm", "tlc_gated_rmsnorm_step", "tlc_linear",
+                        "tlc_linear_swiglu", "tlc_glu", "tlc_rope_kv_store", "tlc_attention", "tlc_attention_decode",
+                        "tlc_attention_decode_fused", "tlc_attention_prefill", "tlc_attention_prefill_tc", "tlc_mamba_conv", "tlc_mamba_step",
+                        "tlc_ssm_scan", "tlc_ssm_scan_one_row", "tlc_ssm_scan_chunked", "tlc_ssm_scan_ssd"))
+
+
 class NotedCalls:
     """Calls in the order they were made.  words: the arguments as 64-bit words; pointers: which of them are pointers.
     owned: what the calls were given that no argument keeps alive (scratch, numbers on the host that a call writes).

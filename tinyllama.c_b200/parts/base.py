@@ -333,7 +333,7 @@ def scratch_buf(tag: str, shape, dtype: torch.dtype, device) -> torch.Tensor:
     t = _scratch.get(key)
     if t is None:
         t = _scratch[key] = torch.empty(shape, dtype=dtype, device=device)
-        if _scratch_stream is not None and current_stream(t.device) != _scratch_stream:
+        if _scratch_stream is not None and current_stream(t.device) is not _scratch_stream:
             used_on(_scratch_stream, (t,))
     return t
 
